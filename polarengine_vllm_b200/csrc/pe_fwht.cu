@@ -45,47 +45,291 @@ __global__ void __launch_bounds__(256) pack_nibble_kernel(const int8_t* codes, u
   *reinterpret_cast<uint4*>(packed + i * 16) = r;
 }
 
-// Quantizer: one warp per (weight row, 128-block).  Zero-pad, L2 norm clamped at 1e-10, divide, rotate, scale by
-// sqrt(128), nearest Lloyd-Max level by distance (first minimum wins, as the reference's argmin does), int8 code
-// and fp16 norm out.  The butterfly rotation and the warp-order sum of squares round differently from the
-// reference's matrix product and torch.norm, so a value that sits on a cell boundary to within fp32 rounding can
-// land on the other side: a few codes per million differ from the CPU quantizer.
-__global__ void __launch_bounds__(256) quantize_kernel(const void* w, int w_dtype, int64_t ld_w, int64_t rows, int in_f, int nb,
-                                                       const float* levels, int n_levels, int8_t* codes, int64_t ld_codes,
-                                                       __half* norms, int64_t ld_norms) {
-  extern __shared__ float lv[];
-  for (int i = threadIdx.x; i < n_levels; i += blockDim.x) lv[i] = levels[i];
+// ---- quantizer --------------------------------------------------------------------------------
+// Zero-pad, L2 norm clamped at 1e-10, divide, rotate, scale by sqrt(128), nearest Lloyd-Max level by distance (first
+// minimum wins, as the reference's argmin does), int8 code and fp16 norm out.  The butterfly rotation and the tree
+// sum of squares round differently from the reference's matrix product and torch.norm, so a value that sits on a
+// cell boundary to within fp32 rounding can land on the other side: a few codes per million differ from the CPU
+// quantizer.
+//
+// The launch is bound by instruction issue and the shared-memory port (two exchanges and two lookups per weight), not
+// by memory (two bytes in, one out).  Four lanes share a 128-block, in four pieces of 8 consecutive values each: five
+// of the seven butterfly stages stay in registers, a warp reads and writes whole sectors, the level is found with one
+// table lookup and one comparison instead of a scan of all levels, the quotient is a product with the reciprocal and
+// one correction, and fp32 arithmetic goes two values per instruction.  4096 x 12288 bf16, on 2 resident CTAs per SM
+// with the next trip's loads in flight: to 4 bits 256 -> 61 us (LSU port 70 % busy, issue slots 66 %), 4096 x 4000 to
+// 8 bits 729 -> 32 us against one warp per block, a scan and a full division per value.
+
+// Exact cell edges: the rotated unit-vector element v takes code j when j edges are below it.  edge[j] is the largest
+// float that is still no farther from level j than from level j + 1 by the fp32 distances quant_dist() that a scan
+// compares.  A uniform grid over [-1.06, 1.06] (elements of a unit vector) gives the edges below an element's cell; a
+// cell holds at most one, so one comparison settles the code.
+constexpr float kQuantRange = 1.06f;
+__device__ __forceinline__ float quant_dist(float v, float level) { return fabsf(fmaf(v, 11.313708498984761f, -level)); }  // sqrt(128)
+struct QuantTable {
+  float edge[256];      // edge[n_levels - 1] = +inf
+  uint8_t first[2048];  // edges in lower cells
+  uint16_t cell[256];   // cell of each edge
+};
+
+// the sum with 1.5 * 2^23 has the cell in its low mantissa bits
+__device__ __forceinline__ uint32_t quant_cell(float x, float scale, float magic, uint32_t mask) {
+  return __float_as_uint(fmaf(x, scale, magic)) & mask;
+}
+
+// Returns whether the levels have to be scanned instead: not ascending, closer than fp32 distances or the grid
+// resolve, or far outside the range of the values.
+__device__ __forceinline__ bool build_quant_table(QuantTable& q, float* lv, const float* levels, int n, uint32_t cells, float scale, float magic) {
+  const int tid = threadIdx.x;
+  if (tid < n) lv[tid] = levels[tid];
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (warp >= rows * nb) return;  // whole warps leave together
-  const int64_t r = warp / nb;
-  const int blk = (int)(warp - r * nb);
-  const bool vin = (ld_w % 4 == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
-  float v[4];
-  load4_as_float(w, w_dtype, r * ld_w, blk * kBlock + lane * 4, in_f, vin, v);
-  float ss = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
-#pragma unroll
-  for (int m = 16; m >= 1; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
-  const float nrm = fmaxf(sqrtf(ss), 1e-10f);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] = __fdiv_rn(v[i], nrm);
-  warp_fwht128(v, lane);  // includes the 1/sqrt(128) of the normalised Hadamard matrix
-  const float root = 11.313708498984761f;  // sqrt(128)
-  uint32_t packed = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float x = v[i] * root;
-    int best = 0;
-    float bd = fabsf(x - lv[0]);
-    for (int j = 1; j < n_levels; ++j) {
-      const float d = fabsf(x - lv[j]);
-      if (d < bd) { bd = d; best = j; }
+  bool bad = false;
+  if (tid < n) {
+    float e = __int_as_float(0x7f800000);
+    if (tid + 1 < n) {
+      const float lo = lv[tid], hi = lv[tid + 1];
+      bad = !(hi - lo > 1e-4f && fabsf(lo) < 11.3f && fabsf(hi) < 11.3f);
+      if (!bad) {  // halve [e, above] until the two are neighbours: `above` is nearer to hi, e is not
+        const float m0 = 0.5f * (lo + hi) * 0.08838834764831845f, near_lo = m0 - 1e-6f, near_hi = m0 + 1e-6f;
+        const bool lo_ok = !(quant_dist(near_lo, hi) < quant_dist(near_lo, lo)), hi_ok = quant_dist(near_hi, hi) < quant_dist(near_hi, lo);
+        e = lo_ok ? near_lo : lo * 0.08838834764831845f;
+        float above = hi_ok ? near_hi : hi * 0.08838834764831845f;
+        for (int i = 0; i < 200; ++i) {
+          const float m = 0.5f * (e + above);
+          if (m == e || m == above) break;
+          if (quant_dist(m, hi) < quant_dist(m, lo)) above = m;
+          else e = m;
+        }
+        q.cell[tid] = (uint16_t)quant_cell(e, scale, magic, cells - 1);
+      }
     }
-    packed |= (uint32_t)(best & 0xff) << (8 * i);
+    q.edge[tid] = e;
   }
-  *reinterpret_cast<uint32_t*>(codes + r * ld_codes + blk * kBlock + lane * 4) = packed;
-  if (lane == 0) norms[r * ld_norms + blk] = __float2half_rn(nrm);
+  if (__syncthreads_or(bad)) return true;
+  if (tid < n) {  // edge tid is the first one not below the cells from its lower neighbour's (exclusive) to its own
+    const int c0 = tid ? q.cell[tid - 1] + 1 : 0, c1 = tid + 1 < n ? q.cell[tid] : (int)cells - 1;
+    for (int c = c0; c <= c1; ++c) q.first[c] = (uint8_t)tid;
+    bad = tid && tid + 1 < n && c0 > c1;
+  }
+  return __syncthreads_or(bad);
+}
+
+// two fp32 values per instruction, each rounded on its own
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{.reg .b64 x, y; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; add.rn.f32x2 x, x, y; mov.b64 {%0, %1}, x;}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{.reg .b64 x, y; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mul.rn.f32x2 x, x, y; mov.b64 {%0, %1}, x;}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{.reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7}; fma.rn.f32x2 x, x, y, z; mov.b64 {%0, %1}, x;}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
+// 8 consecutive weights from column `col` of a row, zero from in_f on: the load and the conversion, so that the next
+// trip's loads are in flight while this one's values are worked on
+template <int W_DTYPE> struct Raw8 { uint4 q[W_DTYPE == PE_F32 ? 2 : 1]; };
+
+template <int W_DTYPE>
+__device__ __forceinline__ Raw8<W_DTYPE> load8_raw(const void* w, int64_t row_off, int col, int in_f, bool vec_ok) {
+  constexpr int kSize = W_DTYPE == PE_F32 ? 4 : 2, kQuads = W_DTYPE == PE_F32 ? 2 : 1;
+  Raw8<W_DTYPE> r;
+  const uint8_t* src = static_cast<const uint8_t*>(w) + (row_off + col) * kSize;
+  if (vec_ok && col + 8 <= in_f) {
+#pragma unroll
+    for (int i = 0; i < kQuads; ++i) r.q[i] = ldg_stream(src + 16 * i);
+  } else {
+    uint32_t u[4 * kQuads];
+#pragma unroll
+    for (int i = 0; i < 4 * kQuads; ++i) {
+      if (W_DTYPE == PE_F32) {
+        u[i] = col + i < in_f ? reinterpret_cast<const uint32_t*>(src)[i] : 0u;
+      } else {
+        const uint16_t* h = reinterpret_cast<const uint16_t*>(src);
+        u[i] = (col + 2 * i < in_f ? h[2 * i] : 0u) | (col + 2 * i + 1 < in_f ? (uint32_t)h[2 * i + 1] << 16 : 0u);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kQuads; ++i) r.q[i] = make_uint4(u[4 * i], u[4 * i + 1], u[4 * i + 2], u[4 * i + 3]);
+  }
+  return r;
+}
+
+template <int W_DTYPE>
+__device__ __forceinline__ void cvt8(const Raw8<W_DTYPE>& r, float v[8]) {
+  if (W_DTYPE == PE_F32) {
+    const uint4 a = r.q[0], b = r.q[W_DTYPE == PE_F32 ? 1 : 0];
+    v[0] = __uint_as_float(a.x); v[1] = __uint_as_float(a.y); v[2] = __uint_as_float(a.z); v[3] = __uint_as_float(a.w);
+    v[4] = __uint_as_float(b.x); v[5] = __uint_as_float(b.y); v[6] = __uint_as_float(b.z); v[7] = __uint_as_float(b.w);
+  } else {
+    const uint32_t h[4] = {r.q[0].x, r.q[0].y, r.q[0].z, r.q[0].w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = W_DTYPE == PE_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&h[i]))
+                                         : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&h[i]));
+      v[2 * i] = f.x; v[2 * i + 1] = f.y;
+    }
+  }
+}
+
+template <int W_DTYPE>
+__global__ void __launch_bounds__(256, 2) quantize_kernel(const void* w, int64_t ld_w, int64_t rows, int in_f, int nb,
+                                                          const float* levels, int n_levels, int8_t* codes, int64_t ld_codes,
+                                                          __half* norms, int64_t ld_norms, int vec_out) {
+  __shared__ float lv[256];
+  __shared__ QuantTable q;
+  uint32_t cells = 64;  // at least 16 per level, which Lloyd-Max levels of every width need; 8 per level at 256
+  while ((int)cells < 16 * n_levels && cells < 2048) cells *= 2;
+  const float scale = (float)cells / (2.f * kQuantRange), magic = 12582912.f + (float)(cells / 2);
+  const bool scan = build_quant_table(q, lv, levels, n_levels, cells, scale, magic);
+  const uint32_t mask = cells - 1;
+  const int lane = threadIdx.x & 31, part = lane & 3;
+  const int64_t n_warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const bool vin = ((ld_w * (W_DTYPE == PE_F32 ? 4 : 2)) % 16 == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
+  // block (row r, column block blk) of this lane, and how far one trip of the grid advances it
+  const int64_t first = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 8 + (lane >> 2);
+  int64_t r = first / nb;
+  int blk = (int)(first - r * nb);
+  const int64_t step_r = n_warps * 8 / nb;
+  const int step_b = (int)(n_warps * 8 - step_r * nb);
+  Raw8<W_DTYPE> raw[4];
+  auto request = [&]() {  // block (r, blk) of the weight, zeros past its last row
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+      raw[p] = load8_raw<W_DTYPE>(w, r < rows ? r * ld_w : 0, blk * kBlock + p * 32 + part * 8, r < rows ? in_f : 0, vin);
+  };
+  request();
+  while (__any_sync(0xffffffffu, r < rows)) {
+    const int64_t r_out = r;
+    const int blk_out = blk;
+    // element k of the block: bits 6..5 of k choose one of the lane's four pieces, bits 4..3 the lane, bits 2..0 the
+    // place in the piece; v[4 * piece + i] holds places i and i + 4
+    float2 v[16];
+    float s[2];  // groups of four (places 0..3, 4..7), then a tree over the 32 groups, widest distance first
+    {
+      float u[4][8], g[4][2];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) cvt8<W_DTYPE>(raw[p], u[p]);
+      r += step_r;
+      blk += step_b;
+      if (blk >= nb) { blk -= nb; ++r; }
+      request();
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          g[p][h] = u[p][4 * h] * u[p][4 * h] + u[p][4 * h + 1] * u[p][4 * h + 1] + u[p][4 * h + 2] * u[p][4 * h + 2] + u[p][4 * h + 3] * u[p][4 * h + 3];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[4 * p + i] = make_float2(u[p][i], u[p][i + 4]);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) s[h] = (g[0][h] + g[2][h]) + (g[1][h] + g[3][h]);
+    }
+#pragma unroll
+    for (int m = 2; m >= 1; m >>= 1) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) s[h] += __shfl_xor_sync(0xffffffffu, s[h], m);
+    }
+    const float nrm = fmaxf(sqrtf(s[0] + s[1]), 1e-10f);
+    // v / nrm: with y the rounded reciprocal and d = v * y, the remainder fma(-d, nrm, v) is exact and d + rem * y
+    // is the rounded quotient (P. Markstein, IBM J. Res. Dev. 34, 1990) while nothing over- or underflows
+    if (nrm > 1e-9f && nrm < 1e18f) {
+      const float y = __frcp_rn(nrm);
+      const float2 y2 = make_float2(y, y), n2 = make_float2(-nrm, -nrm);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float2 d = mul2(v[i], y2);
+        v[i] = fma2(fma2(d, n2, v[i]), y2, d);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = make_float2(__fdiv_rn(v[i].x, nrm), __fdiv_rn(v[i].y, nrm));
+    }
+    // FWHT-128 in the order of the strides: 1, 2 between pairs, 4 inside them, 8, 16 between lanes, 32, 64 between pieces
+    const float2 minus = make_float2(-1.f, -1.f);
+    auto between_pairs = [&](int h) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (!(i & h)) {
+          const float2 a = v[i], b = v[i | h];
+          v[i] = add2(a, b);
+          v[i | h] = fma2(b, minus, a);
+        }
+    };
+    between_pairs(1);
+    between_pairs(2);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = make_float2(v[i].x + v[i].y, v[i].x - v[i].y);
+#pragma unroll
+    for (int m = 1; m <= 2; m <<= 1) {
+      const float sgn = (part & m) ? -1.f : 1.f;
+      const float2 sgn2 = make_float2(sgn, sgn);
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        v[i] = fma2(sgn2, v[i], make_float2(__shfl_xor_sync(0xffffffffu, v[i].x, m), __shfl_xor_sync(0xffffffffu, v[i].y, m)));
+    }
+    between_pairs(4);
+    between_pairs(8);
+    const float s128 = 0.08838834764831845f;  // 1/sqrt(128)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = mul2(v[i], make_float2(s128, s128));
+    uint32_t packed[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) packed[i] = 0;
+    if (!scan) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float2 c = fma2(v[i], make_float2(scale, scale), make_float2(magic, magic));  // quant_cell of both
+        uint32_t jx = q.first[__float_as_uint(c.x) & mask], jy = q.first[__float_as_uint(c.y) & mask];
+        jx += v[i].x > q.edge[jx];
+        jy += v[i].y > q.edge[jy];
+        packed[i >> 2 << 1] |= jx << (8 * (i & 3));
+        packed[(i >> 2 << 1) + 1] |= jy << (8 * (i & 3));
+      }
+      if (v[0].x != v[0].x) {  // a NaN reaches the whole block
+#pragma unroll
+        for (int i = 0; i < 8; ++i) packed[i] = 0;
+      }
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < 32; ++i) {
+        float x = 0.f;
+#pragma unroll
+        for (int k = 0; k < 32; ++k)
+          if (k == i) x = (k & 4) ? v[(k >> 3) * 4 + (k & 3)].y : v[(k >> 3) * 4 + (k & 3)].x;
+        uint32_t best = 0;
+        float bd = quant_dist(x, lv[0]);
+        for (int j = 1; j < n_levels; ++j) {
+          const float d = quant_dist(x, lv[j]);
+          if (d < bd) { bd = d; best = j; }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (k == i >> 2) packed[k] |= best << (8 * (i & 3));
+      }
+    }
+    if (r_out < rows) {
+      int8_t* dst = codes + r_out * ld_codes + blk_out * kBlock + part * 8;
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        if (vec_out) {
+          *reinterpret_cast<uint2*>(dst + p * 32) = make_uint2(packed[2 * p], packed[2 * p + 1]);
+        } else {
+          reinterpret_cast<uint32_t*>(dst + p * 32)[0] = packed[2 * p];
+          reinterpret_cast<uint32_t*>(dst + p * 32)[1] = packed[2 * p + 1];
+        }
+      }
+      if (part == 0) norms[r_out * ld_norms + blk_out] = __float2half_rn(nrm);
+    }
+  }
 }
 
 // Quantized embedding lookup: row ids[t] of the table is dequantised on the fly.
@@ -189,11 +433,15 @@ extern "C" int pe_quantize(const void* weight, int w_dtype, int64_t ld_w, int64_
   if (ld_w < in_f || ld_codes < in_f_padded || ld_norms < in_f_padded / kBlock) return PE_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(codes) & 3) || (ld_codes & 3)) return PE_ERR_ALIGN;
   const int nb = in_f_padded / kBlock;
-  const int64_t warps = out_f * nb;
-  const int64_t blocks = (warps + 7) / 8;
-  if (blocks > 0x7fffffff) return PE_ERR_LIMIT;
-  quantize_kernel<<<(unsigned)blocks, 256, n_levels * sizeof(float), static_cast<cudaStream_t>(stream)>>>(
-      weight, w_dtype, ld_w, out_f, in_f, nb, levels, n_levels, codes, ld_codes, static_cast<__half*>(norms), ld_norms);
+  const int64_t ctas = ((int64_t)out_f * nb + 63) / 64;  // a CTA takes 64 blocks per trip
+  const int sms = sm_count();
+  if (sms <= 0) return PE_ERR_CUDA;
+  // the resident CTAs (two per SM); the level table is built once per CTA
+  const unsigned grid = (unsigned)(ctas < 2ll * sms ? ctas : 2ll * sms);
+  auto kfn = w_dtype == PE_F32 ? quantize_kernel<PE_F32> : w_dtype == PE_F16 ? quantize_kernel<PE_F16> : quantize_kernel<PE_BF16>;
+  const int vec_out = (reinterpret_cast<uintptr_t>(codes) & 7) == 0 && ld_codes % 8 == 0;
+  kfn<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(weight, ld_w, out_f, in_f, nb, levels, n_levels, codes, ld_codes,
+                                                           static_cast<__half*>(norms), ld_norms, vec_out);
   PE_CUDA_TRY(cudaGetLastError());
   return PE_OK;
 }

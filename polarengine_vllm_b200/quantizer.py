@@ -9,7 +9,7 @@ reproduces reference checkpoints bit for bit.
 from __future__ import annotations
 
 import math
-from typing import Dict, Mapping, Optional
+from typing import Dict, Mapping, Optional, Tuple
 
 import torch
 import torch.nn.functional as F
@@ -17,6 +17,19 @@ import torch.nn.functional as F
 from .fwht import build_hadamard
 from .utils import DEFAULT_BIT_ASSIGNMENT, get_bits_for_layer, get_centroids, get_ct_scaled
 from .packing import pack_codes_half_block, pack_codes_q5
+
+
+_TABLES: Dict[Tuple[int, torch.device], Tuple[torch.Tensor, torch.Tensor]] = {}
+
+
+def _device_tables(bits: int, dev: torch.device) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Levels and scaled levels of a width on a device, copied there once (a copy from pageable memory waits for the
+    GPU); the scaled table is divided on the host, as the CPU path has it."""
+    tab = _TABLES.get((bits, dev))
+    if tab is None:
+        tab = _TABLES[(bits, dev)] = (get_centroids(bits).to(dev), get_ct_scaled(bits, 128).to(dev))
+        torch.cuda.current_stream(dev).synchronize()  # later calls may run on other streams
+    return tab
 
 
 class PolarQuantizer:
@@ -66,13 +79,13 @@ class PolarQuantizer:
             w = w.contiguous()
         rows, cols = w.shape
         padded = -(-cols // 128) * 128
-        levels = get_centroids(bits).to(dev)
+        levels, scaled = _device_tables(bits, dev)
         codes = torch.empty(rows, padded, dtype=torch.int8, device=dev)
         norms = torch.empty(rows, padded // 128, dtype=torch.float16, device=dev)
         nv.check(nv.lib().pe_quantize(w.data_ptr(), nv.dtype_code(w), w.stride(0), rows, cols, padded, levels.data_ptr(),
                                       levels.numel(), codes.data_ptr(), codes.stride(0), norms.data_ptr(), norms.stride(0),
                                       nv.stream_ptr(dev)), "pe_quantize")
-        return {"codes": codes, "norms": norms, "ct_scaled": get_ct_scaled(bits, 128).to(dev)}  # table divided on the host, as the CPU path has it
+        return {"codes": codes, "norms": norms, "ct_scaled": scaled.clone()}
 
     def quantize_state_dict(self, state: Mapping[str, torch.Tensor], pack: bool = True):
         """Quantize every eligible 2-D ``*.weight``; returns (tensors, polar_config dict)

@@ -43,3 +43,24 @@ def test_gpu_quantizer_half_and_bf16_inputs():
         ref = oracle.quantize_tensor(wd.float(), 4)
         q = PolarQuantizer().quantize_tensor_gpu(wd.cuda(), 4)
         assert (q["codes"].cpu() != ref["codes"]).float().mean() < 1e-3
+
+
+@pytest.mark.parametrize("levels", ["two", "odd", "crowded", "unsorted"])
+def test_gpu_quantizer_levels_of_any_kind(levels):
+    """Few levels, several edges in one cell of the lookup grid, levels too close together or out of order (scanned)."""
+    from polarengine_vllm_b200 import _native as nv
+    g = torch.Generator().manual_seed(5)
+    lv = {"two": torch.tensor([-0.8, 0.8]), "odd": torch.tensor([-2.0, -0.5, 0.1, 0.4, 3.0]),
+          "crowded": torch.cat([torch.linspace(-0.02, 0.02, 40), torch.tensor([5.0, 9.0])]),
+          "unsorted": torch.tensor([1.5, -1.5, 0.4, -0.4])}[levels]
+    w = torch.randn(33, 200, generator=g) * 0.02
+    nv.ensure_init(torch.device("cuda", 0))
+    wd, ld = w.cuda(), lv.cuda()
+    codes = torch.empty(33, 256, dtype=torch.int8, device="cuda")
+    norms = torch.empty(33, 2, dtype=torch.float16, device="cuda")
+    nv.check(nv.lib().pe_quantize(wd.data_ptr(), nv.PE_F32, 200, 33, 200, 256, ld.data_ptr(), ld.numel(), codes.data_ptr(), 256,
+                                  norms.data_ptr(), 2, nv.stream_ptr(wd.device)), "pe_quantize")
+    blocks = torch.nn.functional.pad(w, (0, 56)).view(33, 2, 128)
+    rot = blocks / blocks.norm(dim=2, keepdim=True) @ oracle.hadamard(128) * 128 ** 0.5
+    ref = (rot.unsqueeze(-1) - lv).abs().argmin(-1).view(33, 256)
+    assert int((codes.cpu().view(torch.uint8).int() != ref).sum()) <= 8
