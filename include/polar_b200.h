@@ -34,8 +34,10 @@ enum { PE_F32 = 0, PE_F16 = 1, PE_BF16 = 2 };
 enum {
   PE_X_ROTATED = 0, /* already FWHT-128 rotated and zero padded to in_f_padded
                        (the reference's `x_transformed`, fwht.py:102-108)        */
-  PE_X_RAW = 1      /* un-rotated activations with in_f valid columns; the kernel
+  PE_X_RAW = 1,     /* un-rotated activations with in_f valid columns; the kernel
                        pads and rotates while staging (linear_method.py:186-197) */
+  PE_X_SILU_MUL = 2 /* grouped entry points, fp16: rows are [gate | up] of 2 in_f columns and the
+                       input is half(silu(gate)) * up (pe_silu_mul), then as PE_X_RAW       */
 };
 
 /* glue ops that pe_gemv_pro computes while it stages its input */
@@ -163,15 +165,12 @@ int pe_pack_nibble(const int8_t* codes, uint8_t* packed, int64_t out_f, int64_t 
  *           it is rotated already (in_f_padded columns) or raw (in_f columns)
  *   y       (batch, out_f) row stride ld_y elements, dtype y_dtype
  *   bias    optional fp16 (out_f), may be NULL
- *   workspace / workspace_bytes  scratch of at least pe_gemv_workspace_bytes(...);
- *           its first 256 KB hold per-tile counters that must read zero on entry
- *           (zero-fill the buffer once after allocating it); every call returns
- *           them to zero, so the buffer can be reused by later calls of any shape
- *           on the same stream without refilling.  Calls that share a scratch
- *           buffer must not overlap on the device.  The last int32 of those 256 KB
- *           is a status word: a kernel whose bounded device-side wait ran out stores
- *           a PE_STATUS_* value there (the output is then undefined);
- *           pe_gemv_status() waits for the stream and returns the word (0 = ok),
+ *   workspace / workspace_bytes  16-byte aligned scratch of at least pe_gemv_workspace_bytes(...);
+ *           no initial contents are needed beyond its status word, the last int32 of
+ *           its first 256 KB, which must read zero before the first call: a kernel whose
+ *           bounded device-side wait ran out stores a PE_STATUS_* value there (the output
+ *           is then undefined).  Calls that share a scratch buffer must not overlap on the
+ *           device.  pe_gemv_status() waits for the stream and returns the word (0 = ok),
  *           clearing it when `clear` is non-zero.
  *
  * Replaces polar_matmul's batch==1 branches and (for 2..16 rows) its GEMM branch
@@ -179,10 +178,9 @@ int pe_pack_nibble(const int8_t* codes, uint8_t* packed, int64_t out_f, int64_t 
 size_t pe_gemv_workspace_bytes(int batch, int out_f, int in_f_padded);
 int pe_gemv_status(void* workspace, size_t workspace_bytes, int clear, void* stream);
 
-/* 1 if pe_gemv runs batches of 3..8 rows of this layer on its row-major arrays with the column-owner
- * tensor-core kernel (weights decoded once per step and used for every row of the batch; no scratch
- * memory, no tiled copy of the layer needed), 0 if such batches go to the tile kernel, which streams the
- * tiled copy (pe_retile / pe_gemv_tiled) best.  No launch, no device access beyond the SM count. */
+/* 1 if pe_gemv runs batches of 3..8 rows of this layer as fast on its row-major arrays as pe_gemv_tiled does on the
+ * tiled copy (pe_retile), 0 if the copy is worth having.  It is for every layer: one contiguous bulk copy per stage
+ * instead of sixteen.  No launch, no device access. */
 int pe_gemv_small_batch_takes(int packed, int64_t ld_codes, const void* norms, int64_t ld_norms, int out_f,
                               int in_f_padded);
 int pe_gemv(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms,
@@ -199,10 +197,12 @@ int pe_gemv(const void* codes, int packed, int64_t ld_codes, const void* norms, 
  * `expert` and writes rows first .. of y.  Entries with rows <= 0 are skipped, so the host
  * sizes the launch for the worst case and never reads the routing back.  max_rows (<= 16)
  * bounds the rows of any problem (8 or less selects the lighter kernel); an expert with
- * more rows takes several problems.  No bias.  The scratch
+ * more rows takes several problems.  No bias.  x_kind may also be PE_X_SILU_MUL.  The scratch
  * (pe_gemv_grouped_workspace_bytes; 0 = too many problems) is its own buffer, not the one
- * of pe_gemv: its first 4 MiB must be zero before the first use and are left zero, so
- * calls of any shapes can share it in stream order.
+ * of pe_gemv: the last int32 of its first 4 MiB is the status word and must be zero before the
+ * first use; calls of any shapes can share it in stream order.
+ * pe_gemv_grouped_tiled = pe_gemv_grouped on tiled copies of the matrices (pe_retile each, matrix e
+ * at tiles + e * tiles_stride bytes).
  * Replaces the per-expert loop of the reference's MoE layer (nemotron_offload.py:190-226:
  * for each selected expert, gate/up projection, activation, down projection) with two
  * grouped launches; the reference's vLLM path has no quantized expert arithmetic
@@ -213,6 +213,10 @@ int pe_gemv_grouped(const void* codes, int packed, int64_t ld_codes, int64_t cod
                     int x_kind, int x_dtype, int64_t ld_x, int in_f, const int32_t* x_rows, void* y, int y_dtype,
                     int64_t ld_y, const int32_t* problems, int max_problems, int max_rows, int out_f,
                     int in_f_padded, void* workspace, size_t workspace_bytes, void* stream);
+int pe_gemv_grouped_tiled(const void* tiles, int packed, int64_t tiles_stride, const float* ct_scaled, int n_levels,
+                          const void* x, int x_kind, int x_dtype, int64_t ld_x, int in_f, const int32_t* x_rows, void* y,
+                          int y_dtype, int64_t ld_y, const int32_t* problems, int max_problems, int max_rows, int out_f,
+                          int in_f_padded, void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---- grouped prefill-size matmul: the experts of a mixture layer on the tensor cores -----
  * pe_gemm over a stack of matrices (expert e's codes directly after expert e-1's:
@@ -349,8 +353,7 @@ int pe_gemv_pro(const void* codes, int packed, int64_t ld_codes, const void* nor
  *    up the array's device address (cudaGetSymbolAddress) with that device current;
  *    make that first call outside of any stream capture.
  *  - All calls on a device share the one array and it keeps the previous call's
- *    contents; the entry point clears the counters it needs, in stream order, before
- *    the kernel.  Two calls that overlap on the GPU (different streams) race on it:
+ *    contents.  Two calls that overlap on the GPU (different streams) race on it:
  *    keep them on one stream or order them with events.
  *  - A bounded device-side wait that runs out leaves a PE_STATUS_* value in a word of the
  *    array; pe_gemv_noalloc_status() waits for the stream and returns that word (0 = every

@@ -16,7 +16,7 @@ _LIB_NAME = "libpolar_b200.so"
 _lib: Optional[ctypes.CDLL] = None
 
 PE_F32, PE_F16, PE_BF16 = 0, 1, 2
-PE_X_ROTATED, PE_X_RAW = 0, 1
+PE_X_ROTATED, PE_X_RAW, PE_X_SILU_MUL = 0, 1, 2
 PE_PRO_ADD_RMSNORM, PE_PRO_SILU_MUL = 1, 2
 
 _DTYPE = {torch.float32: PE_F32, torch.float16: PE_F16, torch.bfloat16: PE_BF16}
@@ -39,6 +39,7 @@ SIGNATURES = {
     "pe_gemv_grouped_workspace_bytes": (_sz, [_i, _i, _i]),
     "pe_gemv_grouped": (_i, [_vp, _i, _i64, _i64, _vp, _i64, _i64, _vp, _i, _vp, _i, _i, _i64, _i, _vp, _vp, _i, _i64, _vp,
                             _i, _i, _i, _i, _vp, _sz, _vp]),
+    "pe_gemv_grouped_tiled": (_i, [_vp, _i, _i64, _vp, _i, _vp, _i, _i, _i64, _i, _vp, _vp, _i, _i64, _vp, _i, _i, _i, _i, _vp, _sz, _vp]),
     "pe_moe_route": (_i, [_vp, _i, _i64, _i, _i, _i, _i, _vp, _vp, _vp]),
     "pe_moe_plan": (_i, [_vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp]),
     "pe_gemm_grouped_workspace_bytes": (_sz, [_i, _i, _i, _i]),

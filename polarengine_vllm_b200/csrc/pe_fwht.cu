@@ -114,26 +114,6 @@ __device__ __forceinline__ bool build_quant_table(QuantTable& q, float* lv, cons
   return __syncthreads_or(bad);
 }
 
-// two fp32 values per instruction, each rounded on its own
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 d;
-  asm("{.reg .b64 x, y; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; add.rn.f32x2 x, x, y; mov.b64 {%0, %1}, x;}"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 d;
-  asm("{.reg .b64 x, y; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mul.rn.f32x2 x, x, y; mov.b64 {%0, %1}, x;}"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("{.reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7}; fma.rn.f32x2 x, x, y, z; mov.b64 {%0, %1}, x;}"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return d;
-}
-
 // 8 consecutive weights from column `col` of a row, zero from in_f on: the load and the conversion, so that the next
 // trip's loads are in flight while this one's values are worked on
 template <int W_DTYPE> struct Raw8 { uint4 q[W_DTYPE == PE_F32 ? 2 : 1]; };

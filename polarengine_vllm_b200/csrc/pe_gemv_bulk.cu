@@ -1,0 +1,548 @@
+// Decode-size quantized matmul (1..16 activation rows): bulk-copy kernel.
+//
+//   y[m, r] = sum_blk norm[r, blk] * sum_k ct[code[r, blk, k]] * xt[m, blk, k]   (+ bias[r])
+//
+// One persistent CTA per SM: sixteen math warps and one copy warp.  A stage of the shared-memory ring is one 16-row
+// tile of the weight matrix by up to 32 quantization blocks; the copy warp fills stages with bulk copies (one per
+// stage from the tiled layout of pe_retile, whose records are contiguous; one per weight row from the row-major
+// layout) long before the activations exist: everything up to the ring's size is on its way before the dependency
+// wait of the programmatic launch returns.  (Without a copy warp -- the last warp to finish with a stage refills it,
+// 128 instead of 96 registers -- the refills came later and every warp had to track them: 4 us over four launches.)
+//
+// What bounds it: once the ring runs, the shared-memory port.  A warp takes block cw, cw + 16 of every stage:
+//  * centroid lookup: the table is replicated per lane at a spacing of 256 bytes per entry, so that ONE byte permute
+//    forms the address (code byte in bits 8..15, lane * 4 below) and the load adds the table's constant address;
+//    32 lanes with 32 different codes never meet on a bank.  A nibble layer indexes it with the whole byte and gets
+//    the fp16 pair of both nibbles; a byte layer keeps (c, 0) and (0, c) in the two halves of an entry, and with up
+//    to eight activation rows multiplies both without merging them (the tensor pipe has room, the integer pipe not);
+//  * products on the tensor cores (mma.sync m16n8k16, weights as the 16-row A operand, activation rows as the eight
+//    columns of B): 16 rows x 16 weights per instruction straight from the lookups' registers, which no descriptor-
+//    based tensor-core operation offers (tcgen05 would need the decoded tile written to shared memory and read again);
+//  * activations: a small launch in front (gemv_frags_kernel) pads, rotates and rounds them once and leaves them in
+//    B-operand order in the workspace, so that a warp loads its own blocks with four coalesced reads each and keeps
+//    them in registers.  Rotating inside this kernel was measured too (in registers, 16-point part by MMAs): its
+//    straight-line code cost more in instruction fetches than the extra launch, 13 us over a layer's four launches.
+//    The registers left over let the small launch's blocks be resident, waiting, while the launch before it still runs.
+// Measured, tiled layout, launches of a dependent chain under a CUDA graph, weights from HBM (in brackets the kernels
+// this one replaced, which split K over CTAs or rows over warps and staged codes with per-lane copies):
+//   activation rows      1              8              16
+//   6144 x 4096 Q5    10.3 (10.4)    10.0 (16.5)    13.8 (31.3) us
+//   4096 x 4096 Q6     7.7  (8.0)     8.1 (13.6)     9.6 (29.4)
+//   24576 x 4096 Q3   14.7 (16.9)    16.9 (24.8)    28.0 (56.5)
+//   4096 x 12288 Q4   10.5 (13.5)    11.5 (28.8)    15.9 (41.2)
+//   the four in turn  42.6 (47.2)    46.4 (86.9)    66.7 (171)
+// Inside the ring's steady state the 24576 x 4096 launch moves 4.9 TB/s; the rest is the launch's own latency: about
+// 3.5 us from the launch before it to the first product, 0.5 us from the last one to the stores.
+//
+// The tiles (rows in the row-major layout) of all problems of a launch form one line that is cut into equal
+// contiguous ranges, one per CTA; nothing crosses CTAs.  The sixteen warps' partial sums of a tile go through shared
+// memory and are added in warp order: bit-identical from run to run, and the same bits from either layout.
+#include "pe_gemv_decode.cuh"
+
+namespace pe {
+
+constexpr int kBulkWarps = 16;                        // math warps
+constexpr int kBulkThreads = (kBulkWarps + 1) * 32;   // + the copy warp
+constexpr int kTabAddr = 2048;                        // address of the centroid table in the shared window
+constexpr int kTabReach = 255 * 256 + 256;            // bytes a lookup can reach from there, whatever the code byte is
+constexpr int kBulkMaxStages = 8;
+constexpr unsigned kBulkSmemMax = 231424u;            // 227 KB minus the runtime's 1 KB
+
+struct BulkArgs {
+  const uint8_t* codes; int64_t ld_codes;  // row-major layout: bytes between rows
+  const __half* norms; int64_t ld_norms;
+  const uint8_t* tiles;                    // tiled layout
+  const float* ct; int n_levels;
+  const uint4* frags;                      // activations in B-operand order
+  void* y; int y_dtype; int64_t ld_y;
+  const __half* bias;
+  int batch, N, nb;
+  int n_chunk, chunk_blocks, n_stage;      // chunks of the K range, blocks of a full chunk
+  int units;                               // units (16 rows tiled, 1 row row-major) per problem
+  int pass_rows;                           // rows whose partial sums shared memory holds (a multiple of 16)
+  int part_stride;                         // floats between activation rows of the partial sums
+  int part_rows;                           // activation rows the partial sums have room for
+  int part_off, norm_off, norm_stride, stage_off, stage_bytes, row_stride;
+  int* status;
+  // grouped launch: problem i multiplies rows grp[i].y .. + grp[i].z of the row list with matrix grp[i].x
+  const int4* grp; int n_problems;
+  int64_t codes_stride, norms_stride, tiles_stride;
+};
+
+// ---- barriers and bulk copies ---------------------------------------------------------------------------------
+__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+// Bounded: after about half a second the status word is set and the wait gives up (the output is then undefined).
+__device__ __noinline__ bool bar_wait_slow(uint32_t bar, uint32_t parity, int* status) {
+  const long long t0 = clock64();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i)
+      if (bar_try(bar, parity)) return true;
+    if (clock64() - t0 > (1ll << 30)) {
+      if (status) atomicExch(status, PE_STATUS_SPLITK_TIMEOUT);
+      return false;
+    }
+  }
+}
+__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, int* status) {
+  if (!bar_try(bar, parity)) bar_wait_slow(bar, parity, status);
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void math_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kBulkWarps * 32) : "memory"); }
+
+// ---- tensor-core products -------------------------------------------------------------------------------------
+__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_f16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+// centroid of byte E of a code word; OFF 128: the upper half of the entry
+template <int E, int OFF>
+__device__ __forceinline__ uint32_t centroid(uint32_t w, uint32_t lane4) {
+  uint32_t a, v;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(a) : "r"(w), "r"(lane4), "n"(0x7604 | (E << 4)));
+  asm volatile("ld.shared.b32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(kTabAddr + OFF));
+  return v;
+}
+
+// One block: 16 weight rows x 128 weights x 8 NT activation rows.  pa, pb: this lane's bytes of rows g and g + 8.
+// The k order of the products is the order of the code bytes: nibble byte i of the block (lane t holds 16 t .. 16 t + 15)
+// is the pair (i, i + 64), byte codes are pairs of neighbours.
+template <bool PACKED, int NT>
+__device__ __forceinline__ void block_product(uint32_t pa, uint32_t pb, const uint32_t (&x)[NT][16], uint32_t lane4, float (&d)[NT][4]) {
+  if (PACKED) {
+    const uint4 qa = lds128(pa), qb = lds128(pb);
+    const uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w}, wb[4] = {qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t a0 = centroid<0, 0>(wa[i], lane4), b0 = centroid<0, 0>(wb[i], lane4), a1 = centroid<1, 0>(wa[i], lane4), b1 = centroid<1, 0>(wb[i], lane4);
+      const uint32_t a2 = centroid<2, 0>(wa[i], lane4), b2 = centroid<2, 0>(wb[i], lane4), a3 = centroid<3, 0>(wa[i], lane4), b3 = centroid<3, 0>(wb[i], lane4);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        if (i == 0) mma_f16_first(d[n], a0, b0, a1, b1, x[n][0], x[n][1]);
+        else mma_f16(d[n], a0, b0, a1, b1, x[n][4 * i], x[n][4 * i + 1]);
+        mma_f16(d[n], a2, b2, a3, b3, x[n][4 * i + 2], x[n][4 * i + 3]);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // halves of 64 weights
+      const uint4 qa = lds128(pa + 64 * h), qb = lds128(pb + 64 * h);
+      const uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w}, wb[4] = {qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = 8 * h + 2 * i;
+        const uint32_t a0 = centroid<0, 0>(wa[i], lane4), b0 = centroid<0, 0>(wb[i], lane4), a1 = centroid<2, 0>(wa[i], lane4), b1 = centroid<2, 0>(wb[i], lane4);
+        const uint32_t a2 = centroid<1, 128>(wa[i], lane4), b2 = centroid<1, 128>(wb[i], lane4), a3 = centroid<3, 128>(wa[i], lane4), b3 = centroid<3, 128>(wb[i], lane4);
+        if (NT == 1) {  // (c0, 0), (c2, 0) and (0, c1), (0, c3) against the same activations
+          if (k == 0) mma_f16_first(d[0], a0, b0, a1, b1, x[0][k], x[0][k + 1]);
+          else mma_f16(d[0], a0, b0, a1, b1, x[0][k], x[0][k + 1]);
+          mma_f16(d[0], a2, b2, a3, b3, x[0][k], x[0][k + 1]);
+        } else {
+#pragma unroll
+          for (int n = 0; n < NT; ++n) {
+            if (k == 0) mma_f16_first(d[n], a0 | a2, b0 | b2, a1 | a3, b1 | b3, x[n][k], x[n][k + 1]);
+            else mma_f16(d[n], a0 | a2, b0 | b2, a1 | a3, b1 | b3, x[n][k], x[n][k + 1]);
+          }
+        }
+      }
+    }
+  }
+}
+
+// ---- activations in B-operand order ------------------------------------------------------------------------------
+// Fragments of one block and eight activation rows: four 16-byte pieces per lane, piece q of lane (g, t) holding the
+// operands of MMAs 2 q and 2 q + 1 for activation row g: [problem][set of eight][block][q][lane].  One warp pads,
+// rotates and stores one (row, block).
+struct FragArgs {
+  const void* x; int x_kind, x_dtype; int64_t ld_x; int in_f, nb, batch, sets;  // sets of eight rows per problem
+  uint4* out;
+  const int4* grp; const int32_t* x_rows;
+};
+constexpr int kFragThreads = 128;
+
+template <bool PACKED>
+__global__ void __launch_bounds__(kFragThreads) gemv_frags_kernel(const FragArgs p) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int lane = threadIdx.x & 31, job = blockIdx.x * (kFragThreads / 32) + (threadIdx.x >> 5);
+  const int m = job / p.nb, b = job - m * p.nb, prob = blockIdx.y;
+  if (m >= p.batch) return;
+  int64_t row = m;
+  if (p.grp) {
+    const int4 d = p.grp[prob];
+    if (m >= d.z) return;
+    row = p.x_rows ? p.x_rows[d.y + m] : d.y + m;
+  }
+  const bool vec_ok = (p.ld_x % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.x) & 15) == 0);
+  float v[4];
+  load4_as_float(p.x, p.x_dtype, row * p.ld_x, b * kBlock + lane * 4, p.x_kind == PE_X_ROTATED ? p.nb * kBlock : p.in_f, vec_ok, v);
+  if (p.x_kind == PE_X_SILU_MUL) {  // the row is [gate | up]: half(silu(gate)) * up, the rounding steps of pe_silu_mul
+    float u[4];
+    load4_as_float(p.x, p.x_dtype, row * p.ld_x + p.in_f, b * kBlock + lane * 4, p.in_f, vec_ok && p.in_f % 4 == 0, u);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = __half2float(__hmul(__float2half_rn(v[i] / (1.f + expf(-v[i]))), __float2half_rn(u[i])));
+  }
+  if (p.x_kind != PE_X_ROTATED) warp_fwht128(v, lane);
+  uint4* dst = p.out + ((size_t)(prob * p.sets + (m >> 3)) * p.nb + b) * 128;
+  const int g = m & 7;
+  if (PACKED) {  // nibble byte i of the block is the pair (i, i + 64); lane t of a row holds bytes 16 t .. 16 t + 15
+    float o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = __shfl_xor_sync(0xffffffffu, v[i], 16);
+    if (lane < 16)
+      dst[(lane & 3) * 32 + g * 4 + (lane >> 2)] = make_uint4(pack_half2(v[0], o[0]), pack_half2(v[1], o[1]), pack_half2(v[2], o[2]), pack_half2(v[3], o[3]));
+  } else {       // neighbours; lane t holds codes 16 t .. 16 t + 15 of each half
+    const int k = (lane < 16 ? 0 : 4) + (lane & 3);
+    reinterpret_cast<uint2*>(dst + (k >> 1) * 32 + g * 4 + ((lane & 15) >> 2))[k & 1] = make_uint2(pack_half2(v[0], v[1]), pack_half2(v[2], v[3]));
+  }
+}
+
+// ---- the launch's line of units ---------------------------------------------------------------------------------
+// A pass is a run of units of one problem whose partial sums fit in shared memory.  The copy warp and the math warps
+// walk the same passes.
+template <bool TILED, bool GROUPED>
+struct Pass {
+  static constexpr int kUnit = TILED ? 16 : 1;  // weight rows per unit
+  int left;               // units of this CTA not yet passed
+  int prob, off;          // problem, unit inside it
+  int row0, rows;         // weight rows of this pass
+  __device__ __forceinline__ void start(const BulkArgs& p, int beg, int n) {
+    left = n;
+    prob = GROUPED ? beg / p.units : 0;
+    off = GROUPED ? beg - prob * p.units : beg;
+  }
+  __device__ __forceinline__ bool next(const BulkArgs& p) {  // false at the end; advances past the pass it describes
+    if (left <= 0) return false;
+    int n = min(p.pass_rows / kUnit, left);
+    if (GROUPED) {
+      if (off == p.units) { off = 0; ++prob; }
+      n = min(n, p.units - off);
+    }
+    row0 = off * kUnit;
+    rows = TILED ? min(n * kUnit, p.N - row0) : n;
+    left -= n; off += n;
+    return true;
+  }
+};
+
+template <bool PACKED, int NT, int BPW, bool TILED, bool GROUPED>
+__global__ void __launch_bounds__(kBulkThreads, 1) gemv_bulk_kernel(const BulkArgs p) {
+  extern __shared__ __align__(128) uint8_t smem[];  // no static shared memory: the window starts with it
+  constexpr int kRowBytes = PACKED ? 64 : 128;           // codes of one row's block
+  constexpr int kRecBytes = kRowBytes * 16 + 32;         // tiled record: 16 rows of a block, then their norms
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+  const uint32_t sbase = smem_u32(smem);
+  const uint32_t full = sbase, empty = sbase + 8 * kBulkMaxStages;
+  int& n_live = *reinterpret_cast<int*>(smem + 16 * kBulkMaxStages);
+  asm volatile("griddepcontrol.launch_dependents;");
+  if (sbase > kTabAddr - 256) {  // the table's place is taken: never seen, the host sizes for any base below
+    if (tid == 0 && p.status) atomicExch(p.status, PE_STATUS_SPLITK_TIMEOUT);
+    return;
+  }
+  if (tid == 0) {
+    for (int s = 0; s < p.n_stage; ++s) { bar_init(full + 8 * s, 1); bar_init(empty + 8 * s, kBulkWarps); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    n_live = 0;
+  }
+  __syncthreads();
+  int line = p.units;
+  if (GROUPED) {  // the problem list comes from the launch before this one
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int i = tid; i < p.n_problems; i += kBulkThreads)
+      if (p.grp[i].z > 0) atomicMax(&n_live, i + 1);
+    __syncthreads();
+    line = n_live * p.units;
+  }
+  Pass<TILED, GROUPED> ps;
+  {
+    const int q = line / (int)gridDim.x, r = line - q * (int)gridDim.x, cta = blockIdx.x;
+    const int beg = cta * q + min(cta, r);
+    ps.start(p, beg, q + (cta < r));
+  }
+
+  if (w == kBulkWarps) {  // ---- copy warp
+    int s = 0;
+    uint32_t ph = 1;
+    while (ps.next(p)) {
+      const uint8_t* codes = p.codes;
+      const uint8_t* tiles = p.tiles;
+      if (GROUPED) {
+        const int4 d = p.grp[ps.prob];
+        if (d.z <= 0) continue;
+        codes += d.x * p.codes_stride;
+        tiles += d.x * p.tiles_stride;
+      }
+      for (int c = 0; c < p.n_chunk; ++c) {
+        const int b0 = c * p.chunk_blocks, nblk = min(p.chunk_blocks, p.nb - b0);
+        for (int r0 = 0; r0 < ps.rows; r0 += 16) {
+          bar_wait(empty + 8 * s, ph, p.status);
+          const uint32_t dst = sbase + p.stage_off + s * p.stage_bytes, bar = full + 8 * s;
+          if (TILED) {
+            if (lane == 0) {
+              bar_expect(bar, nblk * kRecBytes);
+              bulk_load(dst, tiles + ((int64_t)((ps.row0 + r0) >> 4) * p.nb + b0) * kRecBytes, nblk * kRecBytes, bar);
+            }
+          } else {
+            const int rows = min(16, ps.rows - r0);
+            if (lane == 0) bar_expect(bar, rows * nblk * kRowBytes);
+            __syncwarp();
+            if (lane < rows)
+              bulk_load(dst + lane * p.row_stride, codes + (int64_t)(ps.row0 + r0 + lane) * p.ld_codes + b0 * kRowBytes, nblk * kRowBytes, bar);
+          }
+          if (++s == p.n_stage) { s = 0; ph ^= 1; }
+        }
+      }
+    }
+    return;
+  }
+
+  // ---- math warps: the table first (it needs nothing from the launch before this one)
+  {
+    uint8_t* tab = smem + (kTabAddr - sbase);
+    const int entries = PACKED ? (p.n_levels <= 8 ? 128 : 256) : p.n_levels;
+#pragma unroll 2
+    for (int e = tid >> 3; e < entries; e += kBulkWarps * 4) {
+      uint32_t u;
+      if (PACKED) {
+        const int a = e & 15, b = e >> 4;
+        u = pack_half2(a < p.n_levels ? __ldg(p.ct + a) : 0.f, b < p.n_levels ? __ldg(p.ct + b) : 0.f);
+      } else {
+        u = __half_as_ushort(__float2half_rn(__ldg(p.ct + e)));
+      }
+      *reinterpret_cast<uint4*>(tab + e * 256 + (tid & 7) * 16) = make_uint4(u, u, u, u);
+      if (!PACKED) *reinterpret_cast<uint4*>(tab + e * 256 + 128 + (tid & 7) * 16) = make_uint4(u << 16, u << 16, u << 16, u << 16);
+    }
+  }
+  auto stage_norms = [&](const __half* norms, int row0, int rows) {  // row-major layout: norms of a pass
+    for (int r = w; r < rows; r += kBulkWarps)
+      for (int b = lane; b < p.nb; b += 32)
+        *reinterpret_cast<__half*>(smem + p.norm_off + r * p.norm_stride + b * 2) = norms[(int64_t)(row0 + r) * p.ld_norms + b];
+  };
+  bool more = ps.next(p);
+  bool fresh = true;  // norms of the first pass are staged before the dependency wait
+  if (!TILED && !GROUPED && more) { stage_norms(p.norms, ps.row0, ps.rows); fresh = false; }
+  if (!GROUPED) asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  const uint32_t lane4 = lane * 4;
+  float* part = reinterpret_cast<float*>(smem + p.part_off);
+  uint32_t x[BPW][NT][16];
+  int x_prob = -1, group_rows = p.batch;
+  int expert = 0, y_row = 0;
+
+  auto load_x = [&](int prob, int c) {
+    const uint4* src = p.frags + (size_t)(prob * NT * p.nb + c * p.chunk_blocks + w) * 128 + lane;
+    const int nblk = p.nb - c * p.chunk_blocks;
+#pragma unroll
+    for (int j = 0; j < BPW; ++j)
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint4 v = make_uint4(0, 0, 0, 0);
+          if (w + kBulkWarps * j < nblk && n * 8 + g < (GROUPED ? group_rows : p.batch)) v = __ldcg(src + (n * p.nb + kBulkWarps * j) * 128 + q * 32);
+          x[j][n][4 * q] = v.x; x[j][n][4 * q + 1] = v.y; x[j][n][4 * q + 2] = v.z; x[j][n][4 * q + 3] = v.w;
+        }
+  };
+
+  int s = 0;
+  uint32_t ph = 0;
+  for (; more; more = ps.next(p)) {
+    if (ps.prob != x_prob) {
+      if (GROUPED) {
+        const int4 d = p.grp[ps.prob];
+        if (d.z <= 0) continue;
+        group_rows = d.z < 8 * NT ? d.z : 8 * NT;
+        y_row = d.y;
+        expert = d.x;
+      }
+      x_prob = ps.prob;
+      if (p.n_chunk == 1) load_x(x_prob, 0);
+    }
+    if (!TILED && fresh) stage_norms(p.norms + expert * p.norms_stride, ps.row0, ps.rows);
+    fresh = true;
+    math_sync();  // table and norms are there; the sums of the pass before are out
+    for (int c = 0; c < p.n_chunk; ++c) {
+      if (p.n_chunk > 1) load_x(x_prob, c);
+      const int b0 = c * p.chunk_blocks, nblk = min(p.chunk_blocks, p.nb - b0);
+      for (int r0 = 0; r0 < ps.rows; r0 += 16) {
+        const uint32_t st = sbase + p.stage_off + s * p.stage_bytes;
+        bar_wait(full + 8 * s, ph, p.status);
+        float acc[NT][4];
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < BPW; ++j) {
+          const int blk = w + kBulkWarps * j;
+          if (blk < nblk) {
+            float d[NT][4];
+            unsigned short ha, hb;
+            if (TILED) {
+              const uint32_t rec = st + blk * kRecBytes, a = rec + g * kRowBytes + t * 16;
+              asm volatile("ld.shared.u16 %0, [%1];" : "=h"(ha) : "r"(rec + 16 * kRowBytes + g * 2));
+              asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hb) : "r"(rec + 16 * kRowBytes + g * 2 + 16));
+              block_product<PACKED, NT>(a, a + 8 * kRowBytes, x[j], lane4, d);
+            } else {
+              const uint32_t a = st + g * p.row_stride + blk * kRowBytes + t * 16, nn = sbase + p.norm_off + (b0 + blk) * 2;
+              const int last = ps.rows - 1;
+              asm volatile("ld.shared.u16 %0, [%1];" : "=h"(ha) : "r"(nn + min(r0 + g, last) * p.norm_stride));
+              asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hb) : "r"(nn + min(r0 + g + 8, last) * p.norm_stride));
+              block_product<PACKED, NT>(a, a + 8 * p.row_stride, x[j], lane4, d);
+            }
+            const float fa = __half2float(__ushort_as_half(ha)), fb = __half2float(__ushort_as_half(hb));
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+              acc[n][0] = fmaf(fa, d[n][0], acc[n][0]); acc[n][1] = fmaf(fa, d[n][1], acc[n][1]);
+              acc[n][2] = fmaf(fb, d[n][2], acc[n][2]); acc[n][3] = fmaf(fb, d[n][3], acc[n][3]);
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0) bar_arrive(empty + 8 * s);
+        if (++s == p.n_stage) { s = 0; ph ^= 1; }
+        float* pp = part + w * p.part_rows * p.part_stride + r0 + g;
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int m = n * 8 + 2 * t + e;
+            if (m < (GROUPED ? group_rows : p.batch)) {
+              float* q = pp + m * p.part_stride;
+              if (c == 0) { q[0] = acc[n][e]; q[8] = acc[n][2 + e]; }
+              else { q[0] += acc[n][e]; q[8] += acc[n][2 + e]; }
+            }
+          }
+      }
+    }
+    math_sync();
+    const int groups = (ps.rows + 31) >> 5, batch = GROUPED ? group_rows : p.batch;
+    for (int e = w; e < groups * batch; e += kBulkWarps) {  // a warp sums 32 rows of one activation row
+      const int m = groups == 1 ? e : e / groups, r = (e - m * groups) * 32 + lane;
+      if (r < ps.rows) {
+        const float* q = part + m * p.part_stride + r;
+        float v[kBulkWarps], sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < kBulkWarps; ++i) v[i] = q[i * p.part_rows * p.part_stride];
+#pragma unroll
+        for (int i = 0; i < kBulkWarps; ++i) sum += v[i];
+        const int row = ps.row0 + r;
+        if (p.bias) sum += __half2float(p.bias[row]);
+        store_from_float(p.y, p.y_dtype, (int64_t)(y_row + m) * p.ld_y + row, sum);
+      }
+    }
+  }
+}
+
+// ---- host side --------------------------------------------------------------------------------------------------
+template <bool PACKED, int NT, int BPW, bool TILED, bool GROUPED>
+static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
+  constexpr int kRowBytes = PACKED ? 64 : 128, kRecBytes = kRowBytes * 16 + 32;
+  a.chunk_blocks = kBulkWarps * BPW;
+  a.n_chunk = (a.nb + a.chunk_blocks - 1) / a.chunk_blocks;
+  const int blocks = a.nb < a.chunk_blocks ? a.nb : a.chunk_blocks;  // of the largest stage
+  constexpr int kUnit = TILED ? 16 : 1;
+  a.units = TILED ? (a.N + 15) / 16 : a.N;
+  const long long line = (long long)a.units * (a.grp ? a.n_problems : 1);
+  if (line >= (1ll << 31)) return PE_ERR_LIMIT;
+  const int G = (int)(line < sms ? line : sms);
+  // Rows per pass: the sums of a pass meet at a barrier, so few and equal passes; 64 rows of 8 activation rows are
+  // 34 KB of partial sums, which the ring would rather have (64 measured best of 32, 64, 96 and 176).
+  a.part_rows = a.batch < 8 * NT ? a.batch : 8 * NT;
+  const int cta_rows = (int)((line + G - 1) / G) * kUnit;
+  const int entries = PACKED ? (a.n_levels <= 8 ? 128 : 256) : a.n_levels;
+  a.part_off = kTabAddr + entries * 256;  // leaves room for the table wherever the window starts
+  a.norm_stride = (a.nb & 1) ? a.nb * 2 : a.nb * 2 + 2;  // an odd number of halves: rows spread over the banks
+  a.row_stride = TILED ? 0 : (blocks * kRowBytes + 127) / 128 * 128 + 64;  // a quarter warp reads two rows: different halves of the banks
+  a.stage_bytes = TILED ? (blocks * kRecBytes + 127) & ~127 : 16 * a.row_stride;
+  for (int cap = a.part_rows <= 2 ? 256 : (NT == 1 ? 64 : 32);; cap /= 2) {  // smaller passes where long rows' norms take the ring's room
+    if (cap < 16) return PE_ERR_LIMIT;
+    const int passes = (cta_rows + cap - 1) / cap;
+    a.pass_rows = GROUPED ? cap : ((cta_rows + passes - 1) / passes + 15) / 16 * 16;
+    a.part_stride = a.pass_rows + 4;  // rows of a stage land on different banks than the activation rows' distance
+    a.norm_off = a.part_off + kBulkWarps * a.part_rows * a.part_stride * 4;
+    a.stage_off = (a.norm_off + (TILED ? 0 : a.pass_rows * a.norm_stride) + 127) & ~127;
+    a.n_stage = a.stage_off < (int)kBulkSmemMax ? ((int)kBulkSmemMax - a.stage_off) / a.stage_bytes : 0;
+    if (a.n_stage >= 2) break;
+  }
+  if (a.n_stage > kBulkMaxStages) a.n_stage = kBulkMaxStages;
+  unsigned dyn = a.stage_off + a.n_stage * a.stage_bytes;
+  if (dyn < (unsigned)(kTabAddr + kTabReach)) dyn = kTabAddr + kTabReach;
+  auto kfn = gemv_bulk_kernel<PACKED, NT, BPW, TILED, GROUPED>;
+  static thread_local unsigned configured[16] = {0};
+  int dev = 0;
+  PE_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev >= 16 || configured[dev] < dyn) {
+    PE_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    if (dev < 16) configured[dev] = dyn;
+  }
+  PE_CUDA_TRY(launch_pdl(kfn, dim3(G), dim3(kBulkThreads), dyn, st, a));
+  return PE_OK;
+}
+
+template <bool PACKED, bool TILED, bool GROUPED>
+static int launch_bulk_shape(BulkArgs& a, int sms, cudaStream_t st) {
+  // Blocks per warp and stage: two when the row is longer than sixteen blocks.  Two sets of activation rows keep one:
+  // their operands for two blocks spill (4096 x 12288 at 16 rows: 18.4 us with two, 15.9 with one).
+  if (a.batch > 8) return launch_bulk<PACKED, 2, 1, TILED, GROUPED>(a, sms, st);
+  return a.nb > kBulkWarps ? launch_bulk<PACKED, 1, 2, TILED, GROUPED>(a, sms, st) : launch_bulk<PACKED, 1, 1, TILED, GROUPED>(a, sms, st);
+}
+
+template <bool PACKED, bool TILED>
+static int launch_bulk_kind(BulkArgs& a, int sms, cudaStream_t st) {
+  return a.grp ? launch_bulk_shape<PACKED, TILED, true>(a, sms, st) : launch_bulk_shape<PACKED, TILED, false>(a, sms, st);
+}
+
+size_t gemv_bulk_frag_bytes(int problems, int batch, int in_f_padded) {
+  return (size_t)problems * (batch > 8 ? 2 : 1) * (in_f_padded / kBlock) * 2048;
+}
+
+int gemv_bulk_run(const GemvBulkCall& q, cudaStream_t st) {
+  const int sms = sm_count();
+  if (sms <= 0) return PE_ERR_CUDA;
+  FragArgs f = {};
+  f.x = q.x; f.x_kind = q.x_kind; f.x_dtype = q.x_dtype; f.ld_x = q.ld_x; f.in_f = q.in_f;
+  f.nb = q.in_f_padded / kBlock; f.batch = q.batch; f.sets = q.batch > 8 ? 2 : 1;
+  f.out = static_cast<uint4*>(q.frags);
+  f.grp = static_cast<const int4*>(q.problems); f.x_rows = q.x_rows;
+  const int warps = kFragThreads / 32;
+  const dim3 grid((q.batch * f.nb + warps - 1) / warps, q.problems ? q.max_problems : 1);
+  PE_CUDA_TRY(launch_pdl(q.packed ? gemv_frags_kernel<true> : gemv_frags_kernel<false>, grid, dim3(kFragThreads), 0, st, f));
+  BulkArgs a = {};
+  a.codes = static_cast<const uint8_t*>(q.codes); a.ld_codes = q.ld_codes;
+  a.norms = static_cast<const __half*>(q.norms); a.ld_norms = q.ld_norms;
+  a.tiles = static_cast<const uint8_t*>(q.tiles);
+  a.ct = q.ct_scaled; a.n_levels = q.n_levels;
+  a.frags = f.out;
+  a.y = q.y; a.y_dtype = q.y_dtype; a.ld_y = q.ld_y;
+  a.bias = static_cast<const __half*>(q.bias);
+  a.batch = q.batch; a.N = q.out_f; a.nb = f.nb;
+  a.status = q.status;
+  a.grp = f.grp; a.n_problems = q.max_problems;
+  a.codes_stride = q.codes_stride; a.norms_stride = q.norms_stride; a.tiles_stride = q.tiles_stride;
+  if (q.packed) return q.tiles ? launch_bulk_kind<true, true>(a, sms, st) : launch_bulk_kind<true, false>(a, sms, st);
+  return q.tiles ? launch_bulk_kind<false, true>(a, sms, st) : launch_bulk_kind<false, false>(a, sms, st);
+}
+
+}  // namespace pe

@@ -126,20 +126,23 @@ __device__ __forceinline__ float reg_dot(const uint4& q, uint32_t lane_base, con
 }
 
 
-// Decides whether the row-owner kernel (pe_gemv_rows.cu) takes a call and launches it.
-// Returns PE_OK after a launch, 1 if the shape is not its kind (the caller goes on to the
-// tile kernel), or a negative error code.
-int gemv_rows_try(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms,
-                  const float* ct_scaled, int n_levels, const void* x, int x_kind, int x_dtype, int64_t ld_x, int in_f,
-                  void* y, int y_dtype, int64_t ld_y, const void* bias, int batch, int out_f, int in_f_padded,
-                  int* status, cudaStream_t stream);
+// The one-token column-owner kernel over row-major codes (pe_gemv_cols.cu).  PE_OK after a launch, 1 if the layer's
+// shape is not its kind (the caller goes on to the bulk-copy kernel), or a negative error code.
+int gemv_cols_run(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms, const float* ct_scaled, int n_levels,
+                  const void* x, int x_kind, int x_dtype, int in_f, void* y, int y_dtype, const void* bias, int out_f, int in_f_padded,
+                  cudaStream_t stream);
 
-// The column-owner kernel for 3..8 activation rows (pe_gemv_cols8.cu), row-major layout only.  Returns PE_OK after a
-// launch, 1 if the shape is not its kind, or a negative error code; gemv_cols8_takes answers the same question
-// without launching.
-int gemv_cols8_try(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms, const float* ct_scaled,
-                   int n_levels, const void* x, int x_kind, int x_dtype, int64_t ld_x, int in_f, void* y, int y_dtype,
-                   int64_t ld_y, const void* bias, int batch, int out_f, int in_f_padded, cudaStream_t stream);
-bool gemv_cols8_takes(int packed, int64_t ld_codes, const void* norms, int64_t ld_norms, int out_f, int in_f_padded);
+// The bulk-copy kernel (pe_gemv_bulk.cu) for 1..16 activation rows: either layout (tiles when not null), one matrix or a
+// grouped launch (problems when not null; batch is then the largest row count of a problem).  Arguments checked by
+// the caller.
+struct GemvBulkCall {
+  const void* codes; int packed; int64_t ld_codes; const void* norms; int64_t ld_norms; const void* tiles;
+  const float* ct_scaled; int n_levels; const void* x; int x_kind; int x_dtype; int64_t ld_x; int in_f;
+  void* y; int y_dtype; int64_t ld_y; const void* bias; int batch; int out_f; int in_f_padded; int* status;
+  void* frags;  // scratch of gemv_bulk_frag_bytes() bytes, 16-byte aligned: the activations in operand order
+  const void* problems; int max_problems; const int32_t* x_rows; int64_t codes_stride, norms_stride, tiles_stride;
+};
+int gemv_bulk_run(const GemvBulkCall& q, cudaStream_t stream);
+size_t gemv_bulk_frag_bytes(int problems, int batch, int in_f_padded);
 
 }  // namespace pe

@@ -22,7 +22,7 @@ from typing import Any, Dict, List, Optional
 
 import torch
 
-from .kernels import SMALL_BATCH_MAX, pack_codes_int4, quant_matmul, retile, small_batch_takes
+from .kernels import GEMV_MAX_BATCH, pack_codes_int4, quant_matmul, retile
 from .packing import unpack_codes_half_block, unpack_codes_q5
 from .utils import get_ct_scaled
 
@@ -81,8 +81,8 @@ class PolarQuantLinearMethod(_Base):
         self.bits = bits
         self.layer_meta = layer_meta or {}
         # The tiled copy of a layer (codes and norms interleaved per 16-row x 128-column tile) serves batches of
-        # 3..16 rows only; it is built the first time such a batch arrives, so a layer that only ever sees one
-        # token at a time, or prefill, keeps a single copy of its codes in HBM.
+        # up to 16 rows; it is built the first time such a batch arrives, so a layer that only ever sees prefill
+        # keeps a single copy of its codes in HBM.  False: one copy always, decode batches read the row-major arrays.
         self.decode_tiled = True
 
     # ------------------------------------------------------------------ weights
@@ -141,10 +141,8 @@ class PolarQuantLinearMethod(_Base):
         x2 = x.reshape(-1, layer.in_f)
         packed = bool(getattr(layer, "packed", False))
         w = layer.codes_packed if packed else layer.codes
-        if (self.decode_tiled and 3 <= x2.shape[0] <= 16 and getattr(layer, "codes_tiled", None) is None
-                and not torch.cuda.is_current_stream_capturing()
-                and not (x2.shape[0] <= SMALL_BATCH_MAX
-                         and small_batch_takes(w.data, packed, layer.norms.data.reshape(layer.out_f, -1), layer.out_f, layer.in_f_padded))):
+        if (self.decode_tiled and 1 <= x2.shape[0] <= GEMV_MAX_BATCH and getattr(layer, "codes_tiled", None) is None
+                and not torch.cuda.is_current_stream_capturing()):
             layer.codes_tiled = retile(w.data, packed, layer.norms.data)
         # one native entry for every batch size: <= 16 rows run the fused decode kernel,
         # more rows the tensor-core kernel (rotation is done by its preparation launch)
