@@ -540,9 +540,12 @@ def main():
     xh = torch.randn(a.batch, HIDDEN, device=dev, generator=g).half()
     xi = torch.randn(a.batch, INTER, device=dev, generator=g).half()
 
-    def launch(layer, name):
+    tiles = {id(layer): {name: kernels.retile(*layer[name][:3]) for name, _, _, _ in PROJ} for layer in layers}
+
+    def launch(layer, name):  # on the tiled copy, as apply() runs a decode-size batch
         w, packed, norms, ct, n, k = layer[name]
-        return kernels.quant_matmul(w, packed, norms, ct, xh if k == HIDDEN else xi, False, n, k, k, torch.float16)
+        return kernels.quant_matmul(w, packed, norms, ct, xh if k == HIDDEN else xi, False, n, k, k, torch.float16,
+                                    tiles=tiles[id(layer)][name] if a.batch <= kernels.GEMV_MAX_BATCH else None)
 
     def ring_pass(names):
         for layer in layers:
@@ -600,35 +603,27 @@ def main():
     value = step_bytes(a.batch) * steps * world / elapsed / 1e9
 
     # ---- end to end through the plugin surface with host buffers
-    method = {}
-    mods = {}
-    for name, n, k, bits in PROJ:
-        m = PolarQuantLinearMethod(128, bits)
+    method = {name: PolarQuantLinearMethod(128, bits) for name, _, _, bits in PROJ}
+
+    def make_module(layer, name, n, k, bits):
         mod = torch.nn.Module()
-        w, packed, norms, ct, _, _ = layers[0][name]
+        w, packed, norms, ct, _, _ = layer[name]
         mod.in_f, mod.out_f, mod.in_f_padded, mod.n_blocks, mod.bits, mod.block_size = k, n, k, k // 128, bits, 128
         mod.packed, mod.norms, mod.ct_scaled = packed, norms, ct
         if packed:
             mod.codes_packed, mod.in_f_half = w, k // 2
         else:
             mod.codes = w
-        method[name], mods[name] = m, mod
+        return mod
+    mods = [{name: make_module(layer, name, n, k, bits) for name, n, k, bits in PROJ} for layer in layers]
     hx = {k: torch.randn(a.batch, k).half().pin_memory() for k in (HIDDEN, INTER)}
     hy = torch.empty(a.batch, HIDDEN, dtype=torch.float16).pin_memory()
     e2e_steps = min(max(steps, 200), 1000)
 
     def e2e_body(i, dx):
-        layer = layers[i % RING]
         y = None
         for name, n, k, bits in PROJ:
-            mod = mods[name]
-            w, packed, norms, ct, _, _ = layer[name]
-            mod.norms = norms
-            if packed:
-                mod.codes_packed = w
-            else:
-                mod.codes = w
-            y = method[name].apply(mod, dx[k])
+            y = method[name].apply(mods[i % RING][name], dx[k])
         return y
 
     def e2e_step_eager(i):
@@ -690,17 +685,16 @@ def main():
     dom_launches = dom_passes * RING
     dom_bytes = sum(alg_bytes(n, k, b, a.batch) for nm, n, k, b in PROJ if nm in dom)
     achieved = dom_bytes / (dom_elapsed / dom_launches) / 1e9
-    dom_kernel = ("gemv_cols_kernel<nibble codes, table, 3 chunks per warp>" if a.batch == 1 else
-                  "gemv_rows_kernel<nibble codes, table>" if a.batch == 2 else "gemv_kernel (tile kernel)<nibble codes, table>")
+    dom_kernel = "gemv_bulk_kernel<nibble codes, tiled>"
     roofline = {"bound": "hbm", "kernel": dom_kernel + " on down_proj 4096x12288 Q4",
                 "achieved": achieved, "peak": peak, "peak_source": "measured (MEASURED_PEAKS.json)" if peaks else "fallback",
                 "unit": "GB/s", "frac": achieved / peak, "avg_launch_us": dom_elapsed / dom_launches * 1e6,
                 "alg_bytes_per_launch": dom_bytes, "launches_timed": dom_launches,
                 "traffic": measured_traffic("down_proj_b1") if a.batch == 1 else None}
     line = dict(base, value=value, ms_per_step=elapsed / steps * 1e3, steps=steps, steps_requested=a.steps, e2e=e2e,
-                gpu_launches=4 * steps, roofline=roofline, clocks=sampler.summary(), frac_of_measured_hbm=value / world / peak,
+                gpu_launches=8 * steps, roofline=roofline, clocks=sampler.summary(), frac_of_measured_hbm=value / world / peak,
                 timed_region_s=elapsed)
-    del layers, mods, graphs
+    del layers, mods, graphs, tiles
     torch.cuda.empty_cache()
 
     if rank == 0 and not a.no_cpu_baseline and world == 1:

@@ -94,6 +94,25 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native host path (csrc/pe_host.cpp), bound to the library :func:`lib` loads.  Its functions return None for
+    whatever is not the plain case; the Python path then does the call."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _host as ext
+        except ImportError as exc:
+            raise RuntimeError("polarengine_vllm_b200/_host.so not found or not loadable: build it with "
+                               "`make -C polarengine_vllm_b200/csrc` (or __graft_entry__.build())") from exc
+        ext.setup(library_path())
+        _host = ext
+    return _host
+
+
 def check(code: int, what: str) -> None:
     if code != 0:
         l = lib()

@@ -53,6 +53,10 @@ def quant_matmul(codes: torch.Tensor, packed: bool, norms: torch.Tensor, ct_scal
     """y (batch, out_f) for x (batch, in_f or in_f_padded); the single entry to the
     native kernels used by everything else in the package.  ``tiles`` (from
     :func:`retile`) lets batches of up to 16 rows stream the tiled copy of the layer."""
+    y = (nv._host or nv.host()).matmul(codes, packed, norms, ct_scaled, x, rotated, out_f, in_f, in_f_padded, out_dtype, bias, tiles)
+    if y is not None:
+        return y
+    # tensors to convert or to lay out, empty batches, errors to report
     dev = nv.require_cuda(codes, norms, ct_scaled, x)
     nv.ensure_init(dev)
     if x.dim() != 2 or x.stride(1) != 1:

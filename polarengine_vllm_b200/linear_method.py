@@ -22,6 +22,7 @@ from typing import Any, Dict, List, Optional
 
 import torch
 
+from . import _native as nv
 from .kernels import GEMV_MAX_BATCH, pack_codes_int4, quant_matmul, retile
 from .packing import unpack_codes_half_block, unpack_codes_q5
 from .utils import get_ct_scaled
@@ -133,21 +134,30 @@ class PolarQuantLinearMethod(_Base):
             layer.codes_packed = packed
             layer.in_f_half = layer.n_blocks * (layer.block_size // 2)
             layer.packed = True
-        layer.codes_tiled = None
+        layer.codes_tiled = layer.codes_tiled_of = None
 
     # ------------------------------------------------------------------ forward
     def apply(self, layer: torch.nn.Module, x: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+        y = (nv._host or nv.host()).apply(layer, x, bias, self.decode_tiled)
+        if y is not None:
+            return y
+        # the first decode-size batch (the tiled copy is made here), tensors to convert or to lay out, errors to report
         lead = x.shape[:-1]
         x2 = x.reshape(-1, layer.in_f)
         packed = bool(getattr(layer, "packed", False))
         w = layer.codes_packed if packed else layer.codes
-        if (self.decode_tiled and 1 <= x2.shape[0] <= GEMV_MAX_BATCH and getattr(layer, "codes_tiled", None) is None
-                and not torch.cuda.is_current_stream_capturing()):
-            layer.codes_tiled = retile(w.data, packed, layer.norms.data)
-        # one native entry for every batch size: <= 16 rows run the fused decode kernel,
+        tiles = None
+        if self.decode_tiled and 1 <= x2.shape[0] <= GEMV_MAX_BATCH:
+            made_of = (w.data_ptr(), layer.norms.data_ptr())
+            if getattr(layer, "codes_tiled_of", None) != made_of and not torch.cuda.is_current_stream_capturing():
+                layer.codes_tiled = retile(w.data, packed, layer.norms.data)
+                layer.codes_tiled_of = made_of
+            if getattr(layer, "codes_tiled_of", None) == made_of:
+                tiles = layer.codes_tiled
+        # one native entry for every batch size: up to 16 rows run the fused decode kernel,
         # more rows the tensor-core kernel (rotation is done by its preparation launch)
         y = quant_matmul(w, packed, layer.norms, layer.ct_scaled, x2, False, layer.out_f, layer.in_f,
-                         layer.in_f_padded, torch.float16, bias, tiles=getattr(layer, "codes_tiled", None))
+                         layer.in_f_padded, torch.float16, bias, tiles=tiles)
         return y.view(*lead, layer.out_f)
 
 

@@ -147,11 +147,45 @@ class PolarQuantMoEMethod:
         ``apply(layer, x, topk_weights, topk_ids, ...)`` (routing done by the caller, vLLM 0.2x) and
         ``apply(layer, x, router_logits, top_k, renormalize, ...)`` (the reference's, moe_method.py:74-78)."""
         if torch.is_tensor(b) and not b.is_floating_point():
+            y = self._moe_native(layer, x, a, b, b.shape[-1], True, expert_map)
+            if y is not None:
+                return y
             topk_weights, topk_ids = a, b
         else:
             renorm = rest[0] if rest else kwargs.get("renormalize", True)
+            y = self._moe_native(layer, x, a, int(b), int(b), bool(renorm), expert_map)
+            if y is not None:
+                return y
             topk_weights, topk_ids = route_softmax_topk(a, int(b), bool(renorm))
         return self.moe_forward(layer, x, topk_weights, topk_ids, expert_map)
+
+    def _moe_native(self, layer, x, a, b, top_k: int, renormalize: bool, expert_map) -> Optional[torch.Tensor]:
+        """The grouped path from routing to the weighted sum in one native call (``a``, ``b``: router logits and top_k, or
+        top-k weights and ids); None when it is not the plain case."""
+        if x.dtype not in (torch.float16, torch.bfloat16):
+            return None
+        n_local = layer.w13_codes.shape[0]
+        pairs = x.numel() // layer.moe_hidden * top_k
+        plan = self._grouped_plan(pairs, n_local, expert_map)
+        if plan is None:
+            return None
+        rpp, max_problems, tensor_cores = plan
+        tiled = not tensor_cores and self._decode_tiles(layer)
+        return (nv._host or nv.host()).moe(
+            x, a, b, renormalize, expert_map,
+            (layer.w13_codes, layer.w13_norms, layer.w13_ct_scaled, layer.w13_tiles if tiled else None, self.w13_bits <= 4),
+            (layer.w2_codes, layer.w2_norms, layer.w2_ct_scaled, layer.w2_tiles if tiled else None, self.w2_bits <= 4),
+            (layer.moe_hidden, layer.moe_inter, layer.moe_hidden_padded, layer.moe_inter_padded), rpp, max_problems, tensor_cores)
+
+    def _grouped_plan(self, pairs: int, n_local: int, expert_map) -> Optional[Tuple[int, int, bool]]:
+        """(rows per problem, problem slots, tensor cores) of the grouped launches for that many (token, expert) pairs;
+        None when every expert has enough rows to fill the tensor-core kernel by itself."""
+        local_pairs = self.expected_local_pairs(pairs, n_local, expert_map)
+        if pairs < 1 or local_pairs > self.GROUPED_MAX_ROWS_PER_EXPERT * n_local:
+            return None
+        # rows per problem: 8 while experts see few tokens (lighter kernel), else 16
+        rpp = 8 if local_pairs <= 6 * n_local else 16
+        return rpp, min(n_local, pairs) + pairs // rpp, local_pairs >= self.TENSOR_CORE_MIN_ROWS_PER_EXPERT * n_local
 
     # average (token, expert) pairs per local expert up to which the grouped launches are
     # used; beyond it every expert has enough rows to fill the tensor-core kernel by itself
@@ -167,12 +201,14 @@ class PolarQuantMoEMethod:
         """y[t] = sum_k w[t,k] * down_e(silu(gate_e(x[t])) * up_e(x[t])), e = ids[t,k]; fp16 out.
         Decode-size batches: two grouped launches over all experts (``pe_gemv_grouped``),
         nothing read back to the host.  Prefill-size batches: per-expert tensor-core matmuls."""
-        n_local = layer.w13_codes.shape[0]
-        if self.expected_local_pairs(topk_ids.numel(), n_local, expert_map) <= self.GROUPED_MAX_ROWS_PER_EXPERT * n_local \
-                and x.dtype in (torch.float16, torch.bfloat16):
-            out = self._moe_forward_grouped(layer, x, topk_weights, topk_ids, expert_map)
-            if out is not None:
-                return out
+        if x.dtype in (torch.float16, torch.bfloat16):
+            y = None
+            if topk_weights.dtype == torch.float32 and topk_ids.dtype == torch.int64:
+                y = self._moe_native(layer, x, topk_weights, topk_ids, topk_ids.shape[-1], True, expert_map)
+            if y is None:
+                y = self._moe_forward_grouped(layer, x, topk_weights, topk_ids, expert_map)
+            if y is not None:
+                return y
         return self._moe_forward_per_expert(layer, x, topk_weights, topk_ids, expert_map)
 
     @staticmethod
@@ -213,10 +249,10 @@ class PolarQuantMoEMethod:
         pairs = t * k
         ids = topk_ids.reshape(-1).to(torch.int64).contiguous()
         emap = expert_map.to(device=dev, dtype=torch.int64).contiguous() if expert_map is not None else None
-        # rows per problem: 8 while experts see few tokens (lighter kernel), else 16
-        local_pairs = self.expected_local_pairs(pairs, n_local, expert_map)
-        rpp = 8 if local_pairs <= 6 * n_local else 16
-        max_problems = min(n_local, pairs) + pairs // rpp
+        plan = self._grouped_plan(pairs, n_local, expert_map)
+        if plan is None:
+            return None
+        rpp, max_problems, tensor_cores = plan
         l = nv.lib()
         if min(l.pe_gemv_grouped_workspace_bytes(max_problems, 2 * i, hp), l.pe_gemv_grouped_workspace_bytes(max_problems, h, ip)) == 0:
             return None  # more problems than the scratch counter zone holds: the caller takes the per-expert path
@@ -231,8 +267,6 @@ class PolarQuantMoEMethod:
                  "pe_moe_plan")
         # many rows per expert: the tensor-core kernel over all experts (tile list built on the device);
         # few: the decode-size kernel, which streams every expert's codes once per 8 or 16 rows
-        tensor_cores = local_pairs >= self.TENSOR_CORE_MIN_ROWS_PER_EXPERT * n_local
-
         tiled = not tensor_cores and self._decode_tiles(layer)
 
         def grouped(codes, packed, norms, ct, xin, x_kind, x_rows, in_f, kp, y, tiles):
