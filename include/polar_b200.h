@@ -337,6 +337,13 @@ int pe_gemv_pro(const void* codes, int packed, int64_t ld_codes, const void* nor
                 int delta_dtype, const void* norm_weight, void* resid_out, float eps, void* y, int y_dtype,
                 const void* bias, int out_f, int in_f_padded, void* stream);
 
+/* The same on a tiled copy of the layer (pe_retile), any shape: the glue op is computed where the activations are
+ * prepared.  Scratch as for pe_gemv with one row. */
+int pe_gemv_pro_tiled(const void* tiles, int packed, const float* ct_scaled, int n_levels, int prologue, const void* x, int in_f,
+                      const void* delta, int delta_dtype, const void* norm_weight, void* resid_out, float eps, void* y,
+                      int y_dtype, const void* bias, int out_f, int in_f_padded, void* workspace, size_t workspace_bytes,
+                      void* stream);
+
 /* ---- decode-size matmul without caller scratch ----------------------------------
  * Same computation and arguments as pe_gemv, minus workspace / workspace_bytes.  It has
  * no counterpart in the reference.  It is meant for integrations that are not in a

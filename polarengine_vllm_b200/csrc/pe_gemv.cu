@@ -11,7 +11,7 @@ namespace pe {
 
 // Scratch layout: [256 KB, last word: status (0 = ok)][activations in operand order].  pe_gemv_workspace_bytes is an
 // upper bound of what a launch touches: callers plan with it, and pe_gemv_noalloc draws its line by it.
-constexpr size_t kCounterBytes = 262144;
+constexpr size_t kCounterBytes = kGemvStatusBytes;
 constexpr int kMaxRowTiles = (int)(kCounterBytes / sizeof(unsigned)) - 1;
 constexpr int kMaxSms = 256;
 

@@ -178,16 +178,35 @@ struct FragArgs {
   const void* x; int x_kind, x_dtype; int64_t ld_x; int in_f, nb, batch, sets;  // sets of eight rows per problem
   uint4* out;
   const int4* grp; const int32_t* x_rows;
+  // one row, fp16: the residual add and the norm in front of the projection (PE_PRO_ADD_RMSNORM)
+  const void* delta; int delta_dtype; const __half* norm_w; __half* resid_out; float eps;
 };
 constexpr int kFragThreads = 128;
 
-template <bool PACKED>
+// Four consecutive fp16 / fp32 values as loaded, and their fp32 form; columns past in_f (a multiple of 4) are zero.
+__device__ __forceinline__ Raw4 raw4(const void* base, int dtype, int col, int in_f) {
+  Raw4 r = {{0u, 0u, 0u, 0u}};
+  if (base && col < in_f) r = load4_raw(base, dtype, 0, col, in_f, true);
+  return r;
+}
+// updated residual half(x + half(delta)) from the raw values
+__device__ __forceinline__ void residual4(const FragArgs& p, const Raw4& x, const Raw4& d, float r[4]) {
+  cvt4(x, PE_F16, r);
+  if (p.delta) {
+    float f[4];
+    cvt4(d, p.delta_dtype, f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = __half2float(__float2half_rn(r[i] + __half2float(__float2half_rn(f[i]))));
+  }
+}
+
+template <bool PACKED, bool NORM>
 __global__ void __launch_bounds__(kFragThreads) gemv_frags_kernel(const FragArgs p) {
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int lane = threadIdx.x & 31, job = blockIdx.x * (kFragThreads / 32) + (threadIdx.x >> 5);
   const int m = job / p.nb, b = job - m * p.nb, prob = blockIdx.y;
-  if (m >= p.batch) return;
+  if (!NORM && m >= p.batch) return;
   int64_t row = m;
   if (p.grp) {
     const int4 d = p.grp[prob];
@@ -196,7 +215,47 @@ __global__ void __launch_bounds__(kFragThreads) gemv_frags_kernel(const FragArgs
   }
   const bool vec_ok = (p.ld_x % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.x) & 15) == 0);
   float v[4];
-  load4_as_float(p.x, p.x_dtype, row * p.ld_x, b * kBlock + lane * 4, p.x_kind == PE_X_ROTATED ? p.nb * kBlock : p.in_f, vec_ok, v);
+  if (NORM) {  // PE_PRO_ADD_RMSNORM, one row
+    // every block of threads sums the row's squares for itself (8 KB from L2, all loads of 4096 columns in flight
+    // together); a warp stores the residual of its own 128 columns
+    __shared__ float sums[kFragThreads / 32];
+    const int col = b * kBlock + lane * 4;
+    const Raw4 own_x = raw4(m == 0 ? p.x : nullptr, PE_F16, col, p.in_f), own_d = raw4(m == 0 ? p.delta : nullptr, p.delta_dtype, col, p.in_f),
+               own_w = raw4(m == 0 ? p.norm_w : nullptr, PE_F16, col, p.in_f);
+    constexpr int U = 8;
+    float ss = 0.f;
+    for (int c0 = threadIdx.x * 4; c0 < p.in_f; c0 += kFragThreads * 4 * U) {
+      Raw4 x[U], d[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        x[u] = raw4(p.x, PE_F16, c0 + u * kFragThreads * 4, p.in_f);
+        d[u] = raw4(p.delta, p.delta_dtype, c0 + u * kFragThreads * 4, p.in_f);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float r[4];
+        residual4(p, x[u], d[u], r);
+        ss += r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3];
+      }
+    }
+#pragma unroll
+    for (int i = 16; i >= 1; i >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, i);
+    if (lane == 0) sums[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    if (m > 0) return;
+    ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < kFragThreads / 32; ++i) ss += sums[i];
+    const float scale = rsqrtf(ss / (float)p.in_f + p.eps);
+    residual4(p, own_x, own_d, v);
+    if (p.resid_out && col < p.in_f) *reinterpret_cast<uint2*>(p.resid_out + col) = make_uint2(pack_half2(v[0], v[1]), pack_half2(v[2], v[3]));
+    float wn[4];
+    cvt4(own_w, PE_F16, wn);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = __half2float(__hmul(__float2half_rn(v[i] * scale), __float2half_rn(wn[i])));
+  } else {
+    load4_as_float(p.x, p.x_dtype, row * p.ld_x, b * kBlock + lane * 4, p.x_kind == PE_X_ROTATED ? p.nb * kBlock : p.in_f, vec_ok, v);
+  }
   if (p.x_kind == PE_X_SILU_MUL) {  // the row is [gate | up]: half(silu(gate)) * up, the rounding steps of pe_silu_mul
     float u[4];
     load4_as_float(p.x, p.x_dtype, row * p.ld_x + p.in_f, b * kBlock + lane * 4, p.in_f, vec_ok && p.in_f % 4 == 0, u);
@@ -526,9 +585,13 @@ int gemv_bulk_run(const GemvBulkCall& q, cudaStream_t st) {
   f.nb = q.in_f_padded / kBlock; f.batch = q.batch; f.sets = q.batch > 8 ? 2 : 1;
   f.out = static_cast<uint4*>(q.frags);
   f.grp = static_cast<const int4*>(q.problems); f.x_rows = q.x_rows;
+  f.delta = q.delta; f.delta_dtype = q.delta_dtype; f.norm_w = static_cast<const __half*>(q.norm_w);
+  f.resid_out = static_cast<__half*>(q.resid_out); f.eps = q.eps;
   const int warps = kFragThreads / 32;
   const dim3 grid((q.batch * f.nb + warps - 1) / warps, q.problems ? q.max_problems : 1);
-  PE_CUDA_TRY(launch_pdl(q.packed ? gemv_frags_kernel<true> : gemv_frags_kernel<false>, grid, dim3(kFragThreads), 0, st, f));
+  auto frags = q.pro == PE_PRO_ADD_RMSNORM ? (q.packed ? gemv_frags_kernel<true, true> : gemv_frags_kernel<false, true>)
+                                           : (q.packed ? gemv_frags_kernel<true, false> : gemv_frags_kernel<false, false>);
+  PE_CUDA_TRY(launch_pdl(frags, grid, dim3(kFragThreads), 0, st, f));
   BulkArgs a = {};
   a.codes = static_cast<const uint8_t*>(q.codes); a.ld_codes = q.ld_codes;
   a.norms = static_cast<const __half*>(q.norms); a.ld_norms = q.ld_norms;

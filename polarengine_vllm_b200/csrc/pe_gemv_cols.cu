@@ -420,23 +420,32 @@ int gemv_cols_run(const void* codes, int packed, int64_t ld_codes, const void* n
 }  // namespace pe
 
 // ---- batch-1 matmul with the glue op in front of it computed while the input is staged ----
-extern "C" int pe_gemv_pro(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms,
-                           const float* ct_scaled, int n_levels, int prologue, const void* x, int in_f, const void* delta,
-                           int delta_dtype, const void* norm_weight, void* resid_out, float eps, void* y, int y_dtype,
-                           const void* bias, int out_f, int in_f_padded, void* stream) {
-  using namespace pe;
-  if (!codes || !norms || !ct_scaled || !x || !y) return PE_ERR_ARG;
+// Checks of the operands that both layouts share.
+static int pro_check(const float* ct_scaled, int n_levels, int packed, int prologue, const void* x, int in_f, const void* delta, int delta_dtype,
+                     const void* norm_weight, const void* resid_out, const void* y, int y_dtype, int out_f, int in_f_padded) {
+  if (!ct_scaled || !x || !y) return PE_ERR_ARG;
   if (prologue != PE_PRO_ADD_RMSNORM && prologue != PE_PRO_SILU_MUL) return PE_ERR_ARG;
   if (prologue == PE_PRO_ADD_RMSNORM && (!norm_weight || (delta && delta_dtype != PE_F16 && delta_dtype != PE_F32))) return PE_ERR_ARG;
   if (out_f < 1 || in_f < 4 || in_f > in_f_padded || y_dtype < PE_F32 || y_dtype > PE_BF16) return PE_ERR_ARG;
   if (n_levels < 2 || n_levels > 256 || (packed && n_levels > 16)) return PE_ERR_ARG;
-  if (in_f_padded % kBlock || in_f % 4) return PE_ERR_SHAPE;
-  if ((reinterpret_cast<uintptr_t>(codes) & 15) || (ld_codes & 15)) return PE_ERR_ALIGN;
+  if (in_f_padded % pe::kBlock || in_f % 4) return PE_ERR_SHAPE;
   // the prologue reads its operands 8 or 16 bytes at a time
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(delta) | reinterpret_cast<uintptr_t>(norm_weight) |
        reinterpret_cast<uintptr_t>(resid_out)) & 15)
     return PE_ERR_ALIGN;
   if (prologue == PE_PRO_SILU_MUL && (in_f % 8)) return PE_ERR_SHAPE;  // the `up` half starts in_f elements in: keep it 16-byte aligned
+  return PE_OK;
+}
+
+extern "C" int pe_gemv_pro(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms,
+                           const float* ct_scaled, int n_levels, int prologue, const void* x, int in_f, const void* delta,
+                           int delta_dtype, const void* norm_weight, void* resid_out, float eps, void* y, int y_dtype,
+                           const void* bias, int out_f, int in_f_padded, void* stream) {
+  using namespace pe;
+  if (!codes || !norms) return PE_ERR_ARG;
+  const int c = pro_check(ct_scaled, n_levels, packed, prologue, x, in_f, delta, delta_dtype, norm_weight, resid_out, y, y_dtype, out_f, in_f_padded);
+  if (c != PE_OK) return c;
+  if ((reinterpret_cast<uintptr_t>(codes) & 15) || (ld_codes & 15)) return PE_ERR_ALIGN;
   if (ld_codes < (packed ? in_f_padded / 2 : in_f_padded) || ld_norms < in_f_padded / kBlock) return PE_ERR_ARG;
   const int sms = sm_count();
   if (sms <= 0) return PE_ERR_CUDA;
@@ -446,3 +455,26 @@ extern "C" int pe_gemv_pro(const void* codes, int packed, int64_t ld_codes, cons
   return r == 1 ? PE_ERR_SHAPE : r;  // shapes the column-owner kernel does not take: the caller runs the separate launches
 }
 
+
+extern "C" int pe_gemv_pro_tiled(const void* tiles, int packed, const float* ct_scaled, int n_levels, int prologue, const void* x, int in_f,
+                                 const void* delta, int delta_dtype, const void* norm_weight, void* resid_out, float eps, void* y,
+                                 int y_dtype, const void* bias, int out_f, int in_f_padded, void* workspace, size_t workspace_bytes,
+                                 void* stream) {
+  using namespace pe;
+  if (!tiles || !workspace) return PE_ERR_ARG;
+  const int c = pro_check(ct_scaled, n_levels, packed, prologue, x, in_f, delta, delta_dtype, norm_weight, resid_out, y, y_dtype, out_f, in_f_padded);
+  if (c != PE_OK) return c;
+  if ((reinterpret_cast<uintptr_t>(tiles) & 15) || (reinterpret_cast<uintptr_t>(workspace) & 15)) return PE_ERR_ALIGN;
+  if (workspace_bytes < kGemvStatusBytes + gemv_bulk_frag_bytes(1, 1, in_f_padded)) return PE_ERR_WORKSPACE;
+  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  GemvBulkCall q = {};
+  q.tiles = tiles; q.packed = packed; q.ct_scaled = ct_scaled; q.n_levels = n_levels;
+  q.x = x; q.x_kind = prologue == PE_PRO_SILU_MUL ? PE_X_SILU_MUL : PE_X_RAW; q.x_dtype = PE_F16; q.ld_x = 2 * (int64_t)in_f; q.in_f = in_f;
+  q.y = y; q.y_dtype = y_dtype; q.ld_y = out_f; q.bias = bias;
+  q.batch = 1; q.out_f = out_f; q.in_f_padded = in_f_padded;
+  q.status = reinterpret_cast<int*>(ws + kGemvStatusBytes - 4);
+  q.frags = ws + kGemvStatusBytes;
+  q.pro = prologue == PE_PRO_ADD_RMSNORM ? prologue : PE_PRO_NONE;
+  q.delta = delta; q.delta_dtype = delta_dtype; q.norm_w = norm_weight; q.resid_out = resid_out; q.eps = eps;
+  return gemv_bulk_run(q, static_cast<cudaStream_t>(stream));
+}

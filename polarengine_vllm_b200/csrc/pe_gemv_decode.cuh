@@ -126,6 +126,8 @@ __device__ __forceinline__ float reg_dot(const uint4& q, uint32_t lane_base, con
 }
 
 
+constexpr size_t kGemvStatusBytes = 262144;  // first part of pe_gemv's scratch; its last word is the status word
+
 // The one-token column-owner kernel over row-major codes (pe_gemv_cols.cu).  PE_OK after a launch, 1 if the layer's
 // shape is not its kind (the caller goes on to the bulk-copy kernel), or a negative error code.
 int gemv_cols_run(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms, const float* ct_scaled, int n_levels,
@@ -141,6 +143,7 @@ struct GemvBulkCall {
   void* y; int y_dtype; int64_t ld_y; const void* bias; int batch; int out_f; int in_f_padded; int* status;
   void* frags;  // scratch of gemv_bulk_frag_bytes() bytes, 16-byte aligned: the activations in operand order
   const void* problems; int max_problems; const int32_t* x_rows; int64_t codes_stride, norms_stride, tiles_stride;
+  int pro; const void* delta; int delta_dtype; const void* norm_w; void* resid_out; float eps;  // PE_PRO_ADD_RMSNORM, one fp16 row
 };
 int gemv_bulk_run(const GemvBulkCall& q, cudaStream_t stream);
 size_t gemv_bulk_frag_bytes(int problems, int batch, int in_f_padded);

@@ -83,12 +83,16 @@ class QWeight:
     def fused(self, prologue: int, x: torch.Tensor, out_dtype=torch.float16, **kw) -> Optional[torch.Tensor]:
         """One token with the glue op in front of the projection folded into the launch; None if the layer's
         shape is not one the batch-1 kernel takes."""
+        self._make_tiles(1)
         return quant_matmul_pro(self.codes, self.packed, self.norms, self.ct, prologue, x, self.in_f, self.out_f, self.in_f,
-                                out_dtype, **kw)
+                                out_dtype, tiles=self.tiles, **kw)
+
+    def _make_tiles(self, rows: int) -> None:
+        if self.tiles is None and 1 <= rows <= GEMV_MAX_BATCH and not torch.cuda.is_current_stream_capturing():
+            self.tiles = retile(self.codes, self.packed, self.norms)
 
     def __call__(self, x: torch.Tensor, out_dtype=torch.float16) -> torch.Tensor:
-        if self.tiles is None and 1 <= x.shape[0] <= GEMV_MAX_BATCH and not torch.cuda.is_current_stream_capturing():
-            self.tiles = retile(self.codes, self.packed, self.norms)
+        self._make_tiles(x.shape[0])
         return quant_matmul(self.codes, self.packed, self.norms, self.ct, x, False, self.out_f, self.in_f, self.in_f, out_dtype,
                             tiles=self.tiles)
 
