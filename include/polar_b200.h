@@ -260,6 +260,11 @@ int pe_moe_route(const void* logits, int dtype, int64_t ld_logits, int n_tokens,
 int pe_moe_plan(const int64_t* topk_ids, const int64_t* expert_map, int n_global_experts, int n_pairs, int top_k, int n_local_experts,
                 int rows_per_problem, int max_problems, int32_t* row_token, int32_t* pos, int32_t* problems,
                 int32_t* expert_rows, void* stream);
+/* pe_moe_route and pe_moe_plan in one launch, for up to 1024 (token, slot) pairs. */
+int pe_moe_route_plan(const void* logits, int dtype, int64_t ld_logits, int n_tokens, int n_experts, int top_k, int renormalize,
+                      float* weights, int64_t* ids, const int64_t* expert_map, int n_global_experts, int n_local_experts,
+                      int rows_per_problem, int max_problems, int32_t* row_token, int32_t* pos, int32_t* problems,
+                      int32_t* expert_rows, void* stream);
 int pe_moe_combine(const float* y, int64_t ld_y, const int32_t* pos, const float* topk_weights, int tokens, int top_k,
                    void* out, int out_dtype, int64_t ld_out, int hidden, void* stream);
 

@@ -30,6 +30,7 @@ struct Api {
   decltype(&pe_gemm_workspace_bytes_splitk) gemm_bytes;
   decltype(&pe_moe_route) moe_route;
   decltype(&pe_moe_plan) moe_plan;
+  decltype(&pe_moe_route_plan) moe_route_plan;
   decltype(&pe_moe_combine) moe_combine;
   decltype(&pe_gemv_grouped) grouped;
   decltype(&pe_gemv_grouped_tiled) grouped_tiled;
@@ -332,12 +333,19 @@ PyObject* host_moe(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const float* weights = given ? a->const_data_ptr<float>() : reinterpret_cast<float*>(base + at_w);
   const int64_t* ids = given ? given->const_data_ptr<int64_t>() : reinterpret_cast<int64_t*>(base + at_ids);
   int rc = PE_OK;
-  if (!given)
-    rc = api.moe_route(a->const_data_ptr(), ad, a->stride(0), (int)tokens, (int)a->size(1), top_k, PyObject_IsTrue(args[3]) == 1,
-                       reinterpret_cast<float*>(base + at_w), reinterpret_cast<int64_t*>(base + at_ids), st);
-  if (rc == PE_OK)
-    rc = api.moe_plan(ids, emap ? emap->const_data_ptr<int64_t>() : nullptr, emap ? (int)emap->numel() : 0, (int)p.pairs, top_k, (int)p.n_local, rpp,
-                      max_problems, tok, pos, problems, rows, st);
+  const int64_t* map = emap ? emap->const_data_ptr<int64_t>() : nullptr;
+  const int n_global = emap ? (int)emap->numel() : 0;
+  float* w_out = reinterpret_cast<float*>(base + at_w);
+  int64_t* ids_out = reinterpret_cast<int64_t*>(base + at_ids);
+  if (!given && p.pairs <= 1024) {
+    rc = api.moe_route_plan(a->const_data_ptr(), ad, a->stride(0), (int)tokens, (int)a->size(1), top_k, PyObject_IsTrue(args[3]) == 1, w_out, ids_out,
+                            map, n_global, (int)p.n_local, rpp, max_problems, tok, pos, problems, rows, st);
+  } else {
+    if (!given)
+      rc = api.moe_route(a->const_data_ptr(), ad, a->stride(0), (int)tokens, (int)a->size(1), top_k, PyObject_IsTrue(args[3]) == 1, w_out, ids_out, st);
+    if (rc == PE_OK)
+      rc = api.moe_plan(ids, map, n_global, (int)p.pairs, top_k, (int)p.n_local, rpp, max_problems, tok, pos, problems, rows, st);
+  }
   const auto half = x->options().dtype(at::kHalf).requires_grad(false);
   const at::Tensor gu = at::empty({p.pairs, 2 * (int64_t)inter}, half);
   const at::Tensor d = at::empty({p.pairs, h}, half.dtype(at::kFloat));
@@ -375,6 +383,7 @@ PyObject* host_setup(PyObject*, PyObject* arg) {
   PE_SYMBOL(gemm_bytes, pe_gemm_workspace_bytes_splitk)
   PE_SYMBOL(moe_route, pe_moe_route)
   PE_SYMBOL(moe_plan, pe_moe_plan)
+  PE_SYMBOL(moe_route_plan, pe_moe_route_plan)
   PE_SYMBOL(moe_combine, pe_moe_combine)
   PE_SYMBOL(grouped, pe_gemv_grouped)
   PE_SYMBOL(grouped_tiled, pe_gemv_grouped_tiled)

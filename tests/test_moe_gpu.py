@@ -139,3 +139,35 @@ def test_routing_kernel_matches_softmax_topk(t, e, k, dtype):
         assert all(len(set(r.tolist())) == k for r in ids)
         if dtype == torch.float32:
             assert torch.equal(ids, rids)
+
+
+@pytest.mark.parametrize("t,e,k,mapped", [(1, 128, 8, False), (32, 60, 32, False), (33, 256, 4, True), (7, 1000, 3, True)])
+def test_joint_routing_and_plan_equals_the_two_launches(t, e, k, mapped):
+    """pe_moe_route_plan against pe_moe_route followed by a plan made on the host: the same weights and ids, every
+    pair's row inside its expert's range, and problems that cover the rows of each expert in pieces of eight."""
+    from polarengine_vllm_b200 import _native as nv
+    from polarengine_vllm_b200.moe_method import route_softmax_topk
+    g = torch.Generator().manual_seed(t * e)
+    logits = torch.randn(t, e, generator=g).cuda()
+    local = (e + 1) // 2 if mapped else e
+    emap = torch.where(torch.arange(e) % 2 == 0, torch.arange(e) // 2, -1) if mapped else torch.arange(e)
+    demap, pairs, cap = emap.cuda(), t * k, min(local, t * k) + t * k // 8
+    w, ids = torch.empty(t, k, device="cuda"), torch.empty(t, k, dtype=torch.int64, device="cuda")
+    tok, pos = (torch.full((pairs,), -7, dtype=torch.int32, device="cuda") for _ in range(2))
+    prob, rows = torch.empty(cap, 4, dtype=torch.int32, device="cuda"), torch.empty(local, 2, dtype=torch.int32, device="cuda")
+    nv.check(nv.lib().pe_moe_route_plan(logits.data_ptr(), 0, e, t, e, k, 1, w.data_ptr(), ids.data_ptr(), demap.data_ptr() if mapped else None,
+                                        e if mapped else 0, local, 8, cap, tok.data_ptr(), pos.data_ptr(), prob.data_ptr(), rows.data_ptr(),
+                                        nv.stream_ptr(logits.device)), "pe_moe_route_plan")
+    rw, rids = route_softmax_topk(logits, k, True)
+    assert torch.equal(w, rw) and torch.equal(ids, rids)
+    own = emap[ids.cpu()].flatten()
+    count = torch.bincount(own[own >= 0], minlength=local)
+    assert torch.equal(rows.cpu()[:, 1].long(), count) and torch.equal(rows.cpu()[:, 0].long(), count.cumsum(0) - count)
+    p, first = pos.cpu().long(), rows.cpu()[:, 0].long()
+    assert torch.equal(p < 0, own < 0)
+    live = own >= 0
+    assert (p[live] >= first[own[live]]).all() and (p[live] < (first + count)[own[live]]).all() and p[live].unique().numel() == int(live.sum())
+    assert torch.equal(tok.cpu().long()[p[live]], torch.arange(pairs)[live] // k)
+    want = [(x, int(first[x]) + 8 * j, min(8, int(count[x]) - 8 * j)) for x in range(local) for j in range(-(-int(count[x]) // 8))]
+    got = [tuple(r[:3]) for r in prob.cpu().tolist()]
+    assert got[:len(want)] == want and all(r[2] == 0 for r in got[len(want):])
