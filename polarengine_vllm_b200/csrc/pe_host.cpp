@@ -35,9 +35,8 @@ struct Api {
   decltype(&pe_gemv_grouped) grouped;
   decltype(&pe_gemv_grouped_tiled) grouped_tiled;
   decltype(&pe_gemv_grouped_workspace_bytes) grouped_bytes;
-  decltype(&pe_gemm_grouped) gemm_grouped;
+  decltype(&pe_gemm_grouped_routed) gemm_grouped;
   decltype(&pe_gemm_grouped_workspace_bytes) gemm_grouped_bytes;
-  decltype(&pe_silu_mul) silu_mul;
 };
 Api api;
 bool ready = false;
@@ -252,14 +251,14 @@ bool plain_experts(const Experts& w, const at::Device& dev, int64_t rows) {
 }
 
 int grouped(const Experts& w, const MoePlan& p, const at::Device& dev, cudaStream_t st, const void* x, int kind, int xd, int64_t ld_x, int in_f,
-            int in_f_padded, const int32_t* x_rows, void* y, int yd, int out_f) {
+            int in_f_padded, int x_total, const int32_t* x_rows, bool silu_mul, void* y, int yd, int out_f) {
   const float* ct = w.ct->const_data_ptr<float>();
   const int levels = (int)w.ct->numel();
   if (p.tensor_cores) {
     const at::Tensor ws = take_scratch(dev, st, 1, api.gemm_grouped_bytes((int)p.n_local, (int)p.pairs, out_f, in_f_padded), false);
     return api.gemm_grouped(w.codes->const_data_ptr(), w.packed, w.codes->stride(1), w.codes->stride(0), w.norms->const_data_ptr(),
-                            w.norms->stride(1), w.norms->stride(0), ct, levels, x, kind, xd, ld_x, in_f, x_rows, y, yd, out_f, p.expert_rows,
-                            (int)p.n_local, (int)p.pairs, out_f, in_f_padded, ws.mutable_data_ptr(), ws.numel(), st);
+                            w.norms->stride(1), w.norms->stride(0), ct, levels, x, kind, xd, ld_x, in_f, x_total, x_rows, silu_mul, y, yd,
+                            silu_mul ? out_f / 2 : out_f, p.expert_rows, (int)p.n_local, (int)p.pairs, out_f, in_f_padded, ws.mutable_data_ptr(), ws.numel(), st);
   }
   const at::Tensor ws = take_scratch(dev, st, 2, api.grouped_bytes((int)p.max_problems, out_f, in_f_padded), true);
   if (w.tiles)
@@ -347,18 +346,16 @@ PyObject* host_moe(PyObject*, PyObject* const* args, Py_ssize_t n) {
       rc = api.moe_plan(ids, map, n_global, (int)p.pairs, top_k, (int)p.n_local, rpp, max_problems, tok, pos, problems, rows, st);
   }
   const auto half = x->options().dtype(at::kHalf).requires_grad(false);
-  const at::Tensor gu = at::empty({p.pairs, 2 * (int64_t)inter}, half);
+  // tensor cores: the activation function is inside the first launch; else it is computed where the second one's input is prepared
+  const int64_t mid = p.tensor_cores ? inter : 2 * (int64_t)inter;
+  const at::Tensor gu = at::empty({p.pairs, mid}, half);
   const at::Tensor d = at::empty({p.pairs, h}, half.dtype(at::kFloat));
   if (rc == PE_OK)
-    rc = grouped(w[0], p, dev, st, x->const_data_ptr(), PE_X_RAW, xd, h, h, hp, tok, gu.mutable_data_ptr(), PE_F16, 2 * inter);
-  if (rc == PE_OK && p.tensor_cores) {
-    const at::Tensor act = at::empty({p.pairs, inter}, half);
-    rc = api.silu_mul(gu.const_data_ptr(), 2 * inter, act.mutable_data_ptr(), inter, (int)p.pairs, inter, st);
-    if (rc == PE_OK)
-      rc = grouped(w[1], p, dev, st, act.const_data_ptr(), PE_X_RAW, PE_F16, inter, inter, ip, nullptr, d.mutable_data_ptr(), PE_F32, h);
-  } else if (rc == PE_OK) {
-    rc = grouped(w[1], p, dev, st, gu.const_data_ptr(), PE_X_SILU_MUL, PE_F16, 2 * inter, inter, ip, nullptr, d.mutable_data_ptr(), PE_F32, h);
-  }
+    rc = grouped(w[0], p, dev, st, x->const_data_ptr(), PE_X_RAW, xd, h, h, hp, (int)tokens, tok, p.tensor_cores, gu.mutable_data_ptr(), PE_F16,
+                 2 * inter);
+  if (rc == PE_OK)
+    rc = grouped(w[1], p, dev, st, gu.const_data_ptr(), p.tensor_cores ? PE_X_RAW : PE_X_SILU_MUL, PE_F16, mid, inter, ip, 0, nullptr, false,
+                 d.mutable_data_ptr(), PE_F32, h);
   at::Tensor out = at::empty(x->sizes(), half);
   if (rc == PE_OK)
     rc = api.moe_combine(d.const_data_ptr<float>(), h, pos, weights, (int)tokens, top_k, out.mutable_data_ptr(), PE_F16, h, h, st);
@@ -388,9 +385,8 @@ PyObject* host_setup(PyObject*, PyObject* arg) {
   PE_SYMBOL(grouped, pe_gemv_grouped)
   PE_SYMBOL(grouped_tiled, pe_gemv_grouped_tiled)
   PE_SYMBOL(grouped_bytes, pe_gemv_grouped_workspace_bytes)
-  PE_SYMBOL(gemm_grouped, pe_gemm_grouped)
+  PE_SYMBOL(gemm_grouped, pe_gemm_grouped_routed)
   PE_SYMBOL(gemm_grouped_bytes, pe_gemm_grouped_workspace_bytes)
-  PE_SYMBOL(silu_mul, pe_silu_mul)
   ready = true;
   Py_RETURN_NONE;
 }

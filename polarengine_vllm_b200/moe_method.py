@@ -16,7 +16,6 @@ from typing import Optional, Tuple
 import torch
 
 from . import _native as nv
-from .decode_ops import silu_mul
 from .kernels import quant_matmul, retile
 from .packing import pack_codes_half_block
 from .utils import get_ct_scaled
@@ -253,6 +252,8 @@ class PolarQuantMoEMethod:
         if plan is None:
             return None
         rpp, max_problems, tensor_cores = plan
+        # the tensor-core launch addresses the experts' code matrices as one: they must follow each other
+        tensor_cores = tensor_cores and all(c.stride(0) == c.shape[1] * c.stride(1) for c in (layer.w13_codes, layer.w2_codes))
         l = nv.lib()
         if min(l.pe_gemv_grouped_workspace_bytes(max_problems, 2 * i, hp), l.pe_gemv_grouped_workspace_bytes(max_problems, h, ip)) == 0:
             return None  # more problems than the scratch counter zone holds: the caller takes the per-expert path
@@ -270,15 +271,15 @@ class PolarQuantMoEMethod:
         tiled = not tensor_cores and self._decode_tiles(layer)
 
         def grouped(codes, packed, norms, ct, xin, x_kind, x_rows, in_f, kp, y, tiles):
-            if tensor_cores and codes.stride(0) == codes.shape[1] * codes.stride(1):
-                need = l.pe_gemm_grouped_workspace_bytes(n_local, pairs, y.shape[1], kp)
+            if tensor_cores:
+                need = l.pe_gemm_grouped_workspace_bytes(n_local, pairs, codes.shape[1], kp)
                 ws = nv.gemm_workspace(dev, need)
-                nv.check(l.pe_gemm_grouped(codes.data_ptr(), int(packed), codes.stride(1) * codes.element_size(),
-                                           codes.stride(0) * codes.element_size(), norms.data_ptr(), norms.stride(1),
-                                           norms.stride(0), ct.data_ptr(), ct.numel(), xin.data_ptr(), nv.PE_X_RAW,
-                                           nv.dtype_code(xin), xin.stride(0), in_f, x_rows.data_ptr() if x_rows is not None else None,
-                                           y.data_ptr(), nv.dtype_code(y), y.stride(0), expert_rows.data_ptr(), n_local, pairs,
-                                           y.shape[1], kp, ws.data_ptr(), ws.numel(), st), "pe_gemm_grouped")
+                nv.check(l.pe_gemm_grouped_routed(codes.data_ptr(), int(packed), codes.stride(1) * codes.element_size(),
+                                                  codes.stride(0) * codes.element_size(), norms.data_ptr(), norms.stride(1),
+                                                  norms.stride(0), ct.data_ptr(), ct.numel(), xin.data_ptr(), nv.PE_X_RAW,
+                                                  nv.dtype_code(xin), xin.stride(0), in_f, t, x_rows.data_ptr() if x_rows is not None else None,
+                                                  int(x_rows is not None), y.data_ptr(), nv.dtype_code(y), y.stride(0), expert_rows.data_ptr(),
+                                                  n_local, pairs, codes.shape[1], kp, ws.data_ptr(), ws.numel(), st), "pe_gemm_grouped_routed")
                 return
             ws = nv.grouped_scratch(dev, l.pe_gemv_grouped_workspace_bytes(max_problems, y.shape[1], kp))
             if tiled:
@@ -294,14 +295,14 @@ class PolarQuantMoEMethod:
                                        in_f, x_rows.data_ptr() if x_rows is not None else None, y.data_ptr(), nv.dtype_code(y),
                                        y.stride(0), desc.data_ptr(), max_problems, rpp, y.shape[1], kp, ws.data_ptr(), ws.numel(), st),
                      "pe_gemv_grouped")
-        gu = torch.empty(pairs, 2 * i, dtype=torch.float16, device=dev)   # rows beyond the local pairs stay unused
+        # Rows beyond the local pairs stay unused.  silu(gate) * up is computed inside the first tensor-core launch, or (decode
+        # size) where the down projection's input is prepared.
+        gu = torch.empty(pairs, i if tensor_cores else 2 * i, dtype=torch.float16, device=dev)
         grouped(layer.w13_codes, self.w13_bits <= 4, layer.w13_norms, layer.w13_ct_scaled, x2, nv.PE_X_RAW, tok_sorted, h, hp, gu,
                 layer.w13_tiles if tiled else None)
         d = torch.empty(pairs, h, dtype=torch.float32, device=dev)
-        # decode size: the activation is computed where the down projection's input is prepared
-        act, kind = (silu_mul(gu, i), nv.PE_X_RAW) if tensor_cores else (gu, nv.PE_X_SILU_MUL)
-        grouped(layer.w2_codes, self.w2_bits <= 4, layer.w2_norms, layer.w2_ct_scaled, act, kind, None, i, ip, d,
-                layer.w2_tiles if tiled else None)
+        grouped(layer.w2_codes, self.w2_bits <= 4, layer.w2_norms, layer.w2_ct_scaled, gu, nv.PE_X_RAW if tensor_cores else nv.PE_X_SILU_MUL,
+                None, i, ip, d, layer.w2_tiles if tiled else None)
         out = torch.empty(t, h, dtype=torch.float16, device=dev)
         wts = topk_weights.reshape(-1).to(torch.float32).contiguous()
         nv.check(l.pe_moe_combine(d.data_ptr(), d.stride(0), pos.data_ptr(), wts.data_ptr(), t, k, out.data_ptr(), nv.PE_F16,
