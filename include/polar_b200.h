@@ -235,15 +235,13 @@ int pe_gemm_grouped(const void* codes, int packed, int64_t ld_codes, int64_t cod
                     int64_t ld_y, const int32_t* expert_rows, int n_experts, int rows, int out_f, int in_f_padded,
                     void* workspace, size_t workspace_bytes, void* stream);
 
-/* The same with two more facts about the launch.  x_total: the rows of x (<= rows); with x_rows given they are prepared
- * once each and gathered by the matmul, instead of once per row of the list.  silu_mul = 1: the first out_f / 2 rows of
- * an expert are the gate and the rest the up projection, and y (fp16, out_f / 2 columns) gets silu(gate) * up
- * (nemotron_offload.py:205-209). */
-int pe_gemm_grouped_routed(const void* codes, int packed, int64_t ld_codes, int64_t codes_stride, const void* norms,
-                           int64_t ld_norms, int64_t norms_stride, const float* ct_scaled, int n_levels, const void* x,
-                           int x_kind, int x_dtype, int64_t ld_x, int in_f, int x_total, const int32_t* x_rows, int silu_mul, void* y,
-                           int y_dtype, int64_t ld_y, const int32_t* expert_rows, int n_experts, int rows, int out_f, int in_f_padded,
-                           void* workspace, size_t workspace_bytes, void* stream);
+/* The same for gate and up projections: the first out_f / 2 rows of an expert are the gate and the rest the up
+ * projection, and y (fp16, out_f / 2 columns) gets silu(gate) * up (nemotron_offload.py:205-209). */
+int pe_gemm_grouped_silu_mul(const void* codes, int packed, int64_t ld_codes, int64_t codes_stride, const void* norms,
+                             int64_t ld_norms, int64_t norms_stride, const float* ct_scaled, int n_levels, const void* x,
+                             int x_kind, int x_dtype, int64_t ld_x, int in_f, const int32_t* x_rows, void* y, int64_t ld_y,
+                             const int32_t* expert_rows, int n_experts, int rows, int out_f, int in_f_padded,
+                             void* workspace, size_t workspace_bytes, void* stream);
 
 /* Routing of a mixture layer as one launch (nemotron_offload.py:180-189): fp32 softmax of the router logits over
  * the experts, the top_k largest in descending order (ties to the lower expert id), kept weights divided by

@@ -6,13 +6,13 @@
 // The weight rows are the M = 128 side of tcgen05.mma and the activation rows its N side, so a tile costs what its
 // tokens cost, rounded up to 16 instead of to 128 or 256.  A tile is 128 * halves weight rows (halves = 1 or 2) by up
 // to 256 / halves (192 for two halves) tokens; both walk K in steps of 64.  Per CTA, one per SM, persistent:
-//   * warp 0 copies the bf16 activations of a step (TMA tiles, or with warp 3 gather4 by token index for routed tokens);
+//   * warp 0 copies the bf16 activations of a step;
 //   * warp 2 copies raw codes, 128 weight rows x 128 K at a time;
 //   * warps 8..23 decode.  Four groups of four warps; group g owns weight stage g.  A thread owns one weight row: it
 //     reads the row's 64 codes, turns them into 32 bf16 pairs (byte permutes for up to eight levels, one table look-up
 //     per code byte otherwise) times the block norm, and stores them with one tcgen05.st: operand A of the MMA is read
 //     from tensor memory, so decoded weights take no shared-memory bandwidth at all, written or read;
-//   * warp 1 issues the MMAs, accumulating in TMEM columns 0..383, weight stages in columns 384..511;
+//   * warps 1 and 3 issue the MMAs, accumulating in TMEM columns 0..383, weight stages in columns 384..511;
 //   * warps 4..7 read finished accumulators back and store them, while the next tile is decoded.  A lane is a weight row,
 //     so the stores of a token are consecutive.  Tiles whose accumulators fit 192 columns alternate between two sets.
 //
@@ -90,13 +90,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
-// four rows of a matrix by index (box of one row), 64 elements from column c0 on
-__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* map, int c0, int4 rows, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(rows.x), "r"(rows.y), "r"(rows.z), "r"(rows.w)
-      : "memory");
-}
 // table entry of code byte BYTE: its address is byte * 256 + lane * 4 (+ the table's), formed by one permute
 template <int BYTE>
 __device__ __forceinline__ uint32_t tab_ld(uint32_t word, uint32_t lane4) {
@@ -134,7 +127,7 @@ template <bool PACKED, bool REGTAB>
 __global__ void __launch_bounds__(kTmThreads, 1)
 gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap cmap) {
   extern __shared__ uint8_t smem_raw[];
-  constexpr int kCodeStage = PACKED ? 8192 : 16384, NC = kTmCBytes / kCodeStage;
+  constexpr int kCodeStage = PACKED ? 8192 : 16384, NC = kTmCBytes / kCodeStage / 2;  // two rings of NC code stages
   const uint32_t raw = smem_u32(smem_raw);
   if (raw > kTmBarAddr || raw < 1024) {  // the fixed addresses would leave the window
     if (threadIdx.x == 0) atomicCAS(p.status, 0, 12);
@@ -152,13 +145,14 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
   auto acc_empty = [&](int s) { return bars + 336 + 8 * s; };  // 2
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + (bars + 352 - raw));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_raw + (bars + 356 - raw));
-  const uint32_t sink = bars + 360;
+  const uint32_t sink = bars + 360, both_here = bars + 368;
 
   if (tid == 0) {
-    for (int s = 0; s < p.nx; ++s) { mbar_init(full_x(s), 1); mbar_init(empty_x(s), 1); }
-    for (int s = 0; s < NC; ++s) { mbar_init(full_c(s), 1); mbar_init(empty_c(s), 8); }  // two groups read a code stage
+    for (int s = 0; s < p.nx; ++s) { mbar_init(full_x(s), 1); mbar_init(empty_x(s), 2); }
+    for (int s = 0; s < 2 * NC; ++s) { mbar_init(full_c(s), 1); mbar_init(empty_c(s), 8); }  // two groups read a code stage
     for (int s = 0; s < 4; ++s) { mbar_init(full_w(s), 4); mbar_init(empty_w(s), 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(acc_full(s), 1); mbar_init(acc_empty(s), 4); }
+    for (int s = 0; s < 2; ++s) { mbar_init(acc_full(s), 2); mbar_init(acc_empty(s), 4); }
+    mbar_init(both_here, 2);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -186,44 +180,21 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
 
   const int n_units = p.gtiles ? *p.n_gtiles : p.tiles_m * p.tiles_n * p.ksplit;
 
-  if (warp == 0 || (warp == 3 && p.x_rows)) {
-    // ---------------- activations: warp 0, with half of the gathers left to warp 3 ----------------
-    const int part = warp == 3 ? 1 : 0;
-    const uint32_t list = kTmTabAddr + 128 + part * 2048;  // row indices of the tile, in the gaps between table entries
+  if (warp == 0) {
+    // ---------------- activations ----------------
     const bool one = elect_one();
     int sx = 0, ph = 0;
     bool ok = true;
     for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
       const TmUnit u = tm_unit(p, unit);
-      const int copies = p.x_rows ? u.tn >> 2 : (u.tn + p.xbox - 1) / p.xbox;
-      if (p.x_rows) {  // rows of the padding repeat the last one
-        __syncwarp();
-        for (int i = part + 2 * lane; i < copies; i += 64) {
-          const int last = u.rows - 1, *src = p.x_rows + u.m0;
-          asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(list + (uint32_t)((i >> 4) * 256 + ((i >> 1) & 7) * 16)),
-                       "r"(__ldg(src + min(4 * i, last))), "r"(__ldg(src + min(4 * i + 1, last))), "r"(__ldg(src + min(4 * i + 2, last))),
-                       "r"(__ldg(src + min(4 * i + 3, last))) : "memory");
-        }
-        __syncwarp();
-      }
+      const int copies = (u.tn + p.xbox - 1) / p.xbox;
       for (int ks = 2 * u.kb0; ks < 2 * u.kb1; ++ks) {
-        ok = mbar_wait(empty_x(sx), ph ^ 1, abort_flag, p.status, 1);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = __all_sync(0xffffffffu, mbar_wait(empty_x(sx), ph ^ 1, abort_flag, p.status, 1));
         if (!ok) break;
         const uint32_t dst = kTmXAddr + sx * p.x_stage;
         if (one) {
-          if (part == 0) mbar_expect_tx(full_x(sx), (p.x_rows ? u.tn : copies * p.xbox) * 128);
-          if (p.x_rows) {
-#pragma unroll 4
-            for (int i = part; i < copies; i += 2) {
-              int4 r;
-              asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-                           : "r"(list + (uint32_t)((i >> 4) * 256 + ((i >> 1) & 7) * 16)) : "memory");
-              tma_gather4(dst + i * 512, &xmap, ks * kStepK, r, full_x(sx));
-            }
-          } else {
-            for (int i = 0; i < copies; ++i) tma_load_2d(dst + i * p.xbox * 128, &xmap, ks * kStepK, u.m0 + i * p.xbox, full_x(sx));
-          }
+          mbar_expect_tx(full_x(sx), copies * p.xbox * 128);
+          for (int i = 0; i < copies; ++i) tma_load_2d(dst + i * p.xbox * 128, &xmap, ks * kStepK, u.m0 + i * p.xbox, full_x(sx));
         }
         __syncwarp();
         if (++sx == p.nx) { sx = 0; ph ^= 1; }
@@ -231,71 +202,107 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
     }
   } else if (warp == 2) {
     // ---------------- codes ----------------
+    // Two rings: the blocks of the first half and those of the second (of a tile of one half: every other block), each
+    // read by the two decode groups of its own.  (A wait on a barrier's parity is sound only when the waiter knows that
+    // the phase before has passed, that is when it took every earlier stage of the ring itself.)
     const bool one = elect_one();
-    int ci = 0;
+    int n[2] = {0, 0};
     bool ok = true;
     for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
       const TmUnit u = tm_unit(p, unit);
-      for (int kb = u.kb0; kb < u.kb1 && ok; ++kb)
-        for (int h = 0; h < u.halves; ++h, ++ci) {
-          const int sc = ci % NC;
-          ok = __all_sync(0xffffffffu, mbar_wait(empty_c(sc), ((ci / NC) & 1) ^ 1, abort_flag, p.status, 6));
-          if (!ok) break;
-          if (one) {
-            mbar_expect_tx(full_c(sc), kCodeStage);
-            tma_load_2d(kTmCAddr + sc * kCodeStage, &cmap, kb * (PACKED ? 64 : 128), u.crow + h * (p.up_row ? p.up_row : 128), full_c(sc));
-          }
-          __syncwarp();
+      for (int i = 0; i < (u.kb1 - u.kb0) * u.halves && ok; ++i) {
+        const int c = i & 1, kb = u.kb0 + (u.halves == 2 ? i >> 1 : i), row = u.crow + (u.halves == 2 && c ? (p.up_row ? p.up_row : 128) : 0);
+        const int at = c ? n[1]++ : n[0]++, sc = c * NC + at % NC;
+        ok = __all_sync(0xffffffffu, mbar_wait(empty_c(sc), ((at / NC) & 1) ^ 1, abort_flag, p.status, 6));
+        if (!ok) break;
+        if (one) {
+          mbar_expect_tx(full_c(sc), kCodeStage);
+          tma_load_2d(kTmCAddr + sc * kCodeStage, &cmap, kb * (PACKED ? 64 : 128), row, full_c(sc));
         }
+        __syncwarp();
+      }
     }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer: the warp stays together and one elected lane issues ----------------
-    // (A lane of its own in a divergent branch took 160 cycles per instruction: it, not the tensor core, was the bound.)
+  } else if (warp == 1 || warp == 3) {
+    // ---------------- MMA issuers: warp 1 for the first half of a tile, warp 3 for the second ----------------
+    // A warp's trip through a step -- two barriers, four MMAs, two commits -- is a serial chain of about 300 cycles, more
+    // than the step's decode or MMAs take; one warp for both halves was what bounded the kernel.  The warp stays together
+    // and one elected lane issues (a lane of its own in a divergent branch took 160 cycles per instruction), and the next
+    // barriers are asked about before the MMAs of a step, so that the answer is there after them.  Tiles of one half: warp 1.
     const bool one = elect_one();
+    const int m = warp >> 1;
     int sx = 0, phx = 0;
-    uint32_t phw = 0, phe = 0;  // one phase bit per weight stage; per accumulator set
+    uint32_t phw = 0, phe = 0;  // one phase bit per pair of weight stages (s, s + 2); per accumulator set
     int next = 0;               // set of the next tile that needs one only
     bool ok = true;
+    auto wait = [&](bool ready, uint32_t bar, uint32_t parity, int code) {
+      if (__all_sync(0xffffffffu, ready)) return true;
+      return (bool)__all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, p.status, code));
+    };
+    int phm = 0;
+    auto meet = [&]() {
+      if (one) mbar_arrive(both_here);
+      const bool r = wait(false, both_here, phm, 13);
+      phm ^= 1;
+      return r;
+    };
     for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
       const TmUnit u = tm_unit(p, unit);
       const bool both = u.halves * u.tn > kTmAcc;
       const int set = both ? 0 : next;
       if (!both) next ^= 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(acc_empty(set), ((phe >> set) & 1) ^ 1, abort_flag, p.status, 9));
+      ok = wait(false, acc_empty(set), ((phe >> set) & 1) ^ 1, 9);
       phe ^= 1u << set;
       if (ok && both) {
-        ok = __all_sync(0xffffffffu, mbar_wait(acc_empty(1), ((phe >> 1) & 1) ^ 1, abort_flag, p.status, 9));
+        ok = wait(false, acc_empty(1), ((phe >> 1) & 1) ^ 1, 9);
         phe ^= 2u;
       }
       if (!ok) break;
+      const int steps = 2 * (u.kb1 - u.kb0);
+      if (u.halves == 1 && !meet()) { ok = false; break; }  // both warps have taken every stage up to here
+      if (u.halves == 1 && m == 1) {  // not this warp's: only its place in the rings moves on
+        for (int i = 0; i < steps; ++i)
+          if (++sx == p.nx) { sx = 0; phx ^= 1; }
+        for (int kb = u.kb0; kb < u.kb1; ++kb) phw ^= 1u << ((kb - u.kb0) & 1);
+        ok = meet();
+        continue;
+      }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t d0 = tmem + set * kTmAcc;
+      const uint32_t d = tmem + set * kTmAcc + m * u.tn;
       // D fp32, A and B bf16, both K-major, M = 128, N = tn
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(u.tn >> 3) << 17) | ((128u >> 4) << 24);
-      const int steps = 2 * (u.kb1 - u.kb0);
-      for (int ks = 0; ks < steps && ok; ++ks) {
-        ok = __all_sync(0xffffffffu, mbar_wait(full_x(sx), phx, abort_flag, p.status, 2));
+      const bool two = u.halves == 2;
+      int s = m;  // weight stage: m, m + 2, m, ... of two halves; 0, 2, 1, 3, 0, ... of one
+      bool rx = false, rw = false;
+      for (int ks = 0; ks < steps; ++ks) {
+        ok = wait(rx, full_x(sx), phx, 2) && wait(rw, full_w(s), (phw >> (s & 1)) & 1, 3);
         if (!ok) break;
-        const uint64_t db = smem_desc_sw128(kTmXAddr + sx * p.x_stage);
-        for (int h = 0; h < u.halves; ++h) {
-          const int s = u.halves == 2 ? 2 * (ks & 1) + h : ks & 3;
-          ok = __all_sync(0xffffffffu, mbar_wait(full_w(s), (phw >> s) & 1, abort_flag, p.status, 3));
-          if (!ok) break;
-          phw ^= 1u << s;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (one) {
-#pragma unroll
-            for (int kk = 0; kk < kStepK / 16; ++kk)
-              mma_tmem_a(d0 + h * u.tn, tmem + kTmW + s * 32 + kk * 8, db + 2 * kk, idesc, ks > 0 || kk > 0);
-            umma_commit(empty_w(s));
-            if (h == u.halves - 1) umma_commit(empty_x(sx));
-          }
-          __syncwarp();
-        }
+        const int sx_now = sx, s_now = s;
         if (++sx == p.nx) { sx = 0; phx ^= 1; }
+        s ^= 2;
+        if (ks & 1) {  // one more round of the stages: all four, or of a tile of one half the pair just used
+          phw ^= two ? 3u : 1u << (s & 1);
+          if (!two) s ^= 1;
+        }
+        rx = mbar_try(full_x(sx), phx);
+        rw = mbar_try(full_w(s), (phw >> (s & 1)) & 1);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (one) {
+          const uint64_t db = smem_desc_sw128(kTmXAddr + sx_now * p.x_stage);
+          const uint32_t a = tmem + kTmW + s_now * 32;
+#pragma unroll
+          for (int kk = 0; kk < kStepK / 16; ++kk) mma_tmem_a(d, a + kk * 8, db + 2 * kk, idesc, ks > 0 || kk > 0);
+          umma_commit(empty_w(s_now));
+          umma_commit(empty_x(sx_now));
+          if (!two) umma_commit(empty_x(sx_now));  // the barrier counts both halves
+        }
+        __syncwarp();
       }
-      if (ok && one) umma_commit(acc_full(set));
+      if (ok && one) {
+        umma_commit(acc_full(set));
+        if (!two) umma_commit(acc_full(set));
+      }
       __syncwarp();
+      if (ok && !two) ok = meet();
     }
   } else if (warp >= 8) {
     // ---------------- decode ----------------
@@ -304,19 +311,19 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
     const uint32_t wdst = tmem + kTmW + g * 32 + ((uint32_t)(q * 32) << 16);
     const int xr = PACKED ? (r >> 1) & 3 : r & 7;  // 16-byte piece j of a row sits at j ^ xr (64- or 128-byte swizzle)
     // the group's sequence of (unit, block of K): every block of its half of two, every other block of one
-    int unit = blockIdx.x, kb = 0, base = 0;
+    const int cls = g & 1, kh = g >> 1;
+    int unit = blockIdx.x, kb = 0, ci = 0;
     TmUnit u = {};
     bool live = unit < n_units;
-    auto first = [&]() { return u.kb0 + (u.halves == 2 ? 0 : g >> 1); };
+    auto first = [&]() { return u.kb0 + (u.halves == 2 ? 0 : cls); };
     auto settle = [&]() {  // to the next unit that has a block for this group
       while (live && kb >= u.kb1) {
-        base += (u.kb1 - u.kb0) * u.halves;
         unit += gridDim.x;
         live = unit < n_units;
         if (live) { u = tm_unit(p, unit); kb = first(); }
       }
     };
-    auto half = [&]() { return u.halves == 2 ? g & 1 : 0; };
+    auto half = [&]() { return u.halves == 2 ? cls : 0; };
     auto norm = [&]() {
       const int row = u.n0 + half() * (p.up_row ? p.up_row : 128) + r, limit = p.up_row ? 2 * p.up_row : p.N;
       return row < limit ? __ldg(reinterpret_cast<const unsigned short*>(p.norms) + u.expert * p.expert_norms + (int64_t)row * p.ld_norms + kb)
@@ -326,15 +333,14 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
     unsigned short nf = live ? norm() : 0;
     int phw = 1;
     while (live) {
-      const int ci = base + (u.halves == 2 ? 2 * (kb - u.kb0) + (g & 1) : kb - u.kb0);
-      const int kh = u.halves == 2 ? g >> 1 : g & 1;
       const uint32_t n2 = pack_bf16(__half2float(__ushort_as_half(nf)), __half2float(__ushort_as_half(nf)));
       kb += u.halves == 2 ? 1 : 2;
       settle();
       nf = live ? norm() : 0;  // on its way during the waits and the decode of this block
-      const int sc = ci % NC;
+      const int sc = cls * NC + ci % NC, phc = (ci / NC) & 1;
+      ++ci;
       {
-        const bool ok = mbar_wait(full_c(sc), (ci / NC) & 1, abort_flag, p.status, 7);
+        const bool ok = mbar_wait(full_c(sc), phc, abort_flag, p.status, 7);
         if (!__all_sync(0xffffffffu, ok)) break;  // leave together or not at all
       }
       constexpr int CW = PACKED ? 2 : 4;
@@ -384,7 +390,7 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t t0 = tmem + set * kTmAcc + ((uint32_t)(q * 32) << 16);
       const int row0 = u.n0 + q * 32 + lane;
-      if (p.up_row) {  // first half: gate, second half: up
+      if (p.up_row) {  // first half: gate, second half: up (the fast exponential and division: errors far below fp16's)
         const bool on = row0 < p.N;
         __half* dst = static_cast<__half*>(p.y) + (int64_t)u.m0 * p.ld_y + row0;
         for (int c = 0; c < u.tn; c += 16) {
@@ -395,7 +401,7 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
 #pragma unroll
           for (int j = 0; j < 16; ++j, dst += p.ld_y) {
             const float f = __uint_as_float(a[j]);
-            if (on && c + j < u.rows) *dst = __float2half_rn(f / (1.f + expf(-f)) * __uint_as_float(b[j]));
+            if (on && c + j < u.rows) *dst = __float2half_rn(__fdividef(f, 1.f + __expf(-f)) * __uint_as_float(b[j]));
           }
         }
       } else {
@@ -455,7 +461,7 @@ int launch_gemm_tmem(TmemGemmArgs& a, const void* codes, int packed, int64_t ld_
   a.nx = kTmXBytes / a.x_stage < kTmMaxX ? kTmXBytes / a.x_stage : kTmMaxX;
   CUtensorMap xmap, cmap;
   const int K = a.nb * kBlock;
-  int rc = encode_map_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, xq, K, x_total, (uint64_t)K * 2, kStepK, a.x_rows ? 1 : a.xbox,
+  int rc = encode_map_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, xq, K, x_total, (uint64_t)K * 2, kStepK, a.xbox,
                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
   if (rc == PE_OK)
     rc = encode_map_2d(&cmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, codes, packed ? K / 2 : K, code_rows, ld_codes, packed ? 64 : 128, 128,
@@ -516,10 +522,9 @@ extern "C" size_t pe_gemm_grouped_workspace_bytes(int n_experts, int rows, int o
   return 512 + list + (size_t)rows * in_f_padded * 2;
 }
 
-// x_total > 0: x has that many rows, prepared once each and gathered by the matmul; 0: unknown, gathered by the preparation
 static int grouped(const void* codes, int packed, int64_t ld_codes, int64_t codes_stride, const void* norms, int64_t ld_norms, int64_t norms_stride,
                    const float* ct_scaled, int n_levels, const void* x, int x_kind, int x_dtype, int64_t ld_x, int in_f, const int32_t* x_rows,
-                   int x_total, int silu_mul, void* y, int y_dtype, int64_t ld_y, const int32_t* expert_rows, int n_experts, int rows, int out_f,
+                   int silu_mul, void* y, int y_dtype, int64_t ld_y, const int32_t* expert_rows, int n_experts, int rows, int out_f,
                    int in_f_padded, void* workspace, size_t workspace_bytes, void* stream) {
   if (!codes || !norms || !ct_scaled || !x || !y || !expert_rows || !workspace) return PE_ERR_ARG;
   if (n_experts < 1 || rows < 1 || out_f < 1 || in_f < 1 || in_f > in_f_padded) return PE_ERR_ARG;
@@ -536,7 +541,6 @@ static int grouped(const void* codes, int packed, int64_t ld_codes, int64_t code
   const int y_cols = silu_mul ? out_f / 2 : out_f;
   if (ld_codes < (packed ? in_f_padded / 2 : in_f_padded) || ld_norms < in_f_padded / kBlock) return PE_ERR_ARG;
   if (ld_x < (x_kind == PE_X_RAW ? in_f : in_f_padded) || ld_y < y_cols) return PE_ERR_ARG;
-  if (x_total < 0 || x_total > rows) return PE_ERR_ARG;
   if ((int64_t)n_experts * out_f > 0x7fffffff) return PE_ERR_LIMIT;
   const size_t need = pe_gemm_grouped_workspace_bytes(n_experts, rows, out_f, in_f_padded);
   if (need == 0) return PE_ERR_SHAPE;
@@ -554,9 +558,9 @@ static int grouped(const void* codes, int packed, int64_t ld_codes, int64_t code
   void* xq = ws + 512 + list_bytes;
   const int tile_rows = silu_mul ? 128 : 256, tiles_n = (y_cols + tile_rows - 1) / tile_rows;
   PE_CUDA_TRY(launch_pdl(gemm_tile_list_kernel, dim3(1), dim3(1024), 0, st, expert_rows, n_experts, tiles_n, tile_rows, max_tiles, tiles, n_tiles));
-  const bool gather = x_rows && x_total > 0;  // (the preparation kernel clears the status word)
-  int rc = launch_gemm_prep(x, x_kind, x_dtype, ld_x, in_f, xq, gather ? x_total : rows, in_f_padded, packed ? 1 : 0, gather ? nullptr : x_rows,
-                            gather ? nullptr : expert_rows + 2 * (n_experts - 1), status, st);
+  // (the preparation kernel clears the status word)
+  const int rc = launch_gemm_prep(x, x_kind, x_dtype, ld_x, in_f, xq, rows, in_f_padded, packed ? 1 : 0, x_rows, expert_rows + 2 * (n_experts - 1),
+                                  status, st);
   if (rc != PE_OK) return rc;
 
   TmemGemmArgs a = {};
@@ -566,11 +570,10 @@ static int grouped(const void* codes, int packed, int64_t ld_codes, int64_t code
   a.M = rows; a.N = y_cols; a.nb = in_f_padded / kBlock;
   a.ksplit = 1;
   a.xbox = 32; a.x_stage = kTmAcc * 128;
-  a.x_rows = gather ? x_rows : nullptr;
   a.gtiles = tiles; a.n_gtiles = n_tiles; a.expert_codes = out_f;
   a.up_row = silu_mul ? y_cols : 0;
   a.status = status;
-  return launch_gemm_tmem(a, codes, packed, ld_codes, (int64_t)n_experts * out_f, xq, gather ? x_total : rows, max_tiles, sms, st);
+  return launch_gemm_tmem(a, codes, packed, ld_codes, (int64_t)n_experts * out_f, xq, rows, max_tiles, sms, st);
 }
 
 extern "C" int pe_gemm_grouped(const void* codes, int packed, int64_t ld_codes, int64_t codes_stride, const void* norms,
@@ -578,16 +581,15 @@ extern "C" int pe_gemm_grouped(const void* codes, int packed, int64_t ld_codes, 
                                int x_kind, int x_dtype, int64_t ld_x, int in_f, const int32_t* x_rows, void* y, int y_dtype,
                                int64_t ld_y, const int32_t* expert_rows, int n_experts, int rows, int out_f, int in_f_padded,
                                void* workspace, size_t workspace_bytes, void* stream) {
-  return grouped(codes, packed, ld_codes, codes_stride, norms, ld_norms, norms_stride, ct_scaled, n_levels, x, x_kind, x_dtype, ld_x, in_f, x_rows, 0,
-                 0, y, y_dtype, ld_y, expert_rows, n_experts, rows, out_f, in_f_padded, workspace, workspace_bytes, stream);
+  return grouped(codes, packed, ld_codes, codes_stride, norms, ld_norms, norms_stride, ct_scaled, n_levels, x, x_kind, x_dtype, ld_x, in_f, x_rows, 0, y,
+                 y_dtype, ld_y, expert_rows, n_experts, rows, out_f, in_f_padded, workspace, workspace_bytes, stream);
 }
 
-extern "C" int pe_gemm_grouped_routed(const void* codes, int packed, int64_t ld_codes, int64_t codes_stride, const void* norms,
-                                      int64_t ld_norms, int64_t norms_stride, const float* ct_scaled, int n_levels, const void* x,
-                                      int x_kind, int x_dtype, int64_t ld_x, int in_f, int x_total, const int32_t* x_rows, int silu_mul, void* y,
-                                      int y_dtype, int64_t ld_y, const int32_t* expert_rows, int n_experts, int rows, int out_f, int in_f_padded,
-                                      void* workspace, size_t workspace_bytes, void* stream) {
-  if (x_rows && x_total < 1) return PE_ERR_ARG;
-  return grouped(codes, packed, ld_codes, codes_stride, norms, ld_norms, norms_stride, ct_scaled, n_levels, x, x_kind, x_dtype, ld_x, in_f, x_rows,
-                 x_rows ? x_total : 0, silu_mul, y, y_dtype, ld_y, expert_rows, n_experts, rows, out_f, in_f_padded, workspace, workspace_bytes, stream);
+extern "C" int pe_gemm_grouped_silu_mul(const void* codes, int packed, int64_t ld_codes, int64_t codes_stride, const void* norms,
+                                        int64_t ld_norms, int64_t norms_stride, const float* ct_scaled, int n_levels, const void* x,
+                                        int x_kind, int x_dtype, int64_t ld_x, int in_f, const int32_t* x_rows, void* y,
+                                        int64_t ld_y, const int32_t* expert_rows, int n_experts, int rows, int out_f, int in_f_padded,
+                                        void* workspace, size_t workspace_bytes, void* stream) {
+  return grouped(codes, packed, ld_codes, codes_stride, norms, ld_norms, norms_stride, ct_scaled, n_levels, x, x_kind, x_dtype, ld_x, in_f, x_rows, 1, y,
+                 PE_F16, ld_y, expert_rows, n_experts, rows, out_f, in_f_padded, workspace, workspace_bytes, stream);
 }

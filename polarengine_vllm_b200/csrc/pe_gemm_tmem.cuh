@@ -16,7 +16,6 @@ struct TmemGemmArgs {
   float* part;           // [ksplit][M][N] fp32 when ksplit > 1
   int xbox;              // activation rows per TMA copy
   int x_stage, nx;       // bytes and number of the activation stages
-  const int* x_rows;     // grouped launch: rows of the prepared matrix to gather (nullptr: consecutive rows)
   const int4* gtiles;    // grouped launch: per tile (first activation row, rows, first weight row inside the expert, expert)
   const int* n_gtiles;
   int64_t expert_norms;  // halves between the norms of consecutive experts

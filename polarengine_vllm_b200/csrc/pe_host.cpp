@@ -35,7 +35,8 @@ struct Api {
   decltype(&pe_gemv_grouped) grouped;
   decltype(&pe_gemv_grouped_tiled) grouped_tiled;
   decltype(&pe_gemv_grouped_workspace_bytes) grouped_bytes;
-  decltype(&pe_gemm_grouped_routed) gemm_grouped;
+  decltype(&pe_gemm_grouped) gemm_grouped;
+  decltype(&pe_gemm_grouped_silu_mul) gemm_silu_mul;
   decltype(&pe_gemm_grouped_workspace_bytes) gemm_grouped_bytes;
 };
 Api api;
@@ -251,14 +252,18 @@ bool plain_experts(const Experts& w, const at::Device& dev, int64_t rows) {
 }
 
 int grouped(const Experts& w, const MoePlan& p, const at::Device& dev, cudaStream_t st, const void* x, int kind, int xd, int64_t ld_x, int in_f,
-            int in_f_padded, int x_total, const int32_t* x_rows, bool silu_mul, void* y, int yd, int out_f) {
+            int in_f_padded, const int32_t* x_rows, bool silu_mul, void* y, int yd, int out_f) {
   const float* ct = w.ct->const_data_ptr<float>();
   const int levels = (int)w.ct->numel();
   if (p.tensor_cores) {
     const at::Tensor ws = take_scratch(dev, st, 1, api.gemm_grouped_bytes((int)p.n_local, (int)p.pairs, out_f, in_f_padded), false);
+    if (silu_mul)
+      return api.gemm_silu_mul(w.codes->const_data_ptr(), w.packed, w.codes->stride(1), w.codes->stride(0), w.norms->const_data_ptr(),
+                               w.norms->stride(1), w.norms->stride(0), ct, levels, x, kind, xd, ld_x, in_f, x_rows, y, out_f / 2, p.expert_rows,
+                               (int)p.n_local, (int)p.pairs, out_f, in_f_padded, ws.mutable_data_ptr(), ws.numel(), st);
     return api.gemm_grouped(w.codes->const_data_ptr(), w.packed, w.codes->stride(1), w.codes->stride(0), w.norms->const_data_ptr(),
-                            w.norms->stride(1), w.norms->stride(0), ct, levels, x, kind, xd, ld_x, in_f, x_total, x_rows, silu_mul, y, yd,
-                            silu_mul ? out_f / 2 : out_f, p.expert_rows, (int)p.n_local, (int)p.pairs, out_f, in_f_padded, ws.mutable_data_ptr(), ws.numel(), st);
+                            w.norms->stride(1), w.norms->stride(0), ct, levels, x, kind, xd, ld_x, in_f, x_rows, y, yd, out_f, p.expert_rows,
+                            (int)p.n_local, (int)p.pairs, out_f, in_f_padded, ws.mutable_data_ptr(), ws.numel(), st);
   }
   const at::Tensor ws = take_scratch(dev, st, 2, api.grouped_bytes((int)p.max_problems, out_f, in_f_padded), true);
   if (w.tiles)
@@ -351,10 +356,10 @@ PyObject* host_moe(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const at::Tensor gu = at::empty({p.pairs, mid}, half);
   const at::Tensor d = at::empty({p.pairs, h}, half.dtype(at::kFloat));
   if (rc == PE_OK)
-    rc = grouped(w[0], p, dev, st, x->const_data_ptr(), PE_X_RAW, xd, h, h, hp, (int)tokens, tok, p.tensor_cores, gu.mutable_data_ptr(), PE_F16,
+    rc = grouped(w[0], p, dev, st, x->const_data_ptr(), PE_X_RAW, xd, h, h, hp, tok, p.tensor_cores, gu.mutable_data_ptr(), PE_F16,
                  2 * inter);
   if (rc == PE_OK)
-    rc = grouped(w[1], p, dev, st, gu.const_data_ptr(), p.tensor_cores ? PE_X_RAW : PE_X_SILU_MUL, PE_F16, mid, inter, ip, 0, nullptr, false,
+    rc = grouped(w[1], p, dev, st, gu.const_data_ptr(), p.tensor_cores ? PE_X_RAW : PE_X_SILU_MUL, PE_F16, mid, inter, ip, nullptr, false,
                  d.mutable_data_ptr(), PE_F32, h);
   at::Tensor out = at::empty(x->sizes(), half);
   if (rc == PE_OK)
@@ -385,7 +390,8 @@ PyObject* host_setup(PyObject*, PyObject* arg) {
   PE_SYMBOL(grouped, pe_gemv_grouped)
   PE_SYMBOL(grouped_tiled, pe_gemv_grouped_tiled)
   PE_SYMBOL(grouped_bytes, pe_gemv_grouped_workspace_bytes)
-  PE_SYMBOL(gemm_grouped, pe_gemm_grouped_routed)
+  PE_SYMBOL(gemm_grouped, pe_gemm_grouped)
+  PE_SYMBOL(gemm_silu_mul, pe_gemm_grouped_silu_mul)
   PE_SYMBOL(gemm_grouped_bytes, pe_gemm_grouped_workspace_bytes)
   ready = true;
   Py_RETURN_NONE;
