@@ -16,10 +16,10 @@
 //   * warps 4..7 read finished accumulators back and store them, while the next tile is decoded.  A lane is a weight row,
 //     so the stores of a token are consecutive.  Tiles whose accumulators fit 192 columns alternate between two sets.
 //
-// What bounds it: with about 128 tokens per tile the decode (13 instructions per 8 weights) and the MMAs take about
-// the same time.  The form before had the weights in shared memory as the N = 256 side, padded tokens to 128 and
-// drained accumulators with the decode warps: 2048 tokens x 8 experts of 128, 2688 -> 2 x 1856 took 492 us, 429 us now, the
-// rest of the time being the step loop itself.
+// What bounds it: with up to about 100 tokens per tile the decode (13 instructions per 8 weights, near 60% of the issue
+// slots), above that the MMAs and the issue of one after the other.  The form before had the weights in shared memory as
+// the N = 256 side, padded tokens to 128 and drained accumulators with the decode warps: 16384 rows over 128 experts of
+// 2688 -> 2 x 1856 took 492 us, 298 us now (343 us with the activation function, which was a pass of 36 us of its own).
 //
 // Every wait is bounded: on time-out a status code is recorded, all roles leave their loops, TMEM is released.
 #include "pe_gemm_tmem.cuh"
@@ -27,14 +27,13 @@
 namespace pe {
 
 constexpr int kTmThreads = 768;
-constexpr int kTmBarAddr = 1536;                   // shared-window addresses: barriers,
-constexpr int kTmTabAddr = 2048;                   // the centroid table (256 B per entry: a byte permute forms the address),
-constexpr int kTmXAddr = kTmTabAddr + 65536;       // activation stages,
-constexpr int kTmXBytes = 98304;
-constexpr int kTmCAddr = kTmXAddr + kTmXBytes;     // code stages
+constexpr int kTmBarAddr = 1536;                // shared-window addresses: barriers,
+constexpr int kTmTabAddr = 2048;                // the centroid table if there is one (256 B per entry: a byte permute forms the address),
+constexpr int kTmTabBytes = 65536;              // activation stages behind it (their depth covers L2's latency: the longer ring without a
+constexpr int kTmCAddr = 165888;                // table is worth a tenth), and code stages
 constexpr int kTmCBytes = 65536;
 constexpr int kTmEnd = kTmCAddr + kTmCBytes;
-constexpr int kTmSmem = kTmEnd - 1024;             // the dynamic window starts at 1024 or above it would not fit
+constexpr int kTmSmem = kTmEnd - 1024;          // the dynamic window starts at 1024; above it would not fit
 constexpr int kTmMaxX = 8;                         // activation stages at most
 constexpr int kTmAcc = 192;                        // columns of one accumulator set
 constexpr int kTmW = 384;                          // first column of the weight stages, 32 columns each
@@ -127,6 +126,7 @@ template <bool PACKED, bool REGTAB>
 __global__ void __launch_bounds__(kTmThreads, 1)
 gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap cmap) {
   extern __shared__ uint8_t smem_raw[];
+  constexpr int kXAddr = kTmTabAddr + (REGTAB ? 0 : kTmTabBytes);
   constexpr int kCodeStage = PACKED ? 8192 : 16384, NC = kTmCBytes / kCodeStage / 2;  // two rings of NC code stages
   const uint32_t raw = smem_u32(smem_raw);
   if (raw > kTmBarAddr || raw < 1024) {  // the fixed addresses would leave the window
@@ -191,7 +191,7 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
       for (int ks = 2 * u.kb0; ks < 2 * u.kb1; ++ks) {
         ok = __all_sync(0xffffffffu, mbar_wait(empty_x(sx), ph ^ 1, abort_flag, p.status, 1));
         if (!ok) break;
-        const uint32_t dst = kTmXAddr + sx * p.x_stage;
+        const uint32_t dst = kXAddr + sx * p.x_stage;
         if (one) {
           mbar_expect_tx(full_x(sx), copies * p.xbox * 128);
           for (int i = 0; i < copies; ++i) tma_load_2d(dst + i * p.xbox * 128, &xmap, ks * kStepK, u.m0 + i * p.xbox, full_x(sx));
@@ -224,85 +224,84 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
     }
   } else if (warp == 1 || warp == 3) {
     // ---------------- MMA issuers: warp 1 for the first half of a tile, warp 3 for the second ----------------
-    // A warp's trip through a step -- two barriers, four MMAs, two commits -- is a serial chain of about 300 cycles, more
-    // than the step's decode or MMAs take; one warp for both halves was what bounded the kernel.  The warp stays together
-    // and one elected lane issues (a lane of its own in a divergent branch took 160 cycles per instruction), and the next
-    // barriers are asked about before the MMAs of a step, so that the answer is there after them.  Tiles of one half: warp 1.
-    const bool one = elect_one();
-    const int m = warp >> 1;
-    int sx = 0, phx = 0;
-    uint32_t phw = 0, phe = 0;  // one phase bit per pair of weight stages (s, s + 2); per accumulator set
-    int next = 0;               // set of the next tile that needs one only
-    bool ok = true;
-    auto wait = [&](bool ready, uint32_t bar, uint32_t parity, int code) {
-      if (__all_sync(0xffffffffu, ready)) return true;
-      return (bool)__all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, p.status, code));
-    };
-    int phm = 0;
-    auto meet = [&]() {
-      if (one) mbar_arrive(both_here);
-      const bool r = wait(false, both_here, phm, 13);
-      phm ^= 1;
-      return r;
-    };
-    for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
-      const TmUnit u = tm_unit(p, unit);
-      const bool both = u.halves * u.tn > kTmAcc;
-      const int set = both ? 0 : next;
-      if (!both) next ^= 1;
-      ok = wait(false, acc_empty(set), ((phe >> set) & 1) ^ 1, 9);
-      phe ^= 1u << set;
-      if (ok && both) {
-        ok = wait(false, acc_empty(1), ((phe >> 1) & 1) ^ 1, 9);
-        phe ^= 2u;
-      }
-      if (!ok) break;
-      const int steps = 2 * (u.kb1 - u.kb0);
-      if (u.halves == 1 && !meet()) { ok = false; break; }  // both warps have taken every stage up to here
-      if (u.halves == 1 && m == 1) {  // not this warp's: only its place in the rings moves on
-        for (int i = 0; i < steps; ++i)
-          if (++sx == p.nx) { sx = 0; phx ^= 1; }
-        for (int kb = u.kb0; kb < u.kb1; ++kb) phw ^= 1u << ((kb - u.kb0) & 1);
-        ok = meet();
-        continue;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t d = tmem + set * kTmAcc + m * u.tn;
-      // D fp32, A and B bf16, both K-major, M = 128, N = tn
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(u.tn >> 3) << 17) | ((128u >> 4) << 24);
-      const bool two = u.halves == 2;
-      int s = m;  // weight stage: m, m + 2, m, ... of two halves; 0, 2, 1, 3, 0, ... of one
-      bool rx = false, rw = false;
-      for (int ks = 0; ks < steps; ++ks) {
-        ok = wait(rx, full_x(sx), phx, 2) && wait(rw, full_w(s), (phw >> (s & 1)) & 1, 3);
+    // A trip through a step -- two barriers, four MMAs, two commits -- is a serial chain that takes as long as the step's
+    // decode or MMAs; one warp for both halves was what bounded the kernel.  The next barriers are asked about before the
+    // MMAs of a step, so that the answer is there after them.  Tiles of one half: warp 1.
+    if (elect_one()) {
+      const int m = warp >> 1;
+      int sx = 0, phx = 0;
+      uint32_t phw = 0, phe = 0;  // one phase bit per pair of weight stages (s, s + 2); per accumulator set
+      int next = 0;               // set of the next tile that needs one only
+      bool ok = true;
+      auto wait = [&](uint32_t bar, uint32_t parity, int code) {
+        return mbar_wait(bar, parity, abort_flag, p.status, code);
+      };
+      int phm = 0;
+      auto meet = [&]() {
+        mbar_arrive(both_here);
+        const bool r = wait(both_here, phm, 13);
+        phm ^= 1;
+        return r;
+      };
+      for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
+        const TmUnit u = tm_unit(p, unit);
+        const bool both = u.halves * u.tn > kTmAcc;
+        const int set = both ? 0 : next;
+        if (!both) next ^= 1;
+        ok = wait(acc_empty(set), ((phe >> set) & 1) ^ 1, 9);
+        phe ^= 1u << set;
+        if (ok && both) {
+          ok = wait(acc_empty(1), ((phe >> 1) & 1) ^ 1, 9);
+          phe ^= 2u;
+        }
         if (!ok) break;
-        const int sx_now = sx, s_now = s;
-        if (++sx == p.nx) { sx = 0; phx ^= 1; }
-        s ^= 2;
-        if (ks & 1) {  // one more round of the stages: all four, or of a tile of one half the pair just used
-          phw ^= two ? 3u : 1u << (s & 1);
-          if (!two) s ^= 1;
+        const bool two = u.halves == 2;
+        if (!two && !meet()) { ok = false; break; }  // both warps have taken every stage up to here
+        if (!two && m == 1) {  // not this warp's: only its place in the rings moves on
+          for (int i = 0; i < 2 * (u.kb1 - u.kb0); ++i) {
+            if (++sx == p.nx) { sx = 0; phx ^= 1; }
+            if (i & 1) phw ^= 1u << ((i >> 1) & 1);
+          }
+          ok = meet();
+          continue;
         }
-        rx = mbar_try(full_x(sx), phx);
-        rw = mbar_try(full_w(s), (phw >> (s & 1)) & 1);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (one) {
-          const uint64_t db = smem_desc_sw128(kTmXAddr + sx_now * p.x_stage);
-          const uint32_t a = tmem + kTmW + s_now * 32;
+        const uint32_t d = tmem + set * kTmAcc + m * u.tn;
+        // D fp32, A and B bf16, both K-major, M = 128, N = tn
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(u.tn >> 3) << 17) | ((128u >> 4) << 24);
+        auto issue = [&](int stage, uint32_t x, uint32_t acc) {
+          const uint64_t db = smem_desc_sw128(x);
+          const uint32_t a = tmem + kTmW + stage * 32;
 #pragma unroll
-          for (int kk = 0; kk < kStepK / 16; ++kk) mma_tmem_a(d, a + kk * 8, db + 2 * kk, idesc, ks > 0 || kk > 0);
-          umma_commit(empty_w(s_now));
-          umma_commit(empty_x(sx_now));
-          if (!two) umma_commit(empty_x(sx_now));  // the barrier counts both halves
+          for (int kk = 0; kk < kStepK / 16; ++kk) mma_tmem_a(d, a + kk * 8, db + 2 * kk, idesc, kk > 0 ? 1u : acc);
+          umma_commit(empty_w(stage));
+        };
+        int c = m;  // a block's weight stages: c and c + 2; of a tile of one half the two pairs take turns
+        bool ready = false;
+        for (int n = u.kb1 - u.kb0, i = 0; i < n && ok; ++i) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            if (!ready) ok = wait(full_x(sx), phx, 2) && wait(full_w(c + 2 * j), (phw >> c) & 1, 3);
+            if (!ok) break;
+            const uint32_t x = kXAddr + sx * p.x_stage, done_x = empty_x(sx), stage = c + 2 * j;
+            if (++sx == p.nx) { sx = 0; phx ^= 1; }
+            if (j == 1) {
+              phw ^= two ? 3u : 1u << c;
+              if (!two) c ^= 1;
+            }
+            ready = mbar_test(full_x(sx), phx) & mbar_test(full_w(c + 2 * (j ^ 1)), (phw >> c) & 1);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            issue(stage, x, i > 0 || j > 0);
+            umma_commit(done_x);
+            if (!two) umma_commit(done_x);  // the barrier counts both halves
+          }
         }
-        __syncwarp();
+        if (ok) {
+          umma_commit(acc_full(set));
+          if (!two) umma_commit(acc_full(set));
+        }
+        if (ok && !two) ok = meet();
       }
-      if (ok && one) {
-        umma_commit(acc_full(set));
-        if (!two) umma_commit(acc_full(set));
-      }
-      __syncwarp();
-      if (ok && !two) ok = meet();
     }
   } else if (warp >= 8) {
     // ---------------- decode ----------------
@@ -315,31 +314,37 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
     int unit = blockIdx.x, kb = 0, ci = 0;
     TmUnit u = {};
     bool live = unit < n_units;
-    auto first = [&]() { return u.kb0 + (u.halves == 2 ? 0 : cls); };
-    auto settle = [&]() {  // to the next unit that has a block for this group
-      while (live && kb >= u.kb1) {
+    const unsigned short* np = nullptr;  // norm of (this row, block kb); nullptr: the row does not exist
+    auto enter = [&]() {                 // to the first block of this unit, or of the next that has one for this group
+      while (live) {
+        u = tm_unit(p, unit);
+        kb = u.kb0 + (u.halves == 2 ? 0 : cls);
+        if (kb < u.kb1) break;
         unit += gridDim.x;
         live = unit < n_units;
-        if (live) { u = tm_unit(p, unit); kb = first(); }
       }
+      const int row = u.n0 + (u.halves == 2 && cls ? (p.up_row ? p.up_row : 128) : 0) + r, limit = p.up_row ? 2 * p.up_row : p.N;
+      np = live && row < limit
+               ? reinterpret_cast<const unsigned short*>(p.norms) + u.expert * p.expert_norms + (int64_t)row * p.ld_norms + kb
+               : nullptr;
     };
-    auto half = [&]() { return u.halves == 2 ? cls : 0; };
-    auto norm = [&]() {
-      const int row = u.n0 + half() * (p.up_row ? p.up_row : 128) + r, limit = p.up_row ? 2 * p.up_row : p.N;
-      return row < limit ? __ldg(reinterpret_cast<const unsigned short*>(p.norms) + u.expert * p.expert_norms + (int64_t)row * p.ld_norms + kb)
-                         : (unsigned short)0;
-    };
-    if (live) { u = tm_unit(p, unit); kb = first(); settle(); }
-    unsigned short nf = live ? norm() : 0;
+    enter();
+    unsigned short nf = np ? __ldg(np) : 0;
     int phw = 1;
     while (live) {
       const uint32_t n2 = pack_bf16(__half2float(__ushort_as_half(nf)), __half2float(__ushort_as_half(nf)));
-      kb += u.halves == 2 ? 1 : 2;
-      settle();
-      nf = live ? norm() : 0;  // on its way during the waits and the decode of this block
+      const int by = u.halves == 2 ? 1 : 2;
+      kb += by;
+      if (np) np += by;
+      if (kb >= u.kb1) {
+        unit += gridDim.x;
+        live = unit < n_units;
+        enter();
+      }
+      nf = np ? __ldg(np) : 0;  // on its way during the waits and the decode of this block
       const int sc = cls * NC + ci % NC, phc = (ci / NC) & 1;
       ++ci;
-      {
+      if (!__all_sync(0xffffffffu, mbar_try(full_c(sc), phc))) {
         const bool ok = mbar_wait(full_c(sc), phc, abort_flag, p.status, 7);
         if (!__all_sync(0xffffffffu, ok)) break;  // leave together or not at all
       }
@@ -360,7 +365,7 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
       if (lane == 0) mbar_arrive(empty_c(sc));
       uint32_t o[32];
       decode64<PACKED, REGTAB>(c, n2, lane * 4, tb, o);
-      {
+      if (!__all_sync(0xffffffffu, mbar_try(empty_w(g), phw))) {
         const bool ok = mbar_wait(empty_w(g), phw, abort_flag, p.status, 4);
         if (!__all_sync(0xffffffffu, ok)) break;
       }
@@ -458,7 +463,9 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
 
 int launch_gemm_tmem(TmemGemmArgs& a, const void* codes, int packed, int64_t ld_codes, int64_t code_rows, const void* xq, int64_t x_total, int units,
                      int sms, cudaStream_t st) {
-  a.nx = kTmXBytes / a.x_stage < kTmMaxX ? kTmXBytes / a.x_stage : kTmMaxX;
+  const bool regtab = packed && a.n_levels <= 8;
+  const int x_bytes = kTmCAddr - kTmTabAddr - (regtab ? 0 : kTmTabBytes);
+  a.nx = x_bytes / a.x_stage < kTmMaxX ? x_bytes / a.x_stage : kTmMaxX;
   CUtensorMap xmap, cmap;
   const int K = a.nb * kBlock;
   int rc = encode_map_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, xq, K, x_total, (uint64_t)K * 2, kStepK, a.xbox,
@@ -467,7 +474,7 @@ int launch_gemm_tmem(TmemGemmArgs& a, const void* codes, int packed, int64_t ld_
     rc = encode_map_2d(&cmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, codes, packed ? K / 2 : K, code_rows, ld_codes, packed ? 64 : 128, 128,
                        packed ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
   if (rc != PE_OK) return rc;
-  auto kfn = !packed ? gemm_tmem_kernel<false, false> : a.n_levels <= 8 ? gemm_tmem_kernel<true, true> : gemm_tmem_kernel<true, false>;
+  auto kfn = !packed ? gemm_tmem_kernel<false, false> : regtab ? gemm_tmem_kernel<true, true> : gemm_tmem_kernel<true, false>;
   PE_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTmSmem));
   PE_CUDA_TRY(launch_pdl(kfn, dim3((unsigned)(units < sms ? units : sms)), dim3(kTmThreads), kTmSmem, st, a, xmap, cmap));
   return PE_OK;
