@@ -36,7 +36,7 @@ enum {
                        (the reference's `x_transformed`, fwht.py:102-108)        */
   PE_X_RAW = 1,     /* un-rotated activations with in_f valid columns; the kernel
                        pads and rotates while staging (linear_method.py:186-197) */
-  PE_X_SILU_MUL = 2 /* grouped entry points, fp16: rows are [gate | up] of 2 in_f columns and the
+  PE_X_SILU_MUL = 2 /* pe_gemm and the grouped decode entry points, fp16: rows are [gate | up] of 2 in_f columns and the
                        input is half(silu(gate)) * up (pe_silu_mul), then as PE_X_RAW       */
 };
 
@@ -61,7 +61,7 @@ enum {
 
 /* values a kernel leaves in a status word when a bounded device-side wait ran out */
 enum {
-  PE_STATUS_SPLITK_TIMEOUT = 1 /* pe_gemv tile kernel: a split-K partial never arrived */
+  PE_STATUS_SPLITK_TIMEOUT = 1 /* pe_gemv: a wait inside the launch ran out */
 };
 
 int pe_version(void);
@@ -110,20 +110,23 @@ int pe_embedding(const void* codes, int packed, int64_t ld_codes, const void* no
  *   scalar, for graph replay) else pos_host.  Rotate-half rotary embedding of the query and
  *   key heads (frequencies theta^(-2j/d)); queries go to q_out (batch, hq, t, head_dim),
  *   rotated keys and the values into the caches (batch, hkv, max_len, head_dim) at their
- *   positions (positions outside [0, max_len) are dropped).
+ *   positions (positions outside [0, max_len) are dropped).  pe_rope_cache_token_major: the same
+ *   with q_out (batch, t, hq, head_dim).
  * pe_silu_mul: out[r, i] = fp16(silu(gate_up[r, i])) * gate_up[r, inter + i].
  * pe_decode_attention: one new token per sequence.  q (batch, hq, head_dim), caches as
  *   above holding positions 0 .. pos (pos = *pos_dev or pos_host, the token just written);
  *   out (batch, hq * head_dim) = softmax(q K^T / sqrt(head_dim)) V per query head, query head
  *   i reading kv head i / (hq / hkv).  head_dim = 128, hq / hkv in {1, 2, 4, 8}.  With a
  *   workspace (pe_decode_attention_workspace_bytes; its first 4 KB zero before the first call,
- *   left zero) the cache positions are split over up to 16 CTAs per kv head; NULL = one CTA.
+ *   left zero) the cache positions are split over a cluster of up to 8 CTAs per kv head; NULL = one CTA.
  * pe_rope_attention: pe_rope_cache (t = 1) and pe_decode_attention as ONE launch: qkv (batch,
  *   (hq + 2 hkv) * head_dim) holds the raw fused projection of the new token; queries and the new
  *   key are rotated in registers, key and value are written into the caches at the position, and
  *   the attention uses them without reading them back.  Same output as the two calls. */
 int pe_add_rmsnorm(void* x, const void* delta, int delta_dtype, const void* weight, void* out, int rows, int hidden,
                    float eps, void* stream);
+int pe_rope_cache_token_major(const void* qkv, int64_t ld_qkv, const int64_t* pos_dev, int64_t pos_host, void* q_out, void* k_cache,
+                              void* v_cache, int batch, int t, int hq, int hkv, int head_dim, int max_len, float theta, void* stream);
 int pe_rope_cache(const void* qkv, int64_t ld_qkv, const int64_t* pos_dev, int64_t pos_host, void* q_out, void* k_cache,
                   void* v_cache, int batch, int t, int hq, int hkv, int head_dim, int max_len, float theta, void* stream);
 int pe_silu_mul(const void* gate_up, int64_t ld_gu, void* out, int64_t ld_out, int rows, int inter, void* stream);

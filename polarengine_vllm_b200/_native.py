@@ -59,6 +59,7 @@ SIGNATURES = {
     "pe_gemm": (_i, [_vp, _i, _i64, _vp, _i64, _vp, _i, _vp, _i, _i, _i64, _i, _vp, _i, _i64, _vp, _i, _i, _i,
                      _vp, _sz, _vp]),
     "pe_add_rmsnorm": (_i, [_vp, _vp, _i, _vp, _vp, _i, _i, ctypes.c_float, _vp]),
+    "pe_rope_cache_token_major": (_i, [_vp, _i64, _vp, _i64, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, ctypes.c_float, _vp]),
     "pe_rope_cache": (_i, [_vp, _i64, _vp, _i64, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, ctypes.c_float, _vp]),
     "pe_silu_mul": (_i, [_vp, _i64, _vp, _i64, _i, _i, _vp]),
     "pe_decode_attention_workspace_bytes": (_sz, [_i, _i, _i, _i]),

@@ -92,16 +92,17 @@ __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_kernel(__half* x, co
 }
 
 // One block per token: the angles' sines and cosines once, then every head's pairs (j, j + d/2) (rotate-half form), two
-// neighbouring pairs per thread and step.  (A block per head computed them anew for every head, in blocks of two warps:
-// 26 us for 512 tokens of 48 heads, 7.5 us now.)
-// Query heads go to q_out (batch, hq, t, d); key heads (rotated) and value heads (copied)
+// eight neighbouring pairs per thread and step where the rows are aligned for 16-byte accesses.  (A block per head
+// computed them anew for every head, in blocks of two warps: 26 us for 512 tokens of 48 heads, 7.5 us with one block
+// per token and two pairs per step.)
+// Query heads go to q_out (head stride q_head, token stride q_tok, a sequence after the other); key heads (rotated) and value heads (copied)
 // go into the caches (batch, hkv, max_len, d) at position base + token index.
 constexpr int kRopeThreads = 256;
 constexpr int kRopeMaxHalf = 1024;  // head_dim <= 2048
 
 __global__ void __launch_bounds__(kRopeThreads) rope_cache_kernel(const __half* qkv, int64_t ld_qkv, const int64_t* pos_dev, int64_t pos_host, __half* q_out,
                                   __half* k_cache, __half* v_cache, int t, int hq, int hkv, int d, int max_len,
-                                  float theta) {
+                                  float theta, int64_t q_head, int64_t q_tok) {
   __shared__ float cs[kRopeMaxHalf], sn[kRopeMaxHalf];
   const int tok = blockIdx.x, b = tok / t, i = tok - b * t;
   const int half_d = d >> 1;
@@ -116,13 +117,37 @@ __global__ void __launch_bounds__(kRopeThreads) rope_cache_kernel(const __half* 
   const bool room = pos >= 0 && pos < max_len;
   const __half* row = qkv + (int64_t)tok * ld_qkv;
   auto head_dst = [&](int head) -> __half* {  // null: dropped
-    if (head < hq) return q_out + (((int64_t)b * hq + head) * t + i) * d;
+    if (head < hq) return q_out + (int64_t)b * hq * t * d + head * q_head + i * q_tok;
     const bool key = head < hq + hkv;
     return room ? (key ? k_cache : v_cache) + (((int64_t)b * hkv + (head - hq - (key ? 0 : hkv))) * max_len + pos) * d : nullptr;
   };
+  const uintptr_t all = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_cache) |
+                        reinterpret_cast<uintptr_t>(v_cache);
+  if ((half_d & 7) == 0 && (ld_qkv & 7) == 0 && (all & 15) == 0) {
+    const int per_head = half_d >> 3;
+    for (int e = threadIdx.x; e < (hq + 2 * hkv) * per_head; e += kRopeThreads) {
+      const int head = e / per_head, j = (e - head * per_head) * 8;
+      __half* dst = head_dst(head);
+      if (!dst) continue;
+      const __half* src = row + (int64_t)head * d;
+      uint4 a = *reinterpret_cast<const uint4*>(src + j), c = *reinterpret_cast<const uint4*>(src + j + half_d);
+      if (head < hq + hkv) {
+        __half2 *h1 = reinterpret_cast<__half2*>(&a), *h2 = reinterpret_cast<__half2*>(&c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 x1 = __half22float2(h1[k]), x2 = __half22float2(h2[k]);
+          const float2 co = *reinterpret_cast<const float2*>(cs + j + 2 * k), si = *reinterpret_cast<const float2*>(sn + j + 2 * k);
+          h1[k] = __floats2half2_rn(x1.x * co.x - x2.x * si.x, x1.y * co.y - x2.y * si.y);
+          h2[k] = __floats2half2_rn(x2.x * co.x + x1.x * si.x, x2.y * co.y + x1.y * si.y);
+        }
+      }
+      *reinterpret_cast<uint4*>(dst + j) = a;
+      *reinterpret_cast<uint4*>(dst + j + half_d) = c;
+    }
+    return;
+  }
   // pairs of neighbours where every row is aligned for them
-  const bool two = (half_d & 1) == 0 && (ld_qkv & 1) == 0 && ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) |
-                   reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 3) == 0;
+  const bool two = (half_d & 1) == 0 && (ld_qkv & 1) == 0 && (all & 3) == 0;
   const int step = two ? 2 : 1, per_head = half_d / step, items = (hq + 2 * hkv) * per_head;
   for (int e = threadIdx.x; e < items; e += kRopeThreads) {
     const int head = e / per_head, j = (e - head * per_head) * step;
@@ -642,9 +667,8 @@ extern "C" int pe_add_rmsnorm(void* x, const void* delta, int delta_dtype, const
   return PE_OK;
 }
 
-extern "C" int pe_rope_cache(const void* qkv, int64_t ld_qkv, const int64_t* pos_dev, int64_t pos_host, void* q_out,
-                             void* k_cache, void* v_cache, int batch, int t, int hq, int hkv, int head_dim, int max_len,
-                             float theta, void* stream) {
+static int rope_cache(const void* qkv, int64_t ld_qkv, const int64_t* pos_dev, int64_t pos_host, void* q_out, void* k_cache, void* v_cache, int batch,
+                      int t, int hq, int hkv, int head_dim, int max_len, float theta, bool token_major, void* stream) {
   if (!qkv || !q_out || !k_cache || !v_cache || batch < 1 || t < 1 || hq < 1 || hkv < 1 || max_len < 1) return PE_ERR_ARG;
   if (head_dim < 2 || head_dim > 2048 || (head_dim & 1)) return PE_ERR_SHAPE;
   if (ld_qkv < (int64_t)(hq + 2 * hkv) * head_dim) return PE_ERR_ARG;
@@ -652,8 +676,21 @@ extern "C" int pe_rope_cache(const void* qkv, int64_t ld_qkv, const int64_t* pos
   PE_CUDA_TRY(launch_pdl(rope_cache_kernel, dim3((unsigned)(batch * t)), dim3(kRopeThreads), 0,
                          static_cast<cudaStream_t>(stream), static_cast<const __half*>(qkv), ld_qkv, pos_dev, pos_host,
                          static_cast<__half*>(q_out), static_cast<__half*>(k_cache), static_cast<__half*>(v_cache), t, hq, hkv,
-                         head_dim, max_len, theta));
+                         head_dim, max_len, theta, token_major ? (int64_t)head_dim : (int64_t)t * head_dim,
+                         token_major ? (int64_t)hq * head_dim : (int64_t)head_dim));
   return PE_OK;
+}
+
+extern "C" int pe_rope_cache(const void* qkv, int64_t ld_qkv, const int64_t* pos_dev, int64_t pos_host, void* q_out,
+                             void* k_cache, void* v_cache, int batch, int t, int hq, int hkv, int head_dim, int max_len,
+                             float theta, void* stream) {
+  return rope_cache(qkv, ld_qkv, pos_dev, pos_host, q_out, k_cache, v_cache, batch, t, hq, hkv, head_dim, max_len, theta, false, stream);
+}
+
+extern "C" int pe_rope_cache_token_major(const void* qkv, int64_t ld_qkv, const int64_t* pos_dev, int64_t pos_host, void* q_out,
+                                         void* k_cache, void* v_cache, int batch, int t, int hq, int hkv, int head_dim, int max_len,
+                                         float theta, void* stream) {
+  return rope_cache(qkv, ld_qkv, pos_dev, pos_host, q_out, k_cache, v_cache, batch, t, hq, hkv, head_dim, max_len, theta, true, stream);
 }
 
 extern "C" int pe_silu_mul(const void* gate_up, int64_t ld_gu, void* out, int64_t ld_out, int rows, int inter, void* stream) {

@@ -38,9 +38,12 @@ struct GemmArgs {
   int tiles_m, tiles_n;
   int lut_bytes;  // n_levels (256 for nibble pairs) x table stride
   int nc;         // code stages
-  int ksplit;     // K ranges per tile (1 = none); partial results in `part`
-  float* part;    // [ksplit][M][N] fp32
-  int y_tma;      // the output leaves through TMA stores (16-bit output, 16-byte aligned rows)
+  int full;       // tiles 0 .. full - 1 are computed whole, the others in ksplit K ranges each
+  int ksplit;
+  int col0;       // first column of the split tiles
+  float* part;    // [ksplit][M][N - col0] fp32
+  int y_tma;      // the output leaves through TMA stores (16-byte aligned rows)
+  int part_tma;   // ... and so do the partials
   int* status;
 };
 
@@ -145,7 +148,7 @@ __device__ __forceinline__ uint32_t glut_s(uint32_t word, uint32_t lane_base) {
 template <bool PACKED>
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const GemmArgs p, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap cmap,
-                 const __grid_constant__ CUtensorMap ymap) {
+                 const __grid_constant__ CUtensorMap ymap, const __grid_constant__ CUtensorMap partmap) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023) & ~1023u;
@@ -216,12 +219,13 @@ gemm_pair_kernel(const GemmArgs p, const __grid_constant__ CUtensorMap xmap, con
   pdl_enter();
 
   const int ksteps = p.K / kStepK;
-  // A unit of work is a tile or, when the launch has few tiles, one of `ksplit` K ranges of a tile (fp32 partials
-  // in the workspace, summed by a second kernel).
-  const int n_tiles = p.tiles_m * p.tiles_n * p.ksplit;
+  // A unit of work is a tile or, for the tiles of a last wave that would leave pairs idle, one of `ksplit` K ranges of a
+  // tile (fp32 partials in the workspace, summed by a second kernel).  Whole tiles come first: split = -1.
+  const int n_tiles = p.full + (p.tiles_m * p.tiles_n - p.full) * p.ksplit;
   auto unit_of = [&](int unit, int& split, int& ks0, int& ks1) {
-    const int tile = unit / p.ksplit;
-    split = unit - tile * p.ksplit;
+    if (unit < p.full) { split = -1; ks0 = 0; ks1 = ksteps; return unit; }
+    const int u = unit - p.full, tile = p.full + u / p.ksplit;
+    split = u % p.ksplit;
     ks0 = (int)((long long)split * ksteps / p.ksplit);
     ks1 = (int)((long long)(split + 1) * ksteps / p.ksplit);
     return tile;
@@ -322,18 +326,20 @@ gemm_pair_kernel(const GemmArgs p, const __grid_constant__ CUtensorMap xmap, con
     const uint32_t wrow = (uint32_t)((r >> 3) * 1024 + (r & 7) * 128);
     const int sw7 = r & 7;
     const uint32_t lead = map_to_cta(bars, 0) - bars;
-    int it = 0, tcount = 0;
+    int it = 0, tcount = 0, stg_phase = 0;
     for (int unit = pair; unit < n_tiles && !*abort_flag; unit += n_pairs, ++tcount) {
       int split, ks0, ks1;
       const int tile = unit_of(unit, split, ks0, ks1);
       const int m0 = (tile % p.tiles_m) * kPairTileM, n0 = (tile / p.tiles_m) * kTileN;
       const bool two = m0 + 256 < p.M;
       // where this unit's result goes: the output, or (K split) the fp32 partial of its K range
-      void* const y_ptr = p.ksplit > 1 ? static_cast<void*>(p.part + (size_t)split * p.M * p.N) : p.y;
-      const int y_dt = p.ksplit > 1 ? (int)PE_F32 : p.y_dtype;
-      const int64_t y_ld = p.ksplit > 1 ? (int64_t)p.N : p.ld_y;
-      const __half* const bias_ptr = p.ksplit > 1 ? nullptr : p.bias;
-      const bool tma_out = p.y_tma && p.ksplit == 1;
+      const bool whole = split < 0;
+      const int64_t part_ld = p.N - p.col0;
+      void* const y_ptr = whole ? p.y : static_cast<void*>(p.part + (int64_t)split * p.M * part_ld - p.col0);
+      const int y_dt = whole ? p.y_dtype : (int)PE_F32;
+      const int64_t y_ld = whole ? p.ld_y : part_ld;
+      const __half* const bias_ptr = whole ? p.bias : nullptr;
+      const bool tma_out = whole ? p.y_tma : p.part_tma;
       int row = n0 + (int)rank * 128 + r;
       const bool row_ok = row < p.N;
       if (!row_ok) row = p.N - 1;
@@ -418,7 +424,40 @@ gemm_pair_kernel(const GemmArgs p, const __grid_constant__ CUtensorMap xmap, con
         if (!__all_sync(0xffffffffu, ok)) break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (tma_out) {
+      if (tma_out && y_dt == PE_F32) {
+        // as below with 32 rows x 32 columns of fp32 (4 KB, 128-byte swizzle) per warp: the output, or the partial of a K range
+        const uint32_t stg = base + kWOff + (uint32_t)(warp - 2) * 4096u;
+        const int swz = lane & 7;
+        if (half == 0 || two) {
+          const int mrow0 = m0 + half * 256 + (int)rank * 128 + q * 32;
+          const uint32_t trow = tmem + half * 256 + ((uint32_t)(q * 32) << 16);
+#pragma unroll 1
+          for (int cc = chalf * 4; cc < chalf * 4 + 4; ++cc) {
+            uint32_t rr[32];
+            tmem_ld32(trow + cc * 32, rr);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            const int nb0 = n0 + cc * 32;
+            if (bias_ptr) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (nb0 + j < p.N) rr[j] = __float_as_uint(__uint_as_float(rr[j]) + __half2float(bias_ptr[nb0 + j]));
+            }
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the previous store has read the buffer
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(stg + (uint32_t)lane * 128u + (uint32_t)((j ^ swz) << 4)), "r"(rr[4 * j]),
+                           "r"(rr[4 * j + 1]), "r"(rr[4 * j + 2]), "r"(rr[4 * j + 3]) : "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0 && mrow0 < p.M && nb0 < p.N) {
+              asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                           ::"l"(whole ? &ymap : &partmap), "r"(stg), "r"(whole ? nb0 : nb0 - p.col0), "r"(mrow0), "r"(whole ? 0 : split) : "memory");
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+          }
+        }
+      } else if (tma_out) {
         // 16-bit output: every warp stages its 32 rows x 32 columns (2 KB, 64-byte swizzle) in its own piece of the
         // weight stages -- idle now: all MMAs are done and no warp decodes before the staging barrier below -- and one
         // lane sends it off as a TMA store, which writes whole 64-byte row pieces and clips at the matrix edges.
@@ -521,7 +560,8 @@ gemm_pair_kernel(const GemmArgs p, const __grid_constant__ CUtensorMap xmap, con
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           mbar_arrive(stg_free);
         }
-        const bool ok = mbar_wait(stg_free, tcount & 1, abort_flag, p.status, 10);
+        const bool ok = mbar_wait(stg_free, stg_phase, abort_flag, p.status, 10);
+        stg_phase ^= 1;
         if (!__all_sync(0xffffffffu, ok)) break;
       }
     }
@@ -561,13 +601,25 @@ static int small_ksplit(int m, int out_f, int in_f_padded, int sms) {
   return s < 2 ? 1 : s;
 }
 
-// K ranges per 512-row pair tile: as many as there are idle pairs, at least eight K steps each; two ranges only for a
-// long K (the fp32 partials and their sum cost about what halving a short tile saves).
-static int pair_ksplit(int ptiles, int ksteps, int sms) {
-  int ks = (sms / 2) / ptiles;
+// Whole and split tiles of a launch over pairs of CTAs.  Fewer tiles than pairs: as many K ranges as there are idle
+// pairs, at least eight K steps each; two ranges only for a long K (the fp32 partials and their sum cost about what halving
+// a short tile saves).  More: the tiles of the last, partly filled wave (rounded up to whole columns of tiles, so that the
+// partials are one matrix) are split over all pairs where that saves more of a tile's ksteps x 0.85 us than the partials
+// cost (up to 18 us).  4096 x 12288 x 4096, 5.2 waves: 382 us as six waves, 368 us.
+struct PairPlan { int full, ksplit, col0; };
+static PairPlan pair_plan(int tiles_m, int tiles_n, int ksteps, int sms) {
+  const int tiles = tiles_m * tiles_n, pairs = sms / 2;
+  if (tiles <= pairs) {
+    int ks = pairs / tiles;
+    if (ks > ksteps / 8) ks = ksteps / 8;
+    if (ks == 2 && ksteps < 128) ks = 1;
+    return ks < 2 ? PairPlan{tiles, 1, 0} : PairPlan{0, ks, 0};
+  }
+  const int cols = (tiles % pairs + tiles_m - 1) / tiles_m, rest = cols * tiles_m;
+  int ks = rest ? pairs / rest : 1;
   if (ks > ksteps / 8) ks = ksteps / 8;
-  if (ks == 2 && ksteps < 128) ks = 1;
-  return ks < 2 ? 1 : ks;
+  if (ks < 2 || ksteps * (ks - 1) < 40 * ks) return {tiles, 1, 0};
+  return {tiles - rest, ks, (tiles_n - cols) * kTileN};
 }
 
 // workspace: [status word, padded to 256 B][bf16 activations M x K]
@@ -581,12 +633,16 @@ extern "C" size_t pe_gemm_workspace_bytes_splitk(int m, int out_f, int in_f_padd
   const size_t base = pe_gemm_workspace_bytes(m, in_f_padded);
   if (base == 0 || out_f < 1) return 0;
   const int sms = sm_count();
-  int ks = sms > 0 && m <= 256 ? small_ksplit(m, out_f, in_f_padded, sms) : 1;
-  if (m > 256 && sms >= 2) {  // pairs of CTAs, 512-row tiles, at least eight K steps per unit
-    const int ptiles = ((m + kPairTileM - 1) / kPairTileM) * ((out_f + kTileN - 1) / kTileN);
-    ks = pair_ksplit(ptiles, in_f_padded / kStepK, sms);
+  if (sms < 2) return base;
+  int ks = 1, cols = out_f;
+  if (m <= 256) {
+    ks = small_ksplit(m, out_f, in_f_padded, sms);
+  } else {
+    const PairPlan p = pair_plan((m + kPairTileM - 1) / kPairTileM, (out_f + kTileN - 1) / kTileN, in_f_padded / kStepK, sms);
+    ks = p.ksplit;
+    cols = out_f - p.col0;
   }
-  return ks > 1 ? ((base + 255) & ~(size_t)255) + (size_t)ks * m * out_f * sizeof(float) : base;
+  return ks > 1 ? ((base + 255) & ~(size_t)255) + (size_t)ks * m * cols * sizeof(float) : base;
 }
 
 extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms,
@@ -595,7 +651,7 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
                        void* workspace, size_t workspace_bytes, void* stream) {
   if (!codes || !norms || !ct_scaled || !x || !y || !workspace) return PE_ERR_ARG;
   if (m < 1 || out_f < 1 || in_f < 1 || in_f > in_f_padded) return PE_ERR_ARG;
-  if (x_kind != PE_X_ROTATED && x_kind != PE_X_RAW) return PE_ERR_ARG;
+  if (x_kind != PE_X_ROTATED && x_kind != PE_X_RAW && !(x_kind == PE_X_SILU_MUL && x_dtype == PE_F16)) return PE_ERR_ARG;
   if (x_dtype < PE_F32 || x_dtype > PE_BF16 || y_dtype < PE_F32 || y_dtype > PE_BF16) return PE_ERR_ARG;
   if (n_levels < 2 || n_levels > 256 || (packed && n_levels > 16)) return PE_ERR_ARG;
   if (in_f_padded % kBlock) return PE_ERR_SHAPE;
@@ -603,7 +659,7 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return PE_ERR_ALIGN;
   if (workspace_bytes < pe_gemm_workspace_bytes(m, in_f_padded)) return PE_ERR_WORKSPACE;
   if (ld_codes < (packed ? in_f_padded / 2 : in_f_padded) || ld_norms < in_f_padded / kBlock) return PE_ERR_ARG;
-  if (ld_x < (x_kind == PE_X_RAW ? in_f : in_f_padded) || ld_y < out_f) return PE_ERR_ARG;
+  if (ld_x < (x_kind == PE_X_RAW ? in_f : x_kind == PE_X_SILU_MUL ? 2 * (int64_t)in_f : in_f_padded) || ld_y < out_f) return PE_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int sms = sm_count();
   if (sms <= 0) return PE_ERR_CUDA;
@@ -614,7 +670,7 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
   if (rc != PE_OK) return rc;
   // few tiles: split K when the caller's workspace has room for the partials
   const size_t part_off = (pe_gemm_workspace_bytes(m, in_f_padded) + 255) & ~(size_t)255;
-  auto fits = [&](int ks) { return ks > 1 && workspace_bytes >= part_off + (size_t)ks * m * out_f * sizeof(float) ? ks : 1; };
+  auto fits = [&](int ks, int cols) { return ks > 1 && workspace_bytes >= part_off + (size_t)ks * m * cols * sizeof(float); };
   float* part = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + part_off);
 
   if (m <= 256) {
@@ -627,7 +683,8 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
     a.halves = small_halves(m, out_f, sms);
     a.tiles_m = 1; a.tok = m;
     a.tiles_n = (out_f + 128 * a.halves - 1) / (128 * a.halves);
-    a.ksplit = fits(small_ksplit(m, out_f, in_f_padded, sms));
+    a.ksplit = small_ksplit(m, out_f, in_f_padded, sms);
+    if (!fits(a.ksplit, out_f)) a.ksplit = 1;
     a.part = a.ksplit > 1 ? part : nullptr;
     a.xbox = (m + 15) & ~15;
     a.x_stage = a.xbox * 128;
@@ -645,8 +702,10 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
     rc = encode_map_2d(&pmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, codes, packed ? in_f_padded / 2 : in_f_padded, out_f, ld_codes, code_row, 128,
                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
   CUtensorMap ymap = pmap;  // a valid map also when the kernel does not use it
-  const bool y_tma = y_dtype != PE_F32 && ld_y % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
-  if (rc == PE_OK && y_tma)
+  const bool y_tma = ld_y % (y_dtype == PE_F32 ? 4 : 8) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+  if (rc == PE_OK && y_tma && y_dtype == PE_F32)
+    rc = encode_map_f32(&ymap, y, out_f, m, 1, (uint64_t)ld_y * 4);
+  else if (rc == PE_OK && y_tma)
     rc = encode_map_2d(&ymap, CU_TENSOR_MAP_DATA_TYPE_UINT16, y, out_f, m, (uint64_t)ld_y * 2, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B,
                        CU_TENSOR_MAP_L2_PROMOTION_NONE);
   if (rc != PE_OK) return rc;
@@ -664,10 +723,15 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
   a.lut_bytes = packed ? 256 * kPairLutStride : n_levels * 128;
   a.nc = kPairCodeStages;
   const unsigned smem_bytes = (packed ? 4 : 3) * 2 * kXTileBytes + kPairWStages * kPairWTileBytes + a.lut_bytes + a.nc * 128 * code_row + 256 + 1024;
-  const int ptiles = a.tiles_m * a.tiles_n;
-  a.ksplit = fits(pair_ksplit(ptiles, in_f_padded / kStepK, sms));
-  a.part = a.ksplit > 1 ? part : nullptr;
-  const int units = ptiles * a.ksplit, pairs = units < sms / 2 ? units : sms / 2;
+  PairPlan plan = pair_plan(a.tiles_m, a.tiles_n, in_f_padded / kStepK, sms);
+  const int tiles = a.tiles_m * a.tiles_n;
+  if (!fits(plan.ksplit, out_f - plan.col0)) plan = {tiles, 1, 0};
+  a.full = plan.full; a.ksplit = plan.ksplit; a.col0 = plan.col0;
+  a.part = part;
+  CUtensorMap partmap = ymap;
+  a.part_tma = plan.ksplit > 1 && (out_f - plan.col0) % 4 == 0;
+  if (a.part_tma && (rc = encode_map_f32(&partmap, part, out_f - plan.col0, m, plan.ksplit, (uint64_t)(out_f - plan.col0) * 4)) != PE_OK) return rc;
+  const int units = plan.full + (tiles - plan.full) * plan.ksplit, pairs = units < sms / 2 ? units : sms / 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs);
   cfg.blockDim = dim3(kPairThreads);
@@ -682,6 +746,9 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
   cfg.numAttrs = 2;
   auto kfn = packed ? gemm_pair_kernel<true> : gemm_pair_kernel<false>;
   PE_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
-  PE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kfn, a, map, pmap, ymap));
-  return a.ksplit > 1 ? launch_splitk_reduce(part, a.ksplit, m, out_f, bias, y, y_dtype, ld_y, sms, st) : PE_OK;
+  PE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kfn, a, map, pmap, ymap, partmap));
+  if (plan.ksplit == 1) return PE_OK;
+  const int c0 = plan.col0;
+  return launch_splitk_reduce(part, plan.ksplit, m, out_f - c0, bias ? static_cast<const __half*>(bias) + c0 : nullptr,
+                              static_cast<uint8_t*>(y) + (int64_t)c0 * (y_dtype == PE_F32 ? 4 : 2), y_dtype, ld_y, sms, st);
 }

@@ -56,7 +56,9 @@ __device__ __forceinline__ void unpack8(const Raw8<XD>& r, float f[8]) {
 // were what bounded the pass: 16384 rows of 1856 took 50 us, 28 us now.)
 // Grouped launches: row m of the prepared matrix is row x_rows[m] of x, and only the first valid_rows[0] +
 // valid_rows[1] rows exist (the rest of the list is undefined and is written as zeros).
-template <int XD>
+// With SILU rows are [gate | up] of `limit` columns each and the input is half(silu(gate)) * up, rounded as pe_silu_mul
+// rounds (a launch and a trip through memory less per layer: 512 rows of 12288 took 8.5 us more).
+template <int XD, bool SILU>
 __global__ void __launch_bounds__(kPrepThreads) gemm_prep_kernel(const void* x, int raw, int64_t ld_x, int limit, __nv_bfloat16* xq, int M, int nb,
                                                                  int pair_layout, const int* x_rows, const int* valid_rows, int* status) {
   asm volatile("griddepcontrol.wait;" ::: "memory");  // first: the matmul behind may then read what older kernels wrote at once
@@ -68,11 +70,25 @@ __global__ void __launch_bounds__(kPrepThreads) gemm_prep_kernel(const void* x, 
   const int m = on ? (int)(item / nb) : 0, blk = on ? (int)(item - (int64_t)m * nb) : 0;
   const bool live = on && (!valid_rows || m < valid_rows[0] + valid_rows[1]);
   const int64_t row = live && x_rows ? x_rows[m] : m;
-  const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (ld_x & (XD == PE_F32 ? 3 : 7)) == 0;
+  const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (ld_x & (XD == PE_F32 ? 3 : 7)) == 0 && (!SILU || (limit & 7) == 0);
   const int lim = live ? limit : 0, col = blk * kBlock + 16 * q;
   Raw8<XD> r[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) r[i] = load8<XD>(x, row * ld_x, col + (i & 1) * 8 + (i >> 1) * 64, lim, vec);
+  if constexpr (SILU) {
+    Raw8<XD> up[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) up[i] = load8<XD>(x, row * ld_x + limit, col + (i & 1) * 8 + (i >> 1) * 64, lim, vec);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      __half2 *g = reinterpret_cast<__half2*>(&r[i].w[0]), *u = reinterpret_cast<__half2*>(&up[i].w[0]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __half22float2(g[j]);
+        g[j] = __hmul2(__floats2half2_rn(f.x / (1.f + expf(-f.x)), f.y / (1.f + expf(-f.y))), u[j]);
+      }
+    }
+  }
   float2 p[16];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
@@ -131,9 +147,12 @@ int launch_gemm_prep(const void* x, int x_kind, int x_dtype, int64_t ld_x, int i
   const int nb = in_f_padded / kBlock;
   const int64_t blocks = ((int64_t)rows * nb + kPrepItems - 1) / kPrepItems;
   if (blocks > 0x7fffffff) return PE_ERR_LIMIT;
-  auto kfn = x_dtype == PE_F32 ? gemm_prep_kernel<PE_F32> : x_dtype == PE_F16 ? gemm_prep_kernel<PE_F16> : gemm_prep_kernel<PE_BF16>;
-  PE_CUDA_TRY(launch_pdl(kfn, dim3((unsigned)blocks), dim3(kPrepThreads), 0, st, x, x_kind == PE_X_RAW ? 1 : 0, ld_x,
-                         x_kind == PE_X_RAW ? in_f : in_f_padded, static_cast<__nv_bfloat16*>(xq), rows, nb, pair_layout, x_rows, valid_rows, status));
+  auto kfn = x_kind == PE_X_SILU_MUL ? gemm_prep_kernel<PE_F16, true>
+             : x_dtype == PE_F32     ? gemm_prep_kernel<PE_F32, false>
+             : x_dtype == PE_F16     ? gemm_prep_kernel<PE_F16, false>
+                                     : gemm_prep_kernel<PE_BF16, false>;
+  PE_CUDA_TRY(launch_pdl(kfn, dim3((unsigned)blocks), dim3(kPrepThreads), 0, st, x, x_kind != PE_X_ROTATED ? 1 : 0, ld_x,
+                         x_kind != PE_X_ROTATED ? in_f : in_f_padded, static_cast<__nv_bfloat16*>(xq), rows, nb, pair_layout, x_rows, valid_rows, status));
   return PE_OK;
 }
 
@@ -210,6 +229,16 @@ static EncodeTiledFn encode_fn() {
       fn = reinterpret_cast<EncodeTiledFn>(p);
   }
   return fn;
+}
+
+// fp32 matrices [depth][height][width] one after the other, boxes of 32 x 32 x 1 with 128-byte swizzle
+int encode_map_f32(CUtensorMap* map, const void* base, uint64_t width, uint64_t height, uint64_t depth, uint64_t row_bytes) {
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) return PE_ERR_CUDA;
+  const cuuint64_t dims[3] = {width, height, depth}, strides[2] = {row_bytes, row_bytes * height};
+  const cuuint32_t box[3] = {32, 32, 1}, estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? PE_OK : PE_ERR_CUDA;
 }
 
 int encode_map_2d(CUtensorMap* map, CUtensorMapDataType type, const void* base, uint64_t width, uint64_t height, uint64_t row_bytes, uint32_t box_w,

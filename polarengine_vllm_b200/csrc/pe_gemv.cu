@@ -2,7 +2,7 @@
 //
 //   y[m, r] = sum_blk norm[r, blk] * sum_k ct[code[r, blk, k]] * xt[m, blk, k]   (+ bias[r])
 //
-// One activation row over row-major codes goes to the column-owner kernel (pe_gemv_rows.cu: 47.2 us for a decoder
+// One activation row over row-major codes goes to the column-owner kernel (pe_gemv_cols.cu: 47.2 us for a decoder
 // layer's four launches, 51 us for the bulk-copy kernel on that layout); everything else, one row over the tiled copy
 // (42.6 us) included, to the bulk-copy kernel (pe_gemv_bulk.cu).
 #include "pe_gemv_decode.cuh"

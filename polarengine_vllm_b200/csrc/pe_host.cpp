@@ -111,7 +111,7 @@ bool plain(const Matrix& w, const at::Device& dev) {
 }
 
 // x (rows, in_f or in_f_padded), last dimension contiguous; nullopt-like undefined tensor when not the plain case
-at::Tensor multiply(const Matrix& w, const at::Tensor& x, int64_t rows, int64_t ld_x, bool rotated, at::ScalarType out, const at::Tensor* bias,
+at::Tensor multiply(const Matrix& w, const at::Tensor& x, int64_t rows, int64_t ld_x, int kind, at::ScalarType out, const at::Tensor* bias,
                     at::IntArrayRef shape) {
   const at::Device dev = x.device();
   const int xd = code_of(x.scalar_type()), yd = code_of(out);
@@ -120,7 +120,7 @@ at::Tensor multiply(const Matrix& w, const at::Tensor& x, int64_t rows, int64_t 
   at::Tensor y = at::empty(shape, x.options().dtype(out).requires_grad(false));
   cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   const void* b = bias ? bias->const_data_ptr() : nullptr;
-  const int kind = rotated ? PE_X_ROTATED : PE_X_RAW, levels = (int)w.ct->numel();
+  const int levels = (int)w.ct->numel();
   const float* ct = w.ct->const_data_ptr<float>();
   int rc;
   if (rows <= kDecodeRows) {
@@ -206,7 +206,7 @@ PyObject* host_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   at::DimVector shape(x->sizes());
   shape.back() = w.out_f;
-  return wrap_or_none(multiply(w, *x, rows, w.in_f, false, at::kHalf, bias, shape));
+  return wrap_or_none(multiply(w, *x, rows, w.in_f, PE_X_RAW, at::kHalf, bias, shape));
   PE_GUARD_END
 }
 
@@ -222,13 +222,18 @@ PyObject* host_matmul(PyObject*, PyObject* const* args, Py_ssize_t n) {
   w.ct = tensor_or_null(args[3]);
   const at::Tensor* x = tensor_or_null(args[4]);
   if (!w.codes || !w.norms || !w.ct || !x || !to_int(args[6], w.out_f) || !to_int(args[7], w.in_f) || !to_int(args[8], w.in_f_padded)) Py_RETURN_NONE;
-  const bool rotated = PyObject_IsTrue(args[5]) == 1;
-  if (x->dim() != 2 || x->stride(1) != 1 || x->size(1) != (rotated ? w.in_f_padded : w.in_f) || !THPDtype_Check(args[9])) Py_RETURN_NONE;
+  // rotated, or not; or a PE_X_* number
+  int kind = PE_X_RAW;
+  if (PyBool_Check(args[5])) kind = args[5] == Py_True ? PE_X_ROTATED : PE_X_RAW;
+  else if (!to_int(args[5], kind)) Py_RETURN_NONE;
+  const int64_t width = kind == PE_X_ROTATED ? w.in_f_padded : kind == PE_X_SILU_MUL ? 2 * (int64_t)w.in_f : w.in_f;
+  if (x->dim() != 2 || x->stride(1) != 1 || x->size(1) != width || !THPDtype_Check(args[9])) Py_RETURN_NONE;
+  if (kind == PE_X_SILU_MUL && x->size(0) <= kDecodeRows) Py_RETURN_NONE;
   const at::Tensor* bias = nullptr;
   if (args[10] != Py_None && !(bias = tensor_or_null(args[10]))) Py_RETURN_NONE;
   if (args[11] != Py_None && !(w.tiles = tensor_or_null(args[11]))) Py_RETURN_NONE;
   const at::ScalarType out = reinterpret_cast<THPDtype*>(args[9])->scalar_type;
-  return wrap_or_none(multiply(w, *x, x->size(0), x->stride(0), rotated, out, bias, {x->size(0), w.out_f}));
+  return wrap_or_none(multiply(w, *x, x->size(0), x->stride(0), kind, out, bias, {x->size(0), w.out_f}));
   PE_GUARD_END
 }
 

@@ -29,22 +29,23 @@ def add_rmsnorm(x: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Te
 
 
 def rope_cache(qkv: torch.Tensor, pos0: Union[int, torch.Tensor], k_cache: torch.Tensor, v_cache: torch.Tensor, batch: int,
-               t: int, hq: int, hkv: int, head_dim: int, theta: float) -> torch.Tensor:
-    """qkv (batch*t, (hq + 2 hkv) * head_dim) fp16 -> rotated queries (batch, hq, t, head_dim);
+               t: int, hq: int, hkv: int, head_dim: int, theta: float, token_major: bool = False) -> torch.Tensor:
+    """qkv (batch*t, (hq + 2 hkv) * head_dim) fp16 -> rotated queries (batch, hq, t, head_dim), in memory
+    (batch, t, hq, head_dim) if ``token_major``;
     rotated keys and values are written into the caches (batch, hkv, max_len, head_dim) at
     positions pos0 .. pos0 + t - 1.  ``pos0`` is an int or a 0-d int64 device tensor."""
     dev = nv.require_cuda(qkv, k_cache, v_cache)
     if qkv.dtype != torch.float16 or qkv.stride(1) != 1 or not k_cache.is_contiguous() or not v_cache.is_contiguous():
         raise ValueError("rope_cache wants fp16 qkv rows and contiguous caches")
-    q = torch.empty(batch, hq, t, head_dim, dtype=torch.float16, device=dev)
+    q = torch.empty((batch, t, hq, head_dim) if token_major else (batch, hq, t, head_dim), dtype=torch.float16, device=dev)
     dev_pos = pos0 if torch.is_tensor(pos0) else None
     if dev_pos is not None and (dev_pos.dtype != torch.int64 or dev_pos.device != dev):
         raise ValueError("a device position must be an int64 tensor on the same device")
-    nv.check(nv.lib().pe_rope_cache(qkv.data_ptr(), qkv.stride(0), dev_pos.data_ptr() if dev_pos is not None else None,
-                                    0 if dev_pos is not None else int(pos0), q.data_ptr(), k_cache.data_ptr(),
-                                    v_cache.data_ptr(), batch, t, hq, hkv, head_dim, k_cache.shape[2], float(theta),
-                                    nv.stream_ptr(dev)), "pe_rope_cache")
-    return q
+    call = nv.lib().pe_rope_cache_token_major if token_major else nv.lib().pe_rope_cache
+    nv.check(call(qkv.data_ptr(), qkv.stride(0), dev_pos.data_ptr() if dev_pos is not None else None,
+                  0 if dev_pos is not None else int(pos0), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), batch, t, hq, hkv,
+                  head_dim, k_cache.shape[2], float(theta), nv.stream_ptr(dev)), "pe_rope_cache")
+    return q.transpose(1, 2) if token_major else q
 
 
 def silu_mul(gate_up: torch.Tensor, inter: int) -> torch.Tensor:

@@ -97,6 +97,15 @@ class QWeight:
                             tiles=self.tiles)
 
 
+    def of_gate_up(self, gate_up: torch.Tensor, out_dtype=torch.float16) -> torch.Tensor:
+        """The matmul of silu(gate) * up; more rows than a decode batch compute the product while they are prepared."""
+        y = None
+        if gate_up.shape[0] > GEMV_MAX_BATCH:
+            y = (nv._host or nv.host()).matmul(self.codes, self.packed, self.norms, self.ct, gate_up, nv.PE_X_SILU_MUL, self.out_f, self.in_f,
+                                               self.in_f, out_dtype, None, None)
+        return y if y is not None else self(silu_mul(gate_up, self.in_f), out_dtype)
+
+
 def shard_fused_rows(codes, norms, sections, rank: int, world: int):
     """Column-parallel shard of a fused projection: the rank's rows of every section (q | k | v, gate | up),
     concatenated in section order -- the slicing vLLM's loader applies to fused ``qkv_proj`` / ``gate_up_proj``
@@ -236,15 +245,15 @@ class QuantDecoder:
                 q = rope_cache(qkv, pos0, self.k_cache[li], self.v_cache[li], b, t, self.hq, self.hkv, d, cfg.rope_theta)
                 att = decode_attention(q, self.k_cache[li], self.v_cache[li], pos0)
             else:
-                q = rope_cache(qkv, pos0, self.k_cache[li], self.v_cache[li], b, t, self.hq, self.hkv, d, cfg.rope_theta)
+                q = rope_cache(qkv, pos0, self.k_cache[li], self.v_cache[li], b, t, self.hq, self.hkv, d, cfg.rope_theta, token_major=True)
                 p0 = int(pos0)
                 att = F.scaled_dot_product_attention(q, self.k_cache[li][:, :, : p0 + t], self.v_cache[li][:, :, : p0 + t],
                                                      is_causal=(p0 == 0 and t > 1), enable_gqa=True)
-                att = att.transpose(1, 2).reshape(b * t, self.hq * d)
+                att = att.transpose(1, 2).reshape(b * t, self.hq * d)  # the output is laid out as q: no copy
             gate_up = norm_proj(L["gate_up"], L["o"](att, torch.float32), L["ln2"])
             delta = L["down"].fused(nv.PE_PRO_SILU_MUL, gate_up, torch.float32) if one else None
             if delta is None:
-                delta = L["down"](silu_mul(gate_up, self.inter), torch.float32)
+                delta = L["down"].of_gate_up(gate_up, torch.float32)
         if fold_norm:
             logits = self.head.fused(nv.PE_PRO_ADD_RMSNORM, x, torch.float32, delta=delta, norm_weight=self.final_ln,
                                      eps=cfg.rms_eps, resid_out=x_alt)

@@ -230,3 +230,41 @@ def test_rope_attention_equals_the_two_launches(batch, hq, hkv, pos, on_device):
         assert torch.equal(out, ref)
     else:
         assert torch.allclose(out.float(), ref.float(), rtol=2e-3, atol=2e-3)
+
+
+@pytest.mark.parametrize("batch,hq,hkv,max_len,pos", [(1, 4, 4, 8, 7), (1, 8, 4, 33, 32), (5, 16, 4, 100, 63), (2, 16, 2, 4100, 4099),
+                                                      (32, 32, 8, 300, 129)])
+def test_decode_attention_split_edges(batch, hq, hkv, max_len, pos):
+    """Caches shorter than a cluster's split, one position past a split, many sequences (no split), 1, 2, 4 and 8 query
+    heads per key head."""
+    from polarengine_vllm_b200.decode_ops import decode_attention
+    d = 128
+    g = torch.Generator(device="cuda").manual_seed(pos)
+    q = torch.randn(batch, hq, 1, d, device="cuda", generator=g).half()
+    kc, vc = (torch.randn(batch, hkv, max_len, d, device="cuda", generator=g).half() for _ in range(2))
+    k, v = (t[:, :, : pos + 1].float().repeat_interleave(hq // hkv, dim=1) for t in (kc, vc))
+    ref = F.scaled_dot_product_attention(q.float(), k, v).transpose(1, 2).reshape(batch, hq * d)
+    for p in (pos, torch.tensor(pos, device="cuda")):
+        assert torch.allclose(decode_attention(q, kc, vc, p).float(), ref, rtol=2e-3, atol=2e-3)
+
+
+@pytest.mark.parametrize("d,shift", [(128, 0), (128, 8), (24, 0), (16, 2), (10, 1)])
+def test_rope_cache_widths_and_token_major(d, shift):
+    """The 16-byte, 4-byte and element paths of pe_rope_cache (head widths, row alignment) against the reference form; the
+    token-major queries are the same values."""
+    from polarengine_vllm_b200.decode_ops import rope_cache
+    from polarengine_vllm_b200.decoder import rope
+    b, t, hq, hkv, max_len, pos0 = 2, 5, 4, 2, 16, 3
+    g = torch.Generator(device="cuda").manual_seed(d)
+    wide = torch.randn(b * t, (hq + 2 * hkv) * d + 8, device="cuda", generator=g).half()
+    qkv = wide[:, shift:shift + (hq + 2 * hkv) * d]
+    caches = [torch.zeros(b, hkv, max_len, d, device="cuda", dtype=torch.float16) for _ in range(4)]
+    q = rope_cache(qkv, pos0, caches[0], caches[1], b, t, hq, hkv, d, 1e4)
+    q2 = rope_cache(qkv, pos0, caches[2], caches[3], b, t, hq, hkv, d, 1e4, token_major=True)
+    assert torch.equal(q, q2) and q2.transpose(1, 2).is_contiguous()
+    assert torch.equal(caches[0], caches[2]) and torch.equal(caches[1], caches[3])
+    heads = qkv.reshape(b, t, hq + 2 * hkv, d).transpose(1, 2)
+    pos = torch.arange(pos0, pos0 + t, device="cuda")
+    assert torch.allclose(q.float(), rope(heads[:, :hq], pos, 1e4).float(), rtol=2e-3, atol=2e-3)
+    assert torch.allclose(caches[0][:, :, pos0:pos0 + t].float(), rope(heads[:, hq:hq + hkv], pos, 1e4).float(), rtol=2e-3, atol=2e-3)
+    assert torch.equal(caches[1][:, :, pos0:pos0 + t], heads[:, hq + hkv:])

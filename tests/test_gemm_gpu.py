@@ -159,3 +159,60 @@ def test_apply_prefill_matches_oracle():
     y = m.apply(layer, x.cuda())
     ref = oracle.apply_forward(x, q["codes"], q["norms"], q["ct_scaled"], in_f)
     assert y.shape == (2, 48, n) and y.dtype == torch.float16 and max_rel(y, ref) <= TOL
+
+
+@pytest.mark.parametrize("m", [17, 32, 129, 191, 192, 193, 256])
+@pytest.mark.parametrize("bits,n,k", [(3, 127, 128), (4, 129, 384), (6, 300, 640), (4, 19000, 256), (3, 5000, 1920)])
+def test_gemm_up_to_256_rows_edges(m, bits, n, k):
+    """Edges of the tensor-memory kernel: token counts around 16, 128 and 192 (two halves), weight rows around 128 and more
+    tiles than SMs, an odd number of K blocks, one block (no split), rows at odd addresses, every output type."""
+    codes, norms, cts = rand_layer(n, k, bits, seed=m + n)
+    in_f = k - 5
+    x = rand_x(m, in_f, seed=m)
+    ref = oracle.linear_dequant(x, codes, norms, cts, in_f=in_f)
+    bias = rand_x(1, n, seed=4).reshape(n)
+    for dt in (torch.float16, torch.float32, torch.bfloat16):
+        y = run_gemm(codes, norms, cts, x, bits, out_dtype=dt, bias=bias, in_f=in_f)
+        assert max_rel(y, ref + bias.float()) <= TOL
+    xt = oracle.fwht(torch.nn.functional.pad(x.float(), (0, k - in_f)))
+    assert max_rel(run_gemm(codes, norms, cts, xt, bits, rotated=True, in_f=in_f), ref) <= TOL
+
+
+@pytest.mark.parametrize("m,in_f", [(17, 300), (200, 304), (513, 384)])
+def test_gemm_of_gate_up_equals_activation_then_gemm(m, in_f):
+    """PE_X_SILU_MUL input: the bits of pe_silu_mul's rounding followed by the same launch, ragged and unaligned widths."""
+    from polarengine_vllm_b200 import _native as nv, packing
+    n, k = 260, 384
+    codes, norms, cts = rand_layer(n, k, 4, seed=m)
+    w, nd, ctd = packing.pack_codes_half_block(codes.cuda()), norms.cuda(), cts.cuda()
+    gu = rand_x(m, 2 * in_f, seed=in_f).cuda()
+    act = torch.nn.functional.silu(gu[:, :in_f]) * gu[:, in_f:]
+    y, ref = ((nv._host or nv.host()).matmul(w, True, nd, ctd, x, kind, n, in_f, k, torch.float32, None, None)
+              for x, kind in ((gu, nv.PE_X_SILU_MUL), (act, False)))
+    assert y is not None and max_rel(y, ref) <= 2e-3
+    assert max_rel(y, oracle.linear_dequant(act.cpu(), codes, norms, cts, in_f=in_f)) <= TOL
+
+
+@pytest.mark.parametrize("m,n,bits,dtype", [(300, 75 * 256 + 40, 4, torch.float16), (600, 37 * 256 + 101, 3, torch.float32),
+                                            (1100, 25 * 256 + 8, 5, torch.bfloat16)])
+def test_gemm_last_wave_split_over_the_pairs(m, n, bits, dtype):
+    """One wave of whole tiles and one or two columns of tiles left, split in K: ragged edges in the split columns, bias, every
+    output type, and the result of the launch without room for the partials."""
+    from polarengine_vllm_b200 import _native as nv, packing
+    k = 4096
+    codes, norms, cts = rand_layer(n, k, bits, seed=m)
+    x, bias = rand_x(m, k, seed=m + 1), rand_x(1, n, seed=2).reshape(n)
+    w, packed = (packing.pack_codes_half_block(codes.cuda()), True) if bits <= 4 else (codes.cuda(), False)
+    nd, ctd, xd, bd = norms.cuda(), cts.cuda(), x.cuda(), bias.cuda()
+    lib, out = nv.lib(), []
+    for room in (lib.pe_gemm_workspace_bytes_splitk(m, n, k), lib.pe_gemm_workspace_bytes(m, k)):
+        y = torch.full((m, n), float("nan"), dtype=dtype, device="cuda")
+        ws = torch.empty(room, dtype=torch.uint8, device="cuda")
+        nv.check(lib.pe_gemm(w.data_ptr(), int(packed), w.stride(0), nd.data_ptr(), nd.stride(0), ctd.data_ptr(), ctd.numel(), xd.data_ptr(),
+                             nv.PE_X_RAW, nv.dtype_code(xd), k, k, y.data_ptr(), nv.dtype_code(y), n, bd.data_ptr(), m, n, k, ws.data_ptr(),
+                             ws.numel(), nv.stream_ptr(xd.device)), "pe_gemm")
+        out.append(y)
+    rows = torch.cat([torch.arange(0, m, 37), torch.arange(m - 3, m)])
+    ref = oracle.linear_dequant(x[rows], codes, norms, cts) + bias.float()
+    assert max_rel(out[0], out[1]) <= 1e-2 and max_rel(out[0][rows.cuda()], ref) <= TOL
+    assert max_rel(out[0][rows.cuda()][:, -400:], ref[:, -400:]) <= TOL

@@ -218,3 +218,88 @@ def test_gemv_row_owner_shapes(batch, bits, n, k):
     xt = oracle.fwht(torch.nn.functional.pad(x.float(), (0, k - in_f)))
     yb = run_native(codes, norms, cts, xt, bits, rotated=True, out_dtype=torch.bfloat16)
     assert max_rel(yb.float(), ref - bias.float()) <= TOL
+
+
+@pytest.mark.parametrize("batch", [2, 8, 9, 16])
+@pytest.mark.parametrize("bits,n,k", [(3, 15, 128), (5, 17, 2048), (4, 33, 2176), (6, 273, 4224), (2, 4737, 384)])
+def test_gemv_bulk_edges(batch, bits, n, k):
+    """Ragged last row tile, odd block counts, the block counts where the split over warps changes (16 and 33 blocks),
+    more tiles than CTAs; raw ragged fp16 and bf16 input in unaligned rows, rotated fp32 input, bias; the tiled copy gives
+    the bits of the row-major arrays."""
+    from polarengine_vllm_b200 import kernels, packing
+    codes, norms, cts = rand_layer(n, k, bits, seed=bits + n + k)
+    in_f, packed = k - 3, bits <= 4
+    w = packing.pack_codes_half_block(codes.cuda()) if packed else codes.cuda()
+    nd, ctd = norms.cuda(), cts.cuda()
+    tiles = kernels.retile(w, packed, nd)
+    bias = rand_x(1, n, seed=9).reshape(n)
+    for dtype in (torch.float16, torch.bfloat16):
+        x = rand_x(batch, in_f, seed=batch, dtype=dtype)
+        ref = oracle.linear_dequant(x, codes, norms, cts, in_f=in_f)
+        wide = torch.zeros(batch, in_f + 5, dtype=dtype, device="cuda")
+        wide[:, 1:1 + in_f] = x.cuda()
+        xs = wide[:, 1:1 + in_f]  # rows that start at odd addresses
+        y = kernels.quant_matmul(w, packed, nd, ctd, xs, False, n, in_f, k, torch.float32, bias.cuda())
+        assert max_rel(y, ref + bias.float()) <= TOL
+        assert torch.equal(y, kernels.quant_matmul(w, packed, nd, ctd, xs, False, n, in_f, k, torch.float32, bias.cuda(), tiles=tiles))
+    xt = oracle.fwht(torch.nn.functional.pad(x.float(), (0, k - in_f)))
+    y = kernels.quant_matmul(w, packed, nd, ctd, xt.cuda(), True, n, in_f, k, torch.float32, tiles=tiles)
+    assert max_rel(y, ref) <= TOL
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17])
+def test_apply_native_call(rows):
+    """The native call of ``apply``: the tiled copy follows the arrays it was made from, non-contiguous input gives the
+    same values and fp64 an error, and a captured call stays right after other calls reused the scratch."""
+    from polarengine_vllm_b200.linear_method import PolarQuantLinearMethod
+    n, in_f, bits = 272, 300, 4
+    method, layer = PolarQuantLinearMethod(128, bits), torch.nn.Module()
+    method.create_weights(layer, in_f, [n], in_f, n, torch.float16)
+    layer = layer.cuda()
+    sets = [rand_layer(n, 384, bits, seed=s) for s in (1, 2)]
+    layer.codes.data.copy_(sets[0][0])
+    layer.norms.data.copy_(sets[0][1])
+    layer.ct_scaled.data.copy_(sets[0][2])
+    method.process_weights_after_loading(layer)
+    x = rand_x(rows, in_f, seed=4).cuda()
+    ref = [oracle.linear_dequant(x.cpu(), *s, in_f=in_f) for s in sets]
+    for _ in range(2):
+        y = method.apply(layer, x)
+        assert max_rel(y, ref[0]) <= TOL
+    assert torch.equal(y, method.apply(layer, torch.stack([x, x], 2)[:, :, 0]))
+    with pytest.raises(TypeError):
+        method.apply(layer, x.double())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        held = method.apply(layer, x)
+    method.apply(layer, torch.zeros_like(x))
+    graph.replay()
+    assert torch.equal(held, y)
+    from polarengine_vllm_b200 import packing
+    layer.codes_packed = packing.pack_codes_half_block(sets[1][0].cuda())  # another matrix under the same layer
+    layer.norms.data = sets[1][1].cuda()
+    assert max_rel(method.apply(layer, x), ref[1]) <= TOL
+
+
+@pytest.mark.parametrize("bits,n,k", [(3, 33, 128), (4, 4097, 2176), (6, 1000, 1152)])
+def test_folded_prologue_over_the_tiled_copy(bits, n, k):
+    """pe_gemv_pro_tiled: add + RMSNorm and silu * up in front of the tiled matmul, ragged shapes included, against the
+    glue launches followed by the same matmul."""
+    from polarengine_vllm_b200 import _native as nv, kernels, packing
+    from polarengine_vllm_b200.decode_ops import add_rmsnorm, silu_mul
+    codes, norms, cts = rand_layer(n, k, bits, seed=n + k)
+    packed = bits <= 4
+    w = packing.pack_codes_half_block(codes.cuda()) if packed else codes.cuda()
+    nd, ctd = norms.cuda(), cts.cuda()
+    tiles = kernels.retile(w, packed, nd)
+    x, delta, lnw = rand_x(1, k, seed=1).cuda(), rand_x(1, k, seed=2).cuda(), (1 + 0.1 * rand_x(1, k, seed=3)[0]).half().cuda()
+    r = x.clone()
+    ref = _gemv_tiled_direct(tiles, packed, ctd, add_rmsnorm(r, delta, lnw, 1e-6), n, k, k)
+    resid = torch.empty_like(x)
+    y = kernels.quant_matmul_pro(w, packed, nd, ctd, nv.PE_PRO_ADD_RMSNORM, x, k, n, k, torch.float32, delta=delta, norm_weight=lnw, eps=1e-6,
+                                 resid_out=resid, tiles=tiles)
+    assert torch.equal(resid, r) and max_rel(y, ref) <= 2e-3
+    gu = rand_x(1, 2 * k, seed=5).cuda()
+    ref = _gemv_tiled_direct(tiles, packed, ctd, silu_mul(gu, k), n, k, k)
+    y = kernels.quant_matmul_pro(w, packed, nd, ctd, nv.PE_PRO_SILU_MUL, gu, k, n, k, torch.float32, tiles=tiles)
+    assert torch.equal(y, ref)

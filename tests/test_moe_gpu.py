@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import polar_oracle as oracle
-from helpers import max_rel
+from helpers import max_rel, rand_layer, rand_x
 
 pytestmark = pytest.mark.gpu
 
@@ -171,3 +171,73 @@ def test_joint_routing_and_plan_equals_the_two_launches(t, e, k, mapped):
     want = [(x, int(first[x]) + 8 * j, min(8, int(count[x]) - 8 * j)) for x in range(local) for j in range(-(-int(count[x]) // 8))]
     got = [tuple(r[:3]) for r in prob.cpu().tolist()]
     assert got[:len(want)] == want and all(r[2] == 0 for r in got[len(want):])
+
+
+@pytest.mark.parametrize("bits", [3, 4, 5])
+@pytest.mark.parametrize("counts", [(0, 1, 15, 16, 17, 0), (96, 97, 128, 129, 0, 3), (192, 193, 384, 385, 0, 0)])
+def test_grouped_tensor_core_launch_edges(counts, bits):
+    """pe_gemm_grouped and pe_gemm_grouped_silu_mul at the edges of their tiles: empty experts, token counts around 16,
+    around the 96 where a tile's accumulators stop alternating, and around 192 where an expert takes two; out columns
+    that are not whole tiles; rows taken by index."""
+    from polarengine_vllm_b200 import _native as nv, packing
+    n, k, in_f, e, rows, tokens = 2 * 200, 384, 300, len(counts), sum(counts), 64
+    dev, packed = torch.device("cuda"), bits <= 4
+    nv.ensure_init(dev)
+    lib = nv.lib()
+    ws_bytes = lib.pe_gemm_grouped_workspace_bytes(e, rows, n, k)
+    layers = [rand_layer(n, k, bits, seed=bits + i) for i in range(e)]
+    codes = torch.stack([packing.pack_codes_half_block(c.cuda()) if packed else c.cuda() for c, _, _ in layers])
+    norms, ct = torch.stack([m for _, m, _ in layers]).cuda(), layers[0][2].cuda()
+    first = torch.tensor(counts).cumsum(0) - torch.tensor(counts)
+    spans = torch.stack([first, torch.tensor(counts)], 1).int().cuda()
+    x, pick = rand_x(tokens, in_f, seed=1), torch.randint(0, tokens, (rows,), generator=torch.Generator().manual_seed(2))
+    pd, xd, ws = pick.int().cuda(), x.cuda(), torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+    y = torch.full((rows, n), float("nan"), device=dev)
+    act = torch.full((rows, n // 2), float("nan"), dtype=torch.float16, device=dev)
+    head = (codes.data_ptr(), int(packed), codes.stride(1), codes.stride(0), norms.data_ptr(), norms.stride(1), norms.stride(0), ct.data_ptr(),
+            ct.numel(), xd.data_ptr(), nv.PE_X_RAW, nv.dtype_code(xd), xd.stride(0), in_f, pd.data_ptr())
+    tail = (spans.data_ptr(), e, rows, n, k, ws.data_ptr(), ws.numel(), nv.stream_ptr(dev))
+    nv.check(lib.pe_gemm_grouped(*head, y.data_ptr(), nv.PE_F32, n, *tail), "pe_gemm_grouped")
+    nv.check(lib.pe_gemm_grouped_silu_mul(*head, act.data_ptr(), n // 2, *tail), "pe_gemm_grouped_silu_mul")
+    assert int(ws[:4].view(torch.int32)) == 0
+    xr = x[pick]
+    ref = torch.cat([oracle.linear_dequant(xr[int(first[i]):int(first[i]) + c], *layers[i], in_f=in_f) for i, c in enumerate(counts) if c])
+    assert max_rel(y, ref) <= 1e-2
+    assert max_rel(act, torch.nn.functional.silu(ref[:, :n // 2]) * ref[:, n // 2:]) <= 1e-2
+
+
+@pytest.mark.parametrize("bits,inter,h", [(4, 296, 257), (5, 1920, 144)])
+def test_grouped_tiled_silu_input_equals_row_major(bits, inter, h):
+    """pe_gemv_grouped_tiled = pe_gemv_grouped bit for bit, with silu(gate) * up computed where the input is prepared equal
+    to the activation launch in front (ragged widths, problems of 0, 1, 8, 9 and 16 rows)."""
+    from polarengine_vllm_b200 import _native as nv, kernels, packing
+    from polarengine_vllm_b200.decode_ops import silu_mul
+    sizes, kp, dev, packed = (1, 8, 0, 9, 16), -(-inter // 128) * 128, torch.device("cuda"), bits <= 4
+    nv.ensure_init(dev)
+    lib = nv.lib()
+    layers = [rand_layer(h, kp, bits, seed=i) for i in range(len(sizes))]
+    codes = torch.stack([packing.pack_codes_half_block(c.cuda()) if packed else c.cuda() for c, _, _ in layers])
+    norms, ct = torch.stack([m for _, m, _ in layers]).cuda(), layers[0][2].cuda()
+    tiles = torch.cat([kernels.retile(codes[i], packed, norms[i]) for i in range(len(sizes))])
+    rows = sum(sizes)
+    first = [sum(sizes[:i]) for i in range(len(sizes))]
+    prob = torch.tensor([[i, first[i], s, 0] for i, s in enumerate(sizes)], dtype=torch.int32).cuda()
+    gu = rand_x(rows, 2 * inter, seed=3).cuda()
+    act = silu_mul(gu, inter)
+    ws = nv.grouped_scratch(dev, lib.pe_gemv_grouped_workspace_bytes(len(sizes), h, kp))
+    out = []
+    for x, kind in ((act, nv.PE_X_RAW), (gu, nv.PE_X_SILU_MUL)):
+        args = (ct.data_ptr(), ct.numel(), x.data_ptr(), kind, nv.dtype_code(x), x.stride(0), inter, None)
+        for tiled in (False, True):
+            y = torch.zeros(rows, h, device=dev)
+            end = (y.data_ptr(), nv.PE_F32, h, prob.data_ptr(), len(sizes), 16, h, kp, ws.data_ptr(), ws.numel(), nv.stream_ptr(dev))
+            if tiled:
+                nv.check(lib.pe_gemv_grouped_tiled(tiles.data_ptr(), int(packed), tiles.numel() // len(sizes), *args, *end), "tiled")
+            else:
+                nv.check(lib.pe_gemv_grouped(codes.data_ptr(), int(packed), codes.stride(1), codes.stride(0), norms.data_ptr(), norms.stride(1),
+                                             norms.stride(0), *args, *end), "row-major")
+            out.append(y)
+    assert all(torch.equal(out[0], y) for y in out[1:])
+    a = act.cpu()
+    ref = torch.cat([oracle.linear_dequant(a[first[i]:first[i] + s], *layers[i], in_f=inter) for i, s in enumerate(sizes) if s])
+    assert max_rel(out[0], ref) <= 1e-2
