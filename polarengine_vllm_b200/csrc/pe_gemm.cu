@@ -602,23 +602,24 @@ static int small_ksplit(int m, int out_f, int in_f_padded, int sms) {
 }
 
 // Whole and split tiles of a launch over pairs of CTAs.  Fewer tiles than pairs: as many K ranges as there are idle
-// pairs, at least eight K steps each; two ranges only for a long K (the fp32 partials and their sum cost about what halving
-// a short tile saves).  More: the tiles of the last, partly filled wave (rounded up to whole columns of tiles, so that the
-// partials are one matrix) are split over all pairs where that saves more of a tile's ksteps x 0.85 us than the partials
-// cost (up to 18 us).  4096 x 12288 x 4096, 5.2 waves: 382 us as six waves, 368 us.
+// pairs, at least eight K steps each; two ranges from 40 steps on (1024 x 4096 rows, K 4096: 58.4 us whole, 48.6 us split; at
+// K 2048 the fp32 partials and their sum cost what halving the tile saves, 34.0 against 35.4 us).  More: the tiles of the
+// last, partly filled wave (rounded up to whole columns of tiles, so that the partials are one matrix) are split over all
+// pairs where that saves 15 steps of a tile's time or more (600 x 13312 rows, K 2048: 16 saved, 63.2 against 59.5 us;
+// 4096 x 12288, K 4096, 5.2 waves: 382 against 368 us).
 struct PairPlan { int full, ksplit, col0; };
 static PairPlan pair_plan(int tiles_m, int tiles_n, int ksteps, int sms) {
   const int tiles = tiles_m * tiles_n, pairs = sms / 2;
   if (tiles <= pairs) {
     int ks = pairs / tiles;
     if (ks > ksteps / 8) ks = ksteps / 8;
-    if (ks == 2 && ksteps < 128) ks = 1;
+    if (ks == 2 && ksteps < 40) ks = 1;
     return ks < 2 ? PairPlan{tiles, 1, 0} : PairPlan{0, ks, 0};
   }
   const int cols = (tiles % pairs + tiles_m - 1) / tiles_m, rest = cols * tiles_m;
   int ks = rest ? pairs / rest : 1;
   if (ks > ksteps / 8) ks = ksteps / 8;
-  if (ks < 2 || ksteps * (ks - 1) < 40 * ks) return {tiles, 1, 0};
+  if (ks < 2 || ksteps * (ks - 1) < 15 * ks) return {tiles, 1, 0};
   return {tiles - rest, ks, (tiles_n - cols) * kTileN};
 }
 
