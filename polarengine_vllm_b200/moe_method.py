@@ -165,7 +165,7 @@ class PolarQuantMoEMethod:
             return None
         n_local = layer.w13_codes.shape[0]
         pairs = x.numel() // layer.moe_hidden * top_k
-        plan = self._grouped_plan(pairs, n_local, expert_map)
+        plan = self._grouped_plan(pairs, n_local, expert_map, layer.moe_hidden_padded // 128)
         if plan is None:
             return None
         rpp, max_problems, tensor_cores = plan
@@ -176,15 +176,20 @@ class PolarQuantMoEMethod:
             (layer.w2_codes, layer.w2_norms, layer.w2_ct_scaled, layer.w2_tiles if tiled else None, self.w2_bits <= 4),
             (layer.moe_hidden, layer.moe_inter, layer.moe_hidden_padded, layer.moe_inter_padded), rpp, max_problems, tensor_cores)
 
-    def _grouped_plan(self, pairs: int, n_local: int, expert_map) -> Optional[Tuple[int, int, bool]]:
+    def _grouped_plan(self, pairs: int, n_local: int, expert_map, blocks: int) -> Optional[Tuple[int, int, bool]]:
         """(rows per problem, problem slots, tensor cores) of the grouped launches for that many (token, expert) pairs;
-        None when every expert has enough rows to fill the tensor-core kernel by itself."""
+        ``blocks``: 128-blocks of the first projection's K.  None when every expert has enough rows to fill the tensor-core
+        kernel by itself."""
         local_pairs = self.expected_local_pairs(pairs, n_local, expert_map)
         if pairs < 1 or local_pairs > self.GROUPED_MAX_ROWS_PER_EXPERT * n_local:
             return None
-        # rows per problem: 8 while experts see few tokens (lighter kernel), else 16
-        rpp = 8 if local_pairs <= 6 * n_local else 16
-        return rpp, min(n_local, pairs) + pairs // rpp, local_pairs >= self.TENSOR_CORE_MIN_ROWS_PER_EXPERT * n_local
+        tensor_cores = local_pairs >= self.TENSOR_CORE_MIN_ROWS_PER_EXPERT * n_local
+        # Rows per problem: 8 while experts see few tokens (lighter kernel), else 16.  For 16 rows a CTA takes 16 blocks of K
+        # per round: where a last round leaves a quarter of those places empty, problems of 8 stay ahead up to the
+        # tensor cores' range (8 rows for each of 128 experts, 21 blocks: 474 us against 592; 16 blocks: 94 against 91).
+        ragged = blocks > 16 and blocks <= 0.75 * 16 * -(-blocks // 16)
+        rpp = 8 if local_pairs <= 6 * n_local or (ragged and not tensor_cores) else 16
+        return rpp, min(n_local, pairs) + pairs // rpp, tensor_cores
 
     # average (token, expert) pairs per local expert up to which the grouped launches are
     # used; beyond it every expert has enough rows to fill the tensor-core kernel by itself
@@ -248,7 +253,7 @@ class PolarQuantMoEMethod:
         pairs = t * k
         ids = topk_ids.reshape(-1).to(torch.int64).contiguous()
         emap = expert_map.to(device=dev, dtype=torch.int64).contiguous() if expert_map is not None else None
-        plan = self._grouped_plan(pairs, n_local, expert_map)
+        plan = self._grouped_plan(pairs, n_local, expert_map, layer.moe_hidden_padded // 128)
         if plan is None:
             return None
         rpp, max_problems, tensor_cores = plan
