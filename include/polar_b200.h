@@ -239,10 +239,12 @@ int pe_gemm_grouped(const void* codes, int packed, int64_t ld_codes, int64_t cod
                     void* workspace, size_t workspace_bytes, void* stream);
 
 /* The same for gate and up projections: the first out_f / 2 rows of an expert are the gate and the rest the up
- * projection, and y (fp16, out_f / 2 columns) gets silu(gate) * up (nemotron_offload.py:205-209). */
+ * projection, and y (fp16, out_f / 2 columns) gets silu(gate) * up (nemotron_offload.py:205-209).  x has n_x rows, and
+ * row i of it is the input of the list's rows x_to[i * fanout] .. x_to[i * fanout + fanout - 1] (negative: of none): the
+ * `pos` output of pe_moe_plan with fanout = top_k.  n_x * fanout <= rows. */
 int pe_gemm_grouped_silu_mul(const void* codes, int packed, int64_t ld_codes, int64_t codes_stride, const void* norms,
                              int64_t ld_norms, int64_t norms_stride, const float* ct_scaled, int n_levels, const void* x,
-                             int x_kind, int x_dtype, int64_t ld_x, int in_f, const int32_t* x_rows, void* y, int64_t ld_y,
+                             int x_kind, int x_dtype, int64_t ld_x, int in_f, const int32_t* x_to, int n_x, int fanout, void* y, int64_t ld_y,
                              const int32_t* expert_rows, int n_experts, int rows, int out_f, int in_f_padded,
                              void* workspace, size_t workspace_bytes, void* stream);
 

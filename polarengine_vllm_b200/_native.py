@@ -46,7 +46,7 @@ SIGNATURES = {
     "pe_gemm_grouped_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "pe_gemm_grouped": (_i, [_vp, _i, _i64, _i64, _vp, _i64, _i64, _vp, _i, _vp, _i, _i, _i64, _i, _vp, _vp, _i, _i64, _vp,
                             _i, _i, _i, _i, _vp, _sz, _vp]),
-    "pe_gemm_grouped_silu_mul": (_i, [_vp, _i, _i64, _i64, _vp, _i64, _i64, _vp, _i, _vp, _i, _i, _i64, _i, _vp, _vp, _i64, _vp,
+    "pe_gemm_grouped_silu_mul": (_i, [_vp, _i, _i64, _i64, _vp, _i64, _i64, _vp, _i, _vp, _i, _i, _i64, _i, _vp, _i, _i, _vp, _i64, _vp,
                                      _i, _i, _i, _i, _vp, _sz, _vp]),
     "pe_moe_combine": (_i, [_vp, _i64, _vp, _vp, _i, _i, _vp, _i, _i64, _i, _vp]),
     "pe_allreduce_buffer_bytes": (_sz, [_i, _i, _i]),

@@ -667,7 +667,7 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
 
   int* status = static_cast<int*>(workspace);
   uint8_t* xq = static_cast<uint8_t*>(workspace) + 256;
-  int rc = launch_gemm_prep(x, x_kind, x_dtype, ld_x, in_f, xq, m, in_f_padded, packed ? 1 : 0, nullptr, nullptr, status, st);
+  int rc = launch_gemm_prep(x, x_kind, x_dtype, ld_x, in_f, xq, m, in_f_padded, packed ? 1 : 0, nullptr, nullptr, nullptr, 0, status, st);
   if (rc != PE_OK) return rc;
   // few tiles: split K when the caller's workspace has room for the partials
   const size_t part_off = (pe_gemm_workspace_bytes(m, in_f_padded) + 255) & ~(size_t)255;

@@ -123,7 +123,7 @@ __device__ __forceinline__ RegTable bf16_reg_table(const float* ct, int n_levels
 
 // ---- host side (pe_gemm_prep.cu) ----
 int launch_gemm_prep(const void* x, int x_kind, int x_dtype, int64_t ld_x, int in_f, void* xq, int rows, int in_f_padded, int pair_layout,
-                     const int* x_rows, const int* valid_rows, int* status, cudaStream_t st);
+                     const int* x_rows, const int* valid_rows, const int* to_rows, int fanout, int* status, cudaStream_t st);
 int launch_splitk_reduce(const float* part, int ksplit, int m, int n, const void* bias, void* y, int y_dtype, int64_t ld_y, int sms, cudaStream_t st);
 int encode_map_f32(CUtensorMap* map, const void* base, uint64_t width, uint64_t height, uint64_t depth, uint64_t row_bytes);
 int encode_map_2d(CUtensorMap* map, CUtensorMapDataType type, const void* base, uint64_t width, uint64_t height, uint64_t row_bytes, uint32_t box_w,

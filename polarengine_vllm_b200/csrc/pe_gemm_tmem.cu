@@ -531,7 +531,7 @@ extern "C" size_t pe_gemm_grouped_workspace_bytes(int n_experts, int rows, int o
 
 static int grouped(const void* codes, int packed, int64_t ld_codes, int64_t codes_stride, const void* norms, int64_t ld_norms, int64_t norms_stride,
                    const float* ct_scaled, int n_levels, const void* x, int x_kind, int x_dtype, int64_t ld_x, int in_f, const int32_t* x_rows,
-                   int silu_mul, void* y, int y_dtype, int64_t ld_y, const int32_t* expert_rows, int n_experts, int rows, int out_f,
+                   const int32_t* x_to, int n_x, int fanout, int silu_mul, void* y, int y_dtype, int64_t ld_y, const int32_t* expert_rows, int n_experts, int rows, int out_f,
                    int in_f_padded, void* workspace, size_t workspace_bytes, void* stream) {
   if (!codes || !norms || !ct_scaled || !x || !y || !expert_rows || !workspace) return PE_ERR_ARG;
   if (n_experts < 1 || rows < 1 || out_f < 1 || in_f < 1 || in_f > in_f_padded) return PE_ERR_ARG;
@@ -566,8 +566,8 @@ static int grouped(const void* codes, int packed, int64_t ld_codes, int64_t code
   const int tile_rows = silu_mul ? 128 : 256, tiles_n = (y_cols + tile_rows - 1) / tile_rows;
   PE_CUDA_TRY(launch_pdl(gemm_tile_list_kernel, dim3(1), dim3(1024), 0, st, expert_rows, n_experts, tiles_n, tile_rows, max_tiles, tiles, n_tiles));
   // (the preparation kernel clears the status word)
-  const int rc = launch_gemm_prep(x, x_kind, x_dtype, ld_x, in_f, xq, rows, in_f_padded, packed ? 1 : 0, x_rows, expert_rows + 2 * (n_experts - 1),
-                                  status, st);
+  const int rc = launch_gemm_prep(x, x_kind, x_dtype, ld_x, in_f, xq, x_to ? n_x : rows, in_f_padded, packed ? 1 : 0, x_rows,
+                                  x_to ? nullptr : expert_rows + 2 * (n_experts - 1), x_to, fanout, status, st);
   if (rc != PE_OK) return rc;
 
   TmemGemmArgs a = {};
@@ -588,15 +588,16 @@ extern "C" int pe_gemm_grouped(const void* codes, int packed, int64_t ld_codes, 
                                int x_kind, int x_dtype, int64_t ld_x, int in_f, const int32_t* x_rows, void* y, int y_dtype,
                                int64_t ld_y, const int32_t* expert_rows, int n_experts, int rows, int out_f, int in_f_padded,
                                void* workspace, size_t workspace_bytes, void* stream) {
-  return grouped(codes, packed, ld_codes, codes_stride, norms, ld_norms, norms_stride, ct_scaled, n_levels, x, x_kind, x_dtype, ld_x, in_f, x_rows, 0, y,
+  return grouped(codes, packed, ld_codes, codes_stride, norms, ld_norms, norms_stride, ct_scaled, n_levels, x, x_kind, x_dtype, ld_x, in_f, x_rows, nullptr, 0, 0, 0, y,
                  y_dtype, ld_y, expert_rows, n_experts, rows, out_f, in_f_padded, workspace, workspace_bytes, stream);
 }
 
 extern "C" int pe_gemm_grouped_silu_mul(const void* codes, int packed, int64_t ld_codes, int64_t codes_stride, const void* norms,
                                         int64_t ld_norms, int64_t norms_stride, const float* ct_scaled, int n_levels, const void* x,
-                                        int x_kind, int x_dtype, int64_t ld_x, int in_f, const int32_t* x_rows, void* y,
+                                        int x_kind, int x_dtype, int64_t ld_x, int in_f, const int32_t* x_to, int n_x, int fanout, void* y,
                                         int64_t ld_y, const int32_t* expert_rows, int n_experts, int rows, int out_f, int in_f_padded,
                                         void* workspace, size_t workspace_bytes, void* stream) {
-  return grouped(codes, packed, ld_codes, codes_stride, norms, ld_norms, norms_stride, ct_scaled, n_levels, x, x_kind, x_dtype, ld_x, in_f, x_rows, 1, y,
+  if (!x_to || n_x < 1 || fanout < 1 || (int64_t)n_x * fanout > rows) return PE_ERR_ARG;
+  return grouped(codes, packed, ld_codes, codes_stride, norms, ld_norms, norms_stride, ct_scaled, n_levels, x, x_kind, x_dtype, ld_x, in_f, nullptr, x_to, n_x, fanout, 1, y,
                  PE_F16, ld_y, expert_rows, n_experts, rows, out_f, in_f_padded, workspace, workspace_bytes, stream);
 }

@@ -244,8 +244,8 @@ struct Experts {
 };
 struct MoePlan {
   int64_t pairs, n_local, max_problems;
-  int rows_per_problem;
-  const int32_t *problems, *expert_rows;
+  int rows_per_problem, top_k;
+  const int32_t *problems, *expert_rows, *pos;
   bool tensor_cores;
 };
 
@@ -264,7 +264,8 @@ int grouped(const Experts& w, const MoePlan& p, const at::Device& dev, cudaStrea
     const at::Tensor ws = take_scratch(dev, st, 1, api.gemm_grouped_bytes((int)p.n_local, (int)p.pairs, out_f, in_f_padded), false);
     if (silu_mul)
       return api.gemm_silu_mul(w.codes->const_data_ptr(), w.packed, w.codes->stride(1), w.codes->stride(0), w.norms->const_data_ptr(),
-                               w.norms->stride(1), w.norms->stride(0), ct, levels, x, kind, xd, ld_x, in_f, x_rows, y, out_f / 2, p.expert_rows,
+                               w.norms->stride(1), w.norms->stride(0), ct, levels, x, kind, xd, ld_x, in_f, p.pos, (int)(p.pairs / p.top_k), p.top_k, y,
+                               out_f / 2, p.expert_rows,
                                (int)p.n_local, (int)p.pairs, out_f, in_f_padded, ws.mutable_data_ptr(), ws.numel(), st);
     return api.gemm_grouped(w.codes->const_data_ptr(), w.packed, w.codes->stride(1), w.codes->stride(0), w.norms->const_data_ptr(),
                             w.norms->stride(1), w.norms->stride(0), ct, levels, x, kind, xd, ld_x, in_f, x_rows, y, yd, out_f, p.expert_rows,
@@ -339,6 +340,8 @@ PyObject* host_moe(PyObject*, PyObject* const* args, Py_ssize_t n) {
   int32_t *rows = reinterpret_cast<int32_t*>(base + at_rows), *tok = reinterpret_cast<int32_t*>(base + at_tok), *pos = reinterpret_cast<int32_t*>(base + at_pos);
   p.problems = problems;
   p.expert_rows = rows;
+  p.pos = pos;
+  p.top_k = top_k;
   const float* weights = given ? a->const_data_ptr<float>() : reinterpret_cast<float*>(base + at_w);
   const int64_t* ids = given ? given->const_data_ptr<int64_t>() : reinterpret_cast<int64_t*>(base + at_ids);
   int rc = PE_OK;

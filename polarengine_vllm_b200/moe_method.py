@@ -281,12 +281,12 @@ class PolarQuantMoEMethod:
                 ws = nv.gemm_workspace(dev, need)
                 head = (codes.data_ptr(), int(packed), codes.stride(1) * codes.element_size(), codes.stride(0) * codes.element_size(),
                         norms.data_ptr(), norms.stride(1), norms.stride(0), ct.data_ptr(), ct.numel(), xin.data_ptr(), nv.PE_X_RAW,
-                        nv.dtype_code(xin), xin.stride(0), in_f, x_rows.data_ptr() if x_rows is not None else None, y.data_ptr())
+                        nv.dtype_code(xin), xin.stride(0), in_f)
                 tail = (y.stride(0), expert_rows.data_ptr(), n_local, pairs, codes.shape[1], kp, ws.data_ptr(), ws.numel(), st)
                 if x_rows is not None:
-                    nv.check(l.pe_gemm_grouped_silu_mul(*head, *tail), "pe_gemm_grouped_silu_mul")
+                    nv.check(l.pe_gemm_grouped_silu_mul(*head, pos.data_ptr(), t, k, y.data_ptr(), *tail), "pe_gemm_grouped_silu_mul")
                 else:
-                    nv.check(l.pe_gemm_grouped(*head, nv.dtype_code(y), *tail), "pe_gemm_grouped")
+                    nv.check(l.pe_gemm_grouped(*head, None, y.data_ptr(), nv.dtype_code(y), *tail), "pe_gemm_grouped")
                 return
             ws = nv.grouped_scratch(dev, l.pe_gemv_grouped_workspace_bytes(max_problems, y.shape[1], kp))
             if tiled:

@@ -178,7 +178,7 @@ def test_joint_routing_and_plan_equals_the_two_launches(t, e, k, mapped):
 def test_grouped_tensor_core_launch_edges(counts, bits):
     """pe_gemm_grouped and pe_gemm_grouped_silu_mul at the edges of their tiles: empty experts, token counts around 16,
     around the 96 where a tile's accumulators stop alternating, and around 192 where an expert takes two; out columns
-    that are not whole tiles; rows taken by index."""
+    that are not whole tiles; rows taken by index, and rows sent to theirs."""
     from polarengine_vllm_b200 import _native as nv, packing
     n, k, in_f, e, rows, tokens = 2 * 200, 384, 300, len(counts), sum(counts), 64
     dev, packed = torch.device("cuda"), bits <= 4
@@ -194,11 +194,15 @@ def test_grouped_tensor_core_launch_edges(counts, bits):
     pd, xd, ws = pick.int().cuda(), x.cuda(), torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
     y = torch.full((rows, n), float("nan"), device=dev)
     act = torch.full((rows, n // 2), float("nan"), dtype=torch.float16, device=dev)
+    # the list as scattered rows of another order: row i of `xs` is row to[i] of the list
+    to = torch.randperm(rows, generator=torch.Generator().manual_seed(3))
+    xs, td = x[pick][to].contiguous().cuda(), to.int().cuda()
     head = (codes.data_ptr(), int(packed), codes.stride(1), codes.stride(0), norms.data_ptr(), norms.stride(1), norms.stride(0), ct.data_ptr(),
-            ct.numel(), xd.data_ptr(), nv.PE_X_RAW, nv.dtype_code(xd), xd.stride(0), in_f, pd.data_ptr())
+            ct.numel())
+    raw = (nv.PE_X_RAW, nv.dtype_code(xd), xd.stride(0), in_f)
     tail = (spans.data_ptr(), e, rows, n, k, ws.data_ptr(), ws.numel(), nv.stream_ptr(dev))
-    nv.check(lib.pe_gemm_grouped(*head, y.data_ptr(), nv.PE_F32, n, *tail), "pe_gemm_grouped")
-    nv.check(lib.pe_gemm_grouped_silu_mul(*head, act.data_ptr(), n // 2, *tail), "pe_gemm_grouped_silu_mul")
+    nv.check(lib.pe_gemm_grouped(*head, xd.data_ptr(), *raw, pd.data_ptr(), y.data_ptr(), nv.PE_F32, n, *tail), "pe_gemm_grouped")
+    nv.check(lib.pe_gemm_grouped_silu_mul(*head, xs.data_ptr(), *raw, td.data_ptr(), rows, 1, act.data_ptr(), n // 2, *tail), "pe_gemm_grouped_silu_mul")
     assert int(ws[:4].view(torch.int32)) == 0
     xr = x[pick]
     ref = torch.cat([oracle.linear_dequant(xr[int(first[i]):int(first[i]) + c], *layers[i], in_f=in_f) for i, c in enumerate(counts) if c])
