@@ -319,7 +319,7 @@ def model_record(a, dev, rank, world, batches=(1, 8)):
     rec["row_parallel_epilogue"] = note
     for b in batches:
         rec[f"batch{b}"] = decode_run(model, dev, rank, world, b, a.prompt, a.new_tokens, not a.no_graph)
-    rec["gpu_launches_per_step"] = 8 * a.layers + 3
+    rec["gpu_launches_per_step"] = 9 * a.layers + 3
     del model
     torch.cuda.empty_cache()
     return rec
@@ -404,7 +404,8 @@ def moe_run(dev, rank, world, tokens, steps=None):
            "hbm_frac_of_measured": active * per_expert / (ms / 1e3) / 1e9 / float(peaks.get("hbm_gbs", 6650.0)) / world,
            "tflops": flops / (ms / 1e3) / 1e12,
            "tensor_frac_of_burst": flops / (ms / 1e3) / 1e12 / float(peaks.get("bf16_tflops", 1590.0)) / world,
-           "gpu_launches": steps * (5 if grouped else 2 * min(active, e_local))}
+           # routing, plan, two matmuls with their activation launch, combine; tensor cores: a tile list each
+           "gpu_launches": steps * ((9 if tensor else 7) if grouped else 2 * min(active, e_local))}
     if graph is not None:
         graph.reset()
     return rec
