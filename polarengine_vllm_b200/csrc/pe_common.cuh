@@ -28,7 +28,9 @@ long long wait_limit_cycles();  // limit of device-side waits on another party (
 
 // Launch with programmatic stream serialization: the grid may start while its predecessor
 // in the stream is still draining.  The kernel must call pdl_enter() (or its own
-// griddepcontrol.wait) before it touches anything the predecessor reads or writes.
+// griddepcontrol.wait) before it touches anything the predecessor reads or writes.  That wait covers the predecessor
+// alone: a kernel that reads weights before it must be launched behind one that waits before it lets its dependents start
+// (gemm_prep_kernel, gemv_frags_kernel), or writes of kernels further back may not be visible.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg = {};

@@ -5,8 +5,8 @@
 // One persistent CTA per SM: sixteen math warps and one copy warp.  A stage of the shared-memory ring is one 16-row
 // tile of the weight matrix by up to 32 quantization blocks; the copy warp fills stages with bulk copies (one per
 // stage from the tiled layout of pe_retile, whose records are contiguous; one per weight row from the row-major
-// layout) long before the activations exist: everything up to the ring's size is on its way before the dependency
-// wait of the programmatic launch returns.  (Without a copy warp -- the last warp to finish with a stage refills it,
+// layout) while the activations are prepared: the dependency wait of the programmatic launch is the math warps' alone
+// (gemv_frags_kernel lets this kernel start once the launches before both are done).  (Without a copy warp -- the last warp to finish with a stage refills it,
 // 128 instead of 96 registers -- the refills came later and every warp had to track them: 4 us over four launches.)
 //
 // What bounds it: once the ring runs, the shared-memory port.  A warp takes block cw, cw + 16 of every stage:
@@ -202,8 +202,10 @@ __device__ __forceinline__ void residual4(const FragArgs& p, const Raw4& x, cons
 
 template <bool PACKED, bool NORM>
 __global__ void __launch_bounds__(kFragThreads) gemv_frags_kernel(const FragArgs p) {
-  asm volatile("griddepcontrol.launch_dependents;");
+  // The wait first: the matmul behind reads codes, norms and table before its own wait, which covers this launch only, so
+  // what older kernels wrote (a layer just loaded, arrays rewritten in place) has to be visible before it may start.
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
   const int lane = threadIdx.x & 31, job = blockIdx.x * (kFragThreads / 32) + (threadIdx.x >> 5);
   const int m = job / p.nb, b = job - m * p.nb, prob = blockIdx.y;
   if (!NORM && m >= p.batch) return;

@@ -118,7 +118,10 @@ __global__ void __launch_bounds__(kRowThreads, 1) gemv_cols_kernel(const ColArgs
   int cnt = (p.n_chunks - w + kRowWarps - 1) / kRowWarps;  // chunks w, w+16, ... of this warp
   cnt = cnt < 0 ? 0 : (cnt > CPW ? CPW : cnt);
 
+  // The wait before the first read: codes, norms and table may be the output of a kernel that is still running (a layer just
+  // loaded, arrays rewritten in place), and the launch in front may have let this one start before it.
   asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   float ct_mine = 0.f;
   {
     const int e = PACKED ? (lane & 15) : (w + 16 * (lane & 15));
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) gemv_cols_kernel(const ColArgs
   }
 
 
-  // ---- centroid table (built before the dependency wait: it needs nothing from the previous kernel)
+  // ---- centroid table
   RegTable tb = {0, 0, 0, 0};
   if (PACKED && REGTAB) {
 #pragma unroll
@@ -197,7 +200,6 @@ __global__ void __launch_bounds__(kRowThreads, 1) gemv_cols_kernel(const ColArgs
 
   // ---- this warp's activation slices: load, rotate, bounce through the warp's scratch
   // into the item layout, keep in registers
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   uint32_t xr[CPW][kXPerChunk];
   {
     const bool raw = p.x_kind == PE_X_RAW;

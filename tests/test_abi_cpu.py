@@ -84,3 +84,21 @@ def test_size_queries_of_the_grouped_and_exchange_entry_points():
     assert lib.pe_moe_plan(None, None, 0, 8, 2, 4, 8, 8, None, None, None, None, None) == -1
     assert lib.pe_add_rmsnorm(None, None, 1, None, None, 1, 4096, 1e-6, None) == -1
     assert lib.pe_allreduce_add_rmsnorm(None, None, None, None, 1, 4096, 1e-6, None, 0, 1, 1, None, None, None) == -1
+
+
+def _body(source: str, kernel: str) -> str:
+    """Text of a __global__ function of csrc, from its name to the closing brace in the first column."""
+    text = open(os.path.join(ROOT, "polarengine_vllm_b200", "csrc", source)).read()
+    start = re.search(r"\b%s\s*\([^;{]*\)\s*\{" % kernel, text).start()
+    return text[start:text.index("\n}", start)]
+
+
+def test_kernels_see_weights_that_older_kernels_wrote():
+    """A programmatic launch may run before the launches in front of it have finished, and its dependency wait covers the
+    one directly in front only.  Kernels that read weights before their wait run behind a preparation kernel: that one
+    has to wait before it lets them start.  A kernel with no preparation in front has to wait before it reads."""
+    for source, kernel in (("pe_gemv_bulk.cu", "gemv_frags_kernel"), ("pe_gemm_prep.cu", "gemm_prep_kernel")):
+        body = _body(source, kernel)
+        assert 0 <= body.find("griddepcontrol.wait") < body.rfind("griddepcontrol.launch_dependents"), kernel
+    body = _body("pe_gemv_cols.cu", "gemv_cols_kernel")
+    assert 0 <= body.find("griddepcontrol.wait") < min(body.find("ld.global"), body.find("fetch_item(st_base"))

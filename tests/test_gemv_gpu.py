@@ -303,3 +303,29 @@ def test_folded_prologue_over_the_tiled_copy(bits, n, k):
     ref = _gemv_tiled_direct(tiles, packed, ctd, silu_mul(gu, k), n, k, k)
     y = kernels.quant_matmul_pro(w, packed, nd, ctd, nv.PE_PRO_SILU_MUL, gu, k, n, k, torch.float32, tiles=tiles)
     assert torch.equal(y, ref)
+
+
+@pytest.mark.parametrize("rows", [1, 4, 16, 17])
+@pytest.mark.parametrize("bits", [4, 5])
+def test_weights_rewritten_by_the_kernel_in_front(bits, rows):
+    """Codes and norms rewritten on the device right before the call, inside one captured graph: every call multiplies by
+    the arrays of its moment (the launches overlap their predecessors, so an early read would see the old ones)."""
+    from polarengine_vllm_b200 import kernels, packing
+    n, k = 4096, 4096
+    packed = bits <= 4
+    sets = []
+    for seed in (1, 2):
+        codes, norms, ct = rand_layer(n, k, bits, seed=seed)
+        sets.append((packing.pack_codes_half_block(codes.cuda()) if packed else codes.cuda(), norms.cuda()))
+    ctd, x = ct.cuda(), rand_x(rows, k, seed=3).cuda()
+    want = [kernels.quant_matmul(w, packed, m, ctd, x, False, n, k, k, torch.float32) for w, m in sets]
+    w, m = sets[0][0].clone(), sets[0][1].clone()
+    kernels.quant_matmul(w, packed, m, ctd, x, False, n, k, k, torch.float32)
+    graph, got = torch.cuda.CUDAGraph(), []
+    with torch.cuda.graph(graph):
+        for i in range(40):
+            torch.add(sets[i % 2][0], 0, out=w)  # a kernel, not a copy node
+            torch.mul(sets[i % 2][1], 1, out=m)
+            got.append(kernels.quant_matmul(w, packed, m, ctd, x, False, n, k, k, torch.float32))
+    graph.replay()
+    assert all(torch.equal(y, want[i % 2]) for i, y in enumerate(got))
