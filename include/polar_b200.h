@@ -182,8 +182,7 @@ size_t pe_gemv_workspace_bytes(int batch, int out_f, int in_f_padded);
 int pe_gemv_status(void* workspace, size_t workspace_bytes, int clear, void* stream);
 
 /* 1 if pe_gemv runs batches of 3..8 rows of this layer as fast on its row-major arrays as pe_gemv_tiled does on the
- * tiled copy (pe_retile), 0 if the copy is worth having.  It is for every layer: one contiguous bulk copy per stage
- * instead of sixteen.  No launch, no device access. */
+ * tiled copy (pe_retile), 0 if the copy is worth having.  1 for every layer.  No launch, no device access. */
 int pe_gemv_small_batch_takes(int packed, int64_t ld_codes, const void* norms, int64_t ld_norms, int out_f,
                               int in_f_padded);
 int pe_gemv(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms,
@@ -355,8 +354,12 @@ int pe_gemv_pro(const void* codes, int packed, int64_t ld_codes, const void* nor
                 int delta_dtype, const void* norm_weight, void* resid_out, float eps, void* y, int y_dtype,
                 const void* bias, int out_f, int in_f_padded, void* stream);
 
-/* The same on a tiled copy of the layer (pe_retile), any shape: the glue op is computed where the activations are
- * prepared.  Scratch as for pe_gemv with one row. */
+/* The same with scratch as for pe_gemv with one row, any shape, on the row-major arrays or on a tiled copy of the layer
+ * (pe_retile): the glue op is computed where the activations are prepared. */
+int pe_gemv_pro_scratch(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms, const float* ct_scaled,
+                        int n_levels, int prologue, const void* x, int in_f, const void* delta, int delta_dtype,
+                        const void* norm_weight, void* resid_out, float eps, void* y, int y_dtype, const void* bias, int out_f,
+                        int in_f_padded, void* workspace, size_t workspace_bytes, void* stream);
 int pe_gemv_pro_tiled(const void* tiles, int packed, const float* ct_scaled, int n_levels, int prologue, const void* x, int in_f,
                       const void* delta, int delta_dtype, const void* norm_weight, void* resid_out, float eps, void* y,
                       int y_dtype, const void* bias, int out_f, int in_f_padded, void* workspace, size_t workspace_bytes,

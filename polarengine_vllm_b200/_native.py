@@ -65,6 +65,7 @@ SIGNATURES = {
     "pe_decode_attention_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "pe_decode_attention": (_i, [_vp, _vp, _vp, _vp, _i64, _vp, _i, _i, _i, _i, _i, _vp, _sz, _vp]),
     "pe_gemv_pro": (_i, [_vp, _i, _i64, _vp, _i64, _vp, _i, _i, _vp, _i, _vp, _i, _vp, _vp, ctypes.c_float, _vp, _i, _vp, _i, _i, _vp]),
+    "pe_gemv_pro_scratch": (_i, [_vp, _i, _i64, _vp, _i64, _vp, _i, _i, _vp, _i, _vp, _i, _vp, _vp, ctypes.c_float, _vp, _i, _vp, _i, _i, _vp, _sz, _vp]),
     "pe_gemv_pro_tiled": (_i, [_vp, _i, _vp, _i, _i, _vp, _i, _vp, _i, _vp, _vp, ctypes.c_float, _vp, _i, _vp, _i, _i, _vp, _sz, _vp]),
     "pe_gemv_status": (_i, [_vp, _sz, _i, _vp]),
     "pe_gemv_small_batch_takes": (_i, [_i, _i64, _vp, _i64, _i, _i]),

@@ -2,9 +2,9 @@
 //
 //   y[m, r] = sum_blk norm[r, blk] * sum_k ct[code[r, blk, k]] * xt[m, blk, k]   (+ bias[r])
 //
-// One activation row over row-major codes goes to the column-owner kernel (pe_gemv_cols.cu: 47.2 us for a decoder
-// layer's four launches, 51 us for the bulk-copy kernel on that layout); everything else, one row over the tiled copy
-// (42.6 us) included, to the bulk-copy kernel (pe_gemv_bulk.cu).
+// Every call goes to the bulk-copy kernel (pe_gemv_bulk.cu), whichever layout it has: a decoder layer's four launches for
+// one row take 48.5 us on row-major arrays, 48.2 us on the tiled copy, and 52.0 us in the column-owner kernel
+// (pe_gemv_cols.cu), which is left for pe_gemv_pro, whose callers give no scratch memory.
 #include "pe_gemv_decode.cuh"
 
 namespace pe {
@@ -68,11 +68,6 @@ static int gemv_dispatch(const void* codes, int packed, int64_t ld_codes, const 
   if (workspace_bytes < kCounterBytes + gemv_bulk_frag_bytes(1, batch, in_f_padded)) return PE_ERR_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(workspace) & 15) return PE_ERR_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (!tiles && batch == 1) {
-    const int r = gemv_cols_run(codes, packed, ld_codes, norms, ld_norms, ct_scaled, n_levels, x, x_kind, x_dtype, in_f, y, y_dtype, bias,
-                                out_f, in_f_padded, st);
-    if (r <= 0) return r;
-  }
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   GemvBulkCall q = {};
   q.codes = codes; q.packed = packed; q.ld_codes = ld_codes; q.norms = norms; q.ld_norms = ld_norms; q.tiles = tiles;
@@ -97,8 +92,8 @@ static int gemv_run(const void* codes, int packed, int64_t ld_codes, const void*
                        bias, batch, out_f, in_f_padded, workspace, workspace_bytes, stream);
 }
 
-// Batches of 2..16 rows stream the tiled copy fastest whatever the layer's shape.
-extern "C" int pe_gemv_small_batch_takes(int, int64_t, const void*, int64_t, int, int) { return 0; }
+// The row-major arrays stream as fast as the tiled copy (8 rows, a decoder layer's four launches: 51.2 and 51.8 us).
+extern "C" int pe_gemv_small_batch_takes(int, int64_t, const void*, int64_t, int, int) { return 1; }
 
 extern "C" int pe_gemv(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms,
                        const float* ct_scaled, int n_levels, const void* x, int x_kind, int x_dtype, int64_t ld_x,

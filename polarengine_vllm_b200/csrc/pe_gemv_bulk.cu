@@ -2,12 +2,16 @@
 //
 //   y[m, r] = sum_blk norm[r, blk] * sum_k ct[code[r, blk, k]] * xt[m, blk, k]   (+ bias[r])
 //
-// One persistent CTA per SM: sixteen math warps and one copy warp.  A stage of the shared-memory ring is one 16-row
-// tile of the weight matrix by up to 32 quantization blocks; the copy warp fills stages with bulk copies (one per
-// stage from the tiled layout of pe_retile, whose records are contiguous; one per weight row from the row-major
-// layout) while the activations are prepared: the dependency wait of the programmatic launch is the math warps' alone
-// (gemv_frags_kernel lets this kernel start once the launches before both are done).  (Without a copy warp -- the last warp to finish with a stage refills it,
-// 128 instead of 96 registers -- the refills came later and every warp had to track them: 4 us over four launches.)
+// One persistent CTA per SM: sixteen math warps, a copy warp and, for row-major codes, a norm warp.  A stage of the shared-
+// memory ring is one 16-row tile of the weight matrix by up to 32 quantization blocks.  The copy warp fills stages with bulk
+// copies (of the row-major layout one or a few rows each, of the tiled layout of pe_retile, whose records are contiguous, one
+// per stage); norms of row-major layers are a strided gather of halves that no bulk copy does, so the norm warp loads them
+// (two stages under way) and stores them beside the codes.  Both start while the activations are prepared: the dependency wait
+// of the programmatic launch is the math warps' alone (gemv_frags_kernel lets this kernel start once the launches before both
+// are done).  (Without a copy warp -- the last warp to finish with a stage refills it, 128 instead of 96 registers -- the
+// refills came later and every warp had to track them: 4 us over four launches.  Norms loaded by the math warps at the head of
+// every pass: 8 us.  Two or three norm warps that take stages in turn are unsound: a wait on a barrier's parity holds only for
+// a waiter that took every earlier phase itself.)
 //
 // What bounds it: once the ring runs, the shared-memory port.  A warp takes block cw, cw + 16 of every stage:
 //  * centroid lookup: the table is replicated per lane at a spacing of 256 bytes per entry, so that ONE byte permute
@@ -23,26 +27,23 @@
 //    them in registers.  Rotating inside this kernel was measured too (in registers, 16-point part by MMAs): its
 //    straight-line code cost more in instruction fetches than the extra launch, 13 us over a layer's four launches.
 //    The registers left over let the small launch's blocks be resident, waiting, while the launch before it still runs.
-// Measured, tiled layout, launches of a dependent chain under a CUDA graph, weights from HBM (in brackets the kernels
-// this one replaced, which split K over CTAs or rows over warps and staged codes with per-lane copies):
+// Measured, row-major layout, launches of a dependent chain under a CUDA graph, weights from HBM (in brackets the tiled layout):
 //   activation rows      1              8              16
-//   6144 x 4096 Q5    10.3 (10.4)    10.0 (16.5)    13.8 (31.3) us
-//   4096 x 4096 Q6     7.7  (8.0)     8.1 (13.6)     9.6 (29.4)
-//   24576 x 4096 Q3   14.7 (16.9)    16.9 (24.8)    28.0 (56.5)
-//   4096 x 12288 Q4   10.5 (13.5)    11.5 (28.8)    15.9 (41.2)
-//   the four in turn  42.6 (47.2)    46.4 (86.9)    66.7 (171)
-// Inside the ring's steady state the 24576 x 4096 launch moves 4.9 TB/s; the rest is the launch's own latency: about
-// 3.5 us from the launch before it to the first product, 0.5 us from the last one to the stores.
+//   6144 x 4096 Q5    11.1 (11.6)    11.3 (11.8)    13.1 (15.3) us
+//   4096 x 4096 Q6     8.7  (9.3)     9.2  (9.5)     9.5 (11.0)
+//   24576 x 4096 Q3   15.9 (15.0)    17.7 (17.7)    29.2 (28.8)
+//   4096 x 12288 Q4   11.5 (12.4)    12.3 (12.9)    16.2 (16.8)
+//   the four in turn  48.5 (48.2)    51.2 (51.8)    68.6 (71.7)
 //
-// The tiles (rows in the row-major layout) of all problems of a launch form one line that is cut into equal
-// contiguous ranges, one per CTA; nothing crosses CTAs.  The sixteen warps' partial sums of a tile go through shared
-// memory and are added in warp order: bit-identical from run to run, and the same bits from either layout.
+// The tiles of all problems of a launch form one line that is cut into equal contiguous ranges, one per CTA; nothing
+// crosses CTAs.  The sixteen warps' partial sums of a tile go through shared memory and are added in warp order: bit-
+// identical from run to run, and the same bits from either layout.
 #include "pe_gemv_decode.cuh"
 
 namespace pe {
 
 constexpr int kBulkWarps = 16;                        // math warps
-constexpr int kBulkThreads = (kBulkWarps + 1) * 32;   // + the copy warp
+__host__ __device__ constexpr int bulk_threads(bool tiled) { return (kBulkWarps + (tiled ? 1 : 2)) * 32; }  // + the copy warp, the norm warp
 constexpr int kTabAddr = 2048;                        // address of the centroid table in the shared window
 constexpr int kTabReach = 255 * 256 + 256;            // bytes a lookup can reach from there, whatever the code byte is
 constexpr int kBulkMaxStages = 8;
@@ -58,11 +59,12 @@ struct BulkArgs {
   const __half* bias;
   int batch, N, nb;
   int n_chunk, chunk_blocks, n_stage;      // chunks of the K range, blocks of a full chunk
-  int units;                               // units (16 rows tiled, 1 row row-major) per problem
+  int units;                               // 16-row tiles per problem
   int pass_rows;                           // rows whose partial sums shared memory holds (a multiple of 16)
   int part_stride;                         // floats between activation rows of the partial sums
   int part_rows;                           // activation rows the partial sums have room for
-  int part_off, norm_off, norm_stride, stage_off, stage_bytes, row_stride;
+  int part_off, stage_off, stage_bytes;
+  int row_stride, copy_rows;               // row-major layout: bytes between rows of a stage, weight rows per bulk copy
   int* status;
   // grouped launch: problem i multiplies rows grp[i].y .. + grp[i].z of the row list with matrix grp[i].x
   const int4* grp; int n_problems;
@@ -97,6 +99,12 @@ __device__ __noinline__ bool bar_wait_slow(uint32_t bar, uint32_t parity, int* s
 }
 __device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, int* status) {
   if (!bar_try(bar, parity)) bar_wait_slow(bar, parity, status);
+}
+// one lane of a converged warp: a bulk copy takes warp-uniform operands and issues fastest from a branch on this
+__device__ __forceinline__ bool elect_lane() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
 }
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -280,11 +288,10 @@ __global__ void __launch_bounds__(kFragThreads) gemv_frags_kernel(const FragArgs
 }
 
 // ---- the launch's line of units ---------------------------------------------------------------------------------
-// A pass is a run of units of one problem whose partial sums fit in shared memory.  The copy warp and the math warps
+// A pass is a run of 16-row tiles of one problem whose partial sums fit in shared memory.  The copy, norm and math warps
 // walk the same passes.
-template <bool TILED, bool GROUPED>
+template <bool GROUPED>
 struct Pass {
-  static constexpr int kUnit = TILED ? 16 : 1;  // weight rows per unit
   int left;               // units of this CTA not yet passed
   int prob, off;          // problem, unit inside it
   int row0, rows;         // weight rows of this pass
@@ -295,20 +302,20 @@ struct Pass {
   }
   __device__ __forceinline__ bool next(const BulkArgs& p) {  // false at the end; advances past the pass it describes
     if (left <= 0) return false;
-    int n = min(p.pass_rows / kUnit, left);
+    int n = min(p.pass_rows / 16, left);
     if (GROUPED) {
       if (off == p.units) { off = 0; ++prob; }
       n = min(n, p.units - off);
     }
-    row0 = off * kUnit;
-    rows = TILED ? min(n * kUnit, p.N - row0) : n;
+    row0 = off * 16;
+    rows = min(n * 16, p.N - row0);
     left -= n; off += n;
     return true;
   }
 };
 
 template <bool PACKED, int NT, int BPW, bool TILED, bool GROUPED>
-__global__ void __launch_bounds__(kBulkThreads, 1) gemv_bulk_kernel(const BulkArgs p) {
+__global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const BulkArgs p) {
   extern __shared__ __align__(128) uint8_t smem[];  // no static shared memory: the window starts with it
   constexpr int kRowBytes = PACKED ? 64 : 128;           // codes of one row's block
   constexpr int kRecBytes = kRowBytes * 16 + 32;         // tiled record: 16 rows of a block, then their norms
@@ -322,7 +329,7 @@ __global__ void __launch_bounds__(kBulkThreads, 1) gemv_bulk_kernel(const BulkAr
     return;
   }
   if (tid == 0) {
-    for (int s = 0; s < p.n_stage; ++s) { bar_init(full + 8 * s, 1); bar_init(empty + 8 * s, kBulkWarps); }
+    for (int s = 0; s < p.n_stage; ++s) { bar_init(full + 8 * s, TILED ? 1 : 2); bar_init(empty + 8 * s, kBulkWarps); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     n_live = 0;
   }
@@ -330,12 +337,12 @@ __global__ void __launch_bounds__(kBulkThreads, 1) gemv_bulk_kernel(const BulkAr
   int line = p.units;
   if (GROUPED) {  // the problem list comes from the launch before this one
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int i = tid; i < p.n_problems; i += kBulkThreads)
+    for (int i = tid; i < p.n_problems; i += bulk_threads(TILED))
       if (p.grp[i].z > 0) atomicMax(&n_live, i + 1);
     __syncthreads();
     line = n_live * p.units;
   }
-  Pass<TILED, GROUPED> ps;
+  Pass<GROUPED> ps;
   {
     const int q = line / (int)gridDim.x, r = line - q * (int)gridDim.x, cta = blockIdx.x;
     const int beg = cta * q + min(cta, r);
@@ -343,6 +350,7 @@ __global__ void __launch_bounds__(kBulkThreads, 1) gemv_bulk_kernel(const BulkAr
   }
 
   if (w == kBulkWarps) {  // ---- copy warp
+    const bool one = elect_lane();
     int s = 0;
     uint32_t ph = 1;
     while (ps.next(p)) {
@@ -359,21 +367,89 @@ __global__ void __launch_bounds__(kBulkThreads, 1) gemv_bulk_kernel(const BulkAr
         for (int r0 = 0; r0 < ps.rows; r0 += 16) {
           bar_wait(empty + 8 * s, ph, p.status);
           const uint32_t dst = sbase + p.stage_off + s * p.stage_bytes, bar = full + 8 * s;
-          if (TILED) {
-            if (lane == 0) {
+          if (one) {
+            if (TILED) {
               bar_expect(bar, nblk * kRecBytes);
               bulk_load(dst, tiles + ((int64_t)((ps.row0 + r0) >> 4) * p.nb + b0) * kRecBytes, nblk * kRecBytes, bar);
+            } else {
+              const int rows = min(16, ps.rows - r0);
+              const uint8_t* src = codes + (int64_t)(ps.row0 + r0) * p.ld_codes + b0 * kRowBytes;
+              bar_expect(bar, rows * nblk * kRowBytes);
+              for (int r = 0; r < rows; r += p.copy_rows)
+                bulk_load(dst + r * p.row_stride + (r >> 3) * 64, src + r * p.ld_codes, min(p.copy_rows, rows - r) * nblk * kRowBytes, bar);
             }
-          } else {
-            const int rows = min(16, ps.rows - r0);
-            if (lane == 0) bar_expect(bar, rows * nblk * kRowBytes);
-            __syncwarp();
-            if (lane < rows)
-              bulk_load(dst + lane * p.row_stride, codes + (int64_t)(ps.row0 + r0 + lane) * p.ld_codes + b0 * kRowBytes, nblk * kRowBytes, bar);
           }
+          __syncwarp();
           if (++s == p.n_stage) { s = 0; ph ^= 1; }
         }
       }
+    }
+    return;
+  }
+
+  if (!TILED && w > kBulkWarps) {  // ---- norm warp: a stage's norms, the 16 rows of a block side by side
+    constexpr int kPlaces = kBulkWarps * BPW, kLaneRows = 16 * kPlaces / 32;
+    const int b = lane % kPlaces, r_lane = lane / kPlaces * kLaneRows, blocks = min(p.nb, p.chunk_blocks);
+    const __half* norms = p.norms;
+    int c = 0, r0 = 0;
+    auto next_pass = [&]() {
+      while (ps.next(p)) {
+        if (GROUPED) {
+          const int4 d = p.grp[ps.prob];
+          if (d.z <= 0) continue;
+          norms = p.norms + d.x * p.norms_stride;
+        }
+        // the whole pass on its way to L2: a stage's loads then wait for L2 and not for HBM
+        const char* span = reinterpret_cast<const char*>(norms + (int64_t)ps.row0 * p.ld_norms);
+        const int64_t bytes = ((int64_t)(ps.rows - 1) * p.ld_norms + p.nb) * 2;
+        for (int64_t o = lane * 128; o < bytes; o += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(span + o));
+        return true;
+      }
+      return false;
+    };
+    auto next_stage = [&]() {
+      r0 += 16;
+      if (r0 < ps.rows) return true;
+      r0 = 0;
+      if (++c < p.n_chunk) return true;
+      c = 0;
+      return next_pass();
+    };
+    auto load = [&](unsigned short (&h)[kLaneRows]) {
+      const int blk = c * p.chunk_blocks + b;
+      const __half* src = norms + (int64_t)(ps.row0 + r0 + r_lane) * p.ld_norms + blk;
+#pragma unroll
+      for (int i = 0; i < kLaneRows; ++i) {
+        h[i] = 0;
+        if (b < blocks && blk < p.nb && r0 + r_lane + i < ps.rows) h[i] = __half_as_ushort(src[(int64_t)i * p.ld_norms]);
+      }
+    };
+    int s = 0;
+    uint32_t ph = 1;
+    auto store = [&](const unsigned short (&h)[kLaneRows]) {
+      bar_wait(empty + 8 * s, ph, p.status);
+      if (b < blocks) {
+        const uint32_t dst = sbase + p.stage_off + s * p.stage_bytes + 16 * p.row_stride + 64 + b * 32 + r_lane * 2;
+#pragma unroll
+        for (int q = 0; q < kLaneRows; q += 8)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + q * 2), "r"(h[q] | h[q + 1] << 16), "r"(h[q + 2] | h[q + 3] << 16),
+                       "r"(h[q + 4] | h[q + 5] << 16), "r"(h[q + 6] | h[q + 7] << 16) : "memory");
+      }
+      __syncwarp();
+      if (lane == 0) bar_arrive(full + 8 * s);
+      if (++s == p.n_stage) { s = 0; ph ^= 1; }
+    };
+    unsigned short h0[kLaneRows], h1[kLaneRows];  // the loads of two stages under way
+    bool more = next_pass();
+    if (more) load(h0);
+    while (more) {
+      const bool second = next_stage();
+      if (second) load(h1);
+      store(h0);
+      if (!second) break;
+      more = next_stage();
+      if (more) load(h0);
+      store(h1);
     }
     return;
   }
@@ -395,21 +471,23 @@ __global__ void __launch_bounds__(kBulkThreads, 1) gemv_bulk_kernel(const BulkAr
       if (!PACKED) *reinterpret_cast<uint4*>(tab + e * 256 + 128 + (tid & 7) * 16) = make_uint4(u << 16, u << 16, u << 16, u << 16);
     }
   }
-  auto stage_norms = [&](const __half* norms, int row0, int rows) {  // row-major layout: norms of a pass
-    for (int r = w; r < rows; r += kBulkWarps)
-      for (int b = lane; b < p.nb; b += 32)
-        *reinterpret_cast<__half*>(smem + p.norm_off + r * p.norm_stride + b * 2) = norms[(int64_t)(row0 + r) * p.ld_norms + b];
-  };
   bool more = ps.next(p);
-  bool fresh = true;  // norms of the first pass are staged before the dependency wait
-  if (!TILED && !GROUPED && more) { stage_norms(p.norms, ps.row0, ps.rows); fresh = false; }
   if (!GROUPED) asm volatile("griddepcontrol.wait;" ::: "memory");
 
+  // Where this lane's codes and norms lie in a stage.  Its operand rows g and g + 8 are weight rows g and g + 8 of a tile's
+  // records, and rows row_a and row_a + 4 of row-major stages: rows of those lie a multiple of 64 bytes apart, rows 0..7 and
+  // 8..15 another 64 bytes, so that a quarter warp, which reads the rows of two neighbouring g, reads both halves of the banks.
+  constexpr int kRowB = TILED ? 8 : 4;
+  const int row_a = TILED ? g : (g >> 1) + (g & 1) * 8;
+  const uint32_t at_a = TILED ? w * kRecBytes + g * kRowBytes + t * 16 : row_a * p.row_stride + (g & 1) * 64 + w * kRowBytes + t * 16;
+  const uint32_t at_b = at_a + kRowB * (TILED ? kRowBytes : p.row_stride);
+  const uint32_t at_n = TILED ? w * kRecBytes + 16 * kRowBytes + g * 2 : 16 * p.row_stride + 64 + w * 32 + row_a * 2;
+  constexpr int kStep = kBulkWarps * (TILED ? kRecBytes : kRowBytes), kNormStep = kBulkWarps * (TILED ? kRecBytes : 32);
   const uint32_t lane4 = lane * 4;
   float* part = reinterpret_cast<float*>(smem + p.part_off);
   uint32_t x[BPW][NT][16];
   int x_prob = -1, group_rows = p.batch;
-  int expert = 0, y_row = 0;
+  int y_row = 0;
 
   auto load_x = [&](int prob, int c) {
     const uint4* src = p.frags + (size_t)(prob * NT * p.nb + c * p.chunk_blocks + w) * 128 + lane;
@@ -435,17 +513,14 @@ __global__ void __launch_bounds__(kBulkThreads, 1) gemv_bulk_kernel(const BulkAr
         if (d.z <= 0) continue;
         group_rows = d.z < 8 * NT ? d.z : 8 * NT;
         y_row = d.y;
-        expert = d.x;
       }
       x_prob = ps.prob;
       if (p.n_chunk == 1) load_x(x_prob, 0);
     }
-    if (!TILED && fresh) stage_norms(p.norms + expert * p.norms_stride, ps.row0, ps.rows);
-    fresh = true;
-    math_sync();  // table and norms are there; the sums of the pass before are out
+    math_sync();  // the table is there; the sums of the pass before are out
     for (int c = 0; c < p.n_chunk; ++c) {
       if (p.n_chunk > 1) load_x(x_prob, c);
-      const int b0 = c * p.chunk_blocks, nblk = min(p.chunk_blocks, p.nb - b0);
+      const int nblk = min(p.chunk_blocks, p.nb - c * p.chunk_blocks);
       for (int r0 = 0; r0 < ps.rows; r0 += 16) {
         const uint32_t st = sbase + p.stage_off + s * p.stage_bytes;
         bar_wait(full + 8 * s, ph, p.status);
@@ -460,18 +535,9 @@ __global__ void __launch_bounds__(kBulkThreads, 1) gemv_bulk_kernel(const BulkAr
           if (blk < nblk) {
             float d[NT][4];
             unsigned short ha, hb;
-            if (TILED) {
-              const uint32_t rec = st + blk * kRecBytes, a = rec + g * kRowBytes + t * 16;
-              asm volatile("ld.shared.u16 %0, [%1];" : "=h"(ha) : "r"(rec + 16 * kRowBytes + g * 2));
-              asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hb) : "r"(rec + 16 * kRowBytes + g * 2 + 16));
-              block_product<PACKED, NT>(a, a + 8 * kRowBytes, x[j], lane4, d);
-            } else {
-              const uint32_t a = st + g * p.row_stride + blk * kRowBytes + t * 16, nn = sbase + p.norm_off + (b0 + blk) * 2;
-              const int last = ps.rows - 1;
-              asm volatile("ld.shared.u16 %0, [%1];" : "=h"(ha) : "r"(nn + min(r0 + g, last) * p.norm_stride));
-              asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hb) : "r"(nn + min(r0 + g + 8, last) * p.norm_stride));
-              block_product<PACKED, NT>(a, a + 8 * p.row_stride, x[j], lane4, d);
-            }
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(ha) : "r"(st + at_n + j * kNormStep));
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hb) : "r"(st + at_n + j * kNormStep + kRowB * 2));
+            block_product<PACKED, NT>(st + at_a + j * kStep, st + at_b + j * kStep, x[j], lane4, d);
             const float fa = __half2float(__ushort_as_half(ha)), fb = __half2float(__ushort_as_half(hb));
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
@@ -500,9 +566,10 @@ __global__ void __launch_bounds__(kBulkThreads, 1) gemv_bulk_kernel(const BulkAr
     math_sync();
     const int groups = (ps.rows + 31) >> 5, batch = GROUPED ? group_rows : p.batch;
     for (int e = w; e < groups * batch; e += kBulkWarps) {  // a warp sums 32 rows of one activation row
-      const int m = groups == 1 ? e : e / groups, r = (e - m * groups) * 32 + lane;
+      const int m = groups == 1 ? e : e / groups, at = (e - m * groups) * 32 + lane;
+      const int r = TILED ? at : (at & ~15) + ((at & 7) >> 1) + (at & 1) * 8 + ((at >> 1) & 4);  // the row that row_a put there
       if (r < ps.rows) {
-        const float* q = part + m * p.part_stride + r;
+        const float* q = part + m * p.part_stride + at;
         float v[kBulkWarps], sum = 0.f;
 #pragma unroll
         for (int i = 0; i < kBulkWarps; ++i) v[i] = q[i * p.part_rows * p.part_stride];
@@ -523,27 +590,30 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
   a.chunk_blocks = kBulkWarps * BPW;
   a.n_chunk = (a.nb + a.chunk_blocks - 1) / a.chunk_blocks;
   const int blocks = a.nb < a.chunk_blocks ? a.nb : a.chunk_blocks;  // of the largest stage
-  constexpr int kUnit = TILED ? 16 : 1;
-  a.units = TILED ? (a.N + 15) / 16 : a.N;
+  a.units = (a.N + 15) / 16;
   const long long line = (long long)a.units * (a.grp ? a.n_problems : 1);
   if (line >= (1ll << 31)) return PE_ERR_LIMIT;
   const int G = (int)(line < sms ? line : sms);
   // Rows per pass: the sums of a pass meet at a barrier, so few and equal passes; 64 rows of 8 activation rows are
   // 34 KB of partial sums, which the ring would rather have (64 measured best of 32, 64, 96 and 176).
   a.part_rows = a.batch < 8 * NT ? a.batch : 8 * NT;
-  const int cta_rows = (int)((line + G - 1) / G) * kUnit;
+  const int cta_rows = (int)((line + G - 1) / G) * 16;
   const int entries = PACKED ? (a.n_levels <= 8 ? 128 : 256) : a.n_levels;
   a.part_off = kTabAddr + entries * 256;  // leaves room for the table wherever the window starts
-  a.norm_stride = (a.nb & 1) ? a.nb * 2 : a.nb * 2 + 2;  // an odd number of halves: rows spread over the banks
-  a.row_stride = TILED ? 0 : (blocks * kRowBytes + 127) / 128 * 128 + 64;  // a quarter warp reads two rows: different halves of the banks
-  a.stage_bytes = TILED ? (blocks * kRecBytes + 127) & ~127 : 16 * a.row_stride;
-  for (int cap = a.part_rows <= 2 ? 256 : (NT == 1 ? 64 : 32);; cap /= 2) {  // smaller passes where long rows' norms take the ring's room
+  // Row-major stages: a copy of its own for every row of 2 KB or more; shorter rows that follow each other in memory share one
+  // (a copy costs about 60 ns whatever its size: 128 experts of 21 and 15 blocks, rows of 1344 and 960 bytes, took 380 us with a
+  // copy a row and 356 us with two or more rows in one; 24576 rows of 2 KB 14.3 us with a copy a row and 15.3 us with two).
+  a.row_stride = blocks * kRowBytes;
+  a.copy_rows = 1;
+  if (a.n_chunk == 1 && a.ld_codes == a.row_stride)
+    while (a.copy_rows < 8 && a.copy_rows * a.row_stride < 2048) a.copy_rows *= 2;
+  a.stage_bytes = TILED ? (blocks * kRecBytes + 127) & ~127 : (16 * a.row_stride + 64 + blocks * 32 + 127) & ~127;
+  for (int cap = a.part_rows <= 2 ? 256 : (NT == 1 ? 64 : 32);; cap /= 2) {
     if (cap < 16) return PE_ERR_LIMIT;
     const int passes = (cta_rows + cap - 1) / cap;
     a.pass_rows = GROUPED ? cap : ((cta_rows + passes - 1) / passes + 15) / 16 * 16;
     a.part_stride = a.pass_rows + 4;  // rows of a stage land on different banks than the activation rows' distance
-    a.norm_off = a.part_off + kBulkWarps * a.part_rows * a.part_stride * 4;
-    a.stage_off = (a.norm_off + (TILED ? 0 : a.pass_rows * a.norm_stride) + 127) & ~127;
+    a.stage_off = (a.part_off + kBulkWarps * a.part_rows * a.part_stride * 4 + 127) & ~127;
     a.n_stage = a.stage_off < (int)kBulkSmemMax ? ((int)kBulkSmemMax - a.stage_off) / a.stage_bytes : 0;
     if (a.n_stage >= 2) break;
   }
@@ -558,7 +628,7 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
     PE_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     if (dev < 16) configured[dev] = dyn;
   }
-  PE_CUDA_TRY(launch_pdl(kfn, dim3(G), dim3(kBulkThreads), dyn, st, a));
+  PE_CUDA_TRY(launch_pdl(kfn, dim3(G), dim3(bulk_threads(TILED)), dyn, st, a));
   return PE_OK;
 }
 

@@ -1,4 +1,4 @@
-// One-token matmul over the row-major layout: column-owner kernel.
+// One-token matmul over the row-major layout that needs no scratch memory (pe_gemv_pro): column-owner kernel.
 //
 //   y[r] = sum_blk norm[r, blk] * sum_k ct[code[r, blk, k]] * xt[blk, k]   (+ bias[r])
 //
@@ -410,15 +410,6 @@ static int gemv_cols_try(const void* codes, int packed, int64_t ld_codes, const 
   return launch_cols_cpw<false, false>(a, cpw, G, stream);
 }
 
-int gemv_cols_run(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms, const float* ct_scaled, int n_levels,
-                  const void* x, int x_kind, int x_dtype, int in_f, void* y, int y_dtype, const void* bias, int out_f, int in_f_padded,
-                  cudaStream_t stream) {
-  const int sms = sm_count();
-  if (sms <= 0) return PE_ERR_CUDA;
-  return gemv_cols_try(codes, packed, ld_codes, norms, ld_norms, ct_scaled, n_levels, x, x_kind, x_dtype, in_f, y, y_dtype, bias, out_f,
-                       in_f_padded, sms, stream);
-}
-
 }  // namespace pe
 
 // ---- batch-1 matmul with the glue op in front of it computed while the input is staged ----
@@ -457,20 +448,17 @@ extern "C" int pe_gemv_pro(const void* codes, int packed, int64_t ld_codes, cons
   return r == 1 ? PE_ERR_SHAPE : r;  // shapes the column-owner kernel does not take: the caller runs the separate launches
 }
 
-
-extern "C" int pe_gemv_pro_tiled(const void* tiles, int packed, const float* ct_scaled, int n_levels, int prologue, const void* x, int in_f,
-                                 const void* delta, int delta_dtype, const void* norm_weight, void* resid_out, float eps, void* y,
-                                 int y_dtype, const void* bias, int out_f, int in_f_padded, void* workspace, size_t workspace_bytes,
-                                 void* stream) {
+// The same over the bulk-copy kernel: the op is computed where the activations are prepared.
+static int pro_bulk(pe::GemvBulkCall& q, int prologue, const float* ct_scaled, int n_levels, const void* x, int in_f, const void* delta, int delta_dtype,
+                    const void* norm_weight, void* resid_out, float eps, void* y, int y_dtype, const void* bias, int out_f, int in_f_padded,
+                    void* workspace, size_t workspace_bytes, void* stream) {
   using namespace pe;
-  if (!tiles || !workspace) return PE_ERR_ARG;
-  const int c = pro_check(ct_scaled, n_levels, packed, prologue, x, in_f, delta, delta_dtype, norm_weight, resid_out, y, y_dtype, out_f, in_f_padded);
+  const int c = pro_check(ct_scaled, n_levels, q.packed, prologue, x, in_f, delta, delta_dtype, norm_weight, resid_out, y, y_dtype, out_f, in_f_padded);
   if (c != PE_OK) return c;
-  if ((reinterpret_cast<uintptr_t>(tiles) & 15) || (reinterpret_cast<uintptr_t>(workspace) & 15)) return PE_ERR_ALIGN;
+  if (reinterpret_cast<uintptr_t>(workspace) & 15) return PE_ERR_ALIGN;
   if (workspace_bytes < kGemvStatusBytes + gemv_bulk_frag_bytes(1, 1, in_f_padded)) return PE_ERR_WORKSPACE;
   uint8_t* ws = static_cast<uint8_t*>(workspace);
-  GemvBulkCall q = {};
-  q.tiles = tiles; q.packed = packed; q.ct_scaled = ct_scaled; q.n_levels = n_levels;
+  q.ct_scaled = ct_scaled; q.n_levels = n_levels;
   q.x = x; q.x_kind = prologue == PE_PRO_SILU_MUL ? PE_X_SILU_MUL : PE_X_RAW; q.x_dtype = PE_F16; q.ld_x = 2 * (int64_t)in_f; q.in_f = in_f;
   q.y = y; q.y_dtype = y_dtype; q.ld_y = out_f; q.bias = bias;
   q.batch = 1; q.out_f = out_f; q.in_f_padded = in_f_padded;
@@ -479,4 +467,29 @@ extern "C" int pe_gemv_pro_tiled(const void* tiles, int packed, const float* ct_
   q.pro = prologue == PE_PRO_ADD_RMSNORM ? prologue : PE_PRO_NONE;
   q.delta = delta; q.delta_dtype = delta_dtype; q.norm_w = norm_weight; q.resid_out = resid_out; q.eps = eps;
   return gemv_bulk_run(q, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int pe_gemv_pro_scratch(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms, const float* ct_scaled,
+                                   int n_levels, int prologue, const void* x, int in_f, const void* delta, int delta_dtype, const void* norm_weight,
+                                   void* resid_out, float eps, void* y, int y_dtype, const void* bias, int out_f, int in_f_padded, void* workspace,
+                                   size_t workspace_bytes, void* stream) {
+  if (!codes || !norms || !workspace) return PE_ERR_ARG;
+  if ((reinterpret_cast<uintptr_t>(codes) & 15) || (ld_codes & 15)) return PE_ERR_ALIGN;
+  if (ld_codes < (packed ? in_f_padded / 2 : in_f_padded) || ld_norms < in_f_padded / pe::kBlock) return PE_ERR_ARG;
+  pe::GemvBulkCall q = {};
+  q.codes = codes; q.packed = packed; q.ld_codes = ld_codes; q.norms = norms; q.ld_norms = ld_norms;
+  return pro_bulk(q, prologue, ct_scaled, n_levels, x, in_f, delta, delta_dtype, norm_weight, resid_out, eps, y, y_dtype, bias, out_f, in_f_padded,
+                  workspace, workspace_bytes, stream);
+}
+
+extern "C" int pe_gemv_pro_tiled(const void* tiles, int packed, const float* ct_scaled, int n_levels, int prologue, const void* x, int in_f,
+                                 const void* delta, int delta_dtype, const void* norm_weight, void* resid_out, float eps, void* y,
+                                 int y_dtype, const void* bias, int out_f, int in_f_padded, void* workspace, size_t workspace_bytes,
+                                 void* stream) {
+  if (!tiles || !workspace) return PE_ERR_ARG;
+  if (reinterpret_cast<uintptr_t>(tiles) & 15) return PE_ERR_ALIGN;
+  pe::GemvBulkCall q = {};
+  q.tiles = tiles; q.packed = packed;
+  return pro_bulk(q, prologue, ct_scaled, n_levels, x, in_f, delta, delta_dtype, norm_weight, resid_out, eps, y, y_dtype, bias, out_f, in_f_padded,
+                  workspace, workspace_bytes, stream);
 }

@@ -128,12 +128,6 @@ __device__ __forceinline__ float reg_dot(const uint4& q, uint32_t lane_base, con
 
 constexpr size_t kGemvStatusBytes = 262144;  // first part of pe_gemv's scratch; its last word is the status word
 
-// The one-token column-owner kernel over row-major codes (pe_gemv_cols.cu).  PE_OK after a launch, 1 if the layer's
-// shape is not its kind (the caller goes on to the bulk-copy kernel), or a negative error code.
-int gemv_cols_run(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms, const float* ct_scaled, int n_levels,
-                  const void* x, int x_kind, int x_dtype, int in_f, void* y, int y_dtype, const void* bias, int out_f, int in_f_padded,
-                  cudaStream_t stream);
-
 // The bulk-copy kernel (pe_gemv_bulk.cu) for 1..16 activation rows: either layout (tiles when not null), one matrix or a
 // grouped launch (problems when not null; batch is then the largest row count of a problem).  Arguments checked by
 // the caller.

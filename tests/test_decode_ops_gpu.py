@@ -268,3 +268,29 @@ def test_rope_cache_widths_and_token_major(d, shift):
     assert torch.allclose(q.float(), rope(heads[:, :hq], pos, 1e4).float(), rtol=2e-3, atol=2e-3)
     assert torch.allclose(caches[0][:, :, pos0:pos0 + t].float(), rope(heads[:, hq:hq + hkv], pos, 1e4).float(), rtol=2e-3, atol=2e-3)
     assert torch.equal(caches[1][:, :, pos0:pos0 + t], heads[:, hq + hkv:])
+
+
+@pytest.mark.parametrize("bits,n,k", [(4, 4096, 4096), (5, 1000, 1024)])
+def test_folded_prologues_without_scratch(bits, n, k):
+    """pe_gemv_pro, which takes no scratch memory: against the entry point that does (it multiplies in fp16 pairs, hence the
+    tolerance of the packed / unpacked comparisons), and the shapes that it leaves to the separate launches."""
+    from helpers import max_rel, rand_layer
+    from polarengine_vllm_b200 import _native as nv, kernels, packing
+    codes, norms, cts = rand_layer(n, k, bits, seed=n)
+    packed = bits <= 4
+    w = packing.pack_codes_half_block(codes.cuda()) if packed else codes.cuda()
+    nd, ctd, lib = norms.cuda(), cts.cuda(), nv.lib()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, delta = (torch.randn(1, k, device="cuda", generator=g).half() for _ in range(2))
+    gu, lnw = torch.randn(1, 2 * k, device="cuda", generator=g).half(), torch.ones(k, device="cuda").half()
+    for prologue, inp, d, resid in ((nv.PE_PRO_ADD_RMSNORM, x, delta, torch.empty_like(x)), (nv.PE_PRO_SILU_MUL, gu, None, None)):
+        kw = dict(delta=d, norm_weight=lnw if d is not None else None, resid_out=resid, eps=1e-6)
+        ref = kernels.quant_matmul_pro(w, packed, nd, ctd, prologue, inp, k, n, k, torch.float32, **kw)
+        want = resid.clone() if resid is not None else None
+        y = torch.full((1, n), float("nan"), device="cuda")
+        args = (w.data_ptr(), int(packed), w.stride(0), nd.data_ptr(), nd.stride(0), ctd.data_ptr(), ctd.numel(), prologue, inp.data_ptr(), k,
+                d.data_ptr() if d is not None else None, nv.PE_F16, lnw.data_ptr() if d is not None else None,
+                resid.data_ptr() if resid is not None else None, 1e-6, y.data_ptr(), nv.PE_F32, None)
+        nv.check(lib.pe_gemv_pro(*args, n, k, nv.stream_ptr(x.device)), "pe_gemv_pro")
+        assert max_rel(y, ref) <= 2e-3 and (resid is None or torch.equal(resid, want))
+        assert lib.pe_gemv_pro(*args, 8, k, nv.stream_ptr(x.device)) == -2  # too few rows for it

@@ -329,3 +329,23 @@ def test_weights_rewritten_by_the_kernel_in_front(bits, rows):
             got.append(kernels.quant_matmul(w, packed, m, ctd, x, False, n, k, k, torch.float32))
     graph.replay()
     assert all(torch.equal(y, want[i % 2]) for i, y in enumerate(got))
+
+
+@pytest.mark.parametrize("rows", [1, 9])
+@pytest.mark.parametrize("bits,n,k", [(4, 17, 128), (3, 40, 640), (4, 2400, 1920), (4, 9, 4224), (5, 23, 1920), (6, 2377, 2048)])
+def test_row_major_stages_follow_the_strides(bits, n, k, rows):
+    """Stages of row-major arrays: rows that share a bulk copy (short ones that follow each other) and rows with one of
+    their own (long ones, two K ranges, codes with a gap between rows), norms at odd addresses; a last tile of one row, of
+    nine, of a half."""
+    from polarengine_vllm_b200 import kernels, packing
+    codes, norms, cts = rand_layer(n, k, bits, seed=n + k)
+    packed = bits <= 4
+    w = packing.pack_codes_half_block(codes.cuda()) if packed else codes.cuda()
+    nd, ctd, x = norms.cuda(), cts.cuda(), rand_x(rows, k, seed=rows).cuda()
+    y = kernels.quant_matmul(w, packed, nd, ctd, x, False, n, k, k, torch.float32)
+    assert max_rel(y, oracle.linear_dequant(x.cpu(), codes, norms, cts)) <= TOL
+    gap = torch.full((n, w.shape[1] + 48), 0x55, dtype=w.dtype, device="cuda")
+    gap[:, 16:16 + w.shape[1]] = w
+    odd = torch.full((n, nd.shape[1] + 3), float("nan"), dtype=torch.float16, device="cuda")
+    odd[:, 1:1 + nd.shape[1]] = nd
+    assert torch.equal(y, kernels.quant_matmul(gap[:, 16:16 + w.shape[1]], packed, odd[:, 1:1 + nd.shape[1]], ctd, x, False, n, k, k, torch.float32))
