@@ -541,12 +541,9 @@ def main():
     xh = torch.randn(a.batch, HIDDEN, device=dev, generator=g).half()
     xi = torch.randn(a.batch, INTER, device=dev, generator=g).half()
 
-    tiles = {id(layer): {name: kernels.retile(*layer[name][:3]) for name, _, _, _ in PROJ} for layer in layers}
-
-    def launch(layer, name):  # on the tiled copy, as apply() runs a decode-size batch
+    def launch(layer, name):
         w, packed, norms, ct, n, k = layer[name]
-        return kernels.quant_matmul(w, packed, norms, ct, xh if k == HIDDEN else xi, False, n, k, k, torch.float16,
-                                    tiles=tiles[id(layer)][name] if a.batch <= kernels.GEMV_MAX_BATCH else None)
+        return kernels.quant_matmul(w, packed, norms, ct, xh if k == HIDDEN else xi, False, n, k, k, torch.float16)
 
     def ring_pass(names):
         for layer in layers:
@@ -686,7 +683,7 @@ def main():
     dom_launches = dom_passes * RING
     dom_bytes = sum(alg_bytes(n, k, b, a.batch) for nm, n, k, b in PROJ if nm in dom)
     achieved = dom_bytes / (dom_elapsed / dom_launches) / 1e9
-    dom_kernel = "gemv_bulk_kernel<nibble codes, tiled>"
+    dom_kernel = "gemv_bulk_kernel<nibble codes, row-major>"
     roofline = {"bound": "hbm", "kernel": dom_kernel + " on down_proj 4096x12288 Q4",
                 "achieved": achieved, "peak": peak, "peak_source": "measured (MEASURED_PEAKS.json)" if peaks else "fallback",
                 "unit": "GB/s", "frac": achieved / peak, "avg_launch_us": dom_elapsed / dom_launches * 1e6,
@@ -695,7 +692,7 @@ def main():
     line = dict(base, value=value, ms_per_step=elapsed / steps * 1e3, steps=steps, steps_requested=a.steps, e2e=e2e,
                 gpu_launches=8 * steps, roofline=roofline, clocks=sampler.summary(), frac_of_measured_hbm=value / world / peak,
                 timed_region_s=elapsed)
-    del layers, mods, graphs, tiles
+    del layers, mods, graphs
     torch.cuda.empty_cache()
 
     if rank == 0 and not a.no_cpu_baseline and world == 1:

@@ -146,7 +146,7 @@ PyObject* wrap_or_none(at::Tensor y) {
 
 // ---- layer attributes ------------------------------------------------------------------------------------------
 struct Names {
-  PyObject *dict, *parameters, *buffers, *packed, *codes_packed, *codes, *norms, *ct_scaled, *in_f, *out_f, *in_f_padded, *tiled, *tiled_of;
+  PyObject *dict, *parameters, *buffers, *packed, *codes_packed, *codes, *norms, *ct_scaled, *in_f, *out_f, *in_f_padded;
 };
 Names names;
 
@@ -175,9 +175,9 @@ bool to_int(PyObject* o, int& out) {
     return nullptr;                                      \
   }
 
-// apply(layer, x, bias, tiled) -> fp16 output, or None
+// apply(layer, x, bias) -> fp16 output, or None
 PyObject* host_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  if (n != 4) { PyErr_SetString(PyExc_TypeError, "apply takes 4 arguments"); return nullptr; }
+  if (n != 3) { PyErr_SetString(PyExc_TypeError, "apply takes 3 arguments"); return nullptr; }
   PE_GUARD_BEGIN
   if (!ready) Py_RETURN_NONE;
   PyObject** pd = _PyObject_GetDictPtr(args[0]);
@@ -196,14 +196,6 @@ PyObject* host_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const at::Tensor* bias = nullptr;
   if (args[2] != Py_None && !(bias = tensor_or_null(args[2]))) Py_RETURN_NONE;
   const int64_t rows = x->numel() / w.in_f;
-  if (rows <= kDecodeRows && args[3] == Py_True) {
-    w.tiles = tensor_or_null(d.find(names.tiled));
-    PyObject* of = d.find(names.tiled_of);  // the codes and norms the copy was made from
-    const bool current = w.tiles && of && PyTuple_Check(of) && PyTuple_GET_SIZE(of) == 2 &&
-                         PyLong_AsVoidPtr(PyTuple_GET_ITEM(of, 0)) == w.codes->const_data_ptr() &&
-                         PyLong_AsVoidPtr(PyTuple_GET_ITEM(of, 1)) == w.norms->const_data_ptr();
-    if (!current) Py_RETURN_NONE;
-  }
   at::DimVector shape(x->sizes());
   shape.back() = w.out_f;
   return wrap_or_none(multiply(w, *x, rows, w.in_f, PE_X_RAW, at::kHalf, bias, shape));
@@ -426,7 +418,5 @@ PyMODINIT_FUNC PyInit__host(void) {
   names.in_f = PyUnicode_InternFromString("in_f");
   names.out_f = PyUnicode_InternFromString("out_f");
   names.in_f_padded = PyUnicode_InternFromString("in_f_padded");
-  names.tiled = PyUnicode_InternFromString("codes_tiled");
-  names.tiled_of = PyUnicode_InternFromString("codes_tiled_of");
   return PyModule_Create(&module);
 }

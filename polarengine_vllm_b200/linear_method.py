@@ -5,8 +5,10 @@ Same three entry points and the same layer attributes (``codes`` / ``codes_packe
 ``norms``, ``ct_scaled``, ``in_f``, ``out_f``, ``in_f_padded``, ``n_blocks``, ``bits``,
 ``block_size``, ``packed``, ``in_f_half``); the forward keeps the reference's meaning
 (flatten, pad, rotate, multiply, cast to fp16, add ``bias.half()``) but is one native
-launch for up to 16 tokens: padding, rotation, dequantisation, dot products, the
-split-K reduction, the cast and the bias all happen inside ``pe_gemv``.
+call for any number of tokens: a launch that pads and rotates the activations, and one
+that decodes the weights, multiplies, casts and adds the bias (``pe_gemv`` up to 16
+tokens, ``pe_gemm`` above).  Every launch reads the layer's own arrays; there is no
+other copy of them.
 
 Differences from the reference that a vLLM integrator should know:
 * the class derives from vLLM's ``LinearMethodBase`` when vLLM is importable, so the
@@ -23,7 +25,7 @@ from typing import Any, Dict, List, Optional
 import torch
 
 from . import _native as nv
-from .kernels import GEMV_MAX_BATCH, pack_codes_int4, quant_matmul, retile
+from .kernels import pack_codes_int4, quant_matmul
 from .packing import unpack_codes_half_block, unpack_codes_q5
 from .utils import get_ct_scaled
 
@@ -81,10 +83,6 @@ class PolarQuantLinearMethod(_Base):
         self.block_size = block_size
         self.bits = bits
         self.layer_meta = layer_meta or {}
-        # The tiled copy of a layer (codes and norms interleaved per 16-row x 128-column tile) serves batches of
-        # up to 16 rows; it is built the first time such a batch arrives, so a layer that only ever sees prefill
-        # keeps a single copy of its codes in HBM.  False: one copy always, decode batches read the row-major arrays.
-        self.decode_tiled = True
 
     # ------------------------------------------------------------------ weights
     def create_weights(self, layer: torch.nn.Module, input_size_per_partition: int,
@@ -134,30 +132,21 @@ class PolarQuantLinearMethod(_Base):
             layer.codes_packed = packed
             layer.in_f_half = layer.n_blocks * (layer.block_size // 2)
             layer.packed = True
-        layer.codes_tiled = layer.codes_tiled_of = None
 
     # ------------------------------------------------------------------ forward
     def apply(self, layer: torch.nn.Module, x: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-        y = (nv._host or nv.host()).apply(layer, x, bias, self.decode_tiled)
+        y = (nv._host or nv.host()).apply(layer, x, bias)
         if y is not None:
             return y
-        # the first decode-size batch (the tiled copy is made here), tensors to convert or to lay out, errors to report
+        # tensors to convert or to lay out, errors to report
         lead = x.shape[:-1]
         x2 = x.reshape(-1, layer.in_f)
         packed = bool(getattr(layer, "packed", False))
         w = layer.codes_packed if packed else layer.codes
-        tiles = None
-        if self.decode_tiled and 1 <= x2.shape[0] <= GEMV_MAX_BATCH:
-            made_of = (w.data_ptr(), layer.norms.data_ptr())
-            if getattr(layer, "codes_tiled_of", None) != made_of and not torch.cuda.is_current_stream_capturing():
-                layer.codes_tiled = retile(w.data, packed, layer.norms.data)
-                layer.codes_tiled_of = made_of
-            if getattr(layer, "codes_tiled_of", None) == made_of:
-                tiles = layer.codes_tiled
         # one native entry for every batch size: up to 16 rows run the fused decode kernel,
         # more rows the tensor-core kernel (rotation is done by its preparation launch)
         y = quant_matmul(w, packed, layer.norms, layer.ct_scaled, x2, False, layer.out_f, layer.in_f,
-                         layer.in_f_padded, torch.float16, bias, tiles=tiles)
+                         layer.in_f_padded, torch.float16, bias)
         return y.view(*lead, layer.out_f)
 
 

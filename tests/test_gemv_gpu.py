@@ -349,3 +349,38 @@ def test_row_major_stages_follow_the_strides(bits, n, k, rows):
     odd = torch.full((n, nd.shape[1] + 3), float("nan"), dtype=torch.float16, device="cuda")
     odd[:, 1:1 + nd.shape[1]] = nd
     assert torch.equal(y, kernels.quant_matmul(gap[:, 16:16 + w.shape[1]], packed, odd[:, 1:1 + nd.shape[1]], ctd, x, False, n, k, k, torch.float32))
+
+
+@pytest.mark.parametrize("bits", [4, 6])
+def test_a_linear_layer_has_one_copy_of_its_weights(bits):
+    """Decode-size batches multiply by what the layer's arrays hold at the call -- rewritten in place included, the first
+    call inside a capture included -- and leave no further memory with the layer."""
+    from polarengine_vllm_b200.linear_method import PolarQuantLinearMethod
+    from polarengine_vllm_b200 import packing
+    n, in_f = 4096, 4096
+    method, layer = PolarQuantLinearMethod(128, bits), torch.nn.Module()
+    method.create_weights(layer, in_f, [n], in_f, n, torch.float16)
+    layer = layer.cuda()
+    sets = [rand_layer(n, in_f, bits, seed=s) for s in (1, 2)]
+    layer.codes.data.copy_(sets[0][0])
+    layer.norms.data.copy_(sets[0][1])
+    method.process_weights_after_loading(layer)
+    x = rand_x(3, in_f, seed=4).cuda()
+    ref = [oracle.linear_dequant(x.cpu(), *s, in_f=in_f) for s in sets]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        held = method.apply(layer, x)  # the layer's first call
+    graph.replay()
+    assert max_rel(held, ref[0]) <= TOL
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    y = method.apply(layer, x)
+    assert torch.equal(y, held)
+    del y
+    codes = layer.codes_packed if layer.packed else layer.codes
+    assert torch.cuda.memory_allocated() - before < codes.numel() // 4  # scratch of the stream, no copy of the codes
+    codes.data.copy_(packing.pack_codes_half_block(sets[1][0].cuda()) if layer.packed else sets[1][0])
+    layer.norms.data.copy_(sets[1][1])
+    assert max_rel(method.apply(layer, x), ref[1]) <= TOL
+    graph.replay()
+    assert max_rel(held, ref[1]) <= TOL
