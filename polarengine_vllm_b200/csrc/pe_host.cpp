@@ -33,7 +33,6 @@ struct Api {
   decltype(&pe_moe_route_plan) moe_route_plan;
   decltype(&pe_moe_combine) moe_combine;
   decltype(&pe_gemv_grouped) grouped;
-  decltype(&pe_gemv_grouped_tiled) grouped_tiled;
   decltype(&pe_gemv_grouped_workspace_bytes) grouped_bytes;
   decltype(&pe_gemm_grouped) gemm_grouped;
   decltype(&pe_gemm_grouped_silu_mul) gemm_silu_mul;
@@ -231,7 +230,7 @@ PyObject* host_matmul(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 // One projection of every expert over the rows that the plan grouped.
 struct Experts {
-  const at::Tensor *codes, *norms, *ct, *tiles;
+  const at::Tensor *codes, *norms, *ct;
   bool packed;
 };
 struct MoePlan {
@@ -244,8 +243,7 @@ struct MoePlan {
 bool plain_experts(const Experts& w, const at::Device& dev, int64_t rows) {
   return w.codes && w.norms && w.ct && w.codes->device() == dev && w.norms->device() == dev && w.ct->device() == dev && w.codes->dim() == 3 &&
          w.codes->element_size() == 1 && w.codes->is_contiguous() && w.codes->size(1) == rows && w.norms->scalar_type() == at::kHalf &&
-         w.norms->dim() == 3 && w.norms->stride(2) == 1 && w.ct->scalar_type() == at::kFloat && w.ct->is_contiguous() &&
-         (!w.tiles || w.tiles->device() == dev);
+         w.norms->dim() == 3 && w.norms->stride(2) == 1 && w.ct->scalar_type() == at::kFloat && w.ct->is_contiguous();
 }
 
 int grouped(const Experts& w, const MoePlan& p, const at::Device& dev, cudaStream_t st, const void* x, int kind, int xd, int64_t ld_x, int in_f,
@@ -264,15 +262,12 @@ int grouped(const Experts& w, const MoePlan& p, const at::Device& dev, cudaStrea
                             (int)p.n_local, (int)p.pairs, out_f, in_f_padded, ws.mutable_data_ptr(), ws.numel(), st);
   }
   const at::Tensor ws = take_scratch(dev, st, 2, api.grouped_bytes((int)p.max_problems, out_f, in_f_padded), true);
-  if (w.tiles)
-    return api.grouped_tiled(w.tiles->const_data_ptr(), w.packed, w.tiles->numel() / p.n_local, ct, levels, x, kind, xd, ld_x, in_f, x_rows, y, yd,
-                             out_f, p.problems, (int)p.max_problems, p.rows_per_problem, out_f, in_f_padded, ws.mutable_data_ptr(), ws.numel(), st);
   return api.grouped(w.codes->const_data_ptr(), w.packed, w.codes->stride(1), w.codes->stride(0), w.norms->const_data_ptr(), w.norms->stride(1),
                      w.norms->stride(0), ct, levels, x, kind, xd, ld_x, in_f, x_rows, y, yd, out_f, p.problems, (int)p.max_problems,
                      p.rows_per_problem, out_f, in_f_padded, ws.mutable_data_ptr(), ws.numel(), st);
 }
 
-// moe(x, a, b, renormalize, expert_map, (codes, norms, ct, tiles, packed) gate/up, (...) down, (hidden, inter, hidden_padded, inter_padded),
+// moe(x, a, b, renormalize, expert_map, (codes, norms, ct, packed) gate/up, (...) down, (hidden, inter, hidden_padded, inter_padded),
 //     rows_per_problem, max_problems, tensor_cores) -> fp16 output, or None.  a, b: router logits and top_k, or top-k weights and ids.
 PyObject* host_moe(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 11) { PyErr_SetString(PyExc_TypeError, "moe takes 11 arguments"); return nullptr; }
@@ -289,9 +284,9 @@ PyObject* host_moe(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Experts w[2];
   for (int i = 0; i < 2; ++i) {
     PyObject* t = args[5 + i];
-    if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 5) Py_RETURN_NONE;
+    if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 4) Py_RETURN_NONE;
     w[i] = {tensor_or_null(PyTuple_GET_ITEM(t, 0)), tensor_or_null(PyTuple_GET_ITEM(t, 1)), tensor_or_null(PyTuple_GET_ITEM(t, 2)),
-            tensor_or_null(PyTuple_GET_ITEM(t, 3)), PyTuple_GET_ITEM(t, 4) == Py_True};
+            PyTuple_GET_ITEM(t, 3) == Py_True};
   }
   int dim[4], rpp, max_problems;
   if (!PyTuple_Check(args[7]) || PyTuple_GET_SIZE(args[7]) != 4) Py_RETURN_NONE;
@@ -388,7 +383,6 @@ PyObject* host_setup(PyObject*, PyObject* arg) {
   PE_SYMBOL(moe_route_plan, pe_moe_route_plan)
   PE_SYMBOL(moe_combine, pe_moe_combine)
   PE_SYMBOL(grouped, pe_gemv_grouped)
-  PE_SYMBOL(grouped_tiled, pe_gemv_grouped_tiled)
   PE_SYMBOL(grouped_bytes, pe_gemv_grouped_workspace_bytes)
   PE_SYMBOL(gemm_grouped, pe_gemm_grouped)
   PE_SYMBOL(gemm_silu_mul, pe_gemm_grouped_silu_mul)

@@ -16,7 +16,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _native as nv
-from .kernels import quant_matmul, retile
+from .kernels import quant_matmul
 from .packing import pack_codes_half_block
 from .utils import get_ct_scaled
 
@@ -97,9 +97,6 @@ class PolarQuantMoEMethod:
 
     def __init__(self, w13_bits: int = 3, w2_bits: int = 4, block_size: int = 128) -> None:
         self.w13_bits, self.w2_bits, self.block_size = w13_bits, w2_bits, block_size
-        # Decode-size batches stream tiled copies of the experts (``kernels.retile``), built when the first such batch
-        # arrives and dropped when an expert is loaded.  False: one copy always, at a third more time per batch.
-        self.decode_tiled = True
 
     @staticmethod
     def _pad(n: int, b: int = 128) -> int:
@@ -133,11 +130,9 @@ class PolarQuantMoEMethod:
         c = down["codes"]
         layer.w2_codes.data[e] = (pack_codes_half_block(c) if self.w2_bits <= 4 else c).to(layer.w2_codes.device)
         layer.w2_norms.data[e] = down["norms"].to(layer.w2_norms.device)
-        layer.w13_tiles = layer.w2_tiles = None
 
     def process_weights_after_loading(self, layer) -> None:
         dev = layer.w13_codes.device
-        layer.w13_tiles = layer.w2_tiles = None
         layer.w13_ct_scaled = layer.w13_ct_scaled.to(dev)
         layer.w2_ct_scaled = layer.w2_ct_scaled.to(dev)
 
@@ -169,11 +164,10 @@ class PolarQuantMoEMethod:
         if plan is None:
             return None
         rpp, max_problems, tensor_cores = plan
-        tiled = not tensor_cores and self._decode_tiles(layer)
         return (nv._host or nv.host()).moe(
             x, a, b, renormalize, expert_map,
-            (layer.w13_codes, layer.w13_norms, layer.w13_ct_scaled, layer.w13_tiles if tiled else None, self.w13_bits <= 4),
-            (layer.w2_codes, layer.w2_norms, layer.w2_ct_scaled, layer.w2_tiles if tiled else None, self.w2_bits <= 4),
+            (layer.w13_codes, layer.w13_norms, layer.w13_ct_scaled, self.w13_bits <= 4),
+            (layer.w2_codes, layer.w2_norms, layer.w2_ct_scaled, self.w2_bits <= 4),
             (layer.moe_hidden, layer.moe_inter, layer.moe_hidden_padded, layer.moe_inter_padded), rpp, max_problems, tensor_cores)
 
     def _grouped_plan(self, pairs: int, n_local: int, expert_map, blocks: int) -> Optional[Tuple[int, int, bool]]:
@@ -222,23 +216,6 @@ class PolarQuantMoEMethod:
         n_global = int(expert_map.numel()) if expert_map is not None else n_local
         return max(1, pairs * n_local // max(n_global, 1))
 
-    def _decode_tiles(self, layer) -> bool:
-        """Whether the layer has tiled copies of its experts; builds them unless a graph is being captured."""
-        if not self.decode_tiled:
-            return False
-        if getattr(layer, "w13_tiles", None) is None:
-            if torch.cuda.is_current_stream_capturing():
-                return False
-            for name, bits in (("w13", self.w13_bits), ("w2", self.w2_bits)):
-                codes, norms = getattr(layer, name + "_codes").data, getattr(layer, name + "_norms").data
-                e, rows = codes.shape[:2]
-                if rows % 16 == 0 and codes.is_contiguous() and norms.is_contiguous():  # experts are whole tiles: one launch
-                    tiles = retile(codes.view(e * rows, -1), bits <= 4, norms.view(e * rows, -1))
-                else:
-                    tiles = torch.cat([retile(codes[i], bits <= 4, norms[i]) for i in range(e)])
-                setattr(layer, name + "_tiles", tiles)
-        return True
-
     def _moe_forward_grouped(self, layer, x, topk_weights, topk_ids, expert_map) -> Optional[torch.Tensor]:
         lead = x.shape[:-1]
         h, i = layer.moe_hidden, layer.moe_inter
@@ -273,9 +250,7 @@ class PolarQuantMoEMethod:
                  "pe_moe_plan")
         # many rows per expert: the tensor-core kernel over all experts (tile list built on the device);
         # few: the decode-size kernel, which streams every expert's codes once per 8 or 16 rows
-        tiled = not tensor_cores and self._decode_tiles(layer)
-
-        def grouped(codes, packed, norms, ct, xin, x_kind, x_rows, in_f, kp, y, tiles):
+        def grouped(codes, packed, norms, ct, xin, x_kind, x_rows, in_f, kp, y):
             if tensor_cores:
                 need = l.pe_gemm_grouped_workspace_bytes(n_local, pairs, codes.shape[1], kp)
                 ws = nv.gemm_workspace(dev, need)
@@ -289,13 +264,6 @@ class PolarQuantMoEMethod:
                     nv.check(l.pe_gemm_grouped(*head, None, y.data_ptr(), nv.dtype_code(y), *tail), "pe_gemm_grouped")
                 return
             ws = nv.grouped_scratch(dev, l.pe_gemv_grouped_workspace_bytes(max_problems, y.shape[1], kp))
-            if tiled:
-                nv.check(l.pe_gemv_grouped_tiled(tiles.data_ptr(), int(packed), tiles.numel() // n_local, ct.data_ptr(), ct.numel(),
-                                                 xin.data_ptr(), x_kind, nv.dtype_code(xin), xin.stride(0), in_f,
-                                                 x_rows.data_ptr() if x_rows is not None else None, y.data_ptr(), nv.dtype_code(y),
-                                                 y.stride(0), desc.data_ptr(), max_problems, rpp, y.shape[1], kp, ws.data_ptr(),
-                                                 ws.numel(), st), "pe_gemv_grouped_tiled")
-                return
             nv.check(l.pe_gemv_grouped(codes.data_ptr(), int(packed), codes.stride(1) * codes.element_size(),
                                        codes.stride(0) * codes.element_size(), norms.data_ptr(), norms.stride(1), norms.stride(0),
                                        ct.data_ptr(), ct.numel(), xin.data_ptr(), x_kind, nv.dtype_code(xin), xin.stride(0),
@@ -305,11 +273,10 @@ class PolarQuantMoEMethod:
         # Rows beyond the local pairs stay unused.  silu(gate) * up is computed inside the first tensor-core launch, or (decode
         # size) where the down projection's input is prepared.
         gu = torch.empty(pairs, i if tensor_cores else 2 * i, dtype=torch.float16, device=dev)
-        grouped(layer.w13_codes, self.w13_bits <= 4, layer.w13_norms, layer.w13_ct_scaled, x2, nv.PE_X_RAW, tok_sorted, h, hp, gu,
-                layer.w13_tiles if tiled else None)
+        grouped(layer.w13_codes, self.w13_bits <= 4, layer.w13_norms, layer.w13_ct_scaled, x2, nv.PE_X_RAW, tok_sorted, h, hp, gu)
         d = torch.empty(pairs, h, dtype=torch.float32, device=dev)
         grouped(layer.w2_codes, self.w2_bits <= 4, layer.w2_norms, layer.w2_ct_scaled, gu, nv.PE_X_RAW if tensor_cores else nv.PE_X_SILU_MUL,
-                None, i, ip, d, layer.w2_tiles if tiled else None)
+                None, i, ip, d)
         out = torch.empty(t, h, dtype=torch.float16, device=dev)
         wts = topk_weights.reshape(-1).to(torch.float32).contiguous()
         nv.check(l.pe_moe_combine(d.data_ptr(), d.stride(0), pos.data_ptr(), wts.data_ptr(), t, k, out.data_ptr(), nv.PE_F16,

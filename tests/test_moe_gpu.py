@@ -245,3 +245,30 @@ def test_grouped_tiled_silu_input_equals_row_major(bits, inter, h):
     a = act.cpu()
     ref = torch.cat([oracle.linear_dequant(a[first[i]:first[i] + s], *layers[i], in_f=inter) for i, s in enumerate(sizes) if s])
     assert max_rel(out[0], ref) <= 1e-2
+
+
+@pytest.mark.parametrize("tokens", [1, 6])
+def test_experts_have_one_copy_of_their_weights(tokens):
+    """Decode-size batches multiply by what the experts' arrays hold at the call -- rewritten in place included, the first
+    call inside a capture included -- and leave no further memory with the layer."""
+    e, h, i, top_k = 16, 640, 384, 4
+    method, layer, _ = build_random_codes(e, h, i, seed=1)
+    _, other, experts = build_random_codes(e, h, i, seed=7)
+    g = torch.Generator().manual_seed(tokens)
+    x = torch.randn(tokens, h, generator=g).half()
+    w, ids = oracle.moe_route(x, (torch.randn(e, h, generator=g) * 0.02).half(), top_k)
+    xd, wd, idd = x.cuda(), w.cuda(), ids.cuda()
+    want = method.apply(other, xd, wd, idd)
+    assert max_rel(want, oracle.moe_forward(x, w, ids, experts)) <= 1e-2
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        held = method.apply(layer, xd, wd, idd)  # the layer's first call
+    graph.replay()
+    y = method.apply(layer, xd, wd, idd)
+    assert torch.equal(y, held)
+    for name in ("w13_codes", "w13_norms", "w2_codes", "w2_norms"):
+        getattr(layer, name).data.copy_(getattr(other, name).data)
+    assert torch.equal(method.apply(layer, xd, wd, idd), want)
+    graph.replay()
+    assert torch.equal(held, want)
+    assert not [k for k, v in vars(layer).items() if torch.is_tensor(v)]  # parameters and buffers only
