@@ -26,7 +26,7 @@ import torch.nn.functional as F
 
 from .decode_ops import add_rmsnorm, decode_attention, rope_attention, rope_cache, silu_mul
 from . import _native as nv
-from .kernels import GEMV_MAX_BATCH, quant_embedding, quant_matmul, quant_matmul_pro, retile
+from .kernels import GEMV_MAX_BATCH, quant_embedding, quant_matmul, quant_matmul_pro
 from .packing import pack_codes_half_block
 from .parallel import PeerExchange, shard_codes_for_tp, shard_norms_for_tp
 from .utils import get_centroids, get_ct_scaled
@@ -74,28 +74,19 @@ class QWeight:
         self.norms = norms.contiguous()
         self.ct = get_ct_scaled(bits).to(codes.device)
         self.out_f, self.in_f = codes.shape
-        self.tiles = None  # streaming copy for batches of up to 16 rows, built the first time one arrives
 
     @classmethod
     def synthetic(cls, out_f: int, in_f: int, bits: int, dev, gen: torch.Generator) -> "QWeight":
         return cls(*synth_weight(out_f, in_f, bits, dev, gen), bits)
 
     def fused(self, prologue: int, x: torch.Tensor, out_dtype=torch.float16, **kw) -> Optional[torch.Tensor]:
-        """One token with the glue op in front of the projection folded into the launch; None if the layer's
-        shape is not one the batch-1 kernel takes."""
-        self._make_tiles(1)
+        """One token with the glue op in front of the projection folded into the launch; None for a layer too small to
+        gain from it."""
         return quant_matmul_pro(self.codes, self.packed, self.norms, self.ct, prologue, x, self.in_f, self.out_f, self.in_f,
-                                out_dtype, tiles=self.tiles, **kw)
-
-    def _make_tiles(self, rows: int) -> None:
-        if self.tiles is None and 1 <= rows <= GEMV_MAX_BATCH and not torch.cuda.is_current_stream_capturing():
-            self.tiles = retile(self.codes, self.packed, self.norms)
+                                out_dtype, **kw)
 
     def __call__(self, x: torch.Tensor, out_dtype=torch.float16) -> torch.Tensor:
-        self._make_tiles(x.shape[0])
-        return quant_matmul(self.codes, self.packed, self.norms, self.ct, x, False, self.out_f, self.in_f, self.in_f, out_dtype,
-                            tiles=self.tiles)
-
+        return quant_matmul(self.codes, self.packed, self.norms, self.ct, x, False, self.out_f, self.in_f, self.in_f, out_dtype)
 
     def of_gate_up(self, gate_up: torch.Tensor, out_dtype=torch.float16) -> torch.Tensor:
         """The matmul of silu(gate) * up; more rows than a decode batch compute the product while they are prepared."""

@@ -82,3 +82,22 @@ def test_folded_glue_ops_give_the_same_tokens():
         assert float((la - lb).abs().max() / lb.abs().max()) <= 5e-3
         assert torch.equal(la.argmax(-1), lb.argmax(-1))
         ids = lb.argmax(-1).view(1, 1)
+
+
+def test_a_decoder_weight_has_one_copy():
+    """Codes and norms rewritten in place are what the next token is multiplied by, folded prologues included, and a
+    decode step leaves no further memory with the weight."""
+    from polarengine_vllm_b200 import _native as nv
+    from polarengine_vllm_b200.decoder import QWeight
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a, b = (QWeight.synthetic(2048, 2048, 4, "cuda", g) for _ in range(2))
+    x, lnw = torch.randn(1, 2048, device="cuda", generator=g).half(), torch.ones(2048, dtype=torch.float16, device="cuda")
+    calls = (lambda w: w(x), lambda w: w.fused(nv.PE_PRO_ADD_RMSNORM, x, norm_weight=lnw, eps=1e-6))
+    want = [c(b) for c in calls]
+    first = [c(a) for c in calls]
+    held = {k for k, v in vars(a).items() if torch.is_tensor(v)}
+    a.codes.copy_(b.codes)
+    a.norms.copy_(b.norms)
+    for c, y, old in zip(calls, want, first):
+        assert torch.equal(c(a), y) and not torch.equal(y, old)
+    assert held == {"codes", "norms", "ct"}
