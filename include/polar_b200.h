@@ -176,6 +176,9 @@ int pe_pack_nibble(const int8_t* codes, uint8_t* packed, int64_t out_f, int64_t 
  *           device.  pe_gemv_status() waits for the stream and returns the word (0 = ok),
  *           clearing it when `clear` is non-zero.
  *
+ * In a stream capture, calls recorded one behind the other read their layers' arrays early: a
+ * layer's arrays must not be the output (y) of another call in front of it in the capture.
+ *
  * Replaces polar_matmul's batch==1 branches and (for 2..16 rows) its GEMM branch
  * (polar_gemm.py:485-534), plus the cast/bias epilogue of linear_method.py:214-221. */
 size_t pe_gemv_workspace_bytes(int batch, int out_f, int in_f_padded);

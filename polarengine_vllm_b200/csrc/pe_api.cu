@@ -8,6 +8,37 @@ thread_local int g_last_cuda_error = 0;
 static long long g_wait_limit_cycles = 2000000000ll;  // about one second at 2 GHz
 long long wait_limit_cycles() { return g_wait_limit_cycles; }
 
+static thread_local unsigned long long g_line_capture = 0;  // capture the thread's line belongs to, 0: none
+static thread_local cudaGraphNode_t g_line_last = nullptr;
+
+// the single node that the stream's next launch will follow; false outside a capture or if there are several
+static bool capture_tip(cudaStream_t stream, unsigned long long* id, cudaGraphNode_t* node) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  const cudaGraphNode_t* deps = nullptr;
+  const cudaGraphEdgeData* edges = nullptr;
+  size_t n = 0;
+  if (cudaStreamGetCaptureInfo_v3(stream, &status, id, nullptr, &deps, &edges, &n) != cudaSuccess) {
+    cudaGetLastError();  // a question, not a launch: leave no error behind
+    return false;
+  }
+  if (status != cudaStreamCaptureStatusActive || n != 1) return false;
+  *node = deps[0];
+  return true;
+}
+
+bool line_holds(cudaStream_t stream) {
+  if (!g_line_capture) return false;
+  unsigned long long id = 0;
+  cudaGraphNode_t tip = nullptr;
+  if (capture_tip(stream, &id, &tip) && id == g_line_capture && tip == g_line_last) return true;
+  g_line_capture = 0;
+  return false;
+}
+
+void line_extend(cudaStream_t stream) {
+  if (!capture_tip(stream, &g_line_capture, &g_line_last)) g_line_capture = 0;
+}
+
 int sm_count() {
   static int cached[64] = {0};
   int dev = 0;

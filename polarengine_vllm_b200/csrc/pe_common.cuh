@@ -26,6 +26,15 @@ inline int cuda_fail(cudaError_t e) {
 int sm_count();  // SM count of the current device (cached per device)
 long long wait_limit_cycles();  // limit of device-side waits on another party (pe_set_wait_limit_us)
 
+// ---- a line of launches inside a stream capture ------------------------------
+// While a stream is captured, the node its next launch will depend on is known.  If that is the node of this thread's last
+// programmatic launch alone, nothing was recorded between the two: they are in one line.  A line begins with a matmul whose
+// preparation launch waited for everything older before it let the matmul start, and its kernels write activations and
+// scratch, never a layer's arrays (the kernels that do are ordinary launches, which end a line).  So the arrays of any later
+// matmul of the line were complete when the line began, and may be read before the launches in front are done.
+bool line_holds(cudaStream_t stream);   // the next launch on the stream would be in this thread's line
+void line_extend(cudaStream_t stream);  // the node just recorded is the line's last; begins a line if there was none
+
 // Launch with programmatic stream serialization: the grid may start while its predecessor
 // in the stream is still draining.  The kernel must call pdl_enter() (or its own
 // griddepcontrol.wait) before it touches anything the predecessor reads or writes.  That wait covers the predecessor
@@ -43,7 +52,10 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  const bool line = line_holds(stream);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  if (line && e == cudaSuccess) line_extend(stream);
+  return e;
 }
 
 // ---- small device helpers ----------------------------------------------------

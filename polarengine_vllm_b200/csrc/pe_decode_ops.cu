@@ -750,7 +750,9 @@ static int attention_launch(AttArgs a, int batch, int head_dim, void* stream) {
       if (dev < 16) configured[dev] = true;
     }
   }
+  const bool line = line_holds(cfg.stream);
   PE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kfn, a));
+  if (line) line_extend(cfg.stream);
   return PE_OK;
 }
 

@@ -3,7 +3,7 @@
 //   y[m, r] = sum_blk norm[r, blk] * sum_k ct[code[r, blk, k]] * xt[m, blk, k]   (+ bias[r])
 //
 // Every call goes to the bulk-copy kernel (pe_gemv_bulk.cu), whichever layout it has: a decoder layer's four launches for
-// one row take 48.5 us on row-major arrays, 48.2 us on the tiled copy, and 52.0 us in the column-owner kernel
+// one row take 40.3 us on row-major arrays, 42.9 us on the tiled copy, and 52.0 us in the column-owner kernel
 // (pe_gemv_cols.cu), which is left for pe_gemv_pro, whose callers give no scratch memory.
 #include "pe_gemv_decode.cuh"
 
@@ -92,7 +92,7 @@ static int gemv_run(const void* codes, int packed, int64_t ld_codes, const void*
                        bias, batch, out_f, in_f_padded, workspace, workspace_bytes, stream);
 }
 
-// The row-major arrays stream as fast as the tiled copy (8 rows, a decoder layer's four launches: 51.2 and 51.8 us).
+// The row-major arrays stream as fast as the tiled copy (8 rows, a decoder layer's four launches: 44.7 and 47.0 us).
 extern "C" int pe_gemv_small_batch_takes(int, int64_t, const void*, int64_t, int, int) { return 1; }
 
 extern "C" int pe_gemv(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms,

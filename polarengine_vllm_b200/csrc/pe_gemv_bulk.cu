@@ -7,8 +7,7 @@
 // copies (of the row-major layout one or a few rows each, of the tiled layout of pe_retile, whose records are contiguous, one
 // per stage); norms of row-major layers are a strided gather of halves that no bulk copy does, so the norm warp loads them
 // (two stages under way) and stores them beside the codes.  Both start while the activations are prepared: the dependency wait
-// of the programmatic launch is the math warps' alone (gemv_frags_kernel lets this kernel start once the launches before both
-// are done).  (Without a copy warp -- the last warp to finish with a stage refills it, 128 instead of 96 registers -- the
+// of the programmatic launch is the math warps' alone (gemv_frags_kernel lets this kernel start once what it reads is there).  (Without a copy warp -- the last warp to finish with a stage refills it, 128 instead of 96 registers -- the
 // refills came later and every warp had to track them: 4 us over four launches.  Norms loaded by the math warps at the head of
 // every pass: 8 us.  Two or three norm warps that take stages in turn are unsound: a wait on a barrier's parity holds only for
 // a waiter that took every earlier phase itself.)
@@ -27,13 +26,16 @@
 //    them in registers.  Rotating inside this kernel was measured too (in registers, 16-point part by MMAs): its
 //    straight-line code cost more in instruction fetches than the extra launch, 13 us over a layer's four launches.
 //    The registers left over let the small launch's blocks be resident, waiting, while the launch before it still runs.
-// Measured, row-major layout, launches of a dependent chain under a CUDA graph, weights from HBM (in brackets the tiled layout):
+// Measured, row-major layout, a line of launches under a CUDA graph, weights from HBM (in brackets the tiled layout):
 //   activation rows      1              8              16
-//   6144 x 4096 Q5    11.1 (11.6)    11.3 (11.8)    13.1 (15.3) us
-//   4096 x 4096 Q6     8.7  (9.3)     9.2  (9.5)     9.5 (11.0)
-//   24576 x 4096 Q3   15.9 (15.0)    17.7 (17.7)    29.2 (28.8)
-//   4096 x 12288 Q4   11.5 (12.4)    12.3 (12.9)    16.2 (16.8)
-//   the four in turn  48.5 (48.2)    51.2 (51.8)    68.6 (71.7)
+//   6144 x 4096 Q5     9.2 (10.1)     9.5 (10.1)    12.4 (14.2) us
+//   4096 x 4096 Q6     7.2  (8.0)     7.5  (8.1)     8.8  (9.8)
+//   24576 x 4096 Q3   14.0 (15.0)    16.2 (16.8)    28.3 (28.3)
+//   4096 x 12288 Q4   10.1 (10.8)    11.3 (11.8)    15.9 (16.0)
+//   the four in turn  40.3 (42.9)    44.7 (47.0)    65.5 (67.6)
+// Inside the ring's steady state the 24576 x 4096 launch moves 4.9 TB/s; the rest is the launch's own latency: about
+// 3.5 us from the launch before it to the first product, 0.5 us from the last one to the stores.  Outside a line (launched
+// eagerly, or with other kernels in between) the ring fills about 2 us later: the four in turn take 48.5, 51.2 and 68.6 us.
 //
 // The tiles of all problems of a launch form one line that is cut into equal contiguous ranges, one per CTA; nothing
 // crosses CTAs.  The sixteen warps' partial sums of a tile go through shared memory and are added in warp order: bit-
@@ -186,6 +188,7 @@ struct FragArgs {
   const void* x; int x_kind, x_dtype; int64_t ld_x; int in_f, nb, batch, sets;  // sets of eight rows per problem
   uint4* out;
   const int4* grp; const int32_t* x_rows;
+  int in_line;
   // one row, fp16: the residual add and the norm in front of the projection (PE_PRO_ADD_RMSNORM)
   const void* delta; int delta_dtype; const __half* norm_w; __half* resid_out; float eps;
 };
@@ -211,9 +214,12 @@ __device__ __forceinline__ void residual4(const FragArgs& p, const Raw4& x, cons
 template <bool PACKED, bool NORM>
 __global__ void __launch_bounds__(kFragThreads) gemv_frags_kernel(const FragArgs p) {
   // The wait first: the matmul behind reads codes, norms and table before its own wait, which covers this launch only, so
-  // what older kernels wrote (a layer just loaded, arrays rewritten in place) has to be visible before it may start.
+  // what older kernels wrote (a layer just loaded, arrays rewritten in place) has to be visible before it may start.  In a
+  // line of captured launches it was when the line began (line_holds), and the ring of the matmul fills while the launch in
+  // front still runs: four launches for one row 48.5 us without, 40.2 us with.
+  if (p.in_line) asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;");
+  if (!p.in_line) asm volatile("griddepcontrol.launch_dependents;");
   const int lane = threadIdx.x & 31, job = blockIdx.x * (kFragThreads / 32) + (threadIdx.x >> 5);
   const int m = job / p.nb, b = job - m * p.nb, prob = blockIdx.y;
   if (!NORM && m >= p.batch) return;
@@ -659,6 +665,7 @@ int gemv_bulk_run(const GemvBulkCall& q, cudaStream_t st) {
   f.grp = static_cast<const int4*>(q.problems); f.x_rows = q.x_rows;
   f.delta = q.delta; f.delta_dtype = q.delta_dtype; f.norm_w = static_cast<const __half*>(q.norm_w);
   f.resid_out = static_cast<__half*>(q.resid_out); f.eps = q.eps;
+  f.in_line = line_holds(st);
   const int warps = kFragThreads / 32;
   const dim3 grid((q.batch * f.nb + warps - 1) / warps, q.problems ? q.max_problems : 1);
   auto frags = q.pro == PE_PRO_ADD_RMSNORM ? (q.packed ? gemv_frags_kernel<true, true> : gemv_frags_kernel<false, true>)
@@ -676,8 +683,10 @@ int gemv_bulk_run(const GemvBulkCall& q, cudaStream_t st) {
   a.status = q.status;
   a.grp = f.grp; a.n_problems = q.max_problems;
   a.codes_stride = q.codes_stride; a.norms_stride = q.norms_stride; a.tiles_stride = q.tiles_stride;
-  if (q.packed) return q.tiles ? launch_bulk_kind<true, true>(a, sms, st) : launch_bulk_kind<true, false>(a, sms, st);
-  return q.tiles ? launch_bulk_kind<false, true>(a, sms, st) : launch_bulk_kind<false, false>(a, sms, st);
+  const int rc = q.packed ? (q.tiles ? launch_bulk_kind<true, true>(a, sms, st) : launch_bulk_kind<true, false>(a, sms, st))
+                          : (q.tiles ? launch_bulk_kind<false, true>(a, sms, st) : launch_bulk_kind<false, false>(a, sms, st));
+  if (rc == PE_OK && !f.in_line) line_extend(st);
+  return rc;
 }
 
 }  // namespace pe

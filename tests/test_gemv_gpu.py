@@ -384,3 +384,34 @@ def test_a_linear_layer_has_one_copy_of_its_weights(bits):
     assert max_rel(method.apply(layer, x), ref[1]) <= TOL
     graph.replay()
     assert max_rel(held, ref[1]) <= TOL
+
+
+@pytest.mark.parametrize("rows", [1, 16])
+def test_a_captured_line_of_matmuls(rows):
+    """Calls recorded one behind the other overlap in the replay; an ordinary kernel between two of them, a rewrite of the
+    next layer's arrays included, ends the line.  Every output as the same calls give it one by one."""
+    from polarengine_vllm_b200 import kernels, packing
+    k, layers = 2048, []
+    for i, (bits, n) in enumerate([(4, 2048), (6, 2048), (3, 4112), (5, 48)] * 2):
+        codes, norms, ct = rand_layer(n, k, bits, seed=i)
+        layers.append((packing.pack_codes_half_block(codes.cuda()) if bits <= 4 else codes.cuda(), bits <= 4, norms.cuda(), ct.cuda(), n))
+    x = rand_x(rows, k, seed=3).cuda()
+
+    def step(rewrite):
+        out = []
+        for i, (w, packed, m, ct, n) in enumerate(layers):
+            if i == rewrite:
+                torch.mul(m, 2, out=m)
+            out.append(kernels.quant_matmul(w, packed, m, ct, x, False, n, k, k, torch.float32))
+        return out
+    want = [y.clone() for y in step(None)]
+    for rewrite in (None, 0, 3):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = step(rewrite)
+        for times in range(1, 4):
+            graph.replay()
+            for i, (a, b) in enumerate(zip(got, want)):
+                assert torch.equal(a, b * 2 ** times if i == rewrite else b)
+        if rewrite is not None:
+            layers[rewrite][2].div_(8)
