@@ -5,12 +5,13 @@
 // One persistent CTA per SM: sixteen math warps, a copy warp and, for row-major codes, a norm warp.  A stage of the shared-
 // memory ring is one 16-row tile of the weight matrix by up to 32 quantization blocks.  The copy warp fills stages with bulk
 // copies (of the row-major layout one or a few rows each, of the tiled layout of pe_retile, whose records are contiguous, one
-// per stage); norms of row-major layers are a strided gather of halves that no bulk copy does, so the norm warp loads them
-// (two stages under way) and stores them beside the codes.  Both start while the activations are prepared: the dependency wait
-// of the programmatic launch is the math warps' alone (gemv_frags_kernel lets this kernel start once what it reads is there).  (Without a copy warp -- the last warp to finish with a stage refills it, 128 instead of 96 registers -- the
-// refills came later and every warp had to track them: 4 us over four launches.  Norms loaded by the math warps at the head of
-// every pass: 8 us.  Two or three norm warps that take stages in turn are unsound: a wait on a barrier's parity holds only for
-// a waiter that took every earlier phase itself.)
+// per stage).  Norms of row-major layers are a strided gather of halves: the norm warp loads them, two stages under way (with
+// four its registers spill and 128 experts take 382 instead of 351 us), and stores them beside the codes.  Both warps start
+// while the activations are prepared: the dependency wait of the programmatic launch is the math warps' alone
+// (gemv_frags_kernel lets this kernel start once what it reads is there).  (Without a copy warp -- the last warp to finish with
+// a stage refills it, 128 instead of 96 registers -- the refills came later and every warp had to track them: 4 us over four
+// launches.  Norms loaded by the math warps at the head of every pass: 8 us.  There is one norm warp, not several taking stages
+// in turn: a wait on a barrier's parity holds only for a waiter that took every earlier phase itself.)
 //
 // What bounds it: once the ring runs, the shared-memory port.  A warp takes block cw, cw + 16 of every stage:
 //  * centroid lookup: the table is replicated per lane at a spacing of 256 bytes per entry, so that ONE byte permute
@@ -67,6 +68,7 @@ struct BulkArgs {
   int part_rows;                           // activation rows the partial sums have room for
   int part_off, stage_off, stage_bytes;
   int row_stride, copy_rows;               // row-major layout: bytes between rows of a stage, weight rows per bulk copy
+  int norm_stride;                         // grouped, row-major: bytes between the norms of two rows where a stage's are one bulk copy, else 0
   int* status;
   // grouped launch: problem i multiplies rows grp[i].y .. + grp[i].z of the row list with matrix grp[i].x
   const int4* grp; int n_problems;
@@ -325,6 +327,7 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
   extern __shared__ __align__(128) uint8_t smem[];  // no static shared memory: the window starts with it
   constexpr int kRowBytes = PACKED ? 64 : 128;           // codes of one row's block
   constexpr int kRecBytes = kRowBytes * 16 + 32;         // tiled record: 16 rows of a block, then their norms
+  const bool norms_copied = !TILED && GROUPED && p.norm_stride;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
   const uint32_t sbase = smem_u32(smem);
   const uint32_t full = sbase, empty = sbase + 8 * kBulkMaxStages;
@@ -335,7 +338,7 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
     return;
   }
   if (tid == 0) {
-    for (int s = 0; s < p.n_stage; ++s) { bar_init(full + 8 * s, TILED ? 1 : 2); bar_init(empty + 8 * s, kBulkWarps); }
+    for (int s = 0; s < p.n_stage; ++s) { bar_init(full + 8 * s, TILED || norms_copied ? 1 : 2); bar_init(empty + 8 * s, kBulkWarps); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     n_live = 0;
   }
@@ -362,11 +365,13 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
     while (ps.next(p)) {
       const uint8_t* codes = p.codes;
       const uint8_t* tiles = p.tiles;
+      const __half* norms = p.norms;
       if (GROUPED) {
         const int4 d = p.grp[ps.prob];
         if (d.z <= 0) continue;
         codes += d.x * p.codes_stride;
         tiles += d.x * p.tiles_stride;
+        norms += d.x * p.norms_stride;
       }
       for (int c = 0; c < p.n_chunk; ++c) {
         const int b0 = c * p.chunk_blocks, nblk = min(p.chunk_blocks, p.nb - b0);
@@ -380,7 +385,8 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
             } else {
               const int rows = min(16, ps.rows - r0);
               const uint8_t* src = codes + (int64_t)(ps.row0 + r0) * p.ld_codes + b0 * kRowBytes;
-              bar_expect(bar, rows * nblk * kRowBytes);
+              bar_expect(bar, rows * (nblk * kRowBytes + (norms_copied ? p.norm_stride : 0)));
+              if (norms_copied) bulk_load(dst + 16 * p.row_stride + 64, norms + (int64_t)(ps.row0 + r0) * p.nb, rows * p.norm_stride, bar);
               for (int r = 0; r < rows; r += p.copy_rows)
                 bulk_load(dst + r * p.row_stride + (r >> 3) * 64, src + r * p.ld_codes, min(p.copy_rows, rows - r) * nblk * kRowBytes, bar);
             }
@@ -393,6 +399,7 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
     return;
   }
 
+  if (!TILED && w > kBulkWarps && norms_copied) return;
   if (!TILED && w > kBulkWarps) {  // ---- norm warp: a stage's norms, the 16 rows of a block side by side
     constexpr int kPlaces = kBulkWarps * BPW, kLaneRows = 16 * kPlaces / 32;
     const int b = lane % kPlaces, r_lane = lane / kPlaces * kLaneRows, blocks = min(p.nb, p.chunk_blocks);
@@ -487,8 +494,9 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
   const int row_a = TILED ? g : (g >> 1) + (g & 1) * 8;
   const uint32_t at_a = TILED ? w * kRecBytes + g * kRowBytes + t * 16 : row_a * p.row_stride + (g & 1) * 64 + w * kRowBytes + t * 16;
   const uint32_t at_b = at_a + kRowB * (TILED ? kRowBytes : p.row_stride);
-  const uint32_t at_n = TILED ? w * kRecBytes + 16 * kRowBytes + g * 2 : 16 * p.row_stride + 64 + w * 32 + row_a * 2;
-  constexpr int kStep = kBulkWarps * (TILED ? kRecBytes : kRowBytes), kNormStep = kBulkWarps * (TILED ? kRecBytes : 32);
+  const uint32_t at_n = TILED ? w * kRecBytes + 16 * kRowBytes + g * 2 : 16 * p.row_stride + 64 + (norms_copied ? w * 2 + row_a * p.norm_stride : w * 32 + row_a * 2);
+  constexpr int kStep = kBulkWarps * (TILED ? kRecBytes : kRowBytes);
+  const int norm_step = kBulkWarps * (TILED ? kRecBytes : norms_copied ? 2 : 32), norm_b = kRowB * (norms_copied ? p.norm_stride : 2);
   const uint32_t lane4 = lane * 4;
   float* part = reinterpret_cast<float*>(smem + p.part_off);
   uint32_t x[BPW][NT][16];
@@ -541,8 +549,8 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
           if (blk < nblk) {
             float d[NT][4];
             unsigned short ha, hb;
-            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(ha) : "r"(st + at_n + j * kNormStep));
-            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hb) : "r"(st + at_n + j * kNormStep + kRowB * 2));
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(ha) : "r"(st + at_n + j * norm_step));
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hb) : "r"(st + at_n + j * norm_step + norm_b));
             block_product<PACKED, NT>(st + at_a + j * kStep, st + at_b + j * kStep, x[j], lane4, d);
             const float fa = __half2float(__ushort_as_half(ha)), fb = __half2float(__ushort_as_half(hb));
 #pragma unroll
@@ -613,6 +621,12 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
   a.copy_rows = 1;
   if (a.n_chunk == 1 && a.ld_codes == a.row_stride)
     while (a.copy_rows < 8 && a.copy_rows * a.row_stride < 2048) a.copy_rows *= 2;
+  // Grouped launches meet new rows all the time, and the norm warp's sixteen loads a stage are what paces them: where the norms of
+  // a tile follow each other and their bytes are whole 16s, they come as one more bulk copy (128 experts, 2688 -> 2 x 1856, 64
+  // tokens: 354 and 349 us; one token 41.1 and 39.0).  Their rows then share banks where the block count is even, which the
+  // long rows of a dense layer feel more than the loads (24576 x 4096 at 8 rows: 16.4 us by the norm warp, 17.0 copied).
+  a.norm_stride = GROUPED && !TILED && a.n_chunk == 1 && a.ld_norms == a.nb && (reinterpret_cast<uintptr_t>(a.norms) & 15) == 0 &&
+                  a.norms_stride % 8 == 0 && (a.N % 16) * a.nb % 8 == 0 ? a.nb * 2 : 0;
   a.stage_bytes = TILED ? (blocks * kRecBytes + 127) & ~127 : (16 * a.row_stride + 64 + blocks * 32 + 127) & ~127;
   for (int cap = a.part_rows <= 2 ? 256 : (NT == 1 ? 64 : 32);; cap /= 2) {
     if (cap < 16) return PE_ERR_LIMIT;

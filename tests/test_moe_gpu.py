@@ -272,3 +272,35 @@ def test_experts_have_one_copy_of_their_weights(tokens):
     graph.replay()
     assert torch.equal(held, want)
     assert not [k for k, v in vars(layer).items() if torch.is_tensor(v)]  # parameters and buffers only
+
+
+@pytest.mark.parametrize("rows,kp,bits", [(257, 384, 4), (40, 1024, 3), (33, 1152, 5), (16, 4224, 4), (8, 640, 6)])
+def test_grouped_norms_however_they_lie(rows, kp, bits):
+    """pe_gemv_grouped with the norms of a tile in one piece (a last tile whose norms are not whole 16 bytes, or two K
+    ranges, excepted) and with a gap between rows, between experts, or at an odd address: the same bits, and the oracle's
+    values."""
+    from polarengine_vllm_b200 import _native as nv, packing
+    sizes, dev, packed = (3, 0, 8), torch.device("cuda"), bits <= 4
+    nv.ensure_init(dev)
+    lib, nb = nv.lib(), kp // 128
+    layers = [rand_layer(rows, kp, bits, seed=i) for i in range(len(sizes))]
+    codes = torch.stack([packing.pack_codes_half_block(c.cuda()) if packed else c.cuda() for c, _, _ in layers])
+    dense, ct = torch.stack([m for _, m, _ in layers]).cuda(), layers[0][2].cuda()
+    first, total = [0, 3, 3], sum(sizes)
+    prob = torch.tensor([[i, first[i], s, 0] for i, s in enumerate(sizes)], dtype=torch.int32).cuda()
+    x = rand_x(total, kp, seed=3).cuda()
+    ws = nv.grouped_scratch(dev, lib.pe_gemv_grouped_workspace_bytes(len(sizes), rows, kp))
+    out = []
+    for gap_row, gap_expert, shift in ((0, 0, 0), (1, 0, 0), (0, 3, 0), (0, 0, 1)):
+        buf = torch.full((len(sizes) * (rows * (nb + gap_row) + gap_expert) + 8,), float("nan"), dtype=torch.float16, device=dev)
+        m = torch.as_strided(buf, (len(sizes), rows, nb), (rows * (nb + gap_row) + gap_expert, nb + gap_row, 1), shift)
+        m.copy_(dense)
+        y = torch.zeros(total, rows, device=dev)
+        nv.check(lib.pe_gemv_grouped(codes.data_ptr(), int(packed), codes.stride(1), codes.stride(0), m.data_ptr(), m.stride(1), m.stride(0),
+                                     ct.data_ptr(), ct.numel(), x.data_ptr(), nv.PE_X_RAW, nv.dtype_code(x), x.stride(0), kp, None, y.data_ptr(),
+                                     nv.PE_F32, rows, prob.data_ptr(), len(sizes), 8, rows, kp, ws.data_ptr(), ws.numel(), nv.stream_ptr(dev)),
+                 "pe_gemv_grouped")
+        out.append(y)
+    ref = torch.cat([oracle.linear_dequant(x.cpu()[first[i]:first[i] + s], *layers[i]) for i, s in enumerate(sizes) if s])
+    assert max_rel(out[0], ref) <= 1e-2
+    assert all(torch.equal(out[0], y) for y in out[1:])
