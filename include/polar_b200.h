@@ -69,6 +69,13 @@ const char* pe_error_string(int code);
 /* cudaError_t of the last failing runtime call made by this library on this thread */
 int pe_last_cuda_error(void);
 
+/* Every wait inside a kernel is bounded.  One that ran out leaves the output of its launch undefined and a status value
+ * in the launch's scratch, and in a word of the device that this reads: 0 if no wait of this library has run out on the
+ * current device since the word was last cleared, else a status value that one left (whichever launch, stream, captured
+ * graph or scratch it was).  Waits for `stream`, so call it outside captures; clears the word when `clear` is non-zero.
+ * Negative: an error code. */
+int pe_wait_status(int clear, void* stream);
+
 /* Kernels that wait on another party (a peer rank's flag in pe_allreduce_add_rmsnorm) give up after a limit, record a status value and return, so that a
  * missing peer costs a bounded time and never a hung GPU.  The default is about one second; this
  * sets it for launches made afterwards (process-wide).  No counterpart in the reference. */

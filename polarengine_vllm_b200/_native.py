@@ -29,6 +29,7 @@ SIGNATURES = {
     "pe_last_cuda_error": (_i, []),
     "pe_init": (_i, [_i]),
     "pe_set_wait_limit_us": (_i, [_i64]),
+    "pe_wait_status": (_i, [_i, _vp]),
     "pe_fwht128": (_i, [_vp, _i, _i64, _vp, _i, _i64, _i, _i, _i, _vp]),
     "pe_embedding": (_i, [_vp, _i, _i64, _vp, _i64, _vp, _i, _vp, _i64, _vp, _i, _i64, _i, _i, _i, _vp]),
     "pe_quantize": (_i, [_vp, _i, _i64, _i64, _i, _i, _vp, _i, _vp, _i64, _vp, _i64, _vp]),
@@ -154,6 +155,17 @@ def ensure_init(device: torch.device) -> None:
     if idx not in _inited:
         check(lib().pe_init(idx), "pe_init")
         _inited.add(idx)
+
+
+def wait_status(device: Optional[torch.device] = None, clear: bool = True) -> int:
+    """0, or a status value that a bounded wait inside a kernel left on the device since the last clear: the output of that
+    launch is undefined.  Covers every launch of the library, those of captured graphs and of the native host path
+    included, whose scratch the caller does not see.  Waits for the current stream."""
+    with torch.cuda.device(device if device is not None else torch.cuda.current_device()):
+        v = lib().pe_wait_status(int(clear), torch.cuda.current_stream().cuda_stream)
+    if v < 0:
+        check(v, "pe_wait_status")
+    return v
 
 
 # one scratch buffer per (device, stream); zero-filled once, kernels leave it zeroed

@@ -1,5 +1,5 @@
 // Library-wide entry points: version, error strings, per-device set-up.
-#include "pe_common.cuh"
+#include "pe_status.cuh"
 
 namespace pe {
 thread_local int g_last_cuda_error = 0;
@@ -67,6 +67,17 @@ extern "C" const char* pe_error_string(int code) {
     case PE_ERR_LIMIT: return "size beyond a compiled-in maximum";
     default: return "unknown error";
   }
+}
+
+extern "C" int pe_wait_status(int clear, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  int first = 0;
+  for (auto read : {pe::gemv_wait_status, pe::gemm_tmem_wait_status, pe::gemm_wait_status, pe::comm_wait_status}) {
+    const int v = read(clear, st);
+    if (v < 0) return v;
+    if (first == 0) first = v;
+  }
+  return first;
 }
 
 extern "C" int pe_set_wait_limit_us(int64_t microseconds) {

@@ -19,7 +19,7 @@
 // memory (graph replays advance it): a rank can be at most one call ahead of a peer,
 // because finishing a call needs every peer's flag of that call.
 // No multicast, no TMA: ordinary loads and stores on peer-mapped addresses.
-#include "pe_common.cuh"
+#include "pe_status.cuh"
 
 namespace pe {
 
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kArThreads) allreduce_add_rmsnorm_kernel(const
     const long long t0 = clock64();
     while ((int)(ld_acquire_sys(flag) - s) < 0) {
       if (clock64() - t0 > wait_limit) {  // about a second unless the host set another limit: a peer never arrived
-        atomicExch(status, 1);
+        record_timeout(status, 1);
         break;
       }
     }
@@ -138,6 +138,8 @@ __global__ void __launch_bounds__(kArThreads) allreduce_add_rmsnorm_kernel(const
   }
   if (tid == 0) seq[row] = s;
 }
+
+PE_WAIT_STATUS_READER(comm_wait_status)
 
 }  // namespace pe
 

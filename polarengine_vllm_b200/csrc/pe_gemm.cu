@@ -109,7 +109,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
     if (*abort_flag) return false;
     if (clock64() - t0 > kTimeoutCycles) {
       *abort_flag = 1;
-      atomicCAS(status, 0, code);
+      record_timeout(status, code);
       return false;
     }
   }
@@ -582,6 +582,8 @@ gemm_pair_kernel(const GemmArgs p, const __grid_constant__ CUtensorMap xmap, con
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
   }
 }
+
+PE_WAIT_STATUS_READER(gemm_wait_status)
 
 }  // namespace pe
 

@@ -5,6 +5,7 @@
 
 #include "pe_common.cuh"
 #include "pe_gemv_decode.cuh"
+#include "pe_status.cuh"
 
 namespace pe {
 
@@ -55,7 +56,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     if (*abort_flag) return false;
     if (clock64() - t0 > kTimeoutCycles) {
       *abort_flag = 1;
-      atomicCAS(status, 0, code);
+      record_timeout(status, code);
       return false;
     }
   }

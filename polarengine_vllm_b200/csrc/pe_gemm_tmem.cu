@@ -130,7 +130,7 @@ gemm_tmem_kernel(const TmemGemmArgs p, const __grid_constant__ CUtensorMap xmap,
   constexpr int kCodeStage = PACKED ? 8192 : 16384, NC = kTmCBytes / kCodeStage / 2;  // two rings of NC code stages
   const uint32_t raw = smem_u32(smem_raw);
   if (raw > kTmBarAddr || raw < 1024) {  // the fixed addresses would leave the window
-    if (threadIdx.x == 0) atomicCAS(p.status, 0, 12);
+    if (threadIdx.x == 0) record_timeout(p.status, 12);
     return;
   }
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -512,6 +512,8 @@ __global__ void __launch_bounds__(1024) gemm_tile_list_kernel(const int* expert_
     }
   }
 }
+
+PE_WAIT_STATUS_READER(gemm_tmem_wait_status)
 
 }  // namespace pe
 

@@ -42,6 +42,7 @@
 // crosses CTAs.  The sixteen warps' partial sums of a tile go through shared memory and are added in warp order: bit-
 // identical from run to run, and the same bits from either layout.
 #include "pe_gemv_decode.cuh"
+#include "pe_status.cuh"
 
 namespace pe {
 
@@ -96,7 +97,7 @@ __device__ __noinline__ bool bar_wait_slow(uint32_t bar, uint32_t parity, int* s
     for (int i = 0; i < 64; ++i)
       if (bar_try(bar, parity)) return true;
     if (clock64() - t0 > (1ll << 30)) {
-      if (status) atomicExch(status, PE_STATUS_SPLITK_TIMEOUT);
+      record_timeout(status, PE_STATUS_SPLITK_TIMEOUT);
       return false;
     }
   }
@@ -334,7 +335,7 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
   int& n_live = *reinterpret_cast<int*>(smem + 16 * kBulkMaxStages);
   asm volatile("griddepcontrol.launch_dependents;");
   if (sbase > kTabAddr - 256) {  // the table's place is taken: never seen, the host sizes for any base below
-    if (tid == 0 && p.status) atomicExch(p.status, PE_STATUS_SPLITK_TIMEOUT);
+    if (tid == 0) record_timeout(p.status, PE_STATUS_SPLITK_TIMEOUT);
     return;
   }
   if (tid == 0) {
@@ -664,6 +665,8 @@ template <bool PACKED, bool TILED>
 static int launch_bulk_kind(BulkArgs& a, int sms, cudaStream_t st) {
   return a.grp ? launch_bulk_shape<PACKED, TILED, true>(a, sms, st) : launch_bulk_shape<PACKED, TILED, false>(a, sms, st);
 }
+
+PE_WAIT_STATUS_READER(gemv_wait_status)
 
 size_t gemv_bulk_frag_bytes(int problems, int batch, int in_f_padded) {
   return (size_t)problems * (batch > 8 ? 2 : 1) * (in_f_padded / kBlock) * 2048;

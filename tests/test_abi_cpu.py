@@ -102,3 +102,13 @@ def test_kernels_see_weights_that_older_kernels_wrote():
         assert 0 <= body.find("griddepcontrol.wait") < body.rfind("griddepcontrol.launch_dependents"), kernel
     body = _body("pe_gemv_cols.cu", "gemv_cols_kernel")
     assert 0 <= body.find("griddepcontrol.wait") < min(body.find("ld.global"), body.find("fetch_item(st_base"))
+
+
+def test_a_wait_that_runs_out_is_always_recorded_for_the_device():
+    """Kernels store status values through record_timeout alone, which also writes the device's word (pe_wait_status): the
+    scratch of a captured call or of the host path has no other reader."""
+    csrc = os.path.join(ROOT, "polarengine_vllm_b200", "csrc")
+    for name in sorted(os.listdir(csrc)):
+        if name.endswith((".cu", ".cuh")) and name != "pe_status.cuh":
+            text = open(os.path.join(csrc, name)).read()
+            assert not re.search(r"atomic\w+\(\s*&?(p\.|a\.)?status", text), name

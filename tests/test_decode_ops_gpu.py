@@ -294,3 +294,28 @@ def test_folded_prologues_without_scratch(bits, n, k):
         nv.check(lib.pe_gemv_pro(*args, n, k, nv.stream_ptr(x.device)), "pe_gemv_pro")
         assert max_rel(y, ref) <= 2e-3 and (resid is None or torch.equal(resid, want))
         assert lib.pe_gemv_pro(*args, 8, k, nv.stream_ptr(x.device)) == -2  # too few rows for it
+
+
+def test_a_timeout_inside_a_captured_graph_can_be_seen():
+    """pe_wait_status: a wait that runs out in a replayed graph (rank 1 of a world of two local buffers never arrives; limit
+    10 ms) is there to read without the launch's own status word, once, and a launch that waits for nobody leaves it alone."""
+    from polarengine_vllm_b200 import _native as nv
+    dev, lib, hidden = torch.device("cuda"), nv.lib(), 512
+    nbytes = lib.pe_allreduce_buffer_bytes(2, 1, hidden)
+    bufs = [torch.zeros(nbytes, dtype=torch.uint8, device=dev) for _ in range(2)]
+    peers = torch.tensor([b.data_ptr() for b in bufs], dtype=torch.int64, device=dev)
+    seq, status = torch.zeros(1, dtype=torch.int32, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    x, w, part = torch.zeros(1, hidden, device=dev).half(), torch.ones(hidden, device=dev).half(), torch.ones(1, hidden, device=dev)
+    out = torch.empty_like(x)
+    nv.wait_status(dev)
+    assert nv.wait_status(dev) == 0
+    assert lib.pe_set_wait_limit_us(10_000) == 0
+    try:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            nv.check(lib.pe_allreduce_add_rmsnorm(part.data_ptr(), x.data_ptr(), w.data_ptr(), out.data_ptr(), 1, hidden, 1e-6, peers.data_ptr(), 0, 2, 1,
+                                                  seq.data_ptr(), status.data_ptr(), nv.stream_ptr(dev)), "pe_allreduce_add_rmsnorm")
+        graph.replay()
+        assert nv.wait_status(dev, clear=False) == 1 and nv.wait_status(dev) == 1 and nv.wait_status(dev) == 0
+    finally:
+        assert lib.pe_set_wait_limit_us(1_000_000) == 0
