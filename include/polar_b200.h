@@ -175,7 +175,8 @@ int pe_pack_nibble(const int8_t* codes, uint8_t* packed, int64_t out_f, int64_t 
  *           it is rotated already (in_f_padded columns) or raw (in_f columns)
  *   y       (batch, out_f) row stride ld_y elements, dtype y_dtype
  *   bias    optional fp16 (out_f), may be NULL
- *   workspace / workspace_bytes  16-byte aligned scratch of at least pe_gemv_workspace_bytes(...);
+ *   workspace / workspace_bytes  16-byte aligned scratch of at least pe_gemv_scratch_bytes(...) (what a launch
+ *           touches; pe_gemv_workspace_bytes(...) is never less and grows with the layer);
  *           no initial contents are needed beyond its status word, the last int32 of
  *           its first 256 KB, which must read zero before the first call: a kernel whose
  *           bounded device-side wait ran out stores a PE_STATUS_* value there (the output
@@ -189,6 +190,7 @@ int pe_pack_nibble(const int8_t* codes, uint8_t* packed, int64_t out_f, int64_t 
  * Replaces polar_matmul's batch==1 branches and (for 2..16 rows) its GEMM branch
  * (polar_gemm.py:485-534), plus the cast/bias epilogue of linear_method.py:214-221. */
 size_t pe_gemv_workspace_bytes(int batch, int out_f, int in_f_padded);
+size_t pe_gemv_scratch_bytes(int batch, int in_f_padded);
 int pe_gemv_status(void* workspace, size_t workspace_bytes, int clear, void* stream);
 
 /* 1 if pe_gemv runs batches of 3..8 rows of this layer as fast on its row-major arrays as pe_gemv_tiled does on the

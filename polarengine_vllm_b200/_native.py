@@ -35,6 +35,7 @@ SIGNATURES = {
     "pe_quantize": (_i, [_vp, _i, _i64, _i64, _i, _i, _vp, _i, _vp, _i64, _vp, _i64, _vp]),
     "pe_pack_nibble": (_i, [_vp, _vp, _i64, _i64, _vp]),
     "pe_gemv_workspace_bytes": (_sz, [_i, _i, _i]),
+    "pe_gemv_scratch_bytes": (_sz, [_i, _i]),
     "pe_gemv": (_i, [_vp, _i, _i64, _vp, _i64, _vp, _i, _vp, _i, _i, _i64, _i, _vp, _i, _i64, _vp, _i, _i, _i,
                      _vp, _sz, _vp]),
     "pe_gemv_grouped_workspace_bytes": (_sz, [_i, _i, _i]),

@@ -9,8 +9,9 @@
 
 namespace pe {
 
-// Scratch layout: [256 KB, last word: status (0 = ok)][activations in operand order].  pe_gemv_workspace_bytes is an
-// upper bound of what a launch touches: callers plan with it, and pe_gemv_noalloc draws its line by it.
+// Scratch layout: [256 KB, last word: status (0 = ok)][activations in operand order], pe_gemv_scratch_bytes in all.
+// pe_gemv_workspace_bytes is a bound that grows with the layer: it had room for fp32 partial sums of a K split that no kernel
+// makes any more.  Callers planned with it and pe_gemv_noalloc refuses shapes by it, so it stays as it was.
 constexpr size_t kCounterBytes = kGemvStatusBytes;
 constexpr int kMaxRowTiles = (int)(kCounterBytes / sizeof(unsigned)) - 1;
 constexpr int kMaxSms = 256;
@@ -35,6 +36,11 @@ extern "C" size_t pe_gemv_workspace_bytes(int batch, int out_f, int in_f_padded)
   if ((out_f + 15) / 16 > kMaxRowTiles) return 0;
   const size_t part = partial_bytes(batch, out_f, in_f_padded, kMaxSms), frags = gemv_bulk_frag_bytes(1, batch, in_f_padded);
   return kCounterBytes + (part > frags ? part : frags);
+}
+
+extern "C" size_t pe_gemv_scratch_bytes(int batch, int in_f_padded) {
+  if (batch < 1 || batch > 16 || in_f_padded < kBlock || in_f_padded % kBlock) return 0;
+  return kCounterBytes + gemv_bulk_frag_bytes(1, batch, in_f_padded);
 }
 
 // Argument checks shared by every decode-size entry point.
@@ -65,7 +71,7 @@ static int gemv_dispatch(const void* codes, int packed, int64_t ld_codes, const 
                          size_t workspace_bytes, void* stream) {
   if (!workspace) return PE_ERR_ARG;
   if ((out_f + 15) / 16 > kMaxRowTiles) return PE_ERR_LIMIT;
-  if (workspace_bytes < kCounterBytes + gemv_bulk_frag_bytes(1, batch, in_f_padded)) return PE_ERR_WORKSPACE;
+  if (workspace_bytes < pe_gemv_scratch_bytes(batch, in_f_padded)) return PE_ERR_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(workspace) & 15) return PE_ERR_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   uint8_t* ws = static_cast<uint8_t*>(workspace);

@@ -456,7 +456,7 @@ static int pro_bulk(pe::GemvBulkCall& q, int prologue, const float* ct_scaled, i
   const int c = pro_check(ct_scaled, n_levels, q.packed, prologue, x, in_f, delta, delta_dtype, norm_weight, resid_out, y, y_dtype, out_f, in_f_padded);
   if (c != PE_OK) return c;
   if (reinterpret_cast<uintptr_t>(workspace) & 15) return PE_ERR_ALIGN;
-  if (workspace_bytes < kGemvStatusBytes + gemv_bulk_frag_bytes(1, 1, in_f_padded)) return PE_ERR_WORKSPACE;
+  if (workspace_bytes < pe_gemv_scratch_bytes(1, in_f_padded)) return PE_ERR_WORKSPACE;
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   q.ct_scaled = ct_scaled; q.n_levels = n_levels;
   q.x = x; q.x_kind = prologue == PE_PRO_SILU_MUL ? PE_X_SILU_MUL : PE_X_RAW; q.x_dtype = PE_F16; q.ld_x = 2 * (int64_t)in_f; q.in_f = in_f;

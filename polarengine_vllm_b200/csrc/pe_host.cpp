@@ -25,7 +25,7 @@ struct Api {
   decltype(&pe_init) init;
   decltype(&pe_gemv) gemv;
   decltype(&pe_gemv_tiled) gemv_tiled;
-  decltype(&pe_gemv_workspace_bytes) gemv_bytes;
+  decltype(&pe_gemv_scratch_bytes) gemv_bytes;
   decltype(&pe_gemm) gemm;
   decltype(&pe_gemm_workspace_bytes_splitk) gemm_bytes;
   decltype(&pe_moe_route) moe_route;
@@ -123,7 +123,7 @@ at::Tensor multiply(const Matrix& w, const at::Tensor& x, int64_t rows, int64_t 
   const float* ct = w.ct->const_data_ptr<float>();
   int rc;
   if (rows <= kDecodeRows) {
-    const at::Tensor ws = take_scratch(dev, st, 0, api.gemv_bytes((int)rows, w.out_f, w.in_f_padded), true);
+    const at::Tensor ws = take_scratch(dev, st, 0, api.gemv_bytes((int)rows, w.in_f_padded), true);
     rc = w.tiles ? api.gemv_tiled(w.tiles->const_data_ptr(), w.packed, ct, levels, x.const_data_ptr(), kind, xd, ld_x, w.in_f, y.mutable_data_ptr(),
                                   yd, w.out_f, b, (int)rows, w.out_f, w.in_f_padded, ws.mutable_data_ptr(), ws.numel(), st)
                  : api.gemv(w.codes->const_data_ptr(), w.packed, w.codes->stride(0), w.norms->const_data_ptr(), w.norms->stride(0), ct, levels,
@@ -375,7 +375,7 @@ PyObject* host_setup(PyObject*, PyObject* arg) {
   PE_SYMBOL(init, pe_init)
   PE_SYMBOL(gemv, pe_gemv)
   PE_SYMBOL(gemv_tiled, pe_gemv_tiled)
-  PE_SYMBOL(gemv_bytes, pe_gemv_workspace_bytes)
+  PE_SYMBOL(gemv_bytes, pe_gemv_scratch_bytes)
   PE_SYMBOL(gemm, pe_gemm)
   PE_SYMBOL(gemm_bytes, pe_gemm_workspace_bytes_splitk)
   PE_SYMBOL(moe_route, pe_moe_route)

@@ -78,7 +78,7 @@ def quant_matmul(codes: torch.Tensor, packed: bool, norms: torch.Tensor, ct_scal
     l = nv.lib()
     st = nv.stream_ptr(dev)
     if batch <= GEMV_MAX_BATCH:
-        need = l.pe_gemv_workspace_bytes(min(batch, GEMV_MAX_BATCH), out_f, in_f_padded)
+        need = l.pe_gemv_scratch_bytes(min(batch, GEMV_MAX_BATCH), in_f_padded)
         ws = nv.gemv_scratch(dev, need)
         for m0 in range(0, batch, GEMV_MAX_BATCH):
             m1 = min(batch, m0 + GEMV_MAX_BATCH)
@@ -130,7 +130,7 @@ def quant_matmul_pro(codes: torch.Tensor, packed: bool, norms: torch.Tensor, ct_
     y = torch.empty(1, out_f, dtype=out_dtype, device=dev)
     if tiles is None and codes.numel() * codes.element_size() < PRO_MIN_CODE_BYTES:
         return None
-    ws = nv.gemv_scratch(dev, nv.lib().pe_gemv_workspace_bytes(1, out_f, in_f_padded))
+    ws = nv.gemv_scratch(dev, nv.lib().pe_gemv_scratch_bytes(1, in_f_padded))
     mid = (ct_scaled.data_ptr(), ct_scaled.numel(), prologue, x.data_ptr(), in_f, delta.data_ptr() if delta is not None else None,
            nv.dtype_code(delta) if delta is not None else nv.PE_F16, norm_weight.data_ptr() if norm_weight is not None else None,
            resid_out.data_ptr() if resid_out is not None else None, float(eps), y.data_ptr(), nv.dtype_code(y),

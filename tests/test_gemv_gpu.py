@@ -415,3 +415,28 @@ def test_a_captured_line_of_matmuls(rows):
                 assert torch.equal(a, b * 2 ** times if i == rewrite else b)
         if rewrite is not None:
             layers[rewrite][2].div_(8)
+
+
+def test_scratch_is_what_a_launch_touches():
+    """pe_gemv in pe_gemv_scratch_bytes of scratch, the bytes behind it untouched, one byte less refused; a wide layer leaves
+    the stream with a buffer of that order, not one that grows with the layer."""
+    from polarengine_vllm_b200 import _native as nv, kernels
+    n, k, rows, lib = 24576, 2048, 16, nv.lib()
+    codes, norms, cts = rand_layer(n, k, 5, seed=2)
+    w, nd, ctd, x = codes.cuda(), norms.cuda(), cts.cuda(), rand_x(rows, k, seed=1).cuda()
+    need = lib.pe_gemv_scratch_bytes(rows, k)
+    assert (256 << 10) < need <= lib.pe_gemv_workspace_bytes(rows, n, k) and lib.pe_gemv_scratch_bytes(17, k) == 0
+    ws = torch.zeros(need + 4096, dtype=torch.uint8, device="cuda")
+    ws[need:] = 0xA5
+    y = torch.full((rows, n), float("nan"), device="cuda")
+    args = (w.data_ptr(), 0, w.stride(0), nd.data_ptr(), nd.stride(0), ctd.data_ptr(), ctd.numel(), x.data_ptr(), nv.PE_X_RAW, nv.PE_F16, x.stride(0), k,
+            y.data_ptr(), nv.PE_F32, n, None, rows, n, k, ws.data_ptr())
+    assert lib.pe_gemv(*args, need - 1, nv.stream_ptr(x.device)) == -4
+    nv.check(lib.pe_gemv(*args, need, nv.stream_ptr(x.device)), "pe_gemv")
+    assert torch.equal(y, kernels.quant_matmul(w, False, nd, ctd, x, False, n, k, k, torch.float32)) and bool((ws[need:] == 0xA5).all())
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        out = kernels.quant_matmul(w, False, nd, ctd, x, False, n, k, k, torch.float16)
+        assert torch.cuda.memory_allocated() - before - out.numel() * 2 < 2 * need
