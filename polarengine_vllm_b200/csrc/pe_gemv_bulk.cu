@@ -29,14 +29,14 @@
 //    The registers left over let the small launch's blocks be resident, waiting, while the launch before it still runs.
 // Measured, row-major layout, a line of launches under a CUDA graph, weights from HBM (in brackets the tiled layout):
 //   activation rows      1              8              16
-//   6144 x 4096 Q5     9.2 (10.1)     9.5 (10.1)    12.4 (14.2) us
+//   6144 x 4096 Q5     9.2 (10.1)     9.5 (10.1)    11.4 (12.8) us
 //   4096 x 4096 Q6     7.2  (8.0)     7.5  (8.1)     8.8  (9.8)
-//   24576 x 4096 Q3   14.0 (15.0)    16.2 (16.8)    28.3 (28.3)
-//   4096 x 12288 Q4   10.1 (10.8)    11.3 (11.8)    15.9 (16.0)
-//   the four in turn  40.3 (42.9)    44.7 (47.0)    65.5 (67.6)
+//   24576 x 4096 Q3   14.0 (15.0)    16.2 (16.8)    25.0 (24.4)
+//   4096 x 12288 Q4   10.1 (10.8)    11.3 (11.8)    15.9 (15.9)
+//   the four in turn  40.3 (42.9)    44.7 (47.0)    61.3 (62.9)
 // Inside the ring's steady state the 24576 x 4096 launch moves 4.9 TB/s; the rest is the launch's own latency: about
 // 3.5 us from the launch before it to the first product, 0.5 us from the last one to the stores.  Outside a line (launched
-// eagerly, or with other kernels in between) the ring fills about 2 us later: the four in turn take 48.5, 51.2 and 68.6 us.
+// eagerly, or with other kernels in between) the ring fills about 2 us later: the four in turn take 48.5 us for one row, 51.2 for 8.
 //
 // The tiles of all problems of a launch form one line that is cut into equal contiguous ranges, one per CTA; nothing
 // crosses CTAs.  The sixteen warps' partial sums of a tile go through shared memory and are added in warp order: bit-
@@ -609,8 +609,10 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
   const long long line = (long long)a.units * (a.grp ? a.n_problems : 1);
   if (line >= (1ll << 31)) return PE_ERR_LIMIT;
   const int G = (int)(line < sms ? line : sms);
-  // Rows per pass: the sums of a pass meet at a barrier, so few and equal passes; 64 rows of 8 activation rows are
-  // 34 KB of partial sums, which the ring would rather have (64 measured best of 32, 64, 96 and 176).
+  // Rows per pass: the sums of a pass meet at a barrier, and two sets of activation rows read their activations again for
+  // every K range of a pass, so few and equal passes; but 64 rows of 8 activation rows are 34 KB of partial sums (of 16: 68 KB),
+  // which the ring would rather have.  8 rows: 64 best of 32, 64, 96 and 176; 16 rows, 24576 x 4096: 35.9, 28.5 and 25.1 us for
+  // 16, 32 and 64, 6144 x 4096: 14.1, 12.3 and 11.3 us.
   a.part_rows = a.batch < 8 * NT ? a.batch : 8 * NT;
   const int cta_rows = (int)((line + G - 1) / G) * 16;
   const int entries = PACKED ? (a.n_levels <= 8 ? 128 : 256) : a.n_levels;
@@ -629,7 +631,7 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
   a.norm_stride = GROUPED && !TILED && a.n_chunk == 1 && a.ld_norms == a.nb && (reinterpret_cast<uintptr_t>(a.norms) & 15) == 0 &&
                   a.norms_stride % 8 == 0 && (a.N % 16) * a.nb % 8 == 0 ? a.nb * 2 : 0;
   a.stage_bytes = TILED ? (blocks * kRecBytes + 127) & ~127 : (16 * a.row_stride + 64 + blocks * 32 + 127) & ~127;
-  for (int cap = a.part_rows <= 2 ? 256 : (NT == 1 ? 64 : 32);; cap /= 2) {
+  for (int cap = a.part_rows <= 2 ? 256 : 64;; cap /= 2) {
     if (cap < 16) return PE_ERR_LIMIT;
     const int passes = (cta_rows + cap - 1) / cap;
     a.pass_rows = GROUPED ? cap : ((cta_rows + passes - 1) / passes + 15) / 16 * 16;
