@@ -13,6 +13,7 @@ namespace pe {
 // pe_gemv_workspace_bytes is a bound that grows with the layer: it had room for fp32 partial sums of a K split that no kernel
 // makes any more.  Callers planned with it and pe_gemv_noalloc refuses shapes by it, so it stays as it was.
 constexpr size_t kCounterBytes = kGemvStatusBytes;
+// limit on out_f, from the time when a launch kept one word per row tile there
 constexpr int kMaxRowTiles = (int)(kCounterBytes / sizeof(unsigned)) - 1;
 constexpr int kMaxSms = 256;
 
@@ -131,7 +132,9 @@ extern "C" int pe_gemv_status(void* workspace, size_t workspace_bytes, int clear
 // times matrix `index` of a stack of matrices, written to the same rows of y.  Slots with rows <= 0 have no work, so
 // the caller can size the launch for the worst case without knowing the routing.
 namespace pe {
-constexpr size_t kGroupedZone = 4u << 20;  // last word: status
+// last word: status.  The size, and with it the limit on problems x row tiles below, is that of a counter zone which is gone;
+// both stay: callers size buffers and choose their path by them
+constexpr size_t kGroupedZone = 4u << 20;
 }  // namespace pe
 
 extern "C" size_t pe_gemv_grouped_workspace_bytes(int max_problems, int out_f, int in_f_padded) {
@@ -276,7 +279,7 @@ extern "C" int pe_gemv_tiled(const void* tiles, int packed, const float* ct_scal
 // Some hosts of this library hand every byte of device memory to their own pool at
 // start-up (an inference server sizes its KV cache from "whatever is free" and keeps
 // it), so a cudaMalloc made later on behalf of one linear layer can fail, and the code
-// that calls into the layer has no allocator of its own to ask.  For them the split-K
+// that calls into the layer has no allocator of its own to ask.  For them the
 // scratch lives inside the library image: a fixed array in device global memory that
 // exists on every GPU that loads the library, from load until exit.
 constexpr size_t kNoAllocScratchBytes = 8u << 20;  // 8 MiB

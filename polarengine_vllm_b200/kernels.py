@@ -3,8 +3,8 @@
 Reference: polarengine_vllm/kernels/polar_gemm.py:425-534 (``polar_matmul``),
 polar_gemv.py:181-283 (``polar_gemv``, ``polar_gemv_packed``, ``pack_codes_int4``),
 polar_gemv_splitk.py:421-569, polar_gemm.py:312-418.  Argument order and meaning are
-kept; every one of them ends in the same native entry point, which chooses its own
-split of the K range, so the split-K names are aliases.
+kept; every one of them ends in the same native entry point, which divides the
+work its own way, so the split-K names are aliases.
 """
 from __future__ import annotations
 

@@ -180,7 +180,8 @@ class PolarQuantMoEMethod:
         tensor_cores = local_pairs >= self.TENSOR_CORE_MIN_ROWS_PER_EXPERT * n_local
         # Rows per problem: 8 while experts see few tokens (lighter kernel), else 16.  For 16 rows a CTA takes 16 blocks of K
         # per round: where a last round leaves a quarter of those places empty, problems of 8 stay ahead up to the
-        # tensor cores' range (8 rows for each of 128 experts, 21 blocks: 474 us against 592; 16 blocks: 94 against 91).
+        # tensor cores' range (128 experts of 21 blocks, 8 rows each: 489 us against 598, 12 rows 642 against 645; 64
+        # experts of 16 blocks, 8 rows each: 144 against 135).
         ragged = blocks > 16 and blocks <= 0.75 * 16 * -(-blocks // 16)
         rpp = 8 if local_pairs <= 6 * n_local or (ragged and not tensor_cores) else 16
         return rpp, min(n_local, pairs) + pairs // rpp, tensor_cores
@@ -189,16 +190,17 @@ class PolarQuantMoEMethod:
     # used; beyond it every expert has enough rows to fill the tensor-core kernel by itself
     # (measured on 128 experts: grouped 6.5 ms against 21.8 ms per-expert at 128 rows each)
     GROUPED_MAX_ROWS_PER_EXPERT = 512
-    # average rows per expert from which the grouped launches run on the tensor cores (a 256 x 256
-    # tile per expert and weight tile costs the same for 1 or 256 rows; below this the streaming
-    # decode-size kernel is cheaper)
+    # average rows per expert from which the grouped launches run on the tensor cores.  By time alone the line would lie at
+    # four rows (128 experts of 2688 -> 2 x 1856: 347 us either way at 4 rows, 361 against 489 at 8, 345 against 642 at 12), but
+    # that kernel rounds activations and decoded weights to bf16, where the streaming one multiplies fp16 values and keeps the
+    # norms in fp32: a decode batch gives up no precision for speed, a prompt chunk does
     TENSOR_CORE_MIN_ROWS_PER_EXPERT = 12
 
     def moe_forward(self, layer, x: torch.Tensor, topk_weights: torch.Tensor, topk_ids: torch.Tensor,
                     expert_map: Optional[torch.Tensor] = None) -> torch.Tensor:
         """y[t] = sum_k w[t,k] * down_e(silu(gate_e(x[t])) * up_e(x[t])), e = ids[t,k]; fp16 out.
-        Decode-size batches: two grouped launches over all experts (``pe_gemv_grouped``),
-        nothing read back to the host.  Prefill-size batches: per-expert tensor-core matmuls."""
+        Two grouped launches over all experts, nothing read back to the host: ``pe_gemv_grouped`` for few rows per
+        expert, ``pe_gemm_grouped`` for more; beyond GROUPED_MAX_ROWS_PER_EXPERT a matmul per expert and projection."""
         if x.dtype in (torch.float16, torch.bfloat16):
             y = None
             if topk_weights.dtype == torch.float32 and topk_ids.dtype == torch.int64:
