@@ -193,7 +193,7 @@ def fill_linear(layer, tensors: Dict[str, torch.Tensor]) -> None:
     """Copy a loaded layer into the parameters ``PolarQuantLinearMethod.create_weights``
     registered (``codes`` int8, ``norms`` fp16, ``ct_scaled`` fp32).  Nibble-packed
     checkpoints are attached as ``codes_packed`` directly (``process_weights_after_loading``
-    then only builds the tiled copy)."""
+    then has nothing left to do)."""
     from .packing import unpack_codes_half_block
     if "codes" not in tensors:
         raise ValueError("fill_linear needs a quantized layer (codes / norms / ct_scaled)")

@@ -249,7 +249,7 @@ def test_gemv_bulk_edges(batch, bits, n, k):
 
 @pytest.mark.parametrize("rows", [1, 16, 17])
 def test_apply_native_call(rows):
-    """The native call of ``apply``: the tiled copy follows the arrays it was made from, non-contiguous input gives the
+    """The native call of ``apply``: arrays replaced under the layer are the ones multiplied by, non-contiguous input gives the
     same values and fp64 an error, and a captured call stays right after other calls reused the scratch."""
     from polarengine_vllm_b200.linear_method import PolarQuantLinearMethod
     n, in_f, bits = 272, 300, 4
