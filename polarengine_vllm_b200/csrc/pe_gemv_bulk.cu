@@ -51,6 +51,7 @@ __host__ __device__ constexpr int bulk_threads(bool tiled) { return (kBulkWarps 
 constexpr int kTabAddr = 2048;                        // address of the centroid table in the shared window
 constexpr int kTabReach = 255 * 256 + 256;            // bytes a lookup can reach from there, whatever the code byte is
 constexpr int kBulkMaxStages = 8;
+constexpr int kNormAhead = 1 << 18;                   // bytes of norms asked for ahead at most
 constexpr unsigned kBulkSmemMax = 231424u;            // 227 KB minus the runtime's 1 KB
 
 struct BulkArgs {
@@ -413,10 +414,11 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
           if (d.z <= 0) continue;
           norms = p.norms + d.x * p.norms_stride;
         }
-        // the whole pass on its way to L2: a stage's loads then wait for L2 and not for HBM
+        // the whole pass on its way to L2 (of arrays with wide gaps between rows, its first part): a stage's loads then wait for
+        // L2 and not for HBM
         const char* span = reinterpret_cast<const char*>(norms + (int64_t)ps.row0 * p.ld_norms);
-        const int64_t bytes = ((int64_t)(ps.rows - 1) * p.ld_norms + p.nb) * 2;
-        for (int64_t o = lane * 128; o < bytes; o += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(span + o));
+        const int bytes = (int)min(((int64_t)(ps.rows - 1) * p.ld_norms + p.nb) * 2, (int64_t)kNormAhead);
+        for (int o = lane * 128; o < bytes; o += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(span + o));
         return true;
       }
       return false;
