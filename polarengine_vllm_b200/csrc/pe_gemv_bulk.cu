@@ -2,7 +2,8 @@
 //
 //   y[m, r] = sum_blk norm[r, blk] * sum_k ct[code[r, blk, k]] * xt[m, blk, k]   (+ bias[r])
 //
-// One persistent CTA per SM: sixteen math warps, a copy warp and, for row-major codes, a norm warp.  A stage of the shared-
+// One persistent CTA per SM: sixteen math warps, a copy warp, for row-major codes a norm warp, and in launches whose CTAs have
+// several passes two sum warps.  A stage of the shared-
 // memory ring is one 16-row tile of the weight matrix by up to 32 quantization blocks.  The copy warp fills stages with bulk
 // copies (of the row-major layout one or a few rows each, of the tiled layout of pe_retile, whose records are contiguous, one
 // per stage).  Norms of row-major layers are a strided gather of halves: the norm warp loads them, two stages under way (with
@@ -22,6 +23,16 @@
 //  * products on the tensor cores (mma.sync m16n8k16, weights as the 16-row A operand, activation rows as the eight
 //    columns of B): 16 rows x 16 weights per instruction straight from the lookups' registers, which no descriptor-
 //    based tensor-core operation offers (tcgen05 would need the decoded tile written to shared memory and read again);
+//  * what a warp does for a tile besides its blocks (barriers, norms, handing its sums over) is about 100 instructions, as
+//    many as one nibble block: 128 experts of 21 and 15 blocks, 64 tokens, took 177 us with no block multiplied and nothing
+//    copied, 345 us in all.  So where rows are short (kGroupBlocks) a warp takes three blocks, fewer warps share a tile, and
+//    the warps left form further groups that work on other tiles: 310 -> 262 us, one token 39.1 -> 37.0, 24576 x 1024 Q6 at
+//    8 rows 11.1 -> 9.9.  (Whole rows per warp, activations read from shared memory for every block: 443 us.  22 warps of one
+//    block: 341.  Q3 look-ups by byte permutes of register tables instead of loads: 352 to 362.)
+//  * the sums of a pass: with all warps meeting at a barrier, adding and meeting again, 64 tokens of 128 experts took 345 us;
+//    given to warps of their own, with two sets of partial sums so that the next pass runs meanwhile, 310 (four rows a lane and
+//    one 16-byte load per warp's share; with a row a lane two sum warps did not keep up: 326).  24576 x 4096 at 8 rows
+//    16.4 -> 15.8 us, 16 rows 25.2 -> 24.2.  The last pass of a CTA is added by all its warps.
 //  * activations: a small launch in front (gemv_frags_kernel) pads, rotates and rounds them once and leaves them in
 //    B-operand order in the workspace, so that a warp loads its own blocks with four coalesced reads each and keeps
 //    them in registers.  Rotating inside this kernel was measured too (in registers, 16-point part by MMAs): its
@@ -29,11 +40,10 @@
 //    The registers left over let the small launch's blocks be resident, waiting, while the launch before it still runs.
 // Measured, row-major layout, a line of launches under a CUDA graph, weights from HBM (in brackets the tiled layout):
 //   activation rows      1              8              16
-//   6144 x 4096 Q5     9.2 (10.1)     9.5 (10.1)    11.4 (12.8) us
-//   4096 x 4096 Q6     7.2  (8.0)     7.5  (8.1)     8.8  (9.8)
-//   24576 x 4096 Q3   14.0 (15.0)    16.2 (16.8)    25.0 (24.4)
-//   4096 x 12288 Q4   10.1 (10.8)    11.3 (11.8)    15.9 (15.9)
-//   the four in turn  40.3 (42.9)    44.7 (47.0)    61.3 (62.9)
+//   6144 x 4096 Q5     9.4 (10.1)     9.7 (10.1)    11.7 (12.8) us
+//   4096 x 4096 Q6     7.4  (8.0)     7.9  (8.1)     9.2  (9.8)
+//   24576 x 4096 Q3   13.9 (15.0)    15.8 (16.8)    24.2 (24.4)
+//   4096 x 12288 Q4   10.3 (10.8)    11.3 (11.8)    16.2 (15.9)
 // Inside the ring's steady state the 24576 x 4096 launch moves 4.9 TB/s; the rest is the launch's own latency: about
 // 3.5 us from the launch before it to the first product, 0.5 us from the last one to the stores.  Outside a line (launched
 // eagerly, or with other kernels in between) the ring fills about 2 us later: the four in turn take 48.5 us for one row, 51.2 for 8.
@@ -46,8 +56,14 @@
 
 namespace pe {
 
-constexpr int kBulkWarps = 16;                        // math warps
-__host__ __device__ constexpr int bulk_threads(bool tiled) { return (kBulkWarps + (tiled ? 1 : 2)) * 32; }  // + the copy warp, the norm warp
+// Math warps.  Three blocks a warp (BPW) need the registers of a CTA of sixteen warps in all.
+__host__ __device__ constexpr int bulk_warps(int bpw) { return bpw == 3 ? 14 : 16; }
+__host__ __device__ constexpr int sum_warps(int bpw, bool passes) { return !passes ? 0 : bpw == 3 ? 1 : 2; }
+// ... + the copy warp, the sum warps of launches of several passes, the norm warp of row-major layers (never with BPW 3)
+__host__ __device__ constexpr int bulk_threads(int bpw, bool tiled, bool passes) {
+  return (bulk_warps(bpw) + 1 + sum_warps(bpw, passes) + (!tiled && bpw < 3)) * 32;
+}
+constexpr int kGroupBlocks = 21;                      // blocks of a row, at most, where a warp takes three: two groups of seven warps
 constexpr int kTabAddr = 2048;                        // address of the centroid table in the shared window
 constexpr int kTabReach = 255 * 256 + 256;            // bytes a lookup can reach from there, whatever the code byte is
 constexpr int kBulkMaxStages = 8;
@@ -60,7 +76,7 @@ struct BulkArgs {
   const uint8_t* tiles;                    // tiled layout
   const float* ct; int n_levels;
   const uint4* frags;                      // activations in B-operand order
-  void* y; int y_dtype; int64_t ld_y;
+  void* y; int y_dtype, y_vec; int64_t ld_y;  // y_vec: four rows from a multiple of 16 on are one store
   const __half* bias;
   int batch, N, nb;
   int n_chunk, chunk_blocks, n_stage;      // chunks of the K range, blocks of a full chunk
@@ -68,6 +84,8 @@ struct BulkArgs {
   int pass_rows;                           // rows whose partial sums shared memory holds (a multiple of 16)
   int part_stride;                         // floats between activation rows of the partial sums
   int part_rows;                           // activation rows the partial sums have room for
+  int groups, group_warps;                 // three blocks a warp: groups of warps, warps of one
+  int part_bufs, part_floats;              // sets of partial sums, floats of one
   int part_off, stage_off, stage_bytes;
   int row_stride, copy_rows;               // row-major layout: bytes between rows of a stage, weight rows per bulk copy
   int norm_stride;                         // grouped, row-major: bytes between the norms of two rows where a stage's are one bulk copy, else 0
@@ -119,7 +137,8 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 __device__ __forceinline__ void bar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void math_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kBulkWarps * 32) : "memory"); }
+template <int WARPS>
+__device__ __forceinline__ void math_sync() { asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory"); }
 
 // ---- tensor-core products -------------------------------------------------------------------------------------
 __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -324,23 +343,28 @@ struct Pass {
   }
 };
 
-template <bool PACKED, int NT, int BPW, bool TILED, bool GROUPED>
-__global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const BulkArgs p) {
+template <bool PACKED, int NT, int BPW, bool TILED, bool GROUPED, bool PASSES>
+__global__ void __launch_bounds__(bulk_threads(BPW, TILED, PASSES), 1) gemv_bulk_kernel(const BulkArgs p) {
   extern __shared__ __align__(128) uint8_t smem[];  // no static shared memory: the window starts with it
+  constexpr int kWarps = bulk_warps(BPW), kSumWarps = sum_warps(BPW, PASSES), kThreads = bulk_threads(BPW, TILED, PASSES);
   constexpr int kRowBytes = PACKED ? 64 : 128;           // codes of one row's block
+  constexpr int kGroupWarps = kGroupBlocks / 3;
   constexpr int kRecBytes = kRowBytes * 16 + 32;         // tiled record: 16 rows of a block, then their norms
-  const bool norms_copied = !TILED && GROUPED && p.norm_stride;
+  const bool norms_copied = !TILED && (GROUPED || BPW == 3) && p.norm_stride;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
   const uint32_t sbase = smem_u32(smem);
   const uint32_t full = sbase, empty = sbase + 8 * kBulkMaxStages;
   int& n_live = *reinterpret_cast<int*>(smem + 16 * kBulkMaxStages);
+  const uint32_t part_full = sbase + 16 * kBulkMaxStages + 16, part_empty = part_full + 16;
   asm volatile("griddepcontrol.launch_dependents;");
   if (sbase > kTabAddr - 256) {  // the table's place is taken: never seen, the host sizes for any base below
     if (tid == 0) record_timeout(p.status, PE_STATUS_SPLITK_TIMEOUT);
     return;
   }
   if (tid == 0) {
-    for (int s = 0; s < p.n_stage; ++s) { bar_init(full + 8 * s, TILED || norms_copied ? 1 : 2); bar_init(empty + 8 * s, kBulkWarps); }
+    for (int s = 0; s < p.n_stage; ++s) { bar_init(full + 8 * s, TILED || norms_copied ? 1 : 2); bar_init(empty + 8 * s, BPW == 3 ? p.group_warps : kWarps); }
+    if (PASSES)
+      for (int b = 0; b < 2; ++b) { bar_init(part_full + 8 * b, kWarps); bar_init(part_empty + 8 * b, kSumWarps); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     n_live = 0;
   }
@@ -348,7 +372,7 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
   int line = p.units;
   if (GROUPED) {  // the problem list comes from the launch before this one
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int i = tid; i < p.n_problems; i += bulk_threads(TILED))
+    for (int i = tid; i < p.n_problems; i += kThreads)
       if (p.grp[i].z > 0) atomicMax(&n_live, i + 1);
     __syncthreads();
     line = n_live * p.units;
@@ -360,7 +384,7 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
     ps.start(p, beg, q + (cta < r));
   }
 
-  if (w == kBulkWarps) {  // ---- copy warp
+  if (w == kWarps) {  // ---- copy warp
     const bool one = elect_lane();
     int s = 0;
     uint32_t ph = 1;
@@ -394,6 +418,15 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
             }
           }
           __syncwarp();
+          if (BPW == 3 && !TILED && !norms_copied) {  // no norm warp: norms that are no single copy, by this one
+            const __half* src = norms + (int64_t)(ps.row0 + r0) * p.ld_norms;
+            for (int e = lane; e < min(16, ps.rows - r0) * p.nb; e += 32) {
+              const int r = e / p.nb, b = e - r * p.nb;
+              asm volatile("st.shared.u16 [%0], %1;" ::"r"(dst + 16 * p.row_stride + 64 + b * 32 + r * 2), "h"(__half_as_ushort(src[r * p.ld_norms + b])) : "memory");
+            }
+            __syncwarp();
+            if (one) bar_arrive(bar);
+          }
           if (++s == p.n_stage) { s = 0; ph ^= 1; }
         }
       }
@@ -401,9 +434,64 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
     return;
   }
 
-  if (!TILED && w > kBulkWarps && norms_copied) return;
-  if (!TILED && w > kBulkWarps) {  // ---- norm warp: a stage's norms, the 16 rows of a block side by side
-    constexpr int kPlaces = kBulkWarps * BPW, kLaneRows = 16 * kPlaces / 32;
+  // The sums of a pass by warp `who` of `whos`: a lane adds the warps' shares of four rows of an activation row, in warp order.
+  constexpr int kSlots = BPW == 3 ? kGroupWarps : kWarps;
+  float* part = reinterpret_cast<float*>(smem + p.part_off);
+  auto sum_pass = [&](const float* from, int batch, int y_row, int who, int whos) {
+    const int quads = (ps.rows + 3) >> 2, slot = p.part_rows * p.part_stride;
+    for (int e = who * 32 + lane; e < batch * quads; e += whos * 32) {
+      const int m = e / quads, r = (e - m * quads) * 4;
+      const float* q = from + m * p.part_stride + r;
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < kSlots; ++i)
+        if (BPW < 3 || i < p.group_warps) {
+          const float4 v = *reinterpret_cast<const float4*>(q + i * slot);
+          sum[0] += v.x; sum[1] += v.y; sum[2] += v.z; sum[3] += v.w;
+        }
+      const int row = ps.row0 + r, left = ps.rows - r;
+      if (p.bias)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (k < left) sum[k] += __half2float(p.bias[row + k]);
+      const int64_t at = (int64_t)(y_row + m) * p.ld_y + row;
+      if (p.y_vec && left >= 4) {
+        if (p.y_dtype == PE_F32) *reinterpret_cast<float4*>(static_cast<float*>(p.y) + at) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+        else if (p.y_dtype == PE_F16) *reinterpret_cast<uint2*>(static_cast<__half*>(p.y) + at) = make_uint2(pack_half2(sum[0], sum[1]), pack_half2(sum[2], sum[3]));
+        else
+          for (int k = 0; k < 4; ++k) store_from_float(p.y, PE_BF16, at + k, sum[k]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (k < left) store_from_float(p.y, p.y_dtype, at + k, sum[k]);
+      }
+    }
+  };
+
+  if (PASSES && w > kWarps && w <= kWarps + kSumWarps) {  // ---- sum warps: every pass but the CTA's last
+    if (!GROUPED) asm volatile("griddepcontrol.wait;" ::: "memory");
+    int b = 0, prob = -1, batch = p.batch, y_row = 0;
+    uint32_t ph = 0;
+    while (ps.next(p) && ps.left > 0) {
+      if (GROUPED && ps.prob != prob) {
+        const int4 d = p.grp[ps.prob];
+        prob = ps.prob;
+        batch = d.z < 8 * NT ? d.z : 8 * NT;
+        y_row = d.y;
+      }
+      if (GROUPED && batch <= 0) continue;
+      bar_wait(part_full + 8 * b, ph, p.status);
+      sum_pass(part + b * p.part_floats, batch, y_row, w - kWarps - 1, kSumWarps);
+      __syncwarp();
+      if (lane == 0) bar_arrive(part_empty + 8 * b);
+      if (++b == p.part_bufs) { b = 0; ph ^= 1; }
+    }
+    return;
+  }
+
+  if (!TILED && w > kWarps && norms_copied) return;
+  if (!TILED && w > kWarps) {  // ---- norm warp: a stage's norms, the 16 rows of a block side by side
+    constexpr int kPlaces = BPW == 1 ? 16 : 32, kLaneRows = 16 * kPlaces / 32;
     const int b = lane % kPlaces, r_lane = lane / kPlaces * kLaneRows, blocks = min(p.nb, p.chunk_blocks);
     const __half* norms = p.norms;
     int c = 0, r0 = 0;
@@ -475,7 +563,7 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
     uint8_t* tab = smem + (kTabAddr - sbase);
     const int entries = PACKED ? (p.n_levels <= 8 ? 128 : 256) : p.n_levels;
 #pragma unroll 2
-    for (int e = tid >> 3; e < entries; e += kBulkWarps * 4) {
+    for (int e = tid >> 3; e < entries; e += kWarps * 4) {
       uint32_t u;
       if (PACKED) {
         const int a = e & 15, b = e >> 4;
@@ -493,21 +581,23 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
   // Where this lane's codes and norms lie in a stage.  Its operand rows g and g + 8 are weight rows g and g + 8 of a tile's
   // records, and rows row_a and row_a + 4 of row-major stages: rows of those lie a multiple of 64 bytes apart, rows 0..7 and
   // 8..15 another 64 bytes, so that a quarter warp, which reads the rows of two neighbouring g, reads both halves of the banks.
+  // Three blocks a warp: the warps form groups of group_warps, group q takes the tiles in stages q, q + groups, ...
+  const int gw = BPW == 3 ? p.group_warps : kWarps, group = BPW == 3 ? w / gw : 0, wi = BPW == 3 ? w - group * gw : w;
   constexpr int kRowB = TILED ? 8 : 4;
+  constexpr int kPartB = PASSES ? kRowB : 8;
   const int row_a = TILED ? g : (g >> 1) + (g & 1) * 8;
-  const uint32_t at_a = TILED ? w * kRecBytes + g * kRowBytes + t * 16 : row_a * p.row_stride + (g & 1) * 64 + w * kRowBytes + t * 16;
+  const uint32_t at_a = TILED ? wi * kRecBytes + g * kRowBytes + t * 16 : row_a * p.row_stride + (g & 1) * 64 + wi * kRowBytes + t * 16;
   const uint32_t at_b = at_a + kRowB * (TILED ? kRowBytes : p.row_stride);
-  const uint32_t at_n = TILED ? w * kRecBytes + 16 * kRowBytes + g * 2 : 16 * p.row_stride + 64 + (norms_copied ? w * 2 + row_a * p.norm_stride : w * 32 + row_a * 2);
-  constexpr int kStep = kBulkWarps * (TILED ? kRecBytes : kRowBytes);
-  const int norm_step = kBulkWarps * (TILED ? kRecBytes : norms_copied ? 2 : 32), norm_b = kRowB * (norms_copied ? p.norm_stride : 2);
+  const uint32_t at_n = TILED ? wi * kRecBytes + 16 * kRowBytes + g * 2 : 16 * p.row_stride + 64 + (norms_copied ? wi * 2 + row_a * p.norm_stride : wi * 32 + row_a * 2);
+  const int kStep = gw * (TILED ? kRecBytes : kRowBytes);
+  const int norm_step = gw * (TILED ? kRecBytes : norms_copied ? 2 : 32), norm_b = kRowB * (norms_copied ? p.norm_stride : 2);
   const uint32_t lane4 = lane * 4;
-  float* part = reinterpret_cast<float*>(smem + p.part_off);
   uint32_t x[BPW][NT][16];
   int x_prob = -1, group_rows = p.batch;
   int y_row = 0;
 
   auto load_x = [&](int prob, int c) {
-    const uint4* src = p.frags + (size_t)(prob * NT * p.nb + c * p.chunk_blocks + w) * 128 + lane;
+    const uint4* src = p.frags + (size_t)(prob * NT * p.nb + c * p.chunk_blocks + wi) * 128 + lane;
     const int nblk = p.nb - c * p.chunk_blocks;
 #pragma unroll
     for (int j = 0; j < BPW; ++j)
@@ -516,13 +606,14 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           uint4 v = make_uint4(0, 0, 0, 0);
-          if (w + kBulkWarps * j < nblk && n * 8 + g < (GROUPED ? group_rows : p.batch)) v = __ldcg(src + (n * p.nb + kBulkWarps * j) * 128 + q * 32);
+          if (wi + gw * j < nblk && n * 8 + g < (GROUPED ? group_rows : p.batch)) v = __ldcg(src + (n * p.nb + gw * j) * 128 + q * 32);
           x[j][n][4 * q] = v.x; x[j][n][4 * q + 1] = v.y; x[j][n][4 * q + 2] = v.z; x[j][n][4 * q + 3] = v.w;
         }
   };
 
-  int s = 0;
-  uint32_t ph = 0;
+  int s = 0, b = 0, turn = 0;
+  uint32_t ph = 0, part_ph = 1;
+  if (PASSES) math_sync<kWarps>();  // the table is there
   for (; more; more = ps.next(p)) {
     if (ps.prob != x_prob) {
       if (GROUPED) {
@@ -534,11 +625,21 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
       x_prob = ps.prob;
       if (p.n_chunk == 1) load_x(x_prob, 0);
     }
-    math_sync();  // the table is there; the sums of the pass before are out
+    if (PASSES) bar_wait(part_empty + 8 * b, part_ph, p.status);
+    else math_sync<kWarps>();  // the table is there
+    float* const sums = part + b * p.part_floats;
     for (int c = 0; c < p.n_chunk; ++c) {
       if (p.n_chunk > 1) load_x(x_prob, c);
       const int nblk = min(p.chunk_blocks, p.nb - c * p.chunk_blocks);
       for (int r0 = 0; r0 < ps.rows; r0 += 16) {
+        if (BPW == 3) {
+          const bool mine = turn == group;
+          if (++turn == p.groups) turn = 0;
+          if (!mine) {
+            if (++s == p.n_stage) { s = 0; ph ^= 1; }
+            continue;
+          }
+        }
         const uint32_t st = sbase + p.stage_off + s * p.stage_bytes;
         bar_wait(full + 8 * s, ph, p.status);
         float acc[NT][4];
@@ -548,7 +649,7 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
           for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
 #pragma unroll
         for (int j = 0; j < BPW; ++j) {
-          const int blk = w + kBulkWarps * j;
+          const int blk = wi + gw * j;
           if (blk < nblk) {
             float d[NT][4];
             unsigned short ha, hb;
@@ -566,7 +667,7 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
         __syncwarp();
         if (lane == 0) bar_arrive(empty + 8 * s);
         if (++s == p.n_stage) { s = 0; ph ^= 1; }
-        float* pp = part + w * p.part_rows * p.part_stride + r0 + g;
+        float* pp = sums + wi * p.part_rows * p.part_stride + r0 + (PASSES ? row_a : g);
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
@@ -574,37 +675,49 @@ __global__ void __launch_bounds__(bulk_threads(TILED), 1) gemv_bulk_kernel(const
             const int m = n * 8 + 2 * t + e;
             if (m < (GROUPED ? group_rows : p.batch)) {
               float* q = pp + m * p.part_stride;
-              if (c == 0) { q[0] = acc[n][e]; q[8] = acc[n][2 + e]; }
-              else { q[0] += acc[n][e]; q[8] += acc[n][2 + e]; }
+              if (c == 0) { q[0] = acc[n][e]; q[kPartB] = acc[n][2 + e]; }
+              else { q[0] += acc[n][e]; q[kPartB] += acc[n][2 + e]; }
             }
           }
       }
     }
-    math_sync();
-    const int groups = (ps.rows + 31) >> 5, batch = GROUPED ? group_rows : p.batch;
-    for (int e = w; e < groups * batch; e += kBulkWarps) {  // a warp sums 32 rows of one activation row
-      const int m = groups == 1 ? e : e / groups, at = (e - m * groups) * 32 + lane;
-      const int r = TILED ? at : (at & ~15) + ((at & 7) >> 1) + (at & 1) * 8 + ((at >> 1) & 4);  // the row that row_a put there
-      if (r < ps.rows) {
-        const float* q = part + m * p.part_stride + at;
-        float v[kBulkWarps], sum = 0.f;
+    if (!PASSES) {  // few rows a CTA: a lane each
+      math_sync<kWarps>();
+      const int sets = (ps.rows + 31) >> 5;
+      for (int e = w; e < sets * p.batch; e += kWarps) {
+        const int m = sets == 1 ? e : e / sets, at = (e - m * sets) * 32 + lane;
+        const int r = TILED ? at : (at & ~15) + ((at & 7) >> 1) + (at & 1) * 8 + ((at >> 1) & 4);  // the row that row_a put there
+        if (r < ps.rows) {
+          const float* q = sums + m * p.part_stride + at;
+          float v[kWarps], sum = 0.f;
 #pragma unroll
-        for (int i = 0; i < kBulkWarps; ++i) v[i] = q[i * p.part_rows * p.part_stride];
+          for (int i = 0; i < kWarps; ++i) v[i] = q[i * p.part_rows * p.part_stride];
 #pragma unroll
-        for (int i = 0; i < kBulkWarps; ++i) sum += v[i];
-        const int row = ps.row0 + r;
-        if (p.bias) sum += __half2float(p.bias[row]);
-        store_from_float(p.y, p.y_dtype, (int64_t)(y_row + m) * p.ld_y + row, sum);
+          for (int i = 0; i < kWarps; ++i) sum += v[i];
+          const int row = ps.row0 + r;
+          if (p.bias) sum += __half2float(p.bias[row]);
+          store_from_float(p.y, p.y_dtype, (int64_t)m * p.ld_y + row, sum);
+        }
       }
+      continue;
     }
+    if (ps.left == 0) {  // the last pass: nothing left to overlap, and all warps are faster than two
+      math_sync<kWarps>();
+      sum_pass(sums, GROUPED ? group_rows : p.batch, y_row, w, kWarps);
+      break;
+    }
+    __syncwarp();
+    if (lane == 0) bar_arrive(part_full + 8 * b);
+    if (++b == p.part_bufs) { b = 0; part_ph ^= 1; }
   }
 }
 
 // ---- host side --------------------------------------------------------------------------------------------------
-template <bool PACKED, int NT, int BPW, bool TILED, bool GROUPED>
+template <bool PACKED, int NT, int BPW, bool TILED, bool GROUPED, bool PASSES>
 static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
   constexpr int kRowBytes = PACKED ? 64 : 128, kRecBytes = kRowBytes * 16 + 32;
-  a.chunk_blocks = kBulkWarps * BPW;
+  constexpr int kWarps = bulk_warps(BPW);
+  a.chunk_blocks = kWarps * BPW;
   a.n_chunk = (a.nb + a.chunk_blocks - 1) / a.chunk_blocks;
   const int blocks = a.nb < a.chunk_blocks ? a.nb : a.chunk_blocks;  // of the largest stage
   a.units = (a.N + 15) / 16;
@@ -614,10 +727,14 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
   // Rows per pass: the sums of a pass meet at a barrier, and two sets of activation rows read their activations again for
   // every K range of a pass, so few and equal passes; but 64 rows of 8 activation rows are 34 KB of partial sums (of 16: 68 KB),
   // which the ring would rather have.  8 rows: 64 best of 32, 64, 96 and 176; 16 rows, 24576 x 4096: 35.9, 28.5 and 25.1 us for
-  // 16, 32 and 64, 6144 x 4096: 14.1, 12.3 and 11.3 us.
+  // 16, 32 and 64, 6144 x 4096: 14.1, 12.3 and 11.3 us.  Groups of few warps have room for 128 rows: 128 experts, 64 tokens,
+  // 267 us against 276 with 64.
   a.part_rows = a.batch < 8 * NT ? a.batch : 8 * NT;
   const int cta_rows = (int)((line + G - 1) / G) * 16;
   const int entries = PACKED ? (a.n_levels <= 8 ? 128 : 256) : a.n_levels;
+  // Three blocks a warp (short rows): as few warps a tile as hold it, as many tiles at a time as the warps make groups.
+  a.group_warps = BPW == 3 ? (a.nb + 2) / 3 : kWarps;
+  a.groups = kWarps / a.group_warps;
   a.part_off = kTabAddr + entries * 256;  // leaves room for the table wherever the window starts
   // Row-major stages: a copy of its own for every row of 2 KB or more; shorter rows that follow each other in memory share one
   // (a copy costs about 60 ns whatever its size: 128 experts of 21 and 15 blocks, rows of 1344 and 960 bytes, took 380 us with a
@@ -626,26 +743,28 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
   a.copy_rows = 1;
   if (a.n_chunk == 1 && a.ld_codes == a.row_stride)
     while (a.copy_rows < 8 && a.copy_rows * a.row_stride < 2048) a.copy_rows *= 2;
-  // Grouped launches meet new rows all the time, and the norm warp's sixteen loads a stage are what paces them: where the norms of
-  // a tile follow each other and their bytes are whole 16s, they come as one more bulk copy (128 experts, 2688 -> 2 x 1856, 64
-  // tokens: 354 and 349 us; one token 41.1 and 39.0).  Their rows then share banks where the block count is even, which the
-  // long rows of a dense layer feel more than the loads (24576 x 4096 at 8 rows: 16.4 us by the norm warp, 17.0 copied).
-  a.norm_stride = GROUPED && !TILED && a.n_chunk == 1 && a.ld_norms == a.nb && (reinterpret_cast<uintptr_t>(a.norms) & 15) == 0 &&
-                  a.norms_stride % 8 == 0 && (a.N % 16) * a.nb % 8 == 0 ? a.nb * 2 : 0;
   a.stage_bytes = TILED ? (blocks * kRecBytes + 127) & ~127 : (16 * a.row_stride + 64 + blocks * 32 + 127) & ~127;
-  for (int cap = a.part_rows <= 2 ? 256 : 64;; cap /= 2) {
+  for (int cap = BPW == 3 ? 128 : a.batch <= 2 ? 256 : 64;; cap /= 2) {
     if (cap < 16) return PE_ERR_LIMIT;
     const int passes = (cta_rows + cap - 1) / cap;
     a.pass_rows = GROUPED ? cap : ((cta_rows + passes - 1) / passes + 15) / 16 * 16;
-    a.part_stride = a.pass_rows + 4;  // rows of a stage land on different banks than the activation rows' distance
-    a.stage_off = (a.part_off + kBulkWarps * a.part_rows * a.part_stride * 4 + 127) & ~127;
+    a.part_stride = a.pass_rows + 4;
+    a.part_floats = a.group_warps * a.part_rows * a.part_stride;
+    a.part_bufs = PASSES ? 2 : 1;
+    a.stage_off = (a.part_off + a.part_bufs * a.part_floats * 4 + 127) & ~127;
     a.n_stage = a.stage_off < (int)kBulkSmemMax ? ((int)kBulkSmemMax - a.stage_off) / a.stage_bytes : 0;
     if (a.n_stage >= 2) break;
   }
   if (a.n_stage > kBulkMaxStages) a.n_stage = kBulkMaxStages;
+  if (a.groups > a.n_stage) a.groups = a.n_stage;
+  // Several passes: sums by warps of their own, where two sets of them leave a ring of three stages (15360 x 2560 Q5 at 16 rows
+  // would have two, and takes 20.1 us that way, 18.7 with one set; 24576 x 4096 Q3 has three: 24.2 and 25.2 us).
+  if (!PASSES && a.pass_rows < cta_rows && a.stage_off + a.part_floats * 4 + 3 * a.stage_bytes <= (int)kBulkSmemMax)
+    return launch_bulk<PACKED, NT, BPW, TILED, GROUPED, true>(a, sms, st);
+  a.n_stage -= a.n_stage % a.groups;  // a stage is one group's: a wait on a parity holds for a waiter that took every earlier phase
   unsigned dyn = a.stage_off + a.n_stage * a.stage_bytes;
   if (dyn < (unsigned)(kTabAddr + kTabReach)) dyn = kTabAddr + kTabReach;
-  auto kfn = gemv_bulk_kernel<PACKED, NT, BPW, TILED, GROUPED>;
+  auto kfn = gemv_bulk_kernel<PACKED, NT, BPW, TILED, GROUPED, PASSES>;
   static thread_local unsigned configured[16] = {0};
   int dev = 0;
   PE_CUDA_TRY(cudaGetDevice(&dev));
@@ -653,16 +772,28 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
     PE_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     if (dev < 16) configured[dev] = dyn;
   }
-  PE_CUDA_TRY(launch_pdl(kfn, dim3(G), dim3(bulk_threads(TILED)), dyn, st, a));
+  PE_CUDA_TRY(launch_pdl(kfn, dim3(G), dim3(bulk_threads(BPW, TILED, PASSES)), dyn, st, a));
   return PE_OK;
 }
 
 template <bool PACKED, bool TILED, bool GROUPED>
 static int launch_bulk_shape(BulkArgs& a, int sms, cudaStream_t st) {
+  // Grouped launches meet new rows all the time, and the norm warp's sixteen loads a stage are what paces them: where the norms of
+  // a tile follow each other and their bytes are whole 16s, they come as one more bulk copy (128 experts, 2688 -> 2 x 1856, 64
+  // tokens: 354 and 349 us; one token 41.1 and 39.0).  Their rows then share banks where the block count is even, which the
+  // long rows of a dense layer feel more than the loads (24576 x 4096 at 8 rows: 16.4 us by the norm warp, 17.0 copied).
+  a.norm_stride = !TILED && a.nb <= 16 * (a.batch > 8 ? 1 : 2) && a.ld_norms == a.nb && (reinterpret_cast<uintptr_t>(a.norms) & 15) == 0 &&
+                  a.norms_stride % 8 == 0 && (a.N % 16) * a.nb % 8 == 0 ? a.nb * 2 : 0;
   // Blocks per warp and stage: two when the row is longer than sixteen blocks.  Two sets of activation rows keep one:
   // their operands for two blocks spill (4096 x 12288 at 16 rows: 18.4 us with two, 15.9 with one).
-  if (a.batch > 8) return launch_bulk<PACKED, 2, 1, TILED, GROUPED>(a, sms, st);
-  return a.nb > kBulkWarps ? launch_bulk<PACKED, 1, 2, TILED, GROUPED>(a, sms, st) : launch_bulk<PACKED, 1, 1, TILED, GROUPED>(a, sms, st);
+  if (a.batch > 8) return launch_bulk<PACKED, 2, 1, TILED, GROUPED, GROUPED>(a, sms, st);
+  // Three, and groups of warps, for rows of up to 21 blocks: always in grouped launches; in others where a CTA has six tiles or
+  // more, for the groups to have several each (6400 x 2560 Q5 has 2.7: 7.9 us with two blocks a warp, 8.2 with three;
+  // 10240 x 2048 Q3 4.3: 6.9 and 7.2; 15360 x 2560 Q3 6.5: 9.9 and 9.4), and for one or two activation rows only where one block a warp is
+  // not enough (20480 x 1152 Q4, one row: 7.4 and 7.5; 15360 x 2560 Q3, one row: 9.1 and 8.8).
+  if (a.nb <= kGroupBlocks && (GROUPED || ((a.N + 15) / 16 >= 6 * sms && (a.batch > 2 || a.nb > 16))))
+    return launch_bulk<PACKED, 1, 3, TILED, GROUPED, true>(a, sms, st);
+  return a.nb > 16 ? launch_bulk<PACKED, 1, 2, TILED, GROUPED, GROUPED>(a, sms, st) : launch_bulk<PACKED, 1, 1, TILED, GROUPED, GROUPED>(a, sms, st);
 }
 
 template <bool PACKED, bool TILED>
@@ -699,6 +830,7 @@ int gemv_bulk_run(const GemvBulkCall& q, cudaStream_t st) {
   a.ct = q.ct_scaled; a.n_levels = q.n_levels;
   a.frags = f.out;
   a.y = q.y; a.y_dtype = q.y_dtype; a.ld_y = q.ld_y;
+  a.y_vec = (reinterpret_cast<uintptr_t>(q.y) & 15) == 0 && q.ld_y % 4 == 0;
   a.bias = static_cast<const __half*>(q.bias);
   a.batch = q.batch; a.N = q.out_f; a.nb = f.nb;
   a.status = q.status;

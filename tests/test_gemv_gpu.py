@@ -351,6 +351,28 @@ def test_row_major_stages_follow_the_strides(bits, n, k, rows):
     assert torch.equal(y, kernels.quant_matmul(gap[:, 16:16 + w.shape[1]], packed, odd[:, 1:1 + nd.shape[1]], ctd, x, False, n, k, k, torch.float32))
 
 
+@pytest.mark.parametrize("rows", [1, 3, 8, 16])
+@pytest.mark.parametrize("bits,n,k", [(4, 14213, 128), (6, 14209, 1024), (3, 17001, 2176), (5, 14210, 2688), (3, 21000, 2816), (4, 20000, 4096)])
+def test_several_passes_a_cta(rows, bits, n, k):
+    """Layers that give a CTA six tiles of rows and more: sums by warps of their own, groups of warps for rows of up to 21
+    blocks, a last pass and a last tile that are not full; norms that come as one copy and norms that are gathered give the same
+    bits, and so does every run.  Tolerance as everywhere here: fp16 operands, fp32 sums."""
+    from polarengine_vllm_b200 import kernels, packing
+    codes, norms, cts = rand_layer(n, k, bits, seed=n + k)
+    packed = bits <= 4
+    w = packing.pack_codes_half_block(codes.cuda()) if packed else codes.cuda()
+    nd, ctd, x = norms.cuda(), cts.cuda(), rand_x(rows, k, seed=rows).cuda()
+    bias = rand_x(1, n, seed=5)[0]
+    y = kernels.quant_matmul(w, packed, nd, ctd, x, False, n, k, k, torch.float32, bias.cuda())
+    assert max_rel(y, oracle.linear_dequant(x.cpu(), codes, norms, cts) + bias.float()) <= TOL
+    odd = torch.full((n, nd.shape[1] + 3), float("nan"), dtype=torch.float16, device="cuda")
+    odd[:, 1:1 + nd.shape[1]] = nd
+    assert torch.equal(y, kernels.quant_matmul(w, packed, odd[:, 1:1 + nd.shape[1]], ctd, x, False, n, k, k, torch.float32, bias.cuda()))
+    half = kernels.quant_matmul(w, packed, nd, ctd, x, False, n, k, k, torch.float16, bias.cuda())
+    assert torch.equal(half, y.half())
+    assert torch.equal(y, kernels.quant_matmul(w, packed, nd, ctd, x, False, n, k, k, torch.float32, bias.cuda()))
+
+
 @pytest.mark.parametrize("bits", [4, 6])
 def test_a_linear_layer_has_one_copy_of_its_weights(bits):
     """Decode-size batches multiply by what the layer's arrays hold at the call -- rewritten in place included, the first
