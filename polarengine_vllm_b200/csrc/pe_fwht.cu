@@ -52,13 +52,13 @@ __global__ void __launch_bounds__(256) pack_nibble_kernel(const int8_t* codes, u
 // cell boundary to within fp32 rounding can land on the other side: a few codes per million differ from the CPU
 // quantizer.
 //
-// The launch is bound by instruction issue and the shared-memory port (two exchanges and two lookups per weight), not
-// by memory (two bytes in, one out).  Four lanes share a 128-block, in four pieces of 8 consecutive values each: five
+// fp32 weights (quantize_kernel): the launch is bound by instruction issue and the shared-memory port (two exchanges and two
+// lookups per weight), not by memory (four bytes in, one out).  Four lanes share a 128-block, in four pieces of 8 consecutive values each: five
 // of the seven butterfly stages stay in registers, a warp reads and writes whole sectors, the level is found with one
 // table lookup and one comparison instead of a scan of all levels, the quotient is a product with the reciprocal and
-// one correction, and fp32 arithmetic goes two values per instruction.  4096 x 12288 bf16, on 2 resident CTAs per SM
-// with the next trip's loads in flight: to 4 bits 256 -> 61 us (LSU port 70 % busy, issue slots 66 %), 4096 x 4000 to
-// 8 bits 729 -> 32 us against one warp per block, a scan and a full division per value.
+// one correction, and fp32 arithmetic goes two values per instruction.  4096 x 12288, on 2 resident CTAs per SM
+// with the next trip's loads in flight: to 4 bits 68 us; against one warp per block, a scan and a full division per value 256 -> 61 us
+// on bf16 weights, which now have a kernel of their own.
 
 // Exact cell edges: the rotated unit-vector element v takes code j when j edges are below it.  edge[j] is the largest
 // float that is still no farther from level j than from level j + 1 by the fp32 distances quant_dist() that a scan
@@ -156,6 +156,189 @@ __device__ __forceinline__ void cvt8(const Raw8<W_DTYPE>& r, float v[8]) {
       const float2 f = W_DTYPE == PE_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&h[i]))
                                          : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&h[i]));
       v[2 * i] = f.x; v[2 * i + 1] = f.y;
+    }
+  }
+}
+
+// ---- 16-bit weights: the rotation on the tensor cores ------------------------------------------------------------
+// A value's index in its block is 8 a + j.  Lane (g, t) of a warp has the values of a = 2 t, 2 t + 1, 8 + 2 t and 9 + 2 t of block g
+// (32 bytes at a time, so that a warp reads whole lines), which is what operand A of an m16n8k16 product wants of row g with
+// k = a; rows 8 to 15 stay zero.  Products 2 j and 2 j + 1 are the two halves of the 16-point transform over a of the eight
+// blocks' values j: 16-bit values times +-1, exact, summed in fp32.  The lane gets back the same a of its own block, so that the
+// eight-point transform over j, the norm and sixteen consecutive codes twice need no other lane but for one sum of four.
+// (With the blocks as columns of the product the codes came out four blocks a lane: 59 us where this takes 55.)  The norm is that of
+// the rotated values, which are divided by it afterwards: fewer roundings on the way than dividing first.  Codes that are not
+// the nearest level in 64 bits, of 16.8 million: 16 at 4 bits, 31 at 6 (with the butterflies 15 and 35).
+// What bounds it: the L1 data port, 76 % busy (a cycle per 32-byte sector that comes or goes, two look-ups a value), and the chain of
+// a trip.  4096 x 12288 bf16 against the butterfly kernel: to 4 bits 62 -> 55 us, to 6 bits 67 -> 58.
+template <int W_DTYPE>
+__device__ __forceinline__ void mma_first(float2& d, uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+  float unused0, unused1;
+  if (W_DTYPE == PE_F16)
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%5}, {%7,%8}, {%9,%9,%9,%9};"
+        : "=f"(d.x), "=f"(d.y), "=f"(unused0), "=f"(unused1) : "r"(a0), "r"(0), "r"(a2), "r"(b0), "r"(b1), "f"(0.f));
+  else
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%5}, {%7,%8}, {%9,%9,%9,%9};"
+        : "=f"(d.x), "=f"(d.y), "=f"(unused0), "=f"(unused1) : "r"(a0), "r"(0), "r"(a2), "r"(b0), "r"(b1), "f"(0.f));
+}
+
+// Two CTAs an SM request the next trip's values ahead (116 registers); three do not (80).  FEW: at most 64 levels.
+template <int W_DTYPE, int CTAS, bool FEW>
+__global__ void __launch_bounds__(256, CTAS) quantize16_kernel(const void* w, int64_t ld_w, int64_t rows, int in_f, int nb,
+                                                            const float* levels, int n_levels, int8_t* codes, int64_t ld_codes,
+                                                            __half* norms, int64_t ld_norms, int vec_out) {
+  __shared__ float lv[256];
+  __shared__ QuantTable q;
+  uint32_t cells = 64;  // as quantize_kernel
+  while ((int)cells < 16 * n_levels && cells < 2048) cells *= 2;
+  const float scale = (float)cells / (2.f * kQuantRange), magic = 12582912.f + (float)(cells / 2);
+  const bool scan = build_quant_table(q, lv, levels, n_levels, cells, scale, magic);
+  if (FEW && !scan) {  // up to 64 levels: four times the level, the byte offset of its edge
+    for (int c = threadIdx.x; c < (int)cells; c += blockDim.x) q.first[c] *= 4;
+    __syncthreads();
+  }
+  constexpr uint32_t kOne = FEW ? 4 : 1;
+  auto edge_of = [&](uint32_t j) { return FEW ? *reinterpret_cast<const float*>(reinterpret_cast<const char*>(q.edge) + j) : q.edge[j]; };
+  const uint32_t mask = cells - 1;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int64_t n_warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const bool vin = (ld_w * 2) % 16 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0, vin32 = (ld_w * 2) % 32 == 0 && (reinterpret_cast<uintptr_t>(w) & 31) == 0;
+  const int64_t first = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 8 + g;
+  int64_t r = first / nb;
+  int blk = (int)(first - r * nb);
+  const int64_t step_r = n_warps * 8 / nb;
+  const int step_b = (int)(n_warps * 8 - step_r * nb);
+  // sign of H16: the parity of the bits that column n (g, g + 8) and index a (2 t, 2 t + 1 and 8 further on) share
+  const uint32_t one = W_DTYPE == PE_F16 ? 0x3c00u : 0x3f80u, sign = (uint32_t)(__popc(g & 2 * t) & 1) << 15;
+  const uint32_t h0 = one | sign | (one | (sign ^ ((uint32_t)(g & 1) << 15))) << 16, h1 = h0 ^ 0x80008000u;
+  Raw8<W_DTYPE> raw[4];
+  auto request = [&]() {  // block (r, blk) of the weight, zeros past its last row
+    const int col = blk * kBlock + t * 16;
+    if (vin32 && r < rows && (blk + 1) * kBlock <= in_f) {
+      const uint16_t* src = static_cast<const uint16_t*>(w) + r * ld_w + col;
+#pragma unroll
+      for (int p = 0; p < 4; p += 2)
+        asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(raw[p].q[0].x), "=r"(raw[p].q[0].y), "=r"(raw[p].q[0].z), "=r"(raw[p].q[0].w), "=r"(raw[p + 1].q[0].x),
+                       "=r"(raw[p + 1].q[0].y), "=r"(raw[p + 1].q[0].z), "=r"(raw[p + 1].q[0].w) : "l"(src + 32 * p));
+      return;
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+      raw[p] = load8_raw<W_DTYPE>(w, r < rows ? r * ld_w : 0, col + (p >> 1) * 64 + (p & 1) * 8, r < rows ? in_f : 0, vin);
+  };
+  if (CTAS == 2) request();
+  while (__any_sync(0xffffffffu, r < rows)) {
+    if (CTAS != 2) request();
+    const int64_t r_out = r;
+    const int blk_out = blk;
+    float2 v[8][2];  // values 8 (2 t + 8 h) + j (x) and 8 further on (y)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      uint32_t u[4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) u[p] = j < 2 ? raw[p].q[0].x : j < 4 ? raw[p].q[0].y : j < 6 ? raw[p].q[0].z : raw[p].q[0].w;
+      const uint32_t sel = j & 1 ? 0x7632 : 0x5410;
+      const uint32_t x0 = __byte_perm(u[0], u[1], sel), x1 = __byte_perm(u[2], u[3], sel);
+      mma_first<W_DTYPE>(v[j][0], x0, x1, h0, h0);
+      mma_first<W_DTYPE>(v[j][1], x0, x1, h0, h1);
+    }
+    r += step_r;
+    blk += step_b;
+    if (blk >= nb) { blk -= nb; ++r; }
+    if (CTAS == 2) request();
+    const float2 minus = make_float2(-1.f, -1.f);
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (!(j & o))
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float2 a = v[j][h], b = v[j | o][h];
+            v[j][h] = add2(a, b);
+            v[j | o][h] = fma2(b, minus, a);
+          }
+    // the rotation keeps the norm: the squares of its results, sqrt(128) too large, sum to 128 times the block's
+    auto squares = [&](float f) {
+      float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float2 x = f == 1.f ? v[j][h] : mul2(v[j][h], make_float2(f, f));
+          s = fma2(x, x, s);
+        }
+      float sum = s.x + s.y;
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      return sum + __shfl_xor_sync(0xffffffffu, sum, 2);
+    };
+    const float s128 = 0.08838834764831845f;  // 1/sqrt(128)
+    const float sum = squares(1.f);
+    float nrm = sqrtf(sum) * s128;
+    if (W_DTYPE == PE_BF16 && __any_sync(0xffffffffu, !(sum < 1e38f))) {  // again with halved exponents; a norm whose own square overflows is infinite
+      const float small = sqrtf(squares(5.421010862427522e-20f)) * s128;  // 2^-64
+      if (!(sum < 1e38f)) nrm = small < 1.f ? small * 18446744073709551616.f : small >= 1.f ? __int_as_float(0x7f800000) : small;
+    }
+    nrm = fmaxf(nrm, 1e-10f);
+    const float inv = __fdiv_rn(s128, nrm);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) v[j][h] = mul2(v[j][h], make_float2(inv, inv));
+    uint32_t packed[2][2][2];  // half of the block, a, four codes each
+#pragma unroll
+    for (int i = 0; i < 8; ++i) packed[i >> 2][(i >> 1) & 1][i & 1] = 0;
+    if (!scan) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float2 x = v[j][h], c = fma2(x, make_float2(scale, scale), make_float2(magic, magic));  // quant_cell of both
+          const uint32_t jx = q.first[__float_as_uint(c.x) & mask], jy = q.first[__float_as_uint(c.y) & mask];
+          uint32_t &px = packed[h][0][j >> 2], &py = packed[h][1][j >> 2];
+          px += jx << (8 * (j & 3));
+          py += jy << (8 * (j & 3));
+          if (x.x > edge_of(jx)) px += kOne << (8 * (j & 3));
+          if (x.y > edge_of(jy)) py += kOne << (8 * (j & 3));
+        }
+      if (FEW)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) packed[i >> 2][(i >> 1) & 1][i & 1] >>= 2;
+      if (v[0][0].x != v[0][0].x)  // a NaN reaches the whole block
+#pragma unroll
+        for (int i = 0; i < 8; ++i) packed[i >> 2][(i >> 1) & 1][i & 1] = 0;
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < 32; ++i) {
+        float x = 0.f;
+#pragma unroll
+        for (int k = 0; k < 32; ++k)
+          if (k == i) x = ((k >> 3) & 1) ? v[k & 7][k >> 4].y : v[k & 7][k >> 4].x;
+        uint32_t best = 0;
+        float bd = quant_dist(x, lv[0]);
+        for (int j = 1; j < n_levels; ++j) {
+          const float d = quant_dist(x, lv[j]);
+          if (d < bd) { bd = d; best = j; }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (k == i >> 2) packed[k >> 2][(k >> 1) & 1][k & 1] |= best << (8 * (i & 3));
+      }
+    }
+    if (r_out < rows) {
+      int8_t* dst = codes + r_out * ld_codes + blk_out * kBlock + t * 16;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint4 c = make_uint4(packed[h][0][0], packed[h][0][1], packed[h][1][0], packed[h][1][1]);
+        if (vec_out) {
+          *reinterpret_cast<uint4*>(dst + 64 * h) = c;
+        } else {
+          uint32_t* d = reinterpret_cast<uint32_t*>(dst + 64 * h);
+          d[0] = c.x; d[1] = c.y; d[2] = c.z; d[3] = c.w;
+        }
+      }
+      if (t == 0) norms[r_out * ld_norms + blk_out] = __float2half_rn(nrm);
     }
   }
 }
@@ -417,9 +600,14 @@ extern "C" int pe_quantize(const void* weight, int w_dtype, int64_t ld_w, int64_
   const int sms = sm_count();
   if (sms <= 0) return PE_ERR_CUDA;
   // the resident CTAs (two per SM); the level table is built once per CTA
-  const unsigned grid = (unsigned)(ctas < 2ll * sms ? ctas : 2ll * sms);
-  auto kfn = w_dtype == PE_F32 ? quantize_kernel<PE_F32> : w_dtype == PE_F16 ? quantize_kernel<PE_F16> : quantize_kernel<PE_BF16>;
-  const int vec_out = (reinterpret_cast<uintptr_t>(codes) & 7) == 0 && ld_codes % 8 == 0;
+  const bool wide = n_levels > 16;
+  const long long per = w_dtype == PE_F32 || wide ? 2 : 3;
+  const unsigned grid = (unsigned)(ctas < per * sms ? ctas : per * sms);
+  // 4096 x 12288 bf16 with two / three CTAs an SM: to 4 bits 59 / 55 us, to 6 bits 58 / 60 us
+#define PE_QUANTIZE16(W) (!wide ? quantize16_kernel<W, 3, true> : n_levels <= 64 ? quantize16_kernel<W, 2, true> : quantize16_kernel<W, 2, false>)
+  auto kfn = w_dtype == PE_F32 ? quantize_kernel<PE_F32> : w_dtype == PE_F16 ? PE_QUANTIZE16(PE_F16) : PE_QUANTIZE16(PE_BF16);
+#undef PE_QUANTIZE16
+  const int unit = w_dtype == PE_F32 ? 8 : 16, vec_out = reinterpret_cast<uintptr_t>(codes) % unit == 0 && ld_codes % unit == 0;
   kfn<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(weight, ld_w, out_f, in_f, nb, levels, n_levels, codes, ld_codes,
                                                            static_cast<__half*>(norms), ld_norms, vec_out);
   PE_CUDA_TRY(cudaGetLastError());

@@ -64,3 +64,49 @@ def test_gpu_quantizer_levels_of_any_kind(levels):
     rot = blocks / blocks.norm(dim=2, keepdim=True) @ oracle.hadamard(128) * 128 ** 0.5
     ref = (rot.unsqueeze(-1) - lv).abs().argmin(-1).view(33, 256)
     assert int((codes.cpu().view(torch.uint8).int() != ref).sum()) <= 8
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols,bits", [(1, 8, 3), (3, 129, 4), (65, 1000, 5), (33, 1152, 6), (130, 4100, 8)])
+def test_gpu_quantizer_16_bit_weights(dtype, rows, cols, bits):
+    """16-bit weights of any width, row stride and address, an all-zero block among them: the codes that 64-bit arithmetic gives
+    except next to a cell edge (a value within 2e-6 of it: fp32 sums of 128 values of order one), the norms to one fp16 step."""
+    from polarengine_vllm_b200 import _native as nv
+    from polarengine_vllm_b200.utils import get_centroids
+    g = torch.Generator().manual_seed(rows + bits)
+    wide = (0.02 * torch.randn(rows, cols + 5, generator=g)).to(dtype).cuda()
+    wide[0, :128] = 0
+    lv, padded = get_centroids(bits).cuda(), -(-cols // 128) * 128
+    nv.ensure_init(wide.device)
+    out = []
+    for w, ld in ((wide[:, :cols].contiguous(), cols), (wide[:, 3:3 + cols], cols + 5)):
+        codes = torch.full((rows, padded), 0x55, dtype=torch.int8, device="cuda")
+        norms = torch.empty(rows, padded // 128, dtype=torch.float16, device="cuda")
+        nv.check(nv.lib().pe_quantize(w.data_ptr(), nv.dtype_code(w), ld, rows, cols, padded, lv.data_ptr(), lv.numel(), codes.data_ptr(), padded,
+                                      norms.data_ptr(), padded // 128, nv.stream_ptr(w.device)), "pe_quantize")
+        x = torch.nn.functional.pad(w.double(), (0, padded - cols)).view(-1, 128)
+        n = x.norm(dim=1).clamp_min(1e-10)
+        rot = (x / n[:, None]) @ oracle.hadamard(128).double().cuda() * 128 ** 0.5
+        c = codes.view(torch.uint8).long().view(-1, 128)
+        excess = (rot - lv.double()[c]).abs() - (rot.unsqueeze(-1) - lv.double()).abs().amin(-1)
+        assert float(excess.max()) <= 2e-6
+        assert ((norms.double().view(-1) - n).abs() <= n * 2 ** -10 + 1e-7).all()
+
+
+def test_gpu_quantizer_extreme_values():
+    """bf16 values whose squares overflow fp32, infinities and NaN: code 0 where a block has no finite unit vector, its neighbours
+    as without it."""
+    from polarengine_vllm_b200.quantizer import PolarQuantizer
+    g = torch.Generator().manual_seed(3)
+    w = (0.02 * torch.randn(4, 1024, generator=g)).to(torch.bfloat16).cuda()
+    ref = PolarQuantizer().quantize_tensor_gpu(w, 4)["codes"].view(4, 8, 128)
+    x = w.clone()
+    x[0, 128:256] *= 2.0 ** 66     # norm about 1.7e19: its square overflows on the way, the norm does not
+    x[1, 300], x[2, 5], x[3, 1000] = float("inf"), float("nan"), float("-inf")
+    q = PolarQuantizer().quantize_tensor_gpu(x, 4)
+    codes, norms = q["codes"].view(4, 8, 128), q["norms"]
+    assert torch.equal(codes[0], ref[0]) and bool(torch.isinf(norms[0, 1]))
+    for r, b in ((1, 2), (2, 0), (3, 7)):
+        assert not codes[r, b].any()
+        codes[r, b] = ref[r, b]
+    assert torch.equal(codes, ref)
