@@ -3,7 +3,7 @@
 //
 //   Y[m, n] = sum_k Xt[m, k] * (ct[code[n, k]] * norm[n, k / 128])        (+ bias[n])
 //
-// gemm_pair_kernel: more than 256 rows.  A cluster of two CTAs per 512 tokens x 256 weight rows, one cta_group::2 MMA
+// gemm_pair_kernel: more than 256 rows, where many_rows_plan does not prefer the tensor-memory kernel.  A cluster of two CTAs per 512 tokens x 256 weight rows, one cta_group::2 MMA
 // per pair, each CTA decoding half of the weight tile.  (Up to 256 rows: pe_gemm_tmem.cu.)  It walks K in steps of 64:
 //   * one thread issues TMA (cp.async.bulk.tensor.2d, 128-byte swizzle, no multicast) for the bf16
 //     activation tiles and another for the raw code rows of the step;
@@ -625,6 +625,69 @@ static PairPlan pair_plan(int tiles_m, int tiles_n, int ksteps, int sms) {
   return {tiles - rest, ks, (tiles_n - cols) * kTileN};
 }
 
+// ---- more than 256 rows: which kernel, which tiles ----------------------------------------------------------------
+// A pair of CTAs does the work of a full 512 x 256 tile in 0.69 us per 64 of K, the tensor-memory kernel that of its four 256 x 128
+// tiles in 1.4 on two CTAs; but 512 x 256 is a coarse tile: rows are rounded up to 512, and a launch of a few hundred rows has less
+// than one or just over one wave of them.  So the time of both is estimated, for every tiling that the tensor-memory kernel
+// has, and the shorter one taken; the pair kernel where they are within 5 % (10 % at short K, where the drain of the tiles,
+// of which the estimate knows little, counts most: 16384 x 1280 Q6 at 1300 rows, estimated 5 % ahead, took 80.8 against 71.8 us).  The constants are a fit to 590 launches of nine
+// layer shapes at 24 to 2048 rows (7 % off on average); from 1601 rows on the pair kernel is ahead or level on all of them.
+// Before / now: 4096 x 4096 Q6 at 300 rows 31.8 / 24.9 us, 640: 46.8 / 34.0, 1024: 51.3 / 39.3; 24576 x 4096 Q3 at 400 rows 89 / 71,
+// 640: 156 / 107; 4096 x 12288 Q4 at 300 rows 61 / 43..49, 640: 97 / 68; 2560 x 2560 Q5 at 512 rows 28.4 / 20.9.
+constexpr int kTmemMaxRows = 1600;
+
+static double pair_time_us(int m, int out_f, int in_f_padded, int sms) {
+  const int tiles_m = (m + kPairTileM - 1) / kPairTileM, tiles_n = (out_f + kTileN - 1) / kTileN, steps = in_f_padded / kStepK, pairs = sms / 2;
+  const PairPlan p = pair_plan(tiles_m, tiles_n, steps, sms);
+  double t = 7.8 + 1.26e-6 * m * in_f_padded;  // launch and preparation
+  if (p.full) t += (p.full + pairs - 1) / pairs * (0.69 * steps + 7.1);
+  if (p.ksplit > 1) t += (steps + p.ksplit - 1) / p.ksplit * 0.69 + 7.4 + 1.0e-6 * p.ksplit * m * (out_f - p.col0);
+  return t;
+}
+
+struct TmemPlan { int halves, tiles_m, tok, ksplit; };
+static double tmem_time_us(const TmemPlan& p, int m, int out_f, int in_f_padded, int packed, int sms) {
+  const int nb = in_f_padded / kBlock, tiles_n = (out_f + 128 * p.halves - 1) / (128 * p.halves);
+  const int units = p.tiles_m * tiles_n * p.ksplit, waves = (units + sms - 1) / sms, steps = 2 * ((nb + p.ksplit - 1) / p.ksplit);
+  // a step of 128 weight rows: MMAs, or the decode (of tiles of one half by two of the four groups at a time); or the bytes of a step
+  double half = 127 + 0.92 * p.tok;
+  if (!packed && half < 285) half = 285;
+  if (p.halves == 1 && half < 259) half = 259;
+  const double bytes = 128.0 * p.tok + p.halves * (packed ? 4096 : 8192), step = p.halves * half > bytes * 0.0108 ? p.halves * half : bytes * 0.0108;
+  double unit = steps * step + 1740;  // ns
+  if (p.halves * p.tok > 192) unit += 4.5 * p.tok * p.halves;  // the accumulators fill tensor memory: the drain is not hidden
+  double t = 9.0 + 0.95e-6 * m * in_f_padded + waves * unit * 1e-3;
+  if (p.ksplit > 1) t += 1.5 + 0.71e-6 * p.ksplit * m * out_f;
+  return t;
+}
+
+// Shortest tiling of the tensor-memory kernel with at most `max_split` K ranges; halves = 0: the pair kernel is ahead.
+static TmemPlan many_rows_plan(int m, int out_f, int in_f_padded, int packed, int sms, size_t part_bytes) {
+  TmemPlan best = {0, 0, 0, 1};
+  if (m > kTmemMaxRows) return best;
+  // One row of pair tiles: only where a quarter of the time goes.  The kernels multiply the same values, but another cut of K is another
+  // order of the fp32 sums, and six decoder layers make about 1 % of their logits of that (0.75 % if q/k/v keeps its order, as it
+  // does with this line): no error, each is as far from 64-bit arithmetic as the other, but not worth 10 % of a launch.
+  const double share = m <= kPairTileM ? 0.76 : in_f_padded < 2048 ? 0.9 : 0.95;
+  double least = share * pair_time_us(m, out_f, in_f_padded, sms);
+  for (int halves = 1; halves <= 2; ++halves) {
+    const int most = halves == 1 ? 256 : 192, tiles_n = (out_f + 128 * halves - 1) / (128 * halves), first = (m + most - 1) / most;
+    for (int tiles_m = first; tiles_m < first + 3; ++tiles_m) {
+      TmemPlan p = {halves, tiles_m, ((m + tiles_m - 1) / tiles_m + 15) / 16 * 16, 1};
+      p.tiles_m = (m + p.tok - 1) / p.tok;  // the rounded tiles may be one fewer: none is empty
+      int ks = sms / (tiles_n * p.tiles_m);
+      if (ks > in_f_padded / kBlock / 2) ks = in_f_padded / kBlock / 2;
+      for (int split = 0; split < (ks > 1 ? 2 : 1); ++split) {
+        p.ksplit = split ? ks : 1;
+        if (split && (size_t)ks * m * out_f * sizeof(float) > part_bytes) continue;
+        const double t = tmem_time_us(p, m, out_f, in_f_padded, packed, sms);
+        if (t < least) { least = t; best = p; }
+      }
+    }
+  }
+  return best;
+}
+
 // workspace: [status word, padded to 256 B][bf16 activations M x K]
 extern "C" size_t pe_gemm_workspace_bytes(int m, int in_f_padded) {
   if (m < 1 || in_f_padded < kBlock || in_f_padded % kBlock) return 0;
@@ -637,15 +700,19 @@ extern "C" size_t pe_gemm_workspace_bytes_splitk(int m, int out_f, int in_f_padd
   if (base == 0 || out_f < 1) return 0;
   const int sms = sm_count();
   if (sms < 2) return base;
-  int ks = 1, cols = out_f;
+  size_t floats = 0;
+  auto want = [&](int ks, int cols) {
+    const size_t f = ks > 1 ? (size_t)ks * m * cols : 0;
+    if (f > floats) floats = f;
+  };
   if (m <= 256) {
-    ks = small_ksplit(m, out_f, in_f_padded, sms);
+    want(small_ksplit(m, out_f, in_f_padded, sms), out_f);
   } else {
     const PairPlan p = pair_plan((m + kPairTileM - 1) / kPairTileM, (out_f + kTileN - 1) / kTileN, in_f_padded / kStepK, sms);
-    ks = p.ksplit;
-    cols = out_f - p.col0;
+    want(p.ksplit, out_f - p.col0);
+    for (int packed = 0; packed < 2; ++packed) want(many_rows_plan(m, out_f, in_f_padded, packed, sms, ~(size_t)0).ksplit, out_f);
   }
-  return ks > 1 ? ((base + 255) & ~(size_t)255) + (size_t)ks * m * cols * sizeof(float) : base;
+  return floats ? ((base + 255) & ~(size_t)255) + floats * sizeof(float) : base;
 }
 
 extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms,
@@ -676,26 +743,27 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
   auto fits = [&](int ks, int cols) { return ks > 1 && workspace_bytes >= part_off + (size_t)ks * m * cols * sizeof(float); };
   float* part = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + part_off);
 
-  // One tile of tokens in tensor-memory form (up to 256), pairs of CTAs above.  The line is where the second tile of tokens would
-  // begin: the tensor-memory kernel is launched with one.  Measured at 257 rows with two tiles of 144 against one pair tile of 512:
-  // 4096 x 4096 23.7 and 29.3 us, 24576 x 4096 66 and 82, 12288 x 4096 47 and 58; at 512 rows 28.8 and 34.1, 94 and 97, 64 and 59.
-  if (m <= 256) {
+  // Up to 256 rows: one tile of tokens of the tensor-memory kernel.  Above, whichever is estimated to be shorter.
+  TmemPlan plan = {small_halves(m, out_f, sms), 1, m, 1};
+  if (m > 256) plan = many_rows_plan(m, out_f, in_f_padded, packed, sms, workspace_bytes > part_off ? workspace_bytes - part_off : 0);
+  else plan.ksplit = small_ksplit(m, out_f, in_f_padded, sms);
+  if (plan.halves) {
     TmemGemmArgs a = {};
     a.norms = static_cast<const __half*>(norms); a.ld_norms = ld_norms;
     a.ct = ct_scaled; a.n_levels = n_levels;
     a.y = y; a.y_dtype = y_dtype; a.ld_y = ld_y;
     a.bias = static_cast<const __half*>(bias);
     a.M = m; a.N = out_f; a.nb = in_f_padded / kBlock;
-    a.halves = small_halves(m, out_f, sms);
-    a.tiles_m = 1; a.tok = m;
+    a.halves = plan.halves;
+    a.tiles_m = plan.tiles_m; a.tok = plan.tok;
     a.tiles_n = (out_f + 128 * a.halves - 1) / (128 * a.halves);
-    a.ksplit = small_ksplit(m, out_f, in_f_padded, sms);
+    a.ksplit = plan.ksplit;
     if (!fits(a.ksplit, out_f)) a.ksplit = 1;
     a.part = a.ksplit > 1 ? part : nullptr;
-    a.xbox = (m + 15) & ~15;
+    a.xbox = (a.tok + 15) & ~15;
     a.x_stage = a.xbox * 128;
     a.status = status;
-    rc = launch_gemm_tmem(a, codes, packed, ld_codes, out_f, xq, m, a.tiles_n * a.ksplit, sms, st);
+    rc = launch_gemm_tmem(a, codes, packed, ld_codes, out_f, xq, m, a.tiles_m * a.tiles_n * a.ksplit, sms, st);
     if (rc != PE_OK || a.ksplit == 1) return rc;
     return launch_splitk_reduce(part, a.ksplit, m, out_f, bias, y, y_dtype, ld_y, sms, st);
   }
@@ -729,15 +797,15 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
   a.lut_bytes = packed ? 256 * kPairLutStride : n_levels * 128;
   a.nc = kPairCodeStages;
   const unsigned smem_bytes = (packed ? 4 : 3) * 2 * kXTileBytes + kPairWStages * kPairWTileBytes + a.lut_bytes + a.nc * 128 * code_row + 256 + 1024;
-  PairPlan plan = pair_plan(a.tiles_m, a.tiles_n, in_f_padded / kStepK, sms);
+  PairPlan pairs_of = pair_plan(a.tiles_m, a.tiles_n, in_f_padded / kStepK, sms);
   const int tiles = a.tiles_m * a.tiles_n;
-  if (!fits(plan.ksplit, out_f - plan.col0)) plan = {tiles, 1, 0};
-  a.full = plan.full; a.ksplit = plan.ksplit; a.col0 = plan.col0;
+  if (!fits(pairs_of.ksplit, out_f - pairs_of.col0)) pairs_of = {tiles, 1, 0};
+  a.full = pairs_of.full; a.ksplit = pairs_of.ksplit; a.col0 = pairs_of.col0;
   a.part = part;
   CUtensorMap partmap = ymap;
-  a.part_tma = plan.ksplit > 1 && (out_f - plan.col0) % 4 == 0;
-  if (a.part_tma && (rc = encode_map_f32(&partmap, part, out_f - plan.col0, m, plan.ksplit, (uint64_t)(out_f - plan.col0) * 4)) != PE_OK) return rc;
-  const int units = plan.full + (tiles - plan.full) * plan.ksplit, pairs = units < sms / 2 ? units : sms / 2;
+  a.part_tma = pairs_of.ksplit > 1 && (out_f - pairs_of.col0) % 4 == 0;
+  if (a.part_tma && (rc = encode_map_f32(&partmap, part, out_f - pairs_of.col0, m, pairs_of.ksplit, (uint64_t)(out_f - pairs_of.col0) * 4)) != PE_OK) return rc;
+  const int units = pairs_of.full + (tiles - pairs_of.full) * pairs_of.ksplit, pairs = units < sms / 2 ? units : sms / 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs);
   cfg.blockDim = dim3(kPairThreads);
@@ -753,8 +821,8 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
   auto kfn = packed ? gemm_pair_kernel<true> : gemm_pair_kernel<false>;
   PE_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
   PE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kfn, a, map, pmap, ymap, partmap));
-  if (plan.ksplit == 1) return PE_OK;
-  const int c0 = plan.col0;
-  return launch_splitk_reduce(part, plan.ksplit, m, out_f - c0, bias ? static_cast<const __half*>(bias) + c0 : nullptr,
+  if (pairs_of.ksplit == 1) return PE_OK;
+  const int c0 = pairs_of.col0;
+  return launch_splitk_reduce(part, pairs_of.ksplit, m, out_f - c0, bias ? static_cast<const __half*>(bias) + c0 : nullptr,
                               static_cast<uint8_t*>(y) + (int64_t)c0 * (y_dtype == PE_F32 ? 4 : 2), y_dtype, ld_y, sms, st);
 }

@@ -1,4 +1,5 @@
-// Quantized matmul on the tensor cores with the decoded weights in TENSOR MEMORY: up to 256 activation rows, and the
+// Quantized matmul on the tensor cores with the decoded weights in TENSOR MEMORY: up to 256 activation rows (and more,
+// where many_rows_plan says so), and the
 // grouped launches over the experts of a mixture layer.
 //
 //   Y[m, n] = sum_k X[m, k] * (ct[code[n, k]] * norm[n, k / 128])     (+ bias[n]; or silu(first half) * second half)

@@ -1,4 +1,4 @@
-// Arguments and launcher of the tensor-core matmul for up to 256 activation rows and for grouped launches
+// Arguments and launcher of the tensor-core matmul for some hundred activation rows and for grouped launches
 // (pe_gemm_tmem.cu).
 #pragma once
 #include "pe_gemm.cuh"

@@ -216,3 +216,36 @@ def test_gemm_last_wave_split_over_the_pairs(m, n, bits, dtype):
     ref = oracle.linear_dequant(x[rows], codes, norms, cts) + bias.float()
     assert max_rel(out[0], out[1]) <= 1e-2 and max_rel(out[0][rows.cuda()], ref) <= TOL
     assert max_rel(out[0][rows.cuda()][:, -400:], ref[:, -400:]) <= TOL
+
+
+@pytest.mark.parametrize("m,n,k,bits", [(257, 100, 128, 4), (258, 4096, 1024, 3), (300, 1000, 640, 6), (385, 19000, 256, 4), (512, 2500, 2048, 5), (577, 130, 4096, 3),
+                                        (640, 12300, 512, 4), (769, 2560, 384, 6), (1025, 1536, 1152, 4), (1600, 700, 896, 3), (1601, 700, 896, 3), (1537, 9000, 256, 5)])
+def test_gemm_some_hundred_rows(m, n, k, bits):
+    """257 rows and more: whichever kernel and tiling the estimate picks, with one or several tiles of rows, K ranges or none, ragged
+    edges, a bias, 16- and 32-bit results, and a workspace without room for K ranges."""
+    from polarengine_vllm_b200 import _native as nv, kernels, packing
+    codes, norms, cts = rand_layer(n, k, bits, seed=m + n)
+    packed, in_f = bits <= 4, k - 5
+    w = packing.pack_codes_half_block(codes.cuda()) if packed else codes.cuda()
+    nd, ctd, x, bias = norms.cuda(), cts.cuda(), rand_x(m, in_f, seed=k).cuda(), rand_x(1, n, seed=2)[0].cuda()
+    ref = oracle.linear_dequant(x.cpu(), codes, norms, cts, in_f=in_f) + bias.cpu().float()
+    for dt in (torch.float16, torch.float32):
+        y = kernels.quant_matmul(w, packed, nd, ctd, x, False, n, in_f, k, dt, bias)
+        assert y.dtype == dt and max_rel(y, ref) <= TOL
+    lib, need = nv.lib(), nv.lib().pe_gemm_workspace_bytes(m, k)
+    assert nv.lib().pe_gemm_workspace_bytes_splitk(m, n, k) >= need
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    y = torch.empty(m, n, device="cuda")
+    nv.check(lib.pe_gemm(w.data_ptr(), int(packed), w.stride(0), nd.data_ptr(), nd.stride(0), ctd.data_ptr(), ctd.numel(), x.data_ptr(), nv.PE_X_RAW, nv.PE_F16,
+                         x.stride(0), in_f, y.data_ptr(), nv.PE_F32, n, bias.data_ptr(), m, n, k, ws.data_ptr(), need, nv.stream_ptr(x.device)), "pe_gemm")
+    assert max_rel(y, ref) <= TOL
+
+
+@pytest.mark.parametrize("n,bits,dtype", [(19 * 256 + 40, 4, torch.float16), (18 * 256 + 256, 6, torch.float32), (700, 3, torch.bfloat16)])
+def test_gemm_pairs_last_wave_split(n, bits, dtype):
+    """Rows enough for pairs of CTAs whatever the estimate says: a last, partly filled wave cut into K ranges, and a launch of few tiles."""
+    m, k = 1700, 2048
+    codes, norms, cts = rand_layer(n, k, bits, seed=n)
+    x = rand_x(m, k, seed=4)
+    y = run_gemm(codes, norms, cts, x, bits, out_dtype=dtype)
+    assert max_rel(y, oracle.linear_dequant(x, codes, norms, cts)) <= TOL
