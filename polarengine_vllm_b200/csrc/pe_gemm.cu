@@ -216,7 +216,10 @@ gemm_pair_kernel(const GemmArgs p, const __grid_constant__ CUtensorMap xmap, con
   cluster_sync_all();  // barriers of both CTAs exist before anybody arrives on them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  pdl_enter();
+  // Codes, norms and table may be read at once: the preparation launch waited for whatever wrote them before it let this one start.
+  // Its activations, and what an older launch may still read of the output, wait for it.
+  asm volatile("griddepcontrol.launch_dependents;");
+  if (warp == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 
   const int ksteps = p.K / kStepK;
   // A unit of work is a tile or, for the tiles of a last wave that would leave pairs idle, one of `ksplit` K ranges of a
@@ -419,6 +422,7 @@ gemm_pair_kernel(const GemmArgs p, const __grid_constant__ CUtensorMap xmap, con
       }
       if (dead) break;
       // ---------------- epilogue: this CTA's 128 token rows of both accumulators ----------------
+      asm volatile("griddepcontrol.wait;" ::: "memory");
       {
         const bool ok = mbar_wait_cluster(acc_full, tcount & 1, abort_flag, p.status, 5);
         if (!__all_sync(0xffffffffu, ok)) break;

@@ -249,3 +249,27 @@ def test_gemm_pairs_last_wave_split(n, bits, dtype):
     x = rand_x(m, k, seed=4)
     y = run_gemm(codes, norms, cts, x, bits, out_dtype=dtype)
     assert max_rel(y, oracle.linear_dequant(x, codes, norms, cts)) <= TOL
+
+
+@pytest.mark.parametrize("rows", [40, 300, 1700])
+@pytest.mark.parametrize("bits", [4, 5])
+def test_prefill_weights_rewritten_by_the_kernel_in_front(bits, rows):
+    """Codes and norms rewritten on the device right before the call: the tensor-core kernels read them before their own wait, the
+    preparation launch having waited for what wrote them."""
+    from polarengine_vllm_b200 import kernels, packing
+    n, k, sets = 1024, 1024, []
+    for seed in (1, 2):
+        codes, norms, ct = rand_layer(n, k, bits, seed=seed)
+        sets.append((packing.pack_codes_half_block(codes.cuda()) if bits <= 4 else codes.cuda(), norms.cuda()))
+    packed, ctd, x = bits <= 4, ct.cuda(), rand_x(rows, k, seed=3).cuda()
+    want = [kernels.quant_matmul(w, packed, m, ctd, x, False, n, k, k, torch.float32) for w, m in sets]
+    w, m = sets[0][0].clone(), sets[0][1].clone()
+    kernels.quant_matmul(w, packed, m, ctd, x, False, n, k, k, torch.float32)
+    graph, got = torch.cuda.CUDAGraph(), []
+    with torch.cuda.graph(graph):
+        for i in range(20):
+            torch.add(sets[i % 2][0], 0, out=w)
+            torch.mul(sets[i % 2][1], 1, out=m)
+            got.append(kernels.quant_matmul(w, packed, m, ctd, x, False, n, k, k, torch.float32))
+    graph.replay()
+    assert all(torch.equal(y, want[i % 2]) for i, y in enumerate(got))
