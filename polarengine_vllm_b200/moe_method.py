@@ -180,10 +180,11 @@ class PolarQuantMoEMethod:
         tensor_cores = local_pairs >= self.TENSOR_CORE_MIN_ROWS_PER_EXPERT * n_local
         # Rows per problem: 8 while experts see few tokens (lighter kernel), else 16.  For 16 rows a CTA takes 16 blocks of K
         # per round: where a last round leaves a quarter of those places empty, problems of 8 stay ahead up to the
-        # tensor cores' range (128 experts of 21 blocks, 8 rows each: 489 us against 598, 12 rows 642 against 645; 64
-        # experts of 16 blocks, 8 rows each: 144 against 135).
+        # tensor cores' range (128 experts of 21 blocks, 8 rows each: 373 us against 585, 11.5 rows 463 against 617).  Else the
+        # line lies at nine rows (64 experts of 16 blocks, 8 rows each: 143 against 150; 10: 165 against 158; 128 of 8 blocks,
+        # 8 rows: 176 against 200, 10: 183 against 188, 11.5: 199 against 194).
         ragged = blocks > 16 and blocks <= 0.75 * 16 * -(-blocks // 16)
-        rpp = 8 if local_pairs <= 6 * n_local or (ragged and not tensor_cores) else 16
+        rpp = 8 if local_pairs <= 9 * n_local or (ragged and not tensor_cores) else 16
         return rpp, min(n_local, pairs) + pairs // rpp, tensor_cores
 
     # average (token, expert) pairs per local expert up to which the grouped launches are
@@ -191,7 +192,7 @@ class PolarQuantMoEMethod:
     # (measured on 128 experts: grouped 6.5 ms against 21.8 ms per-expert at 128 rows each)
     GROUPED_MAX_ROWS_PER_EXPERT = 512
     # average rows per expert from which the grouped launches run on the tensor cores.  By time alone the line would lie at
-    # four rows (128 experts of 2688 -> 2 x 1856: 347 us either way at 4 rows, 361 against 489 at 8, 345 against 642 at 12), but
+    # eight rows (128 experts of 2688 -> 2 x 1856: 262 us here against 347 at 4 rows, 373 against 361 at 8, 463 against 345 at 12), but
     # that kernel rounds activations and decoded weights to bf16, where the streaming one multiplies fp16 values and keeps the
     # norms in fp32: a decode batch gives up no precision for speed, a prompt chunk does
     TENSOR_CORE_MIN_ROWS_PER_EXPERT = 12
