@@ -335,12 +335,13 @@ int pe_gemv_tiled(const void* tiles, int packed, const float* ct_scaled, int n_l
  *   workspace  at least pe_gemm_workspace_bytes(m, in_f_padded), 256-byte aligned.  Its
  *              first int32 is a status word written by the kernel: 0 on success, 1..10
  *              if a bounded device-side wait ran out (the output is then undefined).
- * More than 256 rows run on pairs of CTAs (thread-block clusters of two, one tensor-core
- * operation per pair); the launch needs no more than the usual one-CTA-per-SM residency.
+ * More than 256 rows run on single CTAs or on pairs of them (thread-block clusters of two, one tensor-core
+ * operation per pair), whichever is estimated to be faster; either way the launch needs no more than the usual
+ * one-CTA-per-SM residency.
  * Replaces polar_matmul's batched branch: polar_gemm / polar_gemm_packed
  * (polar_gemm.py:312-418, 526-534) and the epilogue of linear_method.py:214-221. */
 size_t pe_gemm_workspace_bytes(int m, int in_f_padded);
-/* Launches of up to 256 rows on layers that give few 256-row tiles split K over the SMs when the workspace also
+/* Launches that give few tiles split K over the SMs when the workspace also
  * holds their fp32 partials: this size (>= pe_gemm_workspace_bytes) makes room for them.  With less, pe_gemm runs
  * unsplit.  Same result either way up to the order of the fp32 sums (fixed for a given shape and GPU). */
 size_t pe_gemm_workspace_bytes_splitk(int m, int out_f, int in_f_padded);
