@@ -164,7 +164,10 @@ __device__ __forceinline__ void cvt8(const Raw8<W_DTYPE>& r, float v[8]) {
 // A value's index in its block is 8 a + j.  Lane (g, t) of a warp has the values of a = 2 t, 2 t + 1, 8 + 2 t and 9 + 2 t of block g
 // (32 bytes at a time, so that a warp reads whole lines), which is what operand A of an m16n8k16 product wants of row g with
 // k = a; rows 8 to 15 stay zero.  Products 2 j and 2 j + 1 are the two halves of the 16-point transform over a of the eight
-// blocks' values j: 16-bit values times +-1, exact, summed in fp32.  The lane gets back the same a of its own block, so that the
+// blocks' values j: 16-bit values times +-1, exact products, added in fp32 by the tensor core, which does not round every sum to
+// the nearest as an addition does.  bf16 values are multiplied by +-2^-8 instead: 128 of the largest then stay finite, so that a
+// finite block has no infinity or NaN among its rotated values however large they are (with +-1 the block of a sum past the
+// largest fp32 number came out as NaN: norm 0, codes 0).  The lane gets back the same a of its own block, so that the
 // eight-point transform over j, the norm and sixteen consecutive codes twice need no other lane but for one sum of four.
 // (With the blocks as columns of the product the codes came out four blocks a lane: 59 us where this takes 55.)  The norm is that of
 // the rotated values, which are divided by it afterwards: fewer roundings on the way than dividing first.  Codes that are not
@@ -209,7 +212,9 @@ __global__ void __launch_bounds__(256, CTAS) quantize16_kernel(const void* w, in
   const int64_t step_r = n_warps * 8 / nb;
   const int step_b = (int)(n_warps * 8 - step_r * nb);
   // sign of H16: the parity of the bits that column n (g, g + 8) and index a (2 t, 2 t + 1 and 8 further on) share
-  const uint32_t one = W_DTYPE == PE_F16 ? 0x3c00u : 0x3f80u, sign = (uint32_t)(__popc(g & 2 * t) & 1) << 15;
+  constexpr uint32_t one = W_DTYPE == PE_F16 ? 0x3c00u : 0x3b80u;  // 1, 2^-8
+  constexpr float kBack = W_DTYPE == PE_F16 ? 1.f : 256.f;
+  const uint32_t sign = (uint32_t)(__popc(g & 2 * t) & 1) << 15;
   const uint32_t h0 = one | sign | (one | (sign ^ ((uint32_t)(g & 1) << 15))) << 16, h1 = h0 ^ 0x80008000u;
   Raw8<W_DTYPE> raw[4];
   auto request = [&]() {  // block (r, blk) of the weight, zeros past its last row
@@ -260,28 +265,35 @@ __global__ void __launch_bounds__(256, CTAS) quantize16_kernel(const void* w, in
             v[j | o][h] = fma2(b, minus, a);
           }
     // the rotation keeps the norm: the squares of its results, sqrt(128) too large, sum to 128 times the block's
-    auto squares = [&](float f) {
-      float2 s = make_float2(0.f, 0.f);
+    const float s128 = 0.08838834764831845f * kBack;  // 1/sqrt(128)
+    float2 squares = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 8; ++j)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const float2 x = f == 1.f ? v[j][h] : mul2(v[j][h], make_float2(f, f));
-          s = fma2(x, x, s);
-        }
-      float sum = s.x + s.y;
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      return sum + __shfl_xor_sync(0xffffffffu, sum, 2);
-    };
-    const float s128 = 0.08838834764831845f;  // 1/sqrt(128)
-    const float sum = squares(1.f);
-    float nrm = sqrtf(sum) * s128;
-    if (W_DTYPE == PE_BF16 && __any_sync(0xffffffffu, !(sum < 1e38f))) {  // again with halved exponents; a norm whose own square overflows is infinite
-      const float small = sqrtf(squares(5.421010862427522e-20f)) * s128;  // 2^-64
-      if (!(sum < 1e38f)) nrm = small < 1.f ? small * 18446744073709551616.f : small >= 1.f ? __int_as_float(0x7f800000) : small;
+      for (int h = 0; h < 2; ++h) squares = fma2(v[j][h], v[j][h], squares);
+    float sum = squares.x + squares.y;
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    float nrm = fmaxf(sqrtf(sum) * s128, 1e-10f), inv = __fdiv_rn(s128, nrm);
+    // A norm whose square overflows, infinities, NaN: the norm and the codes of quantize_kernel, from the block itself.  The square of
+    // the norm is infinite or NaN there; finite values become zero, a value that is not finite makes the whole block NaN.
+    if (__any_sync(0xffffffffu, !(sum < 6.6461399789245794e35f))) {  // 128 * 2^128 / 2^16
+      float own = 0.f, finite = 0.f;
+#pragma unroll 1
+      for (int i = 0; i < 32; ++i) {
+        const int col = blk_out * kBlock + t * 32 + i;
+        const uint16_t h = r_out < rows && col < in_f ? static_cast<const uint16_t*>(w)[r_out * ld_w + col] : (uint16_t)0;
+        const float u = W_DTYPE == PE_F16 ? __half2float(__ushort_as_half(h)) : __uint_as_float((uint32_t)h << 16);
+        own = fmaf(u, u, own);
+        finite = fmaf(u, 0.f, finite);
+      }
+#pragma unroll
+      for (int i = 1; i <= 2; i <<= 1) { own += __shfl_xor_sync(0xffffffffu, own, i); finite += __shfl_xor_sync(0xffffffffu, finite, i); }
+      if (!(sum < 6.6461399789245794e35f)) {
+        nrm = fmaxf(sqrtf(own), 1e-10f);
+        inv = finite == 0.f ? __fdiv_rn(s128, nrm) : finite;
+      }
     }
-    nrm = fmaxf(nrm, 1e-10f);
-    const float inv = __fdiv_rn(s128, nrm);
 #pragma unroll
     for (int j = 0; j < 8; ++j)
 #pragma unroll
@@ -305,7 +317,7 @@ __global__ void __launch_bounds__(256, CTAS) quantize16_kernel(const void* w, in
       if (FEW)
 #pragma unroll
         for (int i = 0; i < 8; ++i) packed[i >> 2][(i >> 1) & 1][i & 1] >>= 2;
-      if (v[0][0].x != v[0][0].x)  // a NaN reaches the whole block
+      if (inv != inv)  // a value that is not finite
 #pragma unroll
         for (int i = 0; i < 8; ++i) packed[i >> 2][(i >> 1) & 1][i & 1] = 0;
     } else {

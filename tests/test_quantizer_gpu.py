@@ -110,3 +110,48 @@ def test_gpu_quantizer_extreme_values():
         assert not codes[r, b].any()
         codes[r, b] = ref[r, b]
     assert torch.equal(codes, ref)
+
+
+@pytest.mark.parametrize("bits", [3, 4, 6, 8])
+def test_gpu_quantizer_sums_beyond_fp32(bits):
+    """Finite bf16 blocks whose rotated values are past the largest fp32 number: an infinite norm and the codes of zero, as 32-bit
+    weights of the same values give them; the blocks beside them and those just below the line as ever."""
+    from polarengine_vllm_b200.quantizer import PolarQuantizer
+    g = torch.Generator().manual_seed(bits)
+    w = (0.02 * torch.randn(6, 640, generator=g)).to(torch.bfloat16).cuda()
+    top = torch.finfo(torch.bfloat16).max
+    x = w.clone()
+    x[0, :128] = top                                   # one rotated value of 128 times the largest, the others cancel
+    x[1, 128:256] = top * torch.sign(w[1, 128:256])    # sums of both signs
+    x[2, 256:272] = -top                               # sixteen neighbours
+    x[3, 384:512:8] = top                              # sixteen values that are added first
+    x[4, 512:640] = 2.0 ** 125 * torch.sign(w[4, 512:640])
+    x[5, 5] = top                                      # a single one: no sum is too large, its square is
+    q, ref = (PolarQuantizer().quantize_tensor_gpu(t, bits) for t in (x, x.float()))
+    assert torch.isinf(q["norms"]).sum() == 6
+    assert torch.equal(q["norms"].isinf(), ref["norms"].isinf())
+    zero = PolarQuantizer().quantize_tensor_gpu(torch.zeros_like(x[:1]), bits)["codes"][0, 0]
+    assert bool((q["codes"].view(6, 5, 128)[q["norms"].isinf()] == zero).all())
+    plain = PolarQuantizer().quantize_tensor_gpu(w, bits)
+    same = ~q["norms"].isinf()
+    assert torch.equal(q["codes"].view(6, 5, 128)[same], plain["codes"].view(6, 5, 128)[same]) and torch.equal(q["norms"][same], plain["norms"][same])
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_gpu_quantizer_several_infinities_in_a_block(dtype):
+    """Infinities that meet in one sum of the rotation, of one sign or both, beside a NaN: code 0 for the block and the norm that
+    32-bit weights of the same values get."""
+    from polarengine_vllm_b200.quantizer import PolarQuantizer
+    inf, nan = float("inf"), float("nan")
+    g = torch.Generator().manual_seed(2)
+    w = (0.02 * torch.randn(5, 200, generator=g)).to(dtype).cuda()
+    x = w.clone()
+    for row, at in enumerate([{5: inf, 13: inf}, {5: inf, 21: -inf}, {0: inf, 1: inf, 2: inf, 3: inf}, {7: nan, 71: inf}, {130: -inf, 199: -inf}]):
+        for i, v in at.items():
+            x[row, i] = v
+    q, ref, plain = (PolarQuantizer().quantize_tensor_gpu(t, 4) for t in (x, x.float(), w))
+    hit = torch.zeros(5, 2, dtype=torch.bool, device="cuda")
+    hit[:4, 0], hit[4, 1] = True, True
+    codes = q["codes"].view(5, 2, 128)
+    assert not codes[hit].any() and torch.equal(codes[~hit], plain["codes"].view(5, 2, 128)[~hit])
+    assert torch.equal(q["norms"], torch.where(hit, ref["norms"], plain["norms"]))
