@@ -59,9 +59,10 @@ namespace pe {
 // Math warps.  Three blocks a warp (BPW) need the registers of a CTA of sixteen warps in all.
 __host__ __device__ constexpr int bulk_warps(int bpw) { return bpw == 3 ? 14 : 16; }
 __host__ __device__ constexpr int sum_warps(int bpw, bool passes) { return !passes ? 0 : bpw == 3 ? 1 : 2; }
-// ... + the copy warp, the sum warps of launches of several passes, the norm warp of row-major layers (never with BPW 3)
-__host__ __device__ constexpr int bulk_threads(int bpw, bool tiled, bool passes) {
-  return (bulk_warps(bpw) + 1 + sum_warps(bpw, passes) + (!tiled && bpw < 3)) * 32;
+// ... + the copy warp, the sum warps of launches of several passes, the norm warp: of row-major layers, with BPW 3 only where norms
+// are no single copy, in an instance of its own (a seventeenth warp leaves 96 registers a thread, and 48 to 120 bytes spill)
+__host__ __device__ constexpr int bulk_threads(int bpw, bool norm_warp, bool passes) {
+  return (bulk_warps(bpw) + 1 + sum_warps(bpw, passes) + norm_warp) * 32;
 }
 constexpr int kGroupBlocks = 21;                      // blocks of a row, at most, where a warp takes three: two groups of seven warps
 constexpr int kTabAddr = 2048;                        // address of the centroid table in the shared window
@@ -343,14 +344,14 @@ struct Pass {
   }
 };
 
-template <bool PACKED, int NT, int BPW, bool TILED, bool GROUPED, bool PASSES>
-__global__ void __launch_bounds__(bulk_threads(BPW, TILED, PASSES), 1) gemv_bulk_kernel(const BulkArgs p) {
+template <bool PACKED, int NT, int BPW, bool TILED, bool GROUPED, bool PASSES, bool NORM_WARP>
+__global__ void __launch_bounds__(bulk_threads(BPW, NORM_WARP, PASSES), 1) gemv_bulk_kernel(const BulkArgs p) {
   extern __shared__ __align__(128) uint8_t smem[];  // no static shared memory: the window starts with it
-  constexpr int kWarps = bulk_warps(BPW), kSumWarps = sum_warps(BPW, PASSES), kThreads = bulk_threads(BPW, TILED, PASSES);
+  constexpr int kWarps = bulk_warps(BPW), kSumWarps = sum_warps(BPW, PASSES), kThreads = bulk_threads(BPW, NORM_WARP, PASSES);
   constexpr int kRowBytes = PACKED ? 64 : 128;           // codes of one row's block
   constexpr int kGroupWarps = kGroupBlocks / 3;
   constexpr int kRecBytes = kRowBytes * 16 + 32;         // tiled record: 16 rows of a block, then their norms
-  const bool norms_copied = !TILED && (GROUPED || BPW == 3) && p.norm_stride;
+  const bool norms_copied = !TILED && (BPW == 3 ? !NORM_WARP : GROUPED) && p.norm_stride;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
   const uint32_t sbase = smem_u32(smem);
   const uint32_t full = sbase, empty = sbase + 8 * kBulkMaxStages;
@@ -418,15 +419,6 @@ __global__ void __launch_bounds__(bulk_threads(BPW, TILED, PASSES), 1) gemv_bulk
             }
           }
           __syncwarp();
-          if (BPW == 3 && !TILED && !norms_copied) {  // no norm warp: norms that are no single copy, by this one
-            const __half* src = norms + (int64_t)(ps.row0 + r0) * p.ld_norms;
-            for (int e = lane; e < min(16, ps.rows - r0) * p.nb; e += 32) {
-              const int r = e / p.nb, b = e - r * p.nb;
-              asm volatile("st.shared.u16 [%0], %1;" ::"r"(dst + 16 * p.row_stride + 64 + b * 32 + r * 2), "h"(__half_as_ushort(src[r * p.ld_norms + b])) : "memory");
-            }
-            __syncwarp();
-            if (one) bar_arrive(bar);
-          }
           if (++s == p.n_stage) { s = 0; ph ^= 1; }
         }
       }
@@ -489,8 +481,8 @@ __global__ void __launch_bounds__(bulk_threads(BPW, TILED, PASSES), 1) gemv_bulk
     return;
   }
 
-  if (!TILED && w > kWarps && norms_copied) return;
-  if (!TILED && w > kWarps) {  // ---- norm warp: a stage's norms, the 16 rows of a block side by side
+  if (NORM_WARP && w > kWarps && norms_copied) return;
+  if (NORM_WARP && w > kWarps) {  // ---- norm warp: a stage's norms, the 16 rows of a block side by side
     constexpr int kPlaces = BPW == 1 ? 16 : 32, kLaneRows = 16 * kPlaces / 32;
     const int b = lane % kPlaces, r_lane = lane / kPlaces * kLaneRows, blocks = min(p.nb, p.chunk_blocks);
     const __half* norms = p.norms;
@@ -713,7 +705,7 @@ __global__ void __launch_bounds__(bulk_threads(BPW, TILED, PASSES), 1) gemv_bulk
 }
 
 // ---- host side --------------------------------------------------------------------------------------------------
-template <bool PACKED, int NT, int BPW, bool TILED, bool GROUPED, bool PASSES>
+template <bool PACKED, int NT, int BPW, bool TILED, bool GROUPED, bool PASSES, bool NORM_WARP = !TILED && (BPW < 3)>
 static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
   constexpr int kRowBytes = PACKED ? 64 : 128, kRecBytes = kRowBytes * 16 + 32;
   constexpr int kWarps = bulk_warps(BPW);
@@ -760,11 +752,11 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
   // Several passes: sums by warps of their own, where two sets of them leave a ring of three stages (15360 x 2560 Q5 at 16 rows
   // would have two, and takes 20.1 us that way, 18.7 with one set; 24576 x 4096 Q3 has three: 24.2 and 25.2 us).
   if (!PASSES && a.pass_rows < cta_rows && a.stage_off + a.part_floats * 4 + 3 * a.stage_bytes <= (int)kBulkSmemMax)
-    return launch_bulk<PACKED, NT, BPW, TILED, GROUPED, true>(a, sms, st);
+    return launch_bulk<PACKED, NT, BPW, TILED, GROUPED, true, NORM_WARP>(a, sms, st);
   a.n_stage -= a.n_stage % a.groups;  // a stage is one group's: a wait on a parity holds for a waiter that took every earlier phase
   unsigned dyn = a.stage_off + a.n_stage * a.stage_bytes;
   if (dyn < (unsigned)(kTabAddr + kTabReach)) dyn = kTabAddr + kTabReach;
-  auto kfn = gemv_bulk_kernel<PACKED, NT, BPW, TILED, GROUPED, PASSES>;
+  auto kfn = gemv_bulk_kernel<PACKED, NT, BPW, TILED, GROUPED, PASSES, NORM_WARP>;
   static thread_local unsigned configured[16] = {0};
   int dev = 0;
   PE_CUDA_TRY(cudaGetDevice(&dev));
@@ -772,7 +764,7 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
     PE_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     if (dev < 16) configured[dev] = dyn;
   }
-  PE_CUDA_TRY(launch_pdl(kfn, dim3(G), dim3(bulk_threads(BPW, TILED, PASSES)), dyn, st, a));
+  PE_CUDA_TRY(launch_pdl(kfn, dim3(G), dim3(bulk_threads(BPW, NORM_WARP, PASSES)), dyn, st, a));
   return PE_OK;
 }
 
@@ -791,8 +783,11 @@ static int launch_bulk_shape(BulkArgs& a, int sms, cudaStream_t st) {
   // more, for the groups to have several each (6400 x 2560 Q5 has 2.7: 7.9 us with two blocks a warp, 8.2 with three;
   // 10240 x 2048 Q3 4.3: 6.9 and 7.2; 15360 x 2560 Q3 6.5: 9.9 and 9.4), and for one or two activation rows only where one block a warp is
   // not enough (20480 x 1152 Q4, one row: 7.4 and 7.5; 15360 x 2560 Q3, one row: 9.1 and 8.8).
+  // Norms with gaps, or that do not start or end on 16 bytes, are gathered by a norm warp there too (by the copy warp, between
+  // its copies: 24576 x 2048 Q4 at 8 rows 17.1 us, 128 experts of 21 blocks at 4 rows 479, 64 of 11 blocks 100; now 12.9, 204 and 52, with
+  // one copy 10.4, 147 and 32.5; two blocks a warp took 11.2, 208 and 44).  The order of the sums is the same.
   if (a.nb <= kGroupBlocks && (GROUPED || ((a.N + 15) / 16 >= 6 * sms && (a.batch > 2 || a.nb > 16))))
-    return launch_bulk<PACKED, 1, 3, TILED, GROUPED, true>(a, sms, st);
+    return TILED || a.norm_stride ? launch_bulk<PACKED, 1, 3, TILED, GROUPED, true>(a, sms, st) : launch_bulk<PACKED, 1, 3, TILED, GROUPED, true, !TILED>(a, sms, st);
   return a.nb > 16 ? launch_bulk<PACKED, 1, 2, TILED, GROUPED, GROUPED>(a, sms, st) : launch_bulk<PACKED, 1, 1, TILED, GROUPED, GROUPED>(a, sms, st);
 }
 

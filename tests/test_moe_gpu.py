@@ -304,3 +304,32 @@ def test_grouped_norms_however_they_lie(rows, kp, bits):
     ref = torch.cat([oracle.linear_dequant(x.cpu()[first[i]:first[i] + s], *layers[i]) for i, s in enumerate(sizes) if s])
     assert max_rel(out[0], ref) <= 1e-2
     assert all(torch.equal(out[0], y) for y in out[1:])
+
+
+@pytest.mark.parametrize("rows,kp,bits", [(2100, 2688, 3), (1000, 2176, 6), (300, 128, 4)])
+def test_grouped_norms_gathered_over_several_passes(rows, kp, bits):
+    """Rows of up to 21 blocks whose norms have gaps, more tiles of rows than SMs: gathered by a warp of their own, the bits of
+    copied norms.  Problems of every size, an empty one and more of them than are used."""
+    from polarengine_vllm_b200 import _native as nv, packing
+    sizes, dev, packed, nb = (8, 1, 0, 5, 7), torch.device("cuda"), bits <= 4, kp // 128
+    nv.ensure_init(dev)
+    lib = nv.lib()
+    layers = [rand_layer(rows, kp, bits, seed=i) for i in range(len(sizes))]
+    codes = torch.stack([packing.pack_codes_half_block(c.cuda()) if packed else c.cuda() for c, _, _ in layers])
+    dense, ct = torch.stack([m for _, m, _ in layers]).cuda(), layers[0][2].cuda()
+    gaps = torch.full((len(sizes), rows, nb + 3), float("nan"), dtype=torch.float16, device=dev)
+    gaps[:, :, 1:1 + nb] = dense
+    first = [sum(sizes[:i]) for i in range(len(sizes))]
+    prob = torch.tensor([[i, first[i], s, 0] for i, s in enumerate(sizes)] + [[0, 0, 0, 0]] * 3, dtype=torch.int32).cuda()
+    x = rand_x(sum(sizes), kp, seed=3).cuda()
+    ws = nv.grouped_scratch(dev, lib.pe_gemv_grouped_workspace_bytes(len(prob), rows, kp))
+    out = []
+    for m in (dense, gaps[:, :, 1:1 + nb]):
+        y = torch.full((sum(sizes), rows), float("nan"), device=dev)
+        nv.check(lib.pe_gemv_grouped(codes.data_ptr(), int(packed), codes.stride(1), codes.stride(0), m.data_ptr(), m.stride(1), m.stride(0),
+                                     ct.data_ptr(), ct.numel(), x.data_ptr(), nv.PE_X_RAW, nv.dtype_code(x), x.stride(0), kp, None, y.data_ptr(),
+                                     nv.PE_F32, rows, prob.data_ptr(), len(prob), 8, rows, kp, ws.data_ptr(), ws.numel(), nv.stream_ptr(dev)),
+                 "pe_gemv_grouped")
+        out.append(y)
+    ref = torch.cat([oracle.linear_dequant(x.cpu()[first[i]:first[i] + s], *layers[i]) for i, s in enumerate(sizes) if s])
+    assert max_rel(out[0], ref) <= 1e-2 and torch.equal(out[0], out[1])
