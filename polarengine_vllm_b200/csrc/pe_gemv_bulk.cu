@@ -576,7 +576,8 @@ __global__ void __launch_bounds__(bulk_threads(BPW, NORM_WARP, PASSES), 1) gemv_
   // Three blocks a warp: the warps form groups of group_warps, group q takes the tiles in stages q, q + groups, ...
   const int gw = BPW == 3 ? p.group_warps : kWarps, group = BPW == 3 ? w / gw : 0, wi = BPW == 3 ? w - group * gw : w;
   constexpr int kRowB = TILED ? 8 : 4;
-  constexpr int kPartB = PASSES ? kRowB : 8;
+  constexpr bool kPlain = PASSES || GROUPED;  // partial sums in the order of the rows
+  constexpr int kPartB = kPlain ? kRowB : 8;
   const int row_a = TILED ? g : (g >> 1) + (g & 1) * 8;
   const uint32_t at_a = TILED ? wi * kRecBytes + g * kRowBytes + t * 16 : row_a * p.row_stride + (g & 1) * 64 + wi * kRowBytes + t * 16;
   const uint32_t at_b = at_a + kRowB * (TILED ? kRowBytes : p.row_stride);
@@ -659,7 +660,7 @@ __global__ void __launch_bounds__(bulk_threads(BPW, NORM_WARP, PASSES), 1) gemv_
         __syncwarp();
         if (lane == 0) bar_arrive(empty + 8 * s);
         if (++s == p.n_stage) { s = 0; ph ^= 1; }
-        float* pp = sums + wi * p.part_rows * p.part_stride + r0 + (PASSES ? row_a : g);
+        float* pp = sums + wi * p.part_rows * p.part_stride + r0 + (kPlain ? row_a : g);
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
@@ -672,6 +673,11 @@ __global__ void __launch_bounds__(bulk_threads(BPW, NORM_WARP, PASSES), 1) gemv_
             }
           }
       }
+    }
+    if (!PASSES && GROUPED) {  // one set of sums: all warps add, and meet again before the next pass
+      math_sync<kWarps>();
+      sum_pass(sums, group_rows, y_row, w, kWarps);
+      continue;
     }
     if (!PASSES) {  // few rows a CTA: a lane each
       math_sync<kWarps>();
@@ -736,8 +742,11 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
   if (a.n_chunk == 1 && a.ld_codes == a.row_stride)
     while (a.copy_rows < 8 && a.copy_rows * a.row_stride < 2048) a.copy_rows *= 2;
   a.stage_bytes = TILED ? (blocks * kRecBytes + 127) & ~127 : (16 * a.row_stride + 64 + blocks * 32 + 127) & ~127;
-  for (int cap = BPW == 3 ? 128 : a.batch <= 2 ? 256 : 64;; cap /= 2) {
-    if (cap < 16) return PE_ERR_LIMIT;
+  // Stages a ring should have before a pass gets more rows: two for every group of warps; three beside two sets of sums
+  // (32 experts of 32 blocks Q4, 4 rows: 80 us with two stages, 74 with 32-row passes; 64 of 20 blocks Q6, 8 rows: 162 with a stage a group,
+  // 126 with two and 64-row passes).  Where no cap gives that many (32 blocks Q5: 160 us with 32 or 64 rows) the first that gives two.
+  const int first_cap = BPW == 3 ? 128 : a.batch <= 2 ? 256 : 64;
+  auto ring = [&](int cap) {
     const int passes = (cta_rows + cap - 1) / cap;
     a.pass_rows = GROUPED ? cap : ((cta_rows + passes - 1) / passes + 15) / 16 * 16;
     a.part_stride = a.pass_rows + 4;
@@ -745,13 +754,19 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
     a.part_bufs = PASSES ? 2 : 1;
     a.stage_off = (a.part_off + a.part_bufs * a.part_floats * 4 + 127) & ~127;
     a.n_stage = a.stage_off < (int)kBulkSmemMax ? ((int)kBulkSmemMax - a.stage_off) / a.stage_bytes : 0;
-    if (a.n_stage >= 2) break;
-  }
+    return a.n_stage;
+  };
+  int cap = first_cap;
+  for (const int want = BPW == 3 ? 2 * a.groups : GROUPED && PASSES ? 3 : 2; cap >= 16 && ring(cap) < want;) cap /= 2;
+  if (cap < 16)
+    for (cap = first_cap; cap >= 16 && ring(cap) < 2;) cap /= 2;
+  if (cap < 16) return PE_ERR_LIMIT;
   if (a.n_stage > kBulkMaxStages) a.n_stage = kBulkMaxStages;
   if (a.groups > a.n_stage) a.groups = a.n_stage;
   // Several passes: sums by warps of their own, where two sets of them leave a ring of three stages (15360 x 2560 Q5 at 16 rows
-  // would have two, and takes 20.1 us that way, 18.7 with one set; 24576 x 4096 Q3 has three: 24.2 and 25.2 us).
-  if (!PASSES && a.pass_rows < cta_rows && a.stage_off + a.part_floats * 4 + 3 * a.stage_bytes <= (int)kBulkSmemMax)
+  // would have two, and takes 20.1 us that way, 18.7 with one set; 24576 x 4096 Q3 has three: 24.2 and 25.2 us; problems of 16
+  // rows, 11.5 on average, 64 experts of 16 blocks Q5: 127 and 119 us, 32 of 32 blocks Q4: 142 and 134, 128 of 8 blocks Q3: 70 and 78).
+  if (!PASSES && (GROUPED || a.pass_rows < cta_rows) && a.stage_off + a.part_floats * 4 + 3 * a.stage_bytes <= (int)kBulkSmemMax)
     return launch_bulk<PACKED, NT, BPW, TILED, GROUPED, true, NORM_WARP>(a, sms, st);
   a.n_stage -= a.n_stage % a.groups;  // a stage is one group's: a wait on a parity holds for a waiter that took every earlier phase
   unsigned dyn = a.stage_off + a.n_stage * a.stage_bytes;
@@ -778,7 +793,7 @@ static int launch_bulk_shape(BulkArgs& a, int sms, cudaStream_t st) {
                   a.norms_stride % 8 == 0 && (a.N % 16) * a.nb % 8 == 0 ? a.nb * 2 : 0;
   // Blocks per warp and stage: two when the row is longer than sixteen blocks.  Two sets of activation rows keep one:
   // their operands for two blocks spill (4096 x 12288 at 16 rows: 18.4 us with two, 15.9 with one).
-  if (a.batch > 8) return launch_bulk<PACKED, 2, 1, TILED, GROUPED, GROUPED>(a, sms, st);
+  if (a.batch > 8) return launch_bulk<PACKED, 2, 1, TILED, GROUPED, false>(a, sms, st);
   // Three, and groups of warps, for rows of up to 21 blocks: always in grouped launches; in others where a CTA has six tiles or
   // more, for the groups to have several each (6400 x 2560 Q5 has 2.7: 7.9 us with two blocks a warp, 8.2 with three;
   // 10240 x 2048 Q3 4.3: 6.9 and 7.2; 15360 x 2560 Q3 6.5: 9.9 and 9.4), and for one or two activation rows only where one block a warp is
@@ -788,7 +803,8 @@ static int launch_bulk_shape(BulkArgs& a, int sms, cudaStream_t st) {
   // one copy 10.4, 147 and 32.5; two blocks a warp took 11.2, 208 and 44).  The order of the sums is the same.
   if (a.nb <= kGroupBlocks && (GROUPED || ((a.N + 15) / 16 >= 6 * sms && (a.batch > 2 || a.nb > 16))))
     return TILED || a.norm_stride ? launch_bulk<PACKED, 1, 3, TILED, GROUPED, true>(a, sms, st) : launch_bulk<PACKED, 1, 3, TILED, GROUPED, true, !TILED>(a, sms, st);
-  return a.nb > 16 ? launch_bulk<PACKED, 1, 2, TILED, GROUPED, GROUPED>(a, sms, st) : launch_bulk<PACKED, 1, 1, TILED, GROUPED, GROUPED>(a, sms, st);
+  if constexpr (GROUPED) return launch_bulk<PACKED, 1, 2, TILED, GROUPED, true>(a, sms, st);
+  else return a.nb > 16 ? launch_bulk<PACKED, 1, 2, TILED, GROUPED, false>(a, sms, st) : launch_bulk<PACKED, 1, 1, TILED, GROUPED, false>(a, sms, st);
 }
 
 template <bool PACKED, bool TILED>

@@ -333,3 +333,35 @@ def test_grouped_norms_gathered_over_several_passes(rows, kp, bits):
         out.append(y)
     ref = torch.cat([oracle.linear_dequant(x.cpu()[first[i]:first[i] + s], *layers[i]) for i, s in enumerate(sizes) if s])
     assert max_rel(out[0], ref) <= 1e-2 and torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("max_rows,rows,kp,bits", [(16, 3000, 2176, 4), (16, 1500, 4224, 3), (16, 1501, 2048, 5), (16, 1200, 2560, 6), (16, 3000, 1024, 4),
+                                                   (8, 3000, 2560, 6), (8, 1500, 4096, 4), (8, 700, 4096, 5)])
+def test_grouped_rings_and_sets_of_sums(max_rows, rows, kp, bits):
+    """Problems of 8 and 16 rows over several passes a CTA, with one set of partial sums and with two, passes of 32, 64 and 128 rows, one
+    and several chunks of K: the oracle's values, the bits of the tiled copy, and the same bits every time."""
+    from polarengine_vllm_b200 import _native as nv, kernels, packing
+    sizes, dev, packed = (max_rows, 1, 0, 7, max_rows, 3), torch.device("cuda"), bits <= 4
+    nv.ensure_init(dev)
+    lib = nv.lib()
+    layers = [rand_layer(rows, kp, bits, seed=i) for i in range(len(sizes))]
+    codes = torch.stack([packing.pack_codes_half_block(c.cuda()) if packed else c.cuda() for c, _, _ in layers])
+    norms, ct = torch.stack([m for _, m, _ in layers]).cuda(), layers[0][2].cuda()
+    tiles = torch.cat([kernels.retile(codes[i], packed, norms[i]) for i in range(len(sizes))])
+    first = [sum(sizes[:i]) for i in range(len(sizes))]
+    prob = torch.tensor([[i, first[i], s, 0] for i, s in enumerate(sizes)], dtype=torch.int32).cuda()
+    x = rand_x(sum(sizes), kp, seed=3).cuda()
+    ws = nv.grouped_scratch(dev, lib.pe_gemv_grouped_workspace_bytes(len(sizes), rows, kp))
+    tail = (prob.data_ptr(), len(sizes), max_rows, rows, kp, ws.data_ptr(), ws.numel(), nv.stream_ptr(dev))
+    out = []
+    for tiled in (False, False, True):
+        y = torch.full((sum(sizes), rows), float("nan"), device=dev)
+        mid = (ct.data_ptr(), ct.numel(), x.data_ptr(), nv.PE_X_RAW, nv.dtype_code(x), x.stride(0), kp, None, y.data_ptr(), nv.PE_F32, rows)
+        if tiled:
+            nv.check(lib.pe_gemv_grouped_tiled(tiles.data_ptr(), int(packed), tiles.numel() // len(sizes), *mid, *tail), "tiled")
+        else:
+            nv.check(lib.pe_gemv_grouped(codes.data_ptr(), int(packed), codes.stride(1), codes.stride(0), norms.data_ptr(), norms.stride(1),
+                                         norms.stride(0), *mid, *tail), "row-major")
+        out.append(y)
+    ref = torch.cat([oracle.linear_dequant(x.cpu()[first[i]:first[i] + s], *layers[i]) for i, s in enumerate(sizes) if s])
+    assert max_rel(out[0], ref) <= 1e-2 and torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
