@@ -178,13 +178,16 @@ class PolarQuantMoEMethod:
         if pairs < 1 or local_pairs > self.GROUPED_MAX_ROWS_PER_EXPERT * n_local:
             return None
         tensor_cores = local_pairs >= self.TENSOR_CORE_MIN_ROWS_PER_EXPERT * n_local
-        # Rows per problem: 8 while experts see few tokens (lighter kernel), else 16.  For 16 rows a CTA takes 16 blocks of K
-        # per round: where a last round leaves a quarter of those places empty, problems of 8 stay ahead up to the
-        # tensor cores' range (128 experts of 21 blocks, 8 rows each: 373 us against 585, 11.5 rows 463 against 617).  Else the
-        # line lies at nine rows (64 experts of 16 blocks, 8 rows each: 143 against 150; 10: 165 against 158; 128 of 8 blocks,
-        # 8 rows: 176 against 200, 10: 183 against 188, 11.5: 199 against 194).
+        # Rows per problem: 8 (lighter kernel, codes streamed once per 8 rows) or 16.  Of the first projection's K a CTA takes 16
+        # blocks a round with 16 rows, 32 with 8, and rows of up to 21 blocks share its warps with 8.  Layers of experts x hidden x
+        # intermediate, 8- against 16-row problems: up to 8 blocks (128 x 1024 x 768: 9 rows each 109 and 122 us, 11.9 rows 128 and 133)
+        # and from two 16-block rounds to one of 32 (64 x 2688 x 1856: 213 and 305, 255 and 337; 32 x 4096 x 1408: 139 and 155, 166 and
+        # 163) 8 stay ahead up to the tensor cores' range, as where a last round leaves a quarter of its places empty.  Else the line
+        # lies at nine rows (64 x 2048 x 1408: 8 rows 146 and 147, 9: 152 and 151, 10: 166 and 152; 64 x 1536 x 1856: 138 and 152,
+        # 156 and 158, 164 and 157; 16 x 5120 x 1536: 111 and 114, 120 and 117, 121 and 117).
         ragged = blocks > 16 and blocks <= 0.75 * 16 * -(-blocks // 16)
-        rpp = 8 if local_pairs <= 9 * n_local or (ragged and not tensor_cores) else 16
+        eight = blocks <= 8 or 16 < blocks <= 32 or ragged
+        rpp = 8 if local_pairs <= 9 * n_local or (eight and not tensor_cores) else 16
         return rpp, min(n_local, pairs) + pairs // rpp, tensor_cores
 
     # average (token, expert) pairs per local expert up to which the grouped launches are

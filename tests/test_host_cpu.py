@@ -164,3 +164,17 @@ def test_quantize_state_dict_layout():
     assert cfg["layers"]["model.layers.0.self_attn.q_proj"]["packed_q5"]
     assert tensors["model.layers.0.self_attn.q_proj.codes"].shape == (32, 160)
     assert tensors["model.layers.0.input_layernorm.weight"].dtype == torch.float16
+
+
+# ---- expert layer: rows per problem of the decode-size launches ------------------
+@pytest.mark.parametrize("blocks,rows,problem", [(8, 9, 8), (8, 11.9, 8), (9, 9, 8), (9, 9.1, 16), (12, 10, 16), (16, 9, 8), (16, 10, 16), (17, 11.9, 8),
+                                                 (21, 11.9, 8), (32, 10, 8), (33, 11.9, 8), (40, 9, 8), (40, 10, 16), (48, 11, 16)])
+def test_rows_per_problem_of_the_expert_layer(blocks, rows, problem):
+    """The measured line between problems of 8 and of 16 rows, enough problem slots for any routing, and the tensor cores from
+    twelve rows an expert on."""
+    from polarengine_vllm_b200.moe_method import PolarQuantMoEMethod
+    experts = 64
+    pairs = int(rows * experts)
+    rpp, slots, tensor_cores = PolarQuantMoEMethod()._grouped_plan(pairs, experts, None, blocks)
+    assert (rpp, tensor_cores) == (problem, False) and slots >= min(experts, pairs) + pairs // rpp
+    assert PolarQuantMoEMethod()._grouped_plan(12 * experts, experts, None, blocks)[2]
