@@ -343,7 +343,8 @@ int pe_gemv_tiled(const void* tiles, int packed, const float* ct_scaled, int n_l
 size_t pe_gemm_workspace_bytes(int m, int in_f_padded);
 /* Launches that give few tiles split K over the SMs when the workspace also
  * holds their fp32 partials: this size (>= pe_gemm_workspace_bytes) makes room for them.  With less, pe_gemm runs
- * unsplit.  Same result either way up to the order of the fp32 sums (fixed for a given shape and GPU). */
+ * unsplit, or in fewer ranges, or (more than 256 rows) with other tiles.  Same result either way up to the order of the
+ * fp32 sums, which is fixed for a given shape, GPU and workspace size. */
 size_t pe_gemm_workspace_bytes_splitk(int m, int out_f, int in_f_padded);
 int pe_gemm(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms,
             const float* ct_scaled, int n_levels, const void* x, int x_kind, int x_dtype, int64_t ld_x,

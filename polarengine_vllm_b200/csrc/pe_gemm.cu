@@ -633,20 +633,43 @@ static PairPlan pair_plan(int tiles_m, int tiles_n, int ksteps, int sms) {
 // A pair of CTAs does the work of a full 512 x 256 tile in 0.69 us per 64 of K, the tensor-memory kernel that of its four 256 x 128
 // tiles in 1.4 on two CTAs; but 512 x 256 is a coarse tile: rows are rounded up to 512, and a launch of a few hundred rows has less
 // than one or just over one wave of them.  So the time of both is estimated, for every tiling that the tensor-memory kernel
-// has, and the shorter one taken; the pair kernel where they are within 5 % (10 % at short K, where the drain of the tiles,
-// of which the estimate knows little, counts most: 16384 x 1280 Q6 at 1300 rows, estimated 5 % ahead, took 80.8 against 71.8 us).  The constants are a fit to 590 launches of nine
-// layer shapes at 24 to 2048 rows (7 % off on average); from 1601 rows on the pair kernel is ahead or level on all of them.
-// Before / now: 4096 x 4096 Q6 at 300 rows 31.8 / 24.9 us, 640: 46.8 / 34.0, 1024: 51.3 / 39.3; 24576 x 4096 Q3 at 400 rows 89 / 71,
-// 640: 156 / 107; 4096 x 12288 Q4 at 300 rows 61 / 43..49, 640: 97 / 68; 2560 x 2560 Q5 at 512 rows 28.4 / 20.9.
+// has, and the shorter one taken.  The constants are a fit to 590 launches of nine layer shapes at 24 to 2048 rows.  Over twelve
+// shapes at 51 row counts to 2049 the estimated ratio of the two is 6 % off on average and 25 % at worst, and that worst is at short K,
+// where the drain of the tiles, of which the estimate knows little, counts most (16384 x 1280 Q6 at 1280 rows: 0.94 estimated,
+// 77.0 against 67.1 us); so a tiling has to be ahead by 10 % below K 2048 and by 5 % from there on.  What that picks there is never
+// slower than the pair kernel by more than the noise (2048 x 7168 Q6 at 1024 rows, 47.0 and 46.8 us).
+// Pair / this, us, weights from HBM: 4096 x 4096 Q6 at 257 rows 30.2 / 23.7, 384: 32.1 / 28.0, 640: 45.7 / 32.9, 1024: 50.0 / 38.1; 24576 x
+// 4096 Q3 at 257 rows 84.0 / 68.7, 640: 161.7 / 107.0; 4096 x 12288 Q4 at 257 rows 59.2 / 43.9, 384: 57.1 / 49.8, 640: 92.4 / 67.9; 12288 x 4096
+// Q4 at 512 rows 57.7 / 47.5; 2560 x 2560 Q5 at 512 rows 26.1 / 19.5.
+//
+// Order of the sums.  Both kernels multiply the same values and add them in the same order within a K range, so a tiling with the pair
+// kernel's K ranges gives its bits.  Other K ranges are another order: as far from 64-bit arithmetic, but six decoder layers
+// turn another order of q/k/v alone (6144 x 4096 Q5: one range for three) into 1.0 to 1.1 % of the logits.  Up to one row of pair tiles,
+// another order is therefore taken only where a quarter of the time goes (0.76 by the estimate; q/k/v stays above that but at
+// 432 rows, 0.7597).  What that leaves: q/k/v at 512 rows 41.1 us where 34.0 would do, 24576 x 4096 Q3 at 384 rows 95.6 (73.3), 2560 x 2560
+// Q5 at 433 rows 25.1 (18.7; 432 rows, 0.746, take it), 2048 x 7168 Q6 at 384 rows 31.1 (23.1).
 constexpr int kTmemMaxRows = 1600;
 
-static double pair_time_us(int m, int out_f, int in_f_padded, int sms) {
-  const int tiles_m = (m + kPairTileM - 1) / kPairTileM, tiles_n = (out_f + kTileN - 1) / kTileN, steps = in_f_padded / kStepK, pairs = sms / 2;
-  const PairPlan p = pair_plan(tiles_m, tiles_n, steps, sms);
+static PairPlan pair_plan_within(int m, int out_f, int in_f_padded, int sms, size_t part_bytes) {
+  const int tiles_m = (m + kPairTileM - 1) / kPairTileM, tiles_n = (out_f + kTileN - 1) / kTileN;
+  const PairPlan p = pair_plan(tiles_m, tiles_n, in_f_padded / kStepK, sms);
+  return p.ksplit > 1 && (size_t)p.ksplit * m * (out_f - p.col0) * sizeof(float) > part_bytes ? PairPlan{tiles_m * tiles_n, 1, 0} : p;
+}
+
+static double pair_time_us(const PairPlan& p, int m, int out_f, int in_f_padded, int sms) {
+  const int steps = in_f_padded / kStepK, pairs = sms / 2;
   double t = 7.8 + 1.26e-6 * m * in_f_padded;  // launch and preparation
   if (p.full) t += (p.full + pairs - 1) / pairs * (0.69 * steps + 7.1);
   if (p.ksplit > 1) t += (steps + p.ksplit - 1) / p.ksplit * 0.69 + 7.4 + 1.0e-6 * p.ksplit * m * (out_f - p.col0);
   return t;
+}
+
+// Does a cut of every tile's nb blocks into `ksplit` ranges give the ranges that p gives them?  (p's are ranges of half blocks.)
+static bool same_ranges(const PairPlan& p, int ksplit, int nb) {
+  if (ksplit != p.ksplit || (ksplit > 1 && p.full)) return false;
+  for (int s = 1; s < ksplit; ++s)
+    if (s * 2 * nb / ksplit != s * nb / ksplit * 2) return false;
+  return true;
 }
 
 struct TmemPlan { int halves, tiles_m, tok, ksplit; };
@@ -665,27 +688,28 @@ static double tmem_time_us(const TmemPlan& p, int m, int out_f, int in_f_padded,
   return t;
 }
 
-// Shortest tiling of the tensor-memory kernel with at most `max_split` K ranges; halves = 0: the pair kernel is ahead.
+// Shortest tiling of the tensor-memory kernel whose partials fit part_bytes; halves = 0: the pair kernel.
 static TmemPlan many_rows_plan(int m, int out_f, int in_f_padded, int packed, int sms, size_t part_bytes) {
   TmemPlan best = {0, 0, 0, 1};
   if (m > kTmemMaxRows) return best;
-  // One row of pair tiles: only where a quarter of the time goes.  The kernels multiply the same values, but another cut of K is another
-  // order of the fp32 sums, and six decoder layers make about 1 % of their logits of that (0.75 % if q/k/v keeps its order, as it
-  // does with this line): no error, each is as far from 64-bit arithmetic as the other, but not worth 10 % of a launch.
-  const double share = m <= kPairTileM ? 0.76 : in_f_padded < 2048 ? 0.9 : 0.95;
-  double least = share * pair_time_us(m, out_f, in_f_padded, sms);
+  const int nb = in_f_padded / kBlock;
+  const PairPlan pairs = pair_plan_within(m, out_f, in_f_padded, sms, part_bytes);
+  const double pair = pair_time_us(pairs, m, out_f, in_f_padded, sms), margin = in_f_padded < 2048 ? 0.9 : 0.95;
+  const double same = margin * pair, other = m <= kPairTileM ? 0.76 * pair : same;
+  double least = same;
   for (int halves = 1; halves <= 2; ++halves) {
     const int most = halves == 1 ? 256 : 192, tiles_n = (out_f + 128 * halves - 1) / (128 * halves), first = (m + most - 1) / most;
     for (int tiles_m = first; tiles_m < first + 3; ++tiles_m) {
       TmemPlan p = {halves, tiles_m, ((m + tiles_m - 1) / tiles_m + 15) / 16 * 16, 1};
       p.tiles_m = (m + p.tok - 1) / p.tok;  // the rounded tiles may be one fewer: none is empty
-      int ks = sms / (tiles_n * p.tiles_m);
-      if (ks > in_f_padded / kBlock / 2) ks = in_f_padded / kBlock / 2;
-      for (int split = 0; split < (ks > 1 ? 2 : 1); ++split) {
-        p.ksplit = split ? ks : 1;
-        if (split && (size_t)ks * m * out_f * sizeof(float) > part_bytes) continue;
+      int idle = sms / (tiles_n * p.tiles_m);
+      if (idle > nb / 2) idle = nb / 2;
+      const int splits[3] = {1, idle, m <= kPairTileM ? pairs.ksplit : 1};  // whole, as many as there are idle SMs, as the pair kernel's
+      for (int i = 0; i < 3; ++i) {
+        p.ksplit = splits[i];
+        if (i && (p.ksplit < 2 || (size_t)p.ksplit * m * out_f * sizeof(float) > part_bytes)) continue;
         const double t = tmem_time_us(p, m, out_f, in_f_padded, packed, sms);
-        if (t < least) { least = t; best = p; }
+        if (t < least && (t < other || same_ranges(pairs, p.ksplit, nb))) { least = t; best = p; }
       }
     }
   }
@@ -698,7 +722,7 @@ extern "C" size_t pe_gemm_workspace_bytes(int m, int in_f_padded) {
   return 256 + (size_t)m * in_f_padded * 2;
 }
 
-// [the above][fp32 partials ksplit x M x N]: with this much room a launch of up to 256 rows on few tiles splits K
+// [the above][fp32 partials ksplit x M x N]: with this much room launches split K as they would like to
 extern "C" size_t pe_gemm_workspace_bytes_splitk(int m, int out_f, int in_f_padded) {
   const size_t base = pe_gemm_workspace_bytes(m, in_f_padded);
   if (base == 0 || out_f < 1) return 0;
@@ -712,7 +736,7 @@ extern "C" size_t pe_gemm_workspace_bytes_splitk(int m, int out_f, int in_f_padd
   if (m <= 256) {
     want(small_ksplit(m, out_f, in_f_padded, sms), out_f);
   } else {
-    const PairPlan p = pair_plan((m + kPairTileM - 1) / kPairTileM, (out_f + kTileN - 1) / kTileN, in_f_padded / kStepK, sms);
+    const PairPlan p = pair_plan_within(m, out_f, in_f_padded, sms, ~(size_t)0);
     want(p.ksplit, out_f - p.col0);
     for (int packed = 0; packed < 2; ++packed) want(many_rows_plan(m, out_f, in_f_padded, packed, sms, ~(size_t)0).ksplit, out_f);
   }
@@ -744,13 +768,14 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
   if (rc != PE_OK) return rc;
   // few tiles: split K when the caller's workspace has room for the partials
   const size_t part_off = (pe_gemm_workspace_bytes(m, in_f_padded) + 255) & ~(size_t)255;
-  auto fits = [&](int ks, int cols) { return ks > 1 && workspace_bytes >= part_off + (size_t)ks * m * cols * sizeof(float); };
+  const size_t part_bytes = workspace_bytes > part_off ? workspace_bytes - part_off : 0;
   float* part = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + part_off);
 
-  // Up to 256 rows: one tile of tokens of the tensor-memory kernel.  Above, whichever is estimated to be shorter.
+  // Up to 256 rows: one tile of tokens of the tensor-memory kernel.  Above, as many_rows_plan says.
   TmemPlan plan = {small_halves(m, out_f, sms), 1, m, 1};
-  if (m > 256) plan = many_rows_plan(m, out_f, in_f_padded, packed, sms, workspace_bytes > part_off ? workspace_bytes - part_off : 0);
+  if (m > 256) plan = many_rows_plan(m, out_f, in_f_padded, packed, sms, part_bytes);
   else plan.ksplit = small_ksplit(m, out_f, in_f_padded, sms);
+  if ((size_t)plan.ksplit * m * out_f * sizeof(float) > part_bytes) plan.ksplit = 1;
   if (plan.halves) {
     TmemGemmArgs a = {};
     a.norms = static_cast<const __half*>(norms); a.ld_norms = ld_norms;
@@ -762,7 +787,6 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
     a.tiles_m = plan.tiles_m; a.tok = plan.tok;
     a.tiles_n = (out_f + 128 * a.halves - 1) / (128 * a.halves);
     a.ksplit = plan.ksplit;
-    if (!fits(a.ksplit, out_f)) a.ksplit = 1;
     a.part = a.ksplit > 1 ? part : nullptr;
     a.xbox = (a.tok + 15) & ~15;
     a.x_stage = a.xbox * 128;
@@ -801,9 +825,8 @@ extern "C" int pe_gemm(const void* codes, int packed, int64_t ld_codes, const vo
   a.lut_bytes = packed ? 256 * kPairLutStride : n_levels * 128;
   a.nc = kPairCodeStages;
   const unsigned smem_bytes = (packed ? 4 : 3) * 2 * kXTileBytes + kPairWStages * kPairWTileBytes + a.lut_bytes + a.nc * 128 * code_row + 256 + 1024;
-  PairPlan pairs_of = pair_plan(a.tiles_m, a.tiles_n, in_f_padded / kStepK, sms);
+  const PairPlan pairs_of = pair_plan_within(m, out_f, in_f_padded, sms, part_bytes);
   const int tiles = a.tiles_m * a.tiles_n;
-  if (!fits(pairs_of.ksplit, out_f - pairs_of.col0)) pairs_of = {tiles, 1, 0};
   a.full = pairs_of.full; a.ksplit = pairs_of.ksplit; a.col0 = pairs_of.col0;
   a.part = part;
   CUtensorMap partmap = ymap;

@@ -273,3 +273,16 @@ def test_prefill_weights_rewritten_by_the_kernel_in_front(bits, rows):
             got.append(kernels.quant_matmul(w, packed, m, ctd, x, False, n, k, k, torch.float32))
     graph.replay()
     assert all(torch.equal(y, want[i % 2]) for i, y in enumerate(got))
+
+
+@pytest.mark.parametrize("n,k,bits,few,many", [(4096, 4096, 6, 384, 512), (4096, 4096, 4, 387, 512), (4096, 12288, 4, 416, 512), (12288, 1024, 4, 400, 4200),
+                                               (1536, 2048, 5, 257, 512), (300, 128, 3, 259, 5000), (2817, 640, 6, 511, 4700)])
+def test_gemm_same_bits_where_k_is_cut_alike(n, k, bits, few, many):
+    """The rows of a launch have the bits they have in a launch of more rows, whose larger number takes it to other tiles or to pairs of
+    CTAs: where both cut K into the same ranges every product is added in the same order."""
+    codes, norms, cts = rand_layer(n, k, bits, seed=n + k)
+    x = rand_x(many, k, seed=few)
+    a, b = run_gemm(codes, norms, cts, x[:few], bits, out_dtype=torch.float32), run_gemm(codes, norms, cts, x, bits, out_dtype=torch.float32)
+    assert torch.equal(a, b[:few])
+    ref = oracle.linear_dequant(x[:few], codes, norms, cts)
+    assert max_rel(a, ref) <= TOL
