@@ -636,11 +636,13 @@ static PairPlan pair_plan(int tiles_m, int tiles_n, int ksteps, int sms) {
 // has, and the shorter one taken.  The constants are a fit to 590 launches of nine layer shapes at 24 to 2048 rows.  Over twelve
 // shapes at 51 row counts to 2049 the estimated ratio of the two is 6 % off on average and 25 % at worst, and that worst is at short K,
 // where the drain of the tiles, of which the estimate knows little, counts most (16384 x 1280 Q6 at 1280 rows: 0.94 estimated,
-// 77.0 against 67.1 us); so a tiling has to be ahead by 10 % below K 2048 and by 5 % from there on.  What that picks there is never
-// slower than the pair kernel by more than the noise (2048 x 7168 Q6 at 1024 rows, 47.0 and 46.8 us).
+// 77.0 against 67.1 us); so a tiling has to be ahead by 10 % below K 2048 and by 5 % from there on, and by 10 % more above 1600 rows,
+// where both have several waves (4096 x 12288 Q4 at 1856 rows: 0.93 estimated, 188 against 172 us).  What that picks of the launches
+// measured is never slower than the pair kernel by more than the noise (2048 x 7168 Q6 at 1024 rows, 47.0 and 46.8 us); above
+// 1600 rows it is 104 of 348, 17 % faster on average.  Not measured and not asked above 4096 rows.
 // Pair / this, us, weights from HBM: 4096 x 4096 Q6 at 257 rows 30.2 / 23.7, 384: 32.1 / 28.0, 640: 45.7 / 32.9, 1024: 50.0 / 38.1; 24576 x
 // 4096 Q3 at 257 rows 84.0 / 68.7, 640: 161.7 / 107.0; 4096 x 12288 Q4 at 257 rows 59.2 / 43.9, 384: 57.1 / 49.8, 640: 92.4 / 67.9; 12288 x 4096
-// Q4 at 512 rows 57.7 / 47.5; 2560 x 2560 Q5 at 512 rows 26.1 / 19.5.
+// Q4 at 512 rows 57.7 / 47.5, 1700: 190 / 151; 2560 x 2560 Q5 at 512 rows 26.1 / 19.5, 1700: 43.2 / 28.7; 2048 x 7168 Q6 at 2112 rows 104.5 / 65.6.
 //
 // Order of the sums.  Both kernels multiply the same values and add them in the same order within a K range, so a tiling with the pair
 // kernel's K ranges gives its bits.  Other K ranges are another order: as far from 64-bit arithmetic, but six decoder layers
@@ -648,7 +650,7 @@ static PairPlan pair_plan(int tiles_m, int tiles_n, int ksteps, int sms) {
 // another order is therefore taken only where a quarter of the time goes (0.76 by the estimate; q/k/v stays above that but at
 // 432 rows, 0.7597).  What that leaves: q/k/v at 512 rows 41.1 us where 34.0 would do, 24576 x 4096 Q3 at 384 rows 95.6 (73.3), 2560 x 2560
 // Q5 at 433 rows 25.1 (18.7; 432 rows, 0.746, take it), 2048 x 7168 Q6 at 384 rows 31.1 (23.1).
-constexpr int kTmemMaxRows = 1600;
+constexpr int kTmemMaxRows = 4096;
 
 static PairPlan pair_plan_within(int m, int out_f, int in_f_padded, int sms, size_t part_bytes) {
   const int tiles_m = (m + kPairTileM - 1) / kPairTileM, tiles_n = (out_f + kTileN - 1) / kTileN;
@@ -694,7 +696,7 @@ static TmemPlan many_rows_plan(int m, int out_f, int in_f_padded, int packed, in
   if (m > kTmemMaxRows) return best;
   const int nb = in_f_padded / kBlock;
   const PairPlan pairs = pair_plan_within(m, out_f, in_f_padded, sms, part_bytes);
-  const double pair = pair_time_us(pairs, m, out_f, in_f_padded, sms), margin = in_f_padded < 2048 ? 0.9 : 0.95;
+  const double pair = pair_time_us(pairs, m, out_f, in_f_padded, sms), margin = (in_f_padded < 2048 ? 0.9 : 0.95) - (m > 1600 ? 0.1 : 0);
   const double same = margin * pair, other = m <= kPairTileM ? 0.76 * pair : same;
   double least = same;
   for (int halves = 1; halves <= 2; ++halves) {

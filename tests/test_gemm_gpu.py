@@ -276,7 +276,8 @@ def test_prefill_weights_rewritten_by_the_kernel_in_front(bits, rows):
 
 
 @pytest.mark.parametrize("n,k,bits,few,many", [(4096, 4096, 6, 384, 512), (4096, 4096, 4, 387, 512), (4096, 12288, 4, 416, 512), (12288, 1024, 4, 400, 4200),
-                                               (1536, 2048, 5, 257, 512), (300, 128, 3, 259, 5000), (2817, 640, 6, 511, 4700)])
+                                               (1536, 2048, 5, 257, 512), (300, 128, 3, 259, 5000), (2817, 640, 6, 511, 4700),
+                                               (2560, 640, 5, 1700, 4200), (300, 1024, 4, 4096, 4097)])
 def test_gemm_same_bits_where_k_is_cut_alike(n, k, bits, few, many):
     """The rows of a launch have the bits they have in a launch of more rows, whose larger number takes it to other tiles or to pairs of
     CTAs: where both cut K into the same ranges every product is added in the same order."""
@@ -286,3 +287,18 @@ def test_gemm_same_bits_where_k_is_cut_alike(n, k, bits, few, many):
     assert torch.equal(a, b[:few])
     ref = oracle.linear_dequant(x[:few], codes, norms, cts)
     assert max_rel(a, ref) <= TOL
+
+
+@pytest.mark.parametrize("m,n,k,bits", [(1601, 1024, 8192, 3), (1700, 12288, 512, 4), (1700, 19 * 256 + 40, 2048, 6), (2050, 1000, 2176, 6), (2049, 2300, 5120, 4),
+                                        (4096, 300, 1024, 5)])
+def test_gemm_some_thousand_rows(m, n, k, bits):
+    """1601 to 4096 rows on layers for which the estimate picks the tensor-memory kernel: many tiles of rows, one or two halves, K ranges
+    or none, ragged edges, a bias, every output type."""
+    codes, norms, cts = rand_layer(n, k, bits, seed=m + n)
+    in_f = k - 5
+    x, bias = rand_x(m, in_f, seed=k), rand_x(1, n, seed=2).reshape(n)
+    rows = torch.cat([torch.arange(0, m, 41), torch.arange(m - 20, m)])
+    ref = oracle.linear_dequant(x[rows], codes, norms, cts, in_f=in_f) + bias.float()
+    for dt in (torch.float16, torch.float32, torch.bfloat16):
+        y = run_gemm(codes, norms, cts, x, bits, out_dtype=dt, bias=bias, in_f=in_f)
+        assert torch.isfinite(y.float()).all() and max_rel(y[rows.cuda()], ref) <= TOL
