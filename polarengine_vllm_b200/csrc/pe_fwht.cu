@@ -57,8 +57,7 @@ __global__ void __launch_bounds__(256) pack_nibble_kernel(const int8_t* codes, u
 // of the seven butterfly stages stay in registers, a warp reads and writes whole sectors, the level is found with one
 // table lookup and one comparison instead of a scan of all levels, the quotient is a product with the reciprocal and
 // one correction, and fp32 arithmetic goes two values per instruction.  4096 x 12288, on 2 resident CTAs per SM
-// with the next trip's loads in flight: to 4 bits 68 us; against one warp per block, a scan and a full division per value 256 -> 61 us
-// on bf16 weights, which now have a kernel of their own.
+// with the next trip's loads in flight: to 4 bits 71 us, to 6 bits 75.
 
 // Exact cell edges: the rotated unit-vector element v takes code j when j edges are below it.  edge[j] is the largest
 // float that is still no farther from level j than from level j + 1 by the fp32 distances quant_dist() that a scan
@@ -141,23 +140,6 @@ __device__ __forceinline__ Raw8<W_DTYPE> load8_raw(const void* w, int64_t row_of
     for (int i = 0; i < kQuads; ++i) r.q[i] = make_uint4(u[4 * i], u[4 * i + 1], u[4 * i + 2], u[4 * i + 3]);
   }
   return r;
-}
-
-template <int W_DTYPE>
-__device__ __forceinline__ void cvt8(const Raw8<W_DTYPE>& r, float v[8]) {
-  if (W_DTYPE == PE_F32) {
-    const uint4 a = r.q[0], b = r.q[W_DTYPE == PE_F32 ? 1 : 0];
-    v[0] = __uint_as_float(a.x); v[1] = __uint_as_float(a.y); v[2] = __uint_as_float(a.z); v[3] = __uint_as_float(a.w);
-    v[4] = __uint_as_float(b.x); v[5] = __uint_as_float(b.y); v[6] = __uint_as_float(b.z); v[7] = __uint_as_float(b.w);
-  } else {
-    const uint32_t h[4] = {r.q[0].x, r.q[0].y, r.q[0].z, r.q[0].w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = W_DTYPE == PE_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&h[i]))
-                                         : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&h[i]));
-      v[2 * i] = f.x; v[2 * i + 1] = f.y;
-    }
-  }
 }
 
 // ---- 16-bit weights: the rotation on the tensor cores ------------------------------------------------------------
@@ -355,7 +337,6 @@ __global__ void __launch_bounds__(256, CTAS) quantize16_kernel(const void* w, in
   }
 }
 
-template <int W_DTYPE>
 __global__ void __launch_bounds__(256, 2) quantize_kernel(const void* w, int64_t ld_w, int64_t rows, int in_f, int nb,
                                                           const float* levels, int n_levels, int8_t* codes, int64_t ld_codes,
                                                           __half* norms, int64_t ld_norms, int vec_out) {
@@ -368,18 +349,18 @@ __global__ void __launch_bounds__(256, 2) quantize_kernel(const void* w, int64_t
   const uint32_t mask = cells - 1;
   const int lane = threadIdx.x & 31, part = lane & 3;
   const int64_t n_warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  const bool vin = ((ld_w * (W_DTYPE == PE_F32 ? 4 : 2)) % 16 == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
+  const bool vin = ld_w * 4 % 16 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
   // block (row r, column block blk) of this lane, and how far one trip of the grid advances it
   const int64_t first = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 8 + (lane >> 2);
   int64_t r = first / nb;
   int blk = (int)(first - r * nb);
   const int64_t step_r = n_warps * 8 / nb;
   const int step_b = (int)(n_warps * 8 - step_r * nb);
-  Raw8<W_DTYPE> raw[4];
+  Raw8<PE_F32> raw[4];
   auto request = [&]() {  // block (r, blk) of the weight, zeros past its last row
 #pragma unroll
     for (int p = 0; p < 4; ++p)
-      raw[p] = load8_raw<W_DTYPE>(w, r < rows ? r * ld_w : 0, blk * kBlock + p * 32 + part * 8, r < rows ? in_f : 0, vin);
+      raw[p] = load8_raw<PE_F32>(w, r < rows ? r * ld_w : 0, blk * kBlock + p * 32 + part * 8, r < rows ? in_f : 0, vin);
   };
   request();
   while (__any_sync(0xffffffffu, r < rows)) {
@@ -392,7 +373,13 @@ __global__ void __launch_bounds__(256, 2) quantize_kernel(const void* w, int64_t
     {
       float u[4][8], g[4][2];
 #pragma unroll
-      for (int p = 0; p < 4; ++p) cvt8<W_DTYPE>(raw[p], u[p]);
+      for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint4 x = raw[p].q[h];
+          u[p][4 * h] = __uint_as_float(x.x); u[p][4 * h + 1] = __uint_as_float(x.y);
+          u[p][4 * h + 2] = __uint_as_float(x.z); u[p][4 * h + 3] = __uint_as_float(x.w);
+        }
       r += step_r;
       blk += step_b;
       if (blk >= nb) { blk -= nb; ++r; }
@@ -611,13 +598,13 @@ extern "C" int pe_quantize(const void* weight, int w_dtype, int64_t ld_w, int64_
   const int64_t ctas = ((int64_t)out_f * nb + 63) / 64;  // a CTA takes 64 blocks per trip
   const int sms = sm_count();
   if (sms <= 0) return PE_ERR_CUDA;
-  // the resident CTAs (two per SM); the level table is built once per CTA
+  // the resident CTAs (two per SM, three for 16-bit weights of up to 16 levels); the level table is built once per CTA
   const bool wide = n_levels > 16;
   const long long per = w_dtype == PE_F32 || wide ? 2 : 3;
   const unsigned grid = (unsigned)(ctas < per * sms ? ctas : per * sms);
   // 4096 x 12288 bf16 with two / three CTAs an SM: to 4 bits 59 / 55 us, to 6 bits 58 / 60 us
 #define PE_QUANTIZE16(W) (!wide ? quantize16_kernel<W, 3, true> : n_levels <= 64 ? quantize16_kernel<W, 2, true> : quantize16_kernel<W, 2, false>)
-  auto kfn = w_dtype == PE_F32 ? quantize_kernel<PE_F32> : w_dtype == PE_F16 ? PE_QUANTIZE16(PE_F16) : PE_QUANTIZE16(PE_BF16);
+  auto kfn = w_dtype == PE_F32 ? quantize_kernel : w_dtype == PE_F16 ? PE_QUANTIZE16(PE_F16) : PE_QUANTIZE16(PE_BF16);
 #undef PE_QUANTIZE16
   const int unit = w_dtype == PE_F32 ? 8 : 16, vec_out = reinterpret_cast<uintptr_t>(codes) % unit == 0 && ld_codes % unit == 0;
   kfn<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(weight, ld_w, out_f, in_f, nb, levels, n_levels, codes, ld_codes,
