@@ -312,14 +312,14 @@ int pe_allreduce_add_rmsnorm(const float* partial, void* x, const void* weight, 
                              void* stream);
 
 /* ---- tiled weight layout for the decode kernel -----------------------------------
- * pe_retile rewrites a layer (codes + norms, the reference's row-major layouts) into the
- * layout the decode kernel streams best: for every 16-row tile and every 128-block, the
+ * pe_retile rewrites a layer (codes + norms, the reference's row-major layouts) into a
+ * layout with one contiguous record per tile: for every 16-row tile and every 128-block, the
  * 16 x 64 B (nibble) or 16 x 128 B (byte) codes followed by the 16 fp16 block norms, tiles
- * of a row tile stored one after the other.  A warp then reads one contiguous region
- * with 512-byte requests instead of sixteen 64-byte row pieces, and the norms travel with
- * the codes.  pe_retile_bytes gives the size of the tiled buffer (rows padded to 16).
- * Done once after loading, next to pack_codes_int4 (linear_method.py:228-258); it has no
- * counterpart in the reference.  pe_gemv_tiled = pe_gemv on such a buffer. */
+ * of a row tile stored one after the other, the norms with the codes.  pe_gemv streams the
+ * row-major arrays about as fast (a layer's four projections in 40 us for one row, 43 from
+ * tiles); the layout is for callers that hold such buffers.  pe_retile_bytes gives the size
+ * of one (rows padded to 16).  No counterpart in the reference.  pe_gemv_tiled = pe_gemv on
+ * such a buffer. */
 size_t pe_retile_bytes(int packed, int64_t out_f, int64_t in_f_padded);
 int pe_retile(const void* codes, int packed, int64_t ld_codes, const void* norms, int64_t ld_norms, void* tiles,
               int64_t out_f, int64_t in_f_padded, void* stream);

@@ -2,8 +2,8 @@
 //
 //   y[m, r] = sum_blk norm[r, blk] * sum_k ct[code[r, blk, k]] * xt[m, blk, k]   (+ bias[r])
 //
-// One persistent CTA per SM: sixteen math warps, a copy warp, for row-major codes a norm warp, and in launches whose CTAs have
-// several passes two sum warps.  A stage of the shared-
+// One persistent CTA per SM: sixteen math warps (fourteen where a warp takes three blocks), a copy warp, for row-major codes whose
+// norms are no single copy a norm warp, and in launches whose CTAs have several passes one or two sum warps.  A stage of the shared-
 // memory ring is one 16-row tile of the weight matrix by up to 32 quantization blocks.  The copy warp fills stages with bulk
 // copies (of the row-major layout one or a few rows each, of the tiled layout of pe_retile, whose records are contiguous, one
 // per stage).  Norms of row-major layers are a strided gather of halves: the norm warp loads them, two stages under way (with
@@ -14,7 +14,8 @@
 // launches.  Norms loaded by the math warps at the head of every pass: 8 us.  There is one norm warp, not several taking stages
 // in turn: a wait on a barrier's parity holds only for a waiter that took every earlier phase itself.)
 //
-// What bounds it: once the ring runs, the shared-memory port.  A warp takes block cw, cw + 16 of every stage:
+// What bounds it: once the ring runs, the shared-memory port.  A warp takes blocks w and w + 16 of every stage or, where rows are
+// short, blocks w, w + n and w + 2 n of every stage that falls to its group of n warps:
 //  * centroid lookup: the table is replicated per lane at a spacing of 256 bytes per entry, so that ONE byte permute
 //    forms the address (code byte in bits 8..15, lane * 4 below) and the load adds the table's constant address;
 //    32 lanes with 32 different codes never meet on a bank.  A nibble layer indexes it with the whole byte and gets
@@ -40,17 +41,18 @@
 //    The registers left over let the small launch's blocks be resident, waiting, while the launch before it still runs.
 // Measured, row-major layout, a line of launches under a CUDA graph, weights from HBM (in brackets the tiled layout):
 //   activation rows      1              8              16
-//   6144 x 4096 Q5     9.4 (10.1)     9.7 (10.1)    11.7 (12.8) us
-//   4096 x 4096 Q6     7.4  (8.0)     7.9  (8.1)     9.2  (9.8)
-//   24576 x 4096 Q3   13.9 (15.0)    15.8 (16.8)    24.2 (24.4)
-//   4096 x 12288 Q4   10.3 (10.8)    11.3 (11.8)    16.2 (15.9)
+//   6144 x 4096 Q5     9.2 (10.4)     9.2 (10.1)    11.2 (12.6) us
+//   4096 x 4096 Q6     7.0  (7.5)     7.2  (8.0)     8.6  (9.4)
+//   24576 x 4096 Q3   14.2 (15.1)    15.8 (15.5)    24.5 (23.2)
+//   4096 x 12288 Q4    9.9 (10.6)    11.1 (11.7)    15.9 (15.9)
+//   the four in turn  40.1 (42.9)    44.0 (46.3)    60.3 (61.6)
 // Inside the ring's steady state the 24576 x 4096 launch moves 4.9 TB/s; the rest is the launch's own latency: about
 // 3.5 us from the launch before it to the first product, 0.5 us from the last one to the stores.  Outside a line (launched
 // eagerly, or with other kernels in between) the ring fills about 2 us later: the four in turn take 48.5 us for one row, 51.2 for 8.
 //
 // The tiles of all problems of a launch form one line that is cut into equal contiguous ranges, one per CTA; nothing
-// crosses CTAs.  The sixteen warps' partial sums of a tile go through shared memory and are added in warp order: bit-
-// identical from run to run, and the same bits from either layout.
+// crosses CTAs.  The partial sums that a tile's warps (all sixteen, or a group's) have of it go through shared memory and are added in
+// warp order: bit-identical from run to run, and the same bits from either layout.
 #include "pe_gemv_decode.cuh"
 #include "pe_status.cuh"
 
@@ -89,7 +91,7 @@ struct BulkArgs {
   int part_bufs, part_floats;              // sets of partial sums, floats of one
   int part_off, stage_off, stage_bytes;
   int row_stride, copy_rows;               // row-major layout: bytes between rows of a stage, weight rows per bulk copy
-  int norm_stride;                         // grouped, row-major: bytes between the norms of two rows where a stage's are one bulk copy, else 0
+  int norm_stride;                         // row-major: bytes between the norms of two rows where a stage's come as one bulk copy, else 0
   int* status;
   // grouped launch: problem i multiplies rows grp[i].y .. + grp[i].z of the row list with matrix grp[i].x
   const int4* grp; int n_problems;
@@ -785,11 +787,12 @@ static int launch_bulk(BulkArgs& a, int sms, cudaStream_t st) {
 
 template <bool PACKED, bool TILED, bool GROUPED>
 static int launch_bulk_shape(BulkArgs& a, int sms, cudaStream_t st) {
-  // Grouped launches meet new rows all the time, and the norm warp's sixteen loads a stage are what paces them: where the norms of
+  // Grouped launches, and others of short rows, meet new rows all the time, and the norm warp's sixteen loads a stage are what paces them: where the norms of
   // a tile follow each other and their bytes are whole 16s, they come as one more bulk copy (128 experts, 2688 -> 2 x 1856, 64
   // tokens: 354 and 349 us; one token 41.1 and 39.0).  Their rows then share banks where the block count is even, which the
   // long rows of a dense layer feel more than the loads (24576 x 4096 at 8 rows: 16.4 us by the norm warp, 17.0 copied).
-  a.norm_stride = !TILED && a.nb <= 16 * (a.batch > 8 ? 1 : 2) && a.ld_norms == a.nb && (reinterpret_cast<uintptr_t>(a.norms) & 15) == 0 &&
+  const bool three = a.batch <= 8 && a.nb <= kGroupBlocks && (GROUPED || ((a.N + 15) / 16 >= 6 * sms && (a.batch > 2 || a.nb > 16)));
+  a.norm_stride = !TILED && (GROUPED || three) && a.nb <= 16 * (a.batch > 8 ? 1 : 2) && a.ld_norms == a.nb && (reinterpret_cast<uintptr_t>(a.norms) & 15) == 0 &&
                   a.norms_stride % 8 == 0 && (a.N % 16) * a.nb % 8 == 0 ? a.nb * 2 : 0;
   // Blocks per warp and stage: two when the row is longer than sixteen blocks.  Two sets of activation rows keep one:
   // their operands for two blocks spill (4096 x 12288 at 16 rows: 18.4 us with two, 15.9 with one).
@@ -801,7 +804,7 @@ static int launch_bulk_shape(BulkArgs& a, int sms, cudaStream_t st) {
   // Norms with gaps, or that do not start or end on 16 bytes, are gathered by a norm warp there too (by the copy warp, between
   // its copies: 24576 x 2048 Q4 at 8 rows 17.1 us, 128 experts of 21 blocks at 4 rows 479, 64 of 11 blocks 100; now 12.9, 204 and 52, with
   // one copy 10.4, 147 and 32.5; two blocks a warp took 11.2, 208 and 44).  The order of the sums is the same.
-  if (a.nb <= kGroupBlocks && (GROUPED || ((a.N + 15) / 16 >= 6 * sms && (a.batch > 2 || a.nb > 16))))
+  if (three)
     return TILED || a.norm_stride ? launch_bulk<PACKED, 1, 3, TILED, GROUPED, true>(a, sms, st) : launch_bulk<PACKED, 1, 3, TILED, GROUPED, true, !TILED>(a, sms, st);
   if constexpr (GROUPED) return launch_bulk<PACKED, 1, 2, TILED, GROUPED, true>(a, sms, st);
   else return a.nb > 16 ? launch_bulk<PACKED, 1, 2, TILED, GROUPED, false>(a, sms, st) : launch_bulk<PACKED, 1, 1, TILED, GROUPED, false>(a, sms, st);
