@@ -75,10 +75,9 @@ def test_gemm_ragged_in_features_bias_and_dtypes():
 
 
 @pytest.mark.parametrize("m,n", [(257, 256), (700, 1000), (513, 2688), (1100, 130)])
-def test_gemm_paired_ctas_ragged_edges_bias_and_dtypes(m, n):
-    """More than 256 tokens run on pairs of CTAs (512-token tiles, each CTA decoding half of the weight tile)
-    with the output leaving through clipped TMA stores: token and weight-row counts off every tile, box and
-    vector boundary, padded K, bias, all output types (fp32 output takes the direct-store path)."""
+def test_gemm_some_hundred_rows_ragged_edges_bias_and_dtypes(m, n):
+    """A few tiles of tokens on the tensor-memory kernel: token and weight-row counts off every tile and
+    vector boundary, padded K, bias, all output types."""
     k, in_f, bits = 1920, 1856, 4
     codes, norms, cts = rand_layer(n, k, bits, seed=m + n)
     bias = rand_x(1, n, seed=4).reshape(n)
@@ -90,6 +89,23 @@ def test_gemm_paired_ctas_ragged_edges_bias_and_dtypes(m, n):
     y5 = run_gemm(*rand_layer(n, k, 5, seed=n)[:3], x, 5, in_f=in_f)
     c5, n5, t5 = rand_layer(n, k, 5, seed=n)
     assert max_rel(y5, oracle.linear_dequant(x, c5, n5, t5, in_f=in_f)) <= TOL
+
+
+@pytest.mark.parametrize("m,n", [(4097, 130), (4200, 1000), (4353, 2689), (4097, 37 * 256 + 101)])
+def test_gemm_paired_ctas_ragged_edges_bias_and_dtypes(m, n):
+    """More than 4096 tokens always run on pairs of CTAs (512-token tiles, each CTA decoding half of the weight tile)
+    with the output leaving through clipped TMA stores where its rows are whole 16 bytes: token and weight-row counts off every tile, box and
+    vector boundary, padded K, bias, all output types; tiles whole, all of them in K ranges (130 rows) or those of a last wave (2689)."""
+    k, in_f = 1920, 1856
+    bias = rand_x(1, n, seed=4).reshape(n)
+    x = rand_x(m, in_f, seed=5, dtype=torch.bfloat16)
+    rows = torch.cat([torch.arange(0, m, 61), torch.arange(m - 20, m)])
+    for bits in (4, 5):
+        codes, norms, cts = rand_layer(n, k, bits, seed=m + n)
+        ref = oracle.linear_dequant(x[rows], codes, norms, cts, in_f=in_f) + bias.float()
+        for ydt in (torch.float16, torch.bfloat16, torch.float32):
+            y = run_gemm(codes, norms, cts, x, bits, out_dtype=ydt, bias=bias, in_f=in_f)
+            assert y.dtype == ydt and y.shape == (m, n) and torch.isfinite(y.float()).all() and max_rel(y[rows.cuda()], ref) <= TOL
 
 
 def test_gemm_few_tiles_with_and_without_room_for_the_k_split():
@@ -193,13 +209,9 @@ def test_gemm_of_gate_up_equals_activation_then_gemm(m, in_f):
     assert max_rel(y, oracle.linear_dequant(act.cpu(), codes, norms, cts, in_f=in_f)) <= TOL
 
 
-@pytest.mark.parametrize("m,n,bits,dtype", [(300, 75 * 256 + 40, 4, torch.float16), (600, 37 * 256 + 101, 3, torch.float32),
-                                            (1100, 25 * 256 + 8, 5, torch.bfloat16)])
-def test_gemm_last_wave_split_over_the_pairs(m, n, bits, dtype):
-    """One wave of whole tiles and one or two columns of tiles left, split in K: ragged edges in the split columns, bias, every
-    output type, and the result of the launch without room for the partials."""
+def with_and_without_room(m, n, k, bits, dtype):
+    """The launch with the workspace it would like and with the smallest one, a bias in both; some rows of it from the oracle."""
     from polarengine_vllm_b200 import _native as nv, packing
-    k = 4096
     codes, norms, cts = rand_layer(n, k, bits, seed=m)
     x, bias = rand_x(m, k, seed=m + 1), rand_x(1, n, seed=2).reshape(n)
     w, packed = (packing.pack_codes_half_block(codes.cuda()), True) if bits <= 4 else (codes.cuda(), False)
@@ -216,6 +228,26 @@ def test_gemm_last_wave_split_over_the_pairs(m, n, bits, dtype):
     ref = oracle.linear_dequant(x[rows], codes, norms, cts) + bias.float()
     assert max_rel(out[0], out[1]) <= 1e-2 and max_rel(out[0][rows.cuda()], ref) <= TOL
     assert max_rel(out[0][rows.cuda()][:, -400:], ref[:, -400:]) <= TOL
+    return out
+
+
+@pytest.mark.parametrize("m,n,bits,dtype", [(300, 75 * 256 + 40, 4, torch.float16), (600, 37 * 256 + 101, 3, torch.float32),
+                                            (1100, 25 * 256 + 8, 5, torch.bfloat16)])
+def test_gemm_some_hundred_rows_with_and_without_room(m, n, bits, dtype):
+    """Just over a wave of pair tiles: ragged edges, bias, every output type, whichever kernel and tiling either workspace leads to."""
+    with_and_without_room(m, n, 4096, bits, dtype)
+
+
+@pytest.mark.parametrize("m,n,bits,dtype", [(4097, 9 * 256 - 103, 4, torch.float32), (4300, 17 * 256 - 152, 3, torch.float16),
+                                            (4150, 17 * 256 - 55, 6, torch.bfloat16), (4097, 25 * 256 - 200, 5, torch.float32)])
+def test_gemm_last_wave_split_over_the_pairs(m, n, bits, dtype):
+    """Waves of whole tiles and one column of tiles left, split in K: ragged edges in the split columns, partials that leave by TMA and
+    that do not, bias, every output type.  The columns before them have the bits of the launch without room for the partials."""
+    from polarengine_vllm_b200 import _native as nv
+    k, split = 4096, (n - 1) // 256 * 256
+    assert nv.lib().pe_gemm_workspace_bytes_splitk(m, n, k) >= nv.lib().pe_gemm_workspace_bytes(m, k) + 8 * m * (n - split) * 4
+    room, none = with_and_without_room(m, n, k, bits, dtype)
+    assert torch.equal(room[:, :split], none[:, :split]) and not torch.equal(room[:, split:], none[:, split:])
 
 
 @pytest.mark.parametrize("m,n,k,bits", [(257, 100, 128, 4), (258, 4096, 1024, 3), (300, 1000, 640, 6), (385, 19000, 256, 4), (512, 2500, 2048, 5), (577, 130, 4096, 3),
@@ -244,14 +276,15 @@ def test_gemm_some_hundred_rows(m, n, k, bits):
 @pytest.mark.parametrize("n,bits,dtype", [(19 * 256 + 40, 4, torch.float16), (18 * 256 + 256, 6, torch.float32), (700, 3, torch.bfloat16)])
 def test_gemm_pairs_last_wave_split(n, bits, dtype):
     """Rows enough for pairs of CTAs whatever the estimate says: a last, partly filled wave cut into K ranges, and a launch of few tiles."""
-    m, k = 1700, 2048
+    m, k = 4200, 2048
     codes, norms, cts = rand_layer(n, k, bits, seed=n)
     x = rand_x(m, k, seed=4)
     y = run_gemm(codes, norms, cts, x, bits, out_dtype=dtype)
-    assert max_rel(y, oracle.linear_dequant(x, codes, norms, cts)) <= TOL
+    rows = torch.cat([torch.arange(0, m, 29), torch.arange(m - 20, m)])
+    assert torch.isfinite(y.float()).all() and max_rel(y[rows.cuda()], oracle.linear_dequant(x[rows], codes, norms, cts)) <= TOL
 
 
-@pytest.mark.parametrize("rows", [40, 300, 1700])
+@pytest.mark.parametrize("rows", [40, 300, 1700, 4200])
 @pytest.mark.parametrize("bits", [4, 5])
 def test_prefill_weights_rewritten_by_the_kernel_in_front(bits, rows):
     """Codes and norms rewritten on the device right before the call: the tensor-core kernels read them before their own wait, the
