@@ -66,7 +66,7 @@ __host__ __device__ constexpr int sum_warps(int bpw, bool passes) { return !pass
 __host__ __device__ constexpr int bulk_threads(int bpw, bool norm_warp, bool passes) {
   return (bulk_warps(bpw) + 1 + sum_warps(bpw, passes) + norm_warp) * 32;
 }
-constexpr int kGroupBlocks = 21;                      // blocks of a row, at most, where a warp takes three: two groups of seven warps
+constexpr int kGroupBlocks = 21;                      // blocks of a row, at most, where a warp takes three: two groups of seven warps (22 would take eight warps: one group)
 constexpr int kTabAddr = 2048;                        // address of the centroid table in the shared window
 constexpr int kTabReach = 255 * 256 + 256;            // bytes a lookup can reach from there, whatever the code byte is
 constexpr int kBulkMaxStages = 8;
